@@ -222,6 +222,14 @@ la_status launch_gemm(la_ctx ctx, int mode, int M, int N, int K, const double* A
 // operands.
 la_status launch_gemm_lower(la_ctx ctx, int M, int K, const double* A, size_t lda,
                             const double* B, size_t ldb, double* C, size_t ldc);
+// Products on the tensor cores by exact splitting (gemm_split.cu): C (M x N) -= A B (mode -1), = A B
+// (0) or += A B (1); A M x K, B K x N, or N x K rows of B' when b_rows; any alignment. tri: the
+// square C's part at or below the diagonal, in tiles. ws: gemm_split_ws bytes of device memory,
+// used until the product is done (same: B' is A). LA_UNSUPPORTED: nothing launched.
+size_t gemm_split_ws(int M, int N, int K, bool same);
+la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
+                            const double* A, size_t lda, const double* B, size_t ldb, bool b_rows,
+                            double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes);
 // C + z * czs = A[:, z kper : (z + 1) kper] B[z kper : (z + 1) kper, :] for z < splits
 // (fused, from zero); kper a multiple of 32, splits * kper >= K > (splits - 1) kper.
 la_status launch_gemm_splitk(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
