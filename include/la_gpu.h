@@ -77,10 +77,12 @@ typedef enum la_option {
   /* 1: record per-phase device times of each LU (la_ctx_last_phase_ms). */
   LA_OPT_PROFILE = 4,
   /* 1 (default): factor the next panel on a second stream while the rest of
-   * the trailing update runs; 0: strictly one phase after the other. */
+   * the trailing update runs (EXACT LU, mixed LU, Cholesky, QR); 0: strictly
+   * one phase after the other. Results are bit-identical either way. */
   LA_OPT_LOOKAHEAD = 5,
-  /* 1 (default): the FP32 panels of the mixed LU run on one thread-block
-   * cluster (distributed shared memory); 0: the cooperative multi-CTA kernel. */
+  /* 1 (default): the FP32 panels of the mixed LU and the panels of the FAST LU
+   * run on one thread-block cluster (distributed shared memory); 0: the
+   * cooperative multi-CTA kernel. The FAST LU's results are the same bits. */
   LA_OPT_CLUSTER_PANEL = 6,
   /* Batch plans (read when a plan is built): largest Krylov basis (0-20) of
    * the GMRES-IR stage that a LA_BATCH_MIXED plan runs on a system whose
@@ -420,7 +422,7 @@ la_status la_mlp_set_gate(la_mlp mlp, const float* coef, float bias);
  * the stream and reads the device error word with a synchronous copy), so it
  * cannot be called while any stream is being captured into a CUDA graph.
  * Limit: m <= 16384 (LA_UNSUPPORTED beyond). Its working memory is one static
- * device array of about 70 KB per device, kept until the process exits and
+ * device array of about 3.3 MB per device, kept until the process exits and
  * shared by every call: calls that overlap on the GPU (other host threads,
  * other streams) race and must be serialized by the caller. The first call on
  * a device looks up that array's device address; after cudaDeviceReset that

@@ -133,6 +133,9 @@ struct la_context {
   int* d_swaps = nullptr;        // [1 + 2*128] composed row moves of one panel
   double* d_small = nullptr;     // [8] small device results (det, flags)
   int* d_solve_sync = nullptr;   // [2 + 2*SOLVE_WAVE_MAX_GROUPS] wavefront solve tickets, progress
+  // Workspace of the split products where nothing may be allocated (noalloc.cu); null: allocate.
+  void* split_ws = nullptr;
+  size_t split_ws_bytes = 0;
   void* h_pinned = nullptr;      // pinned host staging for small readbacks
 };
 
@@ -251,6 +254,11 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
                            size_t ldt, int cols);
 la_status launch_panel(la_ctx ctx, cudaStream_t stream, bool exact, double* A, double* S,
                        size_t ld, int m, int j0, int jb, int* d_ipiv, unsigned* bar_base);
+la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t stream, double* A, size_t ld, int m, int j0,
+                                 int jb, int* d_ipiv);
+// C -= A B with tiles of 16 columns (N <= 64), for narrow updates.
+la_status launch_gemm_narrow(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
+                             const double* B, size_t ldb, double* C, size_t ldc);
 la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int n, int j0,
                        int jb);
 la_status launch_trsm_rowpanel(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int j0,

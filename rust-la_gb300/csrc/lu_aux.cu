@@ -126,6 +126,38 @@ trsm_rowpanel_kernel(T* A, const T* S, size_t ld, int j0, int jb, int c_begin, i
     for (int i = ty; i < jb; i += 8) A[(size_t)(j0 + i) * ld + c] = xa[i][tx];
 }
 
+// FAST FP64 form, jb <= 64: 8 columns per CTA. With two FP64 FMAs per clock an SM needs 16 clocks
+// for one warp's FMA, so the 64 x 64 triangle costs 0.5 us a column and the strip's width sets the
+// latency: the 32-column CTAs of the kernel above took 49 us however few columns there were. Row k
+// is final when step k starts; the rows below take its term, neighbouring items (row, column) on
+// neighbouring threads, so that no lane idles but in the last warp. The same FMAs in the same
+// order as above, so the same bits.
+constexpr int TC8 = 8;
+constexpr int TC8_T = 256;
+__global__ void __launch_bounds__(TC8_T)
+trsm_cols8_kernel(double* A, size_t ld, int j0, int jb, int c_begin, int c_end) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  __shared__ double L[MAX_PANEL_W][MAX_PANEL_W + 1];
+  __shared__ double x[MAX_PANEL_W][TC8];
+  const int tid = threadIdx.x, col = tid % TC8, r0 = tid / TC8;  // r0 0..31
+  const int c = c_begin + blockIdx.x * TC8 + col;
+  const bool ok = c < c_end;
+  for (int idx = tid; idx < jb * MAX_PANEL_W; idx += TC8_T) {
+    const int i = idx / MAX_PANEL_W, k = idx % MAX_PANEL_W;
+    if (k < i) L[i][k] = A[(size_t)(j0 + i) * ld + j0 + k];
+  }
+  for (int i = r0; i < jb; i += TC8_T / TC8) x[i][col] = ok ? A[(size_t)(j0 + i) * ld + c] : 0.0;
+  __syncthreads();
+  for (int k = 0; k + 1 < jb; k++) {
+    const double u = x[k][col];
+    for (int i = k + 1 + r0; i < jb; i += TC8_T / TC8) x[i][col] = fma(-L[i][k], u, x[i][col]);
+    __syncthreads();
+  }
+  if (ok)
+    for (int i = r0; i < jb; i += TC8_T / TC8) A[(size_t)(j0 + i) * ld + c] = x[i][col];
+}
+
 // FP32 form for the mixed LU's 32-row blocks (jb <= 32, FMA): one thread per
 // column holds the column's jb values in registers and applies the terms in
 // ascending k (the same FMAs in the same order as the kernel above, so the
@@ -357,10 +389,6 @@ cudaError_t configure_smem_attrs() {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)trsm_smem<double>(true));
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(trsm_rowpanel_kernel<double, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)trsm_smem<double>(false));
-    if (e == cudaSuccess)
       e = cudaFuncSetAttribute(trsm_rowpanel_kernel<float, false>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)trsm_smem<float>(false));
@@ -431,6 +459,14 @@ template <typename T>
 la_status launch_trsm_t(la_ctx ctx, bool exact, T* A, T* S, size_t ld, int j0, int jb,
                         int c_begin, int c_end) {
   if (c_end <= c_begin) return LA_OK;
+  if (sizeof(T) == 8 && !exact) {
+    const cudaError_t e =
+        la_launch(ctx, trsm_cols8_kernel, dim3((c_end - c_begin + TC8 - 1) / TC8), dim3(TC8_T), 0,
+                  ctx->stream, reinterpret_cast<double*>(A), ld, j0, jb, c_begin, c_end);
+    if (e != cudaSuccess) return la_cuda_fail(ctx, e, "trsm_cols8_kernel launch");
+    ctx->launches++;
+    return la_check_launch(ctx, "trsm_cols8_kernel");
+  }
   LA_CUDA(ctx, configure_smem_attrs());
   dim3 grid((c_end - c_begin + TR_COLS - 1) / TR_COLS);
   if (exact)

@@ -32,7 +32,10 @@ constexpr size_t NA_OFF_CROW = NA_OFF_CPOS + 2 * NA_CTAS * sizeof(int);
 constexpr size_t NA_OFF_DIAGA = NA_OFF_CROW + (size_t)2 * NA_CTAS * MAX_PANEL_W * sizeof(double);
 constexpr size_t NA_OFF_DIAGS = NA_OFF_DIAGA + 2 * MAX_PANEL_W * sizeof(double);
 constexpr size_t NA_OFF_SWAPS = NA_OFF_DIAGS + 2 * MAX_PANEL_W * sizeof(double);
-constexpr size_t NA_BYTES = NA_OFF_SWAPS + 4096;  // about 70 KB in total
+// Digits of an update of 2048 x 1024 elements (K = 64); larger ones go in pieces of whole tiles.
+constexpr size_t NA_OFF_SPLIT = NA_OFF_SWAPS + 4096;
+constexpr size_t NA_SPLIT_BYTES = (size_t)(2048 + 1024) * (64 * 16 + 16) + 16384;
+constexpr size_t NA_BYTES = NA_OFF_SPLIT + NA_SPLIT_BYTES;  // about 3.3 MB in total
 
 static __device__ __align__(256) unsigned char g_lu_scratch[NA_BYTES];
 
@@ -95,6 +98,8 @@ extern "C" la_status la_lu_factor_noalloc(void* stream, double* d_a, size_t lda,
   c.d_diag_a = reinterpret_cast<double*>(base + NA_OFF_DIAGA);
   c.d_diag_s = reinterpret_cast<double*>(base + NA_OFF_DIAGS);
   c.d_swaps = reinterpret_cast<int*>(base + NA_OFF_SWAPS);
+  c.split_ws = base + NA_OFF_SPLIT;
+  c.split_ws_bytes = NA_SPLIT_BYTES;
 
   // The array keeps the previous call's contents: clear the error word (the
   // barrier counter is cleared by the factorization itself).

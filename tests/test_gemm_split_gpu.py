@@ -107,3 +107,15 @@ def test_values_that_are_not_finite(lagpu, ctx_fast):
     ok = np.isfinite(ref)
     a0, b0 = np.where(np.isfinite(a), a, 0), np.where(np.isfinite(b), b, 0)
     assert np.all(np.abs(c - ref)[ok] <= (2 * (k + 1) * U * (np.abs(a0) @ np.abs(b0)))[ok])
+
+
+def test_update_form(lagpu, ctx_fast):
+    # C -= A B, which the factorization runs with K = 64: L U against P A.
+    rng = np.random.default_rng(8)
+    a = rng.standard_normal((321, 321))
+    ref = oracle.lu_factor(a)
+    lu = lagpu.LUDecomposition.new(a, ctx_fast)
+    assert np.array_equal(lu.get_piv(), ref.piv)
+    l, u = lu.get_l().data, lu.get_u().data
+    pa = a[ref.piv.astype(int)]
+    assert np.all(np.abs(l @ u - pa) <= 2 * 323 * U * (np.abs(l) @ np.abs(u)))
