@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(PT) panel_kernel(PanelParams p) {
   // Compose this panel's swaps into a list of row moves (dest <- src) for the
   // columns outside the panel (applied by the row-swap kernel).
   if (g == 0 && warp == 0)
-    compose_swaps_warp(s_pivs, jb, p.j0, false, nullptr, p.swaps, s_atp, s_atr, lane);
+    compose_swaps_warp(s_pivs, jb, p.j0, p.swaps, s_atp, s_atr, lane);
 }
 
 }  // namespace

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(CT, 1) panel_cluster_kernel(ClusterPanelArgs p
     if (c < jb) p.A[(size_t)(row0 + r) * p.ld + p.j0 + c] = va[r * CP + c];
   }
   if (g == 0 && warp == 0)
-    compose_swaps_warp(s_pivs, jb, p.j0, false, nullptr, p.swaps, s_atp, s_atr, lane);
+    compose_swaps_warp(s_pivs, jb, p.j0, p.swaps, s_atp, s_atr, lane);
 }
 
 __device__ __forceinline__ unsigned long long gtimer_ns() {
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(CT, 1) panel_cluster_reg_kernel(ClusterPanelAr
       }
     }
   if (g == 0 && warp == 0)
-    compose_swaps_warp(s_pivs, jb, p.j0, false, nullptr, p.swaps, s_atp, s_atr, lane);
+    compose_swaps_warp(s_pivs, jb, p.j0, p.swaps, s_atp, s_atr, lane);
 }
 
 

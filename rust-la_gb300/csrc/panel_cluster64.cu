@@ -8,10 +8,12 @@
 // kernel of lu_panel.cu exchanges through global memory at 5 to 11 us per column; here
 // up to 16 CTAs of one cluster exchange through distributed shared memory.
 //
-//   * One row per thread, its 32 values in registers for the whole panel, with the
-//     row's current position; a pivot exchange swaps two positions and no data. The
-//     register window rotates by one slot per column, so that the current column is
-//     slot 0 and every register index is static.
+//   * Q threads per row (neighbouring lanes), thread q with the columns k = q mod Q, in
+//     registers for the whole panel, with the row's current position; a pivot exchange
+//     swaps two positions and no data. A warp's FMA takes its sub-partition 64 clocks,
+//     however few of its lanes are active, so Q spreads few rows over the SM's four
+//     pipes: 4 up to 64 rows per CTA, 2 up to 128, else 1. The register window rotates
+//     by one slot every Q columns, so that every register index is static.
 //   * An element takes its updates in ascending k by FMA and its multiplier as
 //     v * (1 / pivot), exactly the operations of lu_panel.cu's FAST form: the two
 //     kernels give the same bits.
@@ -21,10 +23,18 @@
 //     with its multiplier, and the pushing warp applies the missing update (one FMA
 //     per lane).
 //   * Every warp finds the CTA's best candidate for itself and pushes it (row and key,
-//     272 bytes, st.async) into the receive slot of one CTA of the cluster; the bytes
-//     complete on the receiver's mbarrier. Three slots: a CTA pushes column c + 3 only
-//     after it has every push of c + 2, which each CTA sends after its last use of
-//     column c's row.
+//     st.async) into the receive slots of some CTAs of the cluster; a warp without rows
+//     meanwhile divides (the candidate's reciprocal) and pushes that, so that no CTA
+//     divides on its way from the winner to the next candidates. The bytes complete on
+//     the receiver's mbarrier. Three slots: a CTA pushes column c + 3 only after it has
+//     every push of c + 2, which each CTA sends after its last use of column c's row.
+//
+// Measured, 32 columns (R rows, us): R = 24 36, 512 49, 2048 63, 4096 84, 8192 138. With one row
+// per thread at every R, a division in every thread and 128-row CTAs it was 53, 90, 86, 110 and
+// 170; the exchange itself is hidden, and what remains per column is about 550 clocks to
+// find and publish the candidate, 650 to push it, 250 to pick the winner, 350 to scale and
+// form the next column, and the update (64 clocks per FMA and warp of a sub-partition:
+// from 512 rows per CTA on it is half of the time).
 //
 // Waits are bounded (2 s or LA_OPT_WAIT_LIMIT_US): a thread whose wait gives up
 // records DERR_PANEL_TIMEOUT, waits for nothing more and pushes nothing more, but
@@ -36,7 +46,7 @@ namespace {
 
 constexpr int PW = 32;                       // panel width
 constexpr int PMAXC = 16;                    // CTAs of a cluster
-constexpr uint32_t PUSH_BYTES = PW * 8 + 16;  // row, key, position
+constexpr uint32_t PUSH_BYTES = PW * 8 + 16 + 8;  // row; key and position; reciprocal
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 __device__ __forceinline__ uint32_t sm_addr(const void* p) {
@@ -86,20 +96,20 @@ __device__ __forceinline__ unsigned long long key_of(double v, bool diag) {
   if (a > 0x7ff0000000000000ull) return diag ? ~0ull : 0ull;
   return a + 1ull;
 }
-// The best (largest key, then lowest position) of the lanes with pos >= 0; src is its lane, -1
-// without one. Three 32-bit warp reductions.
-__device__ __forceinline__ int warp_best(unsigned long long key, int pos, unsigned long long& bk,
-                                         int& bp) {
+// The best (largest key, then lowest position) of the lanes with pos >= 0: returns its lane, -1
+// without one. One 32-bit warp reduction where the key's high word decides, else three.
+__device__ __forceinline__ int warp_best(unsigned long long key, int pos) {
   const bool in = pos >= 0;
   const unsigned hi = in ? (unsigned)(key >> 32) : 0u;
   const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const bool e1 = in && hi == mh;
-  const unsigned ml = __reduce_max_sync(0xffffffffu, e1 ? (unsigned)key : 0u);
-  const bool e2 = e1 && (unsigned)key == ml;
-  const unsigned mp = __reduce_min_sync(0xffffffffu, e2 ? (unsigned)pos : 0xffffffffu);
-  bk = (unsigned long long)mh << 32 | ml;
-  bp = (int)mp;
-  const unsigned who = __ballot_sync(0xffffffffu, e2 && (unsigned)pos == mp);
+  bool e = in && hi == mh;
+  unsigned who = __ballot_sync(0xffffffffu, e);
+  if (who & (who - 1)) {
+    const unsigned ml = __reduce_max_sync(0xffffffffu, e ? (unsigned)key : 0u);
+    e = e && (unsigned)key == ml;
+    const unsigned mp = __reduce_min_sync(0xffffffffu, e ? (unsigned)pos : 0xffffffffu);
+    who = __ballot_sync(0xffffffffu, e && (unsigned)pos == mp);
+  }
   return who ? __ffs(who) - 1 : -1;
 }
 
@@ -117,20 +127,38 @@ struct __align__(16) PushSlot {
   double row[PW];
   unsigned long long key;
   int pos, pad;
+  double rcp, pad2;
 };
 
-template <int T>
-__global__ void __launch_bounds__(T, 1) panel_cluster64_kernel(const Panel64Args p) {
-  la_pdl_wait();
-  la_pdl_trigger();
+// v[i] = fma(l, u[Q i], v[i]) for 1 <= i < n. A switch into the unrolled sequence: an FMA that a
+// predicate switches off takes the FP64 pipe as long as any other.
+template <int Q, int NV>
+__device__ __forceinline__ void update_tail(double (&v)[NV], double l, const double* u, int n) {
+#define LA_U(i) \
+  case (i) + 1: \
+    if ((i) < NV) v[(i) % NV] = fma(l, u[Q * (i)], v[(i) % NV]); \
+    [[fallthrough]];
+  switch (n) {
+    LA_U(31) LA_U(30) LA_U(29) LA_U(28) LA_U(27) LA_U(26) LA_U(25) LA_U(24)
+    LA_U(23) LA_U(22) LA_U(21) LA_U(20) LA_U(19) LA_U(18) LA_U(17) LA_U(16)
+    LA_U(15) LA_U(14) LA_U(13) LA_U(12) LA_U(11) LA_U(10) LA_U(9) LA_U(8)
+    LA_U(7) LA_U(6) LA_U(5) LA_U(4) LA_U(3) LA_U(2) LA_U(1)
+    default: break;
+  }
+#undef LA_U
+}
+
+// T threads with rows and one more warp, for the reciprocals.
+template <int T, int Q>
+__global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel64Args p) {
   constexpr int NW = T / 32;
+  constexpr int NV = PW / Q;  // values per thread: columns q, q + Q, ...
   __shared__ PushSlot recv[3][PMAXC];
   __shared__ double wrow[2][NW][PW];
   __shared__ double wl[2][NW];  // the published row's multiplier of the previous column
   __shared__ unsigned long long wkey[2][NW];
   __shared__ int wpos[2][NW];
   __shared__ __align__(8) uint64_t rbar[3];
-  __shared__ int s_pivs[PW];
   __shared__ int s_atp[SWAP_SLOTS], s_atr[SWAP_SLOTS];
 
   uint32_t rank;
@@ -140,159 +168,189 @@ __global__ void __launch_bounds__(T, 1) panel_cluster64_kernel(const Panel64Args
   const int jb = p.jb;
   const int row0 = p.j0 + g * p.rpc;
   const int nrows = max(0, min(p.rpc, p.m - row0));
-  bool live = *reinterpret_cast<volatile int*>(p.err) == 0;
 
   if (tid < 3)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm_addr(&rbar[tid])));
   if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 
-  double v[PW];
-  int pos = tid < nrows ? row0 + tid : -1;
+  // Before the wait for the kernel ahead: every CTA's receive barriers are initialised before any
+  // push.
+  cluster_barrier();
+  la_pdl_wait();
+  la_pdl_trigger();
+  bool live = *reinterpret_cast<volatile int*>(p.err) == 0;
+  double v[NV];
+  const int q = lane % Q, lr = tid / Q;
+  int pos = tid < T && lr < nrows ? row0 + lr : -1;
   {
     const double* src = p.A + (size_t)(pos >= 0 ? pos : p.j0) * p.ld + p.j0;
-    if (p.vec && jb == PW) {
+    if (Q == 1 && p.vec && jb == PW) {
 #pragma unroll
-      for (int k = 0; k < PW; k += 2) {
+      for (int k = 0; k < NV; k += 2) {
         const double2 t = pos >= 0 ? *reinterpret_cast<const double2*>(src + k) : make_double2(0, 0);
         v[k] = t.x;
         v[k + 1] = t.y;
       }
     } else {
 #pragma unroll
-      for (int k = 0; k < PW; k++) v[k] = pos >= 0 && k < jb ? src[k] : 0.0;
+      for (int i = 0; i < NV; i++) v[i] = pos >= 0 && q + Q * i < jb ? src[q + Q * i] : 0.0;
     }
   }
-  cluster_barrier();  // every CTA's receive barriers are initialised before any push
 
-  bool act = false;                // this row took part in the previous column's update
-  const double* uprev = nullptr;   // the previous column's pivot row
-  for (int c = 0; c < jb; c++) {
-    const int j = p.j0 + c, par = c & 1, slot = c % 3;
-    // candidates of column c (slot 0 holds it, every update applied)
-    {
-      unsigned long long bk;
-      int bp;
-      const int src =
-          warp_best(key_of(v[0], pos == j), pos >= j ? pos : -1, bk, bp);
-      if (src == lane) {
-        double* dst = wrow[par][warp] + c;
+  // This warp's first target: its receive slots and barriers. The last warp sends the reciprocals,
+  // a lane to each CTA.
+  const uint32_t to0 = (uint32_t)(warp < NW ? warp : lane) % (uint32_t)C;
+  const uint32_t dst0 = peer_addr(&recv[0][g], to0), bar0 = peer_addr(&rbar[0], to0);
+
+  int na = 0;                     // the last warp of CTA 0: slots of the composed interchanges
+  bool act = false;               // this row took part in the previous column's update,
+  double lp = 0.0;                // with this multiplier
+  const double* uprev = nullptr;  // and this pivot row
+  for (int cb = 0; cb < jb; cb += Q) {
+    // one copy of the body (four of them outgrew the instruction cache: 2750 against 2200 clocks
+    // per column with 32 rows per CTA)
+#pragma unroll 1
+    for (int s = 0; s < Q; s++) {  // column c = cb + s: slot 0 of the threads q == s
+      const int c = cb + s;
+      if (c >= jb) break;
+      const int j = p.j0 + c, par = c & 1, slot = c % 3;
+      // this warp's candidate of column c, its row one update behind
+      if (warp < NW) {
+        const bool mine = q == s && pos >= j;
+        const unsigned long long key = key_of(v[0], pos == j);
+        const int src = warp_best(key, mine ? pos : -1);
+        if (src >= 0 && lane / Q == src / Q) {
+          double* dst = wrow[par][warp] + cb + q;
 #pragma unroll
-        for (int q = 0; q < PW; q += 4)
-          if (c + q < jb)
-#pragma unroll
-            for (int i = q; i < q + 4; i++)
-              if (c + i < PW) dst[i] = v[i];
-        wl[par][warp] = c > 0 ? v[PW - 1] : 0.0;
+          for (int i = 0; i < NV; i++)
+            if (cb + Q * i < jb) dst[Q * i] = v[i];
+          if (lane == src) {
+            wl[par][warp] = lp;
+            wkey[par][warp] = key;
+            wpos[par][warp] = pos;
+          }
+        }
+        if (src < 0 && lane == 0) {
+          wkey[par][warp] = 0ull;
+          wpos[par][warp] = -1;
+        }
       }
-      if (lane == 0) {
-        wkey[par][warp] = bk;
-        wpos[par][warp] = src >= 0 ? bp : -1;
-      }
-    }
-    __syncthreads();
-    // the CTA's best, and its row with the previous column's update, to the cluster
-    {
-      unsigned long long bk;
-      int bp;
-      const int w = warp_best(lane < NW ? wkey[par][lane % NW] : 0ull,
-                              lane < NW ? wpos[par][lane % NW] : -1, bk, bp);
-      if (live) {
+      __syncthreads();
+      // the CTA's best, its row with the previous column's update, to the cluster
+      const unsigned long long wk = lane < NW ? wkey[par][lane % NW] : 0ull;
+      const int wp = lane < NW ? wpos[par][lane % NW] : -1;
+      const int w = warp_best(wk, wp);
+      if (live && warp < NW) {
         double t = 0.0;
         if (w >= 0 && lane >= c) {
           t = wrow[par][w][lane];
           if (c > 0 && lane > c) t = fma(-wl[par][w], uprev[lane], t);
         }
         for (int to = warp; to < C; to += NW) {
-          const uint32_t bar = peer_addr(&rbar[slot], (uint32_t)to);
+          uint32_t bar = bar0 + slot * 8, dst = dst0 + slot * (uint32_t)sizeof(recv[0]);
+          if (to != warp) {
+            bar = peer_addr(&rbar[slot], (uint32_t)to);
+            dst = peer_addr(&recv[slot][g], (uint32_t)to);
+          }
           asm volatile(
               "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
-                  peer_addr(&recv[slot][g].row[lane], (uint32_t)to)),
+                  dst + (uint32_t)lane * 8),
               "l"(__double_as_longlong(t)), "r"(bar)
               : "memory");
-          if (lane == 0)
+          if (lane == (w >= 0 ? w : 0))
             asm volatile(
                 "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, "
-                "%4}, [%5];" ::"r"(peer_addr(&recv[slot][g].key, (uint32_t)to)),
-                "r"((unsigned)bk), "r"((unsigned)(bk >> 32)), "r"(w >= 0 ? bp : -1), "r"(0), "r"(bar)
+                "%4}, [%5];" ::"r"(dst + (uint32_t)offsetof(PushSlot, key)),
+                "r"((unsigned)wk), "r"((unsigned)(wk >> 32)), "r"(w >= 0 ? wp : -1), "r"(0), "r"(bar)
                 : "memory");
         }
-        if (tid == 0)
+      } else if (live) {
+        const double rcp = 1.0 / (w >= 0 ? wrow[par][w][c] : 1.0);
+        if (lane < C)
+          asm volatile(
+              "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                  dst0 + slot * (uint32_t)sizeof(recv[0]) + (uint32_t)offsetof(PushSlot, rcp)),
+              "l"(__double_as_longlong(rcp)), "r"(bar0 + slot * 8)
+              : "memory");
+        if (lane == 0)
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                            sm_addr(&rbar[slot])),
                        "r"((uint32_t)(C + p.stall) * PUSH_BYTES)
                        : "memory");
       }
+      // the previous column's update of the columns after c, while the pushes travel
+      if (act) {
+        const double l = -lp;
+        const double* u = uprev + cb + q;
+        if (Q > 1 && s < Q - 1 && q > s) v[0] = fma(l, u[0], v[0]);
+        update_tail<Q, NV>(v, l, u, (jb - cb + Q - 1) / Q);  // slots with cb + Q i < jb
+      }
+      if (live) live = wait_pushes(&rbar[slot], (uint32_t)((c / 3) & 1), p.err, p.wait_ns);
+      live = __all_sync(0xffffffffu, live);
+      // the winner and its row
+      const PushSlot& mine = recv[slot][lane % PMAXC];
+      const int cpos = lane < C && live ? mine.pos : -1;
+      const int src = warp_best(mine.key, cpos);
+      // a failed wait: no use is made of what follows
+      const int piv = src >= 0 ? __shfl_sync(0xffffffffu, cpos, src) : j;
+      const PushSlot& win = recv[slot][src >= 0 ? src : 0];
+      const double* u = win.row;
+      act = false;
+      if (pos == piv) {
+        pos = j;  // the pivot row keeps its values
+      } else {
+        if (pos == j) pos = piv;  // the displaced row takes its place
+        act = pos > j;
+      }
+      // the multiplier, from the row's thread of column c to its others; a zero pivot (key 1)
+      // leaves the column as it is
+      if (act && q == s && win.key != 1ull) v[0] = v[0] * win.rcp;
+      lp = Q == 1 ? v[0] : __shfl_sync(0xffffffffu, v[0], lane / Q * Q + s);
+      if (act && c + 1 < jb) {
+        if (s + 1 < Q) {
+          if (q == s + 1) v[0] = fma(-lp, u[c + 1], v[0]);
+        } else if (q == 0) {
+          v[NV > 1 ? 1 : 0] = fma(-lp, u[c + 1], v[NV > 1 ? 1 : 0]);
+        }
+      }
+      uprev = u;
+      if (g == 0 && warp == NW) {
+        if (lane == 0) p.ipiv[j] = piv;
+        compose_step(j, piv, na, s_atp, s_atr, lane);
+      }
     }
-    // the previous column's update of the columns after c, while the pushes travel
-    if (act) {
-      const double l = -v[PW - 1];
-#pragma unroll
-      for (int q = 0; q < PW; q += 4)
-        if (c + q < jb)
-#pragma unroll
-          for (int i = q; i < q + 4; i++)
-            if (i > 0 && c + i < PW) v[i] = fma(l, uprev[c + i], v[i]);
-    }
-    if (live) live = wait_pushes(&rbar[slot], (uint32_t)((c / 3) & 1), p.err, p.wait_ns);
-    live = __all_sync(0xffffffffu, live);
-    // the winner and its row
-    unsigned long long bk;
-    int piv;
-    const int src = warp_best(lane < C ? recv[slot][lane % PMAXC].key : 0ull,
-                              lane < C && live ? recv[slot][lane % PMAXC].pos : -1, bk, piv);
-    const double* u = recv[slot][src >= 0 ? src : 0].row;
-    if (!live || src < 0) piv = j;  // a failed wait: no use is made of what follows
-    const double d = u[c];
-    const double l = d != 0.0 ? v[0] * (1.0 / d) : v[0];
-    act = false;
-    if (pos == piv) {
-      pos = j;  // the pivot row keeps its values
-    } else {
-      if (pos == j) pos = piv;  // the displaced row takes its place
-      act = pos > j;
-    }
-    if (act) {
-      v[0] = l;
-      if (c + 1 < jb) v[1] = fma(-l, u[c + 1], v[1]);
-    }
-    uprev = u;
     const double t = v[0];
 #pragma unroll
-    for (int k = 0; k < PW - 1; k++) v[k] = v[k + 1];
-    v[PW - 1] = t;
-    if (g == 0 && tid == 0) {
-      p.ipiv[j] = piv;
-      s_pivs[c] = piv;
-    }
+    for (int i = 0; i < NV - 1; i++) v[i] = v[i + 1];
+    v[NV - 1] = t;
   }
   const bool ok = __syncthreads_and(live ? 1 : 0) != 0;
   cluster_barrier();  // no CTA leaves while pushes into its shared memory may be in flight
   if (!ok) return;
-  // jb rotations so far; 32 bring every value back to its column
-  for (int r = jb; r < PW; r++) {
+  // one rotation per Q columns so far; NV bring every value back to its column
+  for (int r = (jb + Q - 1) / Q; r < NV; r++) {
     const double t = v[0];
 #pragma unroll
-    for (int k = 0; k < PW - 1; k++) v[k] = v[k + 1];
-    v[PW - 1] = t;
+    for (int i = 0; i < NV - 1; i++) v[i] = v[i + 1];
+    v[NV - 1] = t;
   }
   if (pos >= 0) {
     double* dst = p.A + (size_t)pos * p.ld + p.j0;
-    if (p.vec && jb == PW) {
+    if (Q == 1 && p.vec && jb == PW) {
 #pragma unroll
-      for (int k = 0; k < PW; k += 2)
+      for (int k = 0; k < NV; k += 2)
         *reinterpret_cast<double2*>(dst + k) = make_double2(v[k], v[k + 1]);
     } else {
 #pragma unroll
-      for (int k = 0; k < PW; k++)
-        if (k < jb) dst[k] = v[k];
+      for (int i = 0; i < NV; i++)
+        if (q + Q * i < jb) dst[q + Q * i] = v[i];
     }
   }
-  if (g == 0 && warp == 0)
-    compose_swaps_warp(s_pivs, jb, p.j0, false, nullptr, p.swaps, s_atp, s_atr, lane);
+  if (g == 0 && warp == NW) compose_emit(na, p.swaps, s_atp, s_atr, lane);
 }
 
 // CTAs per cluster: LA_UNSUPPORTED (nothing launched) where such a cluster cannot be resident.
-template <int T>
+template <int T, int Q>
 la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   static unsigned ok_for[LA_MAX_DEVICES];  // bit C: a cluster of C CTAs can be resident
   static la_device_once once;
@@ -307,12 +365,12 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C);
-  cfg.blockDim = dim3(T);
+  cfg.blockDim = dim3(T + 32);
   cfg.stream = st;
   cfg.attrs = at;
   once.run([](int d) {
     ok_for[d] = 0;
-    if (cudaFuncSetAttribute(panel_cluster64_kernel<T>,
+    if (cudaFuncSetAttribute(panel_cluster64_kernel<T, Q>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
       for (int c = 1; c <= PMAXC; c *= 2) {
         cudaLaunchAttribute ca;
@@ -322,11 +380,11 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
         ca.val.clusterDim.z = 1;
         cudaLaunchConfig_t q = {};
         q.gridDim = dim3(c);
-        q.blockDim = dim3(T);
+        q.blockDim = dim3(T + 32);
         q.attrs = &ca;
         q.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, panel_cluster64_kernel<T>, &q) == cudaSuccess && n > 0)
+        if (cudaOccupancyMaxActiveClusters(&n, panel_cluster64_kernel<T, Q>, &q) == cudaSuccess && n > 0)
           ok_for[d] |= 1u << c;
       }
     cudaGetLastError();
@@ -334,7 +392,7 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   });
   if (!(ok_for[dev] >> C & 1u)) return LA_UNSUPPORTED;
   cfg.numAttrs = ctx->pdl_now ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, panel_cluster64_kernel<T>, a);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, panel_cluster64_kernel<T, Q>, a);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaLaunchKernelEx(panel_cluster64)");
   ctx->launches++;
   return LA_OK;
@@ -349,10 +407,9 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, size_t 
   const int R = m - j0;
   if (R <= 0 || jb <= 0) return LA_OK;
   if (jb > PW || R > PMAXC * 512) return LA_UNSUPPORTED;
-  // 128 rows per CTA until the cluster is full: the FMAs of 128 rows take about as long as an
-  // exchange.
+  // 32 rows per CTA until the cluster is full (R = 256: 51 us, with 128 rows per CTA 82)
   int C = 1;
-  while (C < PMAXC && R > C * 128) C *= 2;
+  while (C < PMAXC && R > C * 32) C *= 2;
   Panel64Args a;
   a.A = A;
   a.ld = ld;
@@ -367,7 +424,8 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, size_t 
   a.swaps = ctx->d_swaps;
   a.err = ctx->d_err;
   a.wait_ns = ctx->wait_limit_us > 0 ? (unsigned long long)ctx->wait_limit_us * 1000ull : WAIT_NS;
-  if (a.rpc <= 128) return launch_t<128>(ctx, st, C, a);
-  if (a.rpc <= 256) return launch_t<256>(ctx, st, C, a);
-  return launch_t<512>(ctx, st, C, a);
+  if (a.rpc <= 64) return launch_t<256, 4>(ctx, st, C, a);
+  if (a.rpc <= 128) return launch_t<256, 2>(ctx, st, C, a);
+  if (a.rpc <= 256) return launch_t<256, 1>(ctx, st, C, a);
+  return launch_t<512, 1>(ctx, st, C, a);
 }

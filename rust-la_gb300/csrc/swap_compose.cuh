@@ -29,42 +29,33 @@ __device__ __forceinline__ int swap_find(const int* arr, int na, int val, int la
   return -1;
 }
 
-// Called by all 32 lanes of one warp. by_row = false: fin[c] is x_c, the
-// position swapped with j0 + c. by_row = true: fin[c] is the ORIGINAL row that
-// must end at position j0 + c; x_c is its position at step c, written to
-// ipiv[j0 + c] when ipiv is non-null. Writes the moves to swaps: swaps[0] =
-// count, swaps[1 + i] = dst, swaps[1 + 2 MAX_PANEL_W + i] = src.
-__device__ __forceinline__ void compose_swaps_warp(const int* fin, int jb, int j0, bool by_row,
-                                                   int* ipiv, int* swaps, int* at_pos,
-                                                   int* at_row, int lane) {
-  int na = 0;
-  for (int c = 0; c < jb; c++) {
-    const int a = j0 + c;
-    int x = fin[c];
-    if (by_row) {
-      const int t = swap_find(at_row, na, x, lane);
-      if (t >= 0) x = at_pos[t];
-    }
-    if (ipiv != nullptr && lane == 0) ipiv[a] = x;
-    if (x == a) continue;
-    int ia = swap_find(at_pos, na, a, lane);
-    int ix = swap_find(at_pos, na, x, lane);
-    if (ia < 0) {
-      if (lane == 0) { at_pos[na] = a; at_row[na] = a; }
-      ia = na++;
-    }
-    if (ix < 0) {
-      if (lane == 0) { at_pos[na] = x; at_row[na] = x; }
-      ix = na++;
-    }
-    __syncwarp();
-    if (lane == 0) {
-      const int t = at_row[ia];
-      at_row[ia] = at_row[ix];
-      at_row[ix] = t;
-    }
-    __syncwarp();
+// One interchange (a, x) on the slot table of na slots; called by all 32 lanes of one warp.
+static __device__ __noinline__ void compose_step(int a, int x, int& na, int* at_pos, int* at_row,
+                                             int lane) {
+  if (x == a) return;
+  int ia = swap_find(at_pos, na, a, lane);
+  int ix = swap_find(at_pos, na, x, lane);
+  if (ia < 0) {
+    if (lane == 0) { at_pos[na] = a; at_row[na] = a; }
+    ia = na++;
   }
+  if (ix < 0) {
+    if (lane == 0) { at_pos[na] = x; at_row[na] = x; }
+    ix = na++;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    const int t = at_row[ia];
+    at_row[ia] = at_row[ix];
+    at_row[ix] = t;
+  }
+  __syncwarp();
+}
+
+// The moves of a slot table of na slots: swaps[0] = count, swaps[1 + i] = dst,
+// swaps[1 + 2 MAX_PANEL_W + i] = src.
+__device__ __forceinline__ void compose_emit(int na, int* swaps, const int* at_pos,
+                                             const int* at_row, int lane) {
   int k = 0;
   for (int s = 0; s * 32 < na; s++) {
     const int t = s * 32 + lane;
@@ -78,4 +69,13 @@ __device__ __forceinline__ void compose_swaps_warp(const int* fin, int jb, int j
     k += __popc(b);
   }
   if (lane == 0) swaps[0] = k;
+}
+
+// Called by all 32 lanes of one warp: the moves of the interchanges (j0 + c, fin[c]), c < jb, in
+// order. (A kernel with a warp to spare calls compose_step as it finds them.)
+__device__ __forceinline__ void compose_swaps_warp(const int* fin, int jb, int j0, int* swaps,
+                                                   int* at_pos, int* at_row, int lane) {
+  int na = 0;
+  for (int c = 0; c < jb; c++) compose_step(j0 + c, fin[c], na, at_pos, at_row, lane);
+  compose_emit(na, swaps, at_pos, at_row, lane);
 }
