@@ -22,23 +22,26 @@
 // So an element has one rounding where an FMA chain has K, plus an error of about
 // sqrt(K) 2^-64 2^(ea_i + eb_j) from the digits left out.
 //
-// Which tiles take this path. That last error is relative to the row's and the
-// column's largest entries, an FMA chain's to sum_k |a_ik b_kj|. The split kernels
-// count, per row and per column, the entries within 2^-5 of the scale; a tile whose
-// smallest row count and smallest column count add up to more than 5/4 K has at least
-// K/4 k where both are large, so sum |a b| >= K/4 2^-10 2^(ea+eb), and for K >= 48 the
-// error left out is below the chain's own (about 0.2 2^-53 sum |a b| for terms of
-// random signs). Every other tile (outliers, graded or sparse rows, values that are
-// not finite or beyond 2^+-400) goes on a list that fma_tiles_kernel, launched right
-// after, works off with FMA chains in ascending k, 64 x 64 tiles as in gemm_f64.cu (it
-// ends at once where the list is empty). The decision is made on the device.
+// Which tiles take this path. That last error is relative to the row's and the column's largest
+// entries, an FMA chain's to sum_k |a_ik b_kj|: about 0.2 2^-53 of it for terms of random signs.
+// So a tile is computed this way where for every element, in units of 2^(ea_i + eb_j),
+//     sum_k |a_ik b_kj| >= 2^-8.9 sqrt(K),
+// where the error left out is no larger than the chain's. guard_kernel decides it per tile, in two
+// steps. The split kernels count, per row and column, the entries within 2^-5 of the scale; if the
+// smallest row count and the smallest column count exceed K by 2 sqrt(K) together, that many k have
+// both entries large, and the sum is at least 2 sqrt(K) 2^-10. Else the sums are formed, in FP32
+// from the leading two digits (8 us for 128 x 64 x 256, where the FMA tile takes 1 ms). Every other
+// tile (graded or sparse operands, values that are not finite or beyond 2^+-400) goes on a list that
+// fma_tiles_kernel, launched after the product, works off with FMA chains in ascending k, 64 x 64
+// tiles as in gemm_f64.cu (it ends at once where the list is empty).
 //
-// Measured on 8192^3 (A and B N(0,1)): 27.9 ms against 876.6 ms by FMA, 36 x 2 x 8192^3 FP16
-// operations in all, 1.42 PFLOP/s; rms error against quadruple precision 5 to 17 times smaller than
-// the FMA chain's (K = 64 to 2049). What bounds it: the MMAs of 128 k (9.2k clocks at the
-// tensor peak) and reading the accumulators after them (about 5k clocks), one after the other, since
-// a tile's accumulators fill the tensor memory. For K = 64 (8192 x 8192, 0.40 ms) the integer
-// instructions of the rounding bound it (ALU pipe 59 % busy, tensor pipe 26 %, DRAM 16 %).
+// Measured on 8192^3 (A and B N(0,1)): 24.0 ms against 876.6 ms by FMA, 36 x 2 x 8192^3 FP16
+// operations in all, 1.65 PFLOP/s; rms error against quadruple precision 5 to 17 times smaller than
+// the FMA chain's (K = 64 to 2049). What bounds it: the MMAs of 128 k (9.2k clocks at the tensor
+// peak) and the part of reading the accumulators (about 5k clocks per 128 k) that does not overlap
+// them. The tile's accumulators fill the tensor memory, so they are handed over in two halves: 0-3
+// while 4-7 are still being computed, and 4-7 while the next k's 0-3 are (28.0 ms in one piece).
+// For K = 64 (8192 x 8192 in 0.37 ms) the epilogue's integer instructions bound it.
 //
 // Layout. 128 x 64 output tiles, one persistent CTA per SM: the eight accumulators of
 // a tile fill its 512 tensor-memory columns. Digits are K-major FP16, [digit][row][k];
@@ -74,6 +77,7 @@ constexpr uint32_t EPI_BYTES = EPI_WARPS * 32 * 8 * 8;  // 32 KB: per warp 32 ro
 constexpr size_t SPLIT_SMEM = (size_t)NST * PST_BYTES + EPI_BYTES + 1024;
 constexpr int EXP_LIMIT = 400;        // |ea|, |eb| the digits are used for
 constexpr int LARGE_BITS = 4;         // "large": exponent within 4 of the largest (2^-5 of the scale)
+constexpr float GUARD = 0.0021f;      // 2^-8.9
 constexpr int CNT_BAD = -(1 << 29);   // count of a row the digits cannot represent
 constexpr int FT = 64, FK = 16;       // FMA tiles: 64 x 64 in slabs of 16 k
 constexpr int FMA_T = 256, FMA_PER_SM = 3;
@@ -118,19 +122,18 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
           smem_u32(bar))
       : "memory");
 }
-// Two columns of an accumulator. The wait takes the registers, so that nothing that uses them
+// Four columns of four accumulators. The wait takes the registers, so that nothing that uses them
 // moves above it.
-__device__ __forceinline__ void tmem_ld2(uint32_t addr, uint32_t (&r)[2]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
-               : "=r"(r[0]), "=r"(r[1])
+constexpr int HG = SL / 2;  // accumulators per half
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr));
 }
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[SL][2]) {
-#define LA_R2(g) "+r"(r[g][0]), "+r"(r[g][1])
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : LA_R2(0), LA_R2(1), LA_R2(2), LA_R2(3), LA_R2(4), LA_R2(5), LA_R2(6), LA_R2(7)::
-                   "memory");
-#undef LA_R2
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[HG][4]) {
+#define LA_R4(g) "+r"(r[g][0]), "+r"(r[g][1]), "+r"(r[g][2]), "+r"(r[g][3])
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : LA_R4(0), LA_R4(1), LA_R4(2), LA_R4(3)::"memory");
+#undef LA_R4
 }
 
 // ---- splitting -------------------------------------------------------------------------------
@@ -190,15 +193,11 @@ __device__ __forceinline__ bool is_denormal(double v) {
 // Rows of X (R x K, pitch ldx) into digits [SL][R][kp], exps[R] (ea) and cnt[R] (large entries).
 // One warp per row, two neighbouring k per lane: a slice's row is written 128 bytes at a time. The
 // row is read twice, the second time from L1 or L2 where K is a panel's width.
-__global__ void __launch_bounds__(256)
-split_rows_kernel(const double* __restrict__ X, size_t ldx, int R, int K, int kp,
-                  __half* __restrict__ dig, int* __restrict__ exps, int* __restrict__ cnt,
-                  int* nlist) {
-  la_pdl_wait();
-  la_pdl_trigger();
-  if (nlist && blockIdx.x == 0 && threadIdx.x == 0) *nlist = 0;
+__device__ __forceinline__ void split_rows(int block, const double* __restrict__ X, size_t ldx,
+                                           int R, int K, int kp, __half* __restrict__ dig,
+                                           int* __restrict__ exps, int* __restrict__ cnt) {
   const int lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int r = block * 8 + (threadIdx.x >> 5);
   if (r >= R) return;
   const double* x = X + (size_t)r * ldx;
   int me = 0;
@@ -254,17 +253,16 @@ col_exp_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kper,
 // time and a digit's k are written 128 bytes at a time. ALL: the CTA sees every k of its columns
 // and finds their exponents itself; else they come from col_exp_kernel and counts are added up.
 template <bool ALL>
-__global__ void __launch_bounds__(256)
-split_cols_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kp, int kper,
-                  const int* __restrict__ maxexp, __half* __restrict__ dig,
-                  int* __restrict__ exps, int* __restrict__ cnt) {
-  la_pdl_wait();
-  la_pdl_trigger();
+__device__ __forceinline__ void split_cols(int block, int yblock, const double* __restrict__ X,
+                                           size_t ldx, int K, int N, int kp, int kper,
+                                           const int* __restrict__ maxexp,
+                                           __half* __restrict__ dig, int* __restrict__ exps,
+                                           int* __restrict__ cnt) {
   __shared__ double tile[64][33];
   __shared__ int s_me[32], s_den[32];
   const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-  const int c0 = blockIdx.x * 32, c = c0 + tx;
-  const int kb = ALL ? 0 : blockIdx.y * kper, ke = ALL ? K : min(K, kb + kper);
+  const int c0 = block * 32, c = c0 + tx;
+  const int kb = ALL ? 0 : yblock * kper, ke = ALL ? K : min(K, kb + kper);
   if (ALL) {
     if (tid < 32) { s_me[tid] = 0; s_den[tid] = 0; }
     __syncthreads();
@@ -317,7 +315,7 @@ split_cols_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kp
       bool bad;
       const int top = top_of(s_me[n], bad);
       bad |= s_me[n] == 0 && s_den[n];
-      if (ALL || blockIdx.y == 0) exps[c0 + n] = top + 1 - 1023;
+      if (ALL || yblock == 0) exps[c0 + n] = top + 1 - 1023;
       const int v = bad ? CNT_BAD : s_me[n] == 0 ? ke - kb : l;
       if (ALL) cnt[c0 + n] = v;
       else if (bad) atomicMin(cnt + c0 + n, CNT_BAD / 2);
@@ -326,10 +324,35 @@ split_cols_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kp
   }
 }
 
+// Rows of A and columns of B in one launch: the first ra CTAs take 8 rows of A each, the next rb 8
+// rows of B' (b_rows) or 32 columns of B. list[0] is zeroed for the guard.
+struct SplitSide {
+  const double* X;
+  size_t ldx;
+  int n;
+  __half* dig;
+  int *exps, *cnt;
+};
+__global__ void __launch_bounds__(256)
+split_kernel(const SplitSide a, const SplitSide b, int K, int kp, int ra, int b_rows, int* list) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  const int block = blockIdx.x;
+  if (block == 0 && threadIdx.x == 0) *list = 0;
+  if (block < ra) split_rows(block, a.X, a.ldx, a.n, K, kp, a.dig, a.exps, a.cnt);
+  else if (b_rows) split_rows(block - ra, b.X, b.ldx, b.n, K, kp, b.dig, b.exps, b.cnt);
+  else split_cols<true>(block - ra, 0, b.X, b.ldx, K, b.n, kp, K, nullptr, b.dig, b.exps, b.cnt);
+}
+__global__ void __launch_bounds__(256)
+split_cols_part_kernel(const SplitSide b, int K, int kp, int kper, const int* __restrict__ maxexp) {
+  split_cols<false>(blockIdx.x, blockIdx.y, b.X, b.ldx, K, b.n, kp, kper, maxexp, b.dig, b.exps,
+                    b.cnt);
+}
+
 // ---- the product -----------------------------------------------------------------------------
 
 struct SplitArgs {
-  int M, N, K, tri, tiles_m, tiles_n, tiles;
+  int M, N, K, tri, tiles_m, tiles_n, tiles, prefetch, per_cta;
   const double* A;   // the operands themselves, for the FMA tiles
   size_t lda;
   const double* B;
@@ -338,6 +361,9 @@ struct SplitArgs {
   double* C;
   size_t ldc;
   const int *ea, *ca, *eb, *cb;
+  const __half *da, *db;  // the digits [SL][rows][kp]
+  int kp, joint;     // joint: 2 sqrt(K), rounded up
+  int* fits;         // per tile: 1 where the digits hold what it needs
   int* list;         // [0] count, then the tiles left to fma_tiles_kernel
   int* err;
 };
@@ -360,41 +386,153 @@ __device__ __forceinline__ void tile_at(const SplitArgs& p, int t, int& tm, int&
   tn = r / rows;
 }
 
-// Whether the tile's digits hold what its products need (see the head of the file). Whole warp.
-__device__ __forceinline__ bool tile_fits(const SplitArgs& p, int tm, int tn, int lane) {
-  int a = 1 << 29, b = 1 << 29;
+// fits[tile] (see the head of the file), and the list of the others. A warp per tile compares the
+// counts; the tiles they do not decide are summed by the whole CTA, one after the other.
+constexpr int GK = 32;        // k per slab of the FP32 sums
+constexpr int GUARD_T = 256;
+__global__ void __launch_bounds__(GUARD_T)
+guard_kernel(const __grid_constant__ SplitArgs p) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  __shared__ int s_sum[GUARD_T / 32];
+  __shared__ __align__(16) float as[GK][PM + 4], bs[GK][PN + 4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  {
+    const int t = blockIdx.x * p.per_cta + warp;
+    int sum = 0;
+    if (warp < p.per_cta && t < p.tiles) {
+      int tm, tn;
+      tile_at(p, t, tm, tn);
+      int a = 1 << 29, b = 1 << 29;
 #pragma unroll
-  for (int i = 0; i < PM / 32; i++) {
-    const int r = tm * PM + i * 32 + lane;
-    if (r < p.M) a = min(a, __ldg(p.ca + r));
-  }
+      for (int i = 0; i < PM / 32; i++) {
+        const int r = tm * PM + i * 32 + lane;
+        if (r < p.M) a = min(a, p.ca[r]);
+      }
 #pragma unroll
-  for (int i = 0; i < PN / 32; i++) {
-    const int c = tn * PN + i * 32 + lane;
-    if (c < p.N) b = min(b, __ldg(p.cb + c));
+      for (int i = 0; i < PN / 32; i++) {
+        const int c = tn * PN + i * 32 + lane;
+        if (c < p.N) b = min(b, p.cb[c]);
+      }
+      a = __reduce_min_sync(0xffffffffu, a);
+      b = __reduce_min_sync(0xffffffffu, b);
+      const bool fit = (long long)a + b >= (long long)p.K + p.joint;
+      sum = !fit && a >= 0 && b >= 0;
+      if (lane == 0 && !sum) {
+        p.fits[t] = fit ? 1 : 0;
+        if (!fit) p.list[1 + atomicAdd(p.list, 1)] = t;
+      }
+    }
+    if (lane == 0) s_sum[warp] = sum;
   }
-  a = __reduce_min_sync(0xffffffffu, a);
-  b = __reduce_min_sync(0xffffffffu, b);
-  return 4 * ((long long)a + b) > 5 * (long long)p.K;
+  __syncthreads();
+  for (int w = 0; w < GUARD_T / 32; w++) {
+    if (!s_sum[w]) continue;
+    const int t = blockIdx.x * p.per_cta + w;
+    int tm, tn;
+    tile_at(p, t, tm, tn);
+    // sum_k |a_ik| |b_kj| in units of 2^(ea + eb), every element of the tile: rows 8 ty.., columns
+    // 4 tx..
+    const int tx = tid & 15, ty = tid >> 4;
+    const size_t sa = (size_t)p.M * p.kp, sb = (size_t)p.N * p.kp;
+    constexpr int LOADS = (PM + PN) * (GK / 4) / GUARD_T;  // 4 k of one row per load
+    uint2 d0[LOADS], d1[LOADS];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int q = 0; q < LOADS; q++) {
+        const int e = tid + q * GUARD_T, row = e / (GK / 4), k = k0 + e % (GK / 4) * 4;
+        const bool ina = row < PM;
+        const int g = ina ? tm * PM + row : tn * PN + row - PM;
+        d0[q] = d1[q] = make_uint2(0u, 0u);
+        if (g < (ina ? p.M : p.N) && k < p.K) {  // rows are kp values, a multiple of 8
+          const __half* d = (ina ? p.da : p.db) + (size_t)g * p.kp + k;
+          d0[q] = *reinterpret_cast<const uint2*>(d);
+          d1[q] = *reinterpret_cast<const uint2*>(d + (ina ? sa : sb));
+        }
+      }
+    };
+    float acc[8][4] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < p.K; k0 += GK) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < LOADS; q++) {
+        const int e = tid + q * GUARD_T, row = e / (GK / 4), k = e % (GK / 4) * 4;
+        const __half* x = reinterpret_cast<const __half*>(&d0[q]);
+        const __half* y = reinterpret_cast<const __half*>(&d1[q]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float v = k0 + k + i < p.K ? fabsf(__half2float(x[i]) * 0.0078125f +
+                                                   __half2float(y[i]) * 3.0517578125e-5f)
+                                           : 0.f;  // what lies between K and kp is not set
+          if (row < PM) as[k + i][row] = v;
+          else bs[k + i][row - PM] = v;
+        }
+      }
+      __syncthreads();
+      if (k0 + GK < p.K) fetch(k0 + GK);
+#pragma unroll 8
+      for (int k = 0; k < GK; k++) {
+        const float4 x0 = *reinterpret_cast<const float4*>(&as[k][8 * ty]);
+        const float4 x1 = *reinterpret_cast<const float4*>(&as[k][8 * ty + 4]);
+        const float4 y0 = *reinterpret_cast<const float4*>(&bs[k][4 * tx]);
+        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+        const float y[4] = {y0.x, y0.y, y0.z, y0.w};
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+      }
+    }
+    const float need = GUARD * sqrtf((float)p.K);
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (tm * PM + 8 * ty + i < p.M && tn * PN + 4 * tx + j < p.N) ok = ok && acc[i][j] >= need;
+    const bool fit = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (tid == 0) {
+      p.fits[t] = fit ? 1 : 0;
+      if (!fit) p.list[1 + atomicAdd(p.list, 1)] = t;
+    }
+  }
 }
 
-// (hi 2^32 + lo) 2^(sc - 70) rounded to nearest (ties away from zero), by integer instructions
-// without branches. The sum is below 2^95; the exponent limits keep the result a normal number.
-__device__ __forceinline__ double round_sum(long long hi, long long lo, int sc) {
-  const long long p = hi + (lo >> 32);  // the sum's upper 64 bits, above 32 in w
-  const long long sg = p >> 63;
-  const unsigned s32 = (unsigned)sg;
-  unsigned w = ((unsigned)lo ^ s32) - s32;
-  unsigned long long m = (unsigned long long)(p ^ sg) + (w == 0u ? (s32 & 1u) : 0u);
-  const bool low = m == 0;
-  m = low ? (unsigned long long)w : m;
-  w = low ? 0u : w;
-  const int z = __clzll((long long)m);
-  const unsigned long long n = (m << z) | (((unsigned long long)w << 32) >> (64 - z));
-  const unsigned long long mant = (n >> 11) + ((n >> 10) & 1u);  // 53 bits, the first one set
-  const int e = (low ? 63 : 95) - z + sc - 70 + 1022;
-  const unsigned long long bits = ((unsigned long long)(unsigned)e << 52) + mant;
-  return __longlong_as_double((long long)(n == 0 ? 0ull : bits | (unsigned long long)sg << 63));
+// A signed 96-bit integer, least significant word first.
+struct Sum96 {
+  unsigned x0, x1, x2;
+};
+__device__ __forceinline__ Sum96 sum96(long long hi, long long lo) {  // hi 2^32 + lo
+  const long long u = hi + (lo >> 32);
+  return {(unsigned)lo, (unsigned)u, (unsigned)(u >> 32)};
+}
+// a 2^(sc - 70) rounded to nearest (ties away from zero), by integer instructions without
+// branches; the exponent limits keep the result a normal number. (The ALU pipe, not the tensor
+// pipe, bounds products of K = 64: every instruction here counts.)
+__device__ __forceinline__ double round_sum(Sum96 a, int sc) {
+  const bool neg = (int)a.x2 < 0;
+  if (neg)
+    asm("sub.cc.u32 %0, 0, %0;\n\tsubc.cc.u32 %1, 0, %1;\n\tsubc.u32 %2, 0, %2;"
+        : "+r"(a.x0), "+r"(a.x1), "+r"(a.x2));
+  // the first word that is not zero leads (a sum below 2^32 is moved up two words, which takes
+  // another look below)
+  const bool s1 = a.x2 == 0u;
+  unsigned hi = s1 ? a.x1 : a.x2, mi = s1 ? a.x0 : a.x1, lo = s1 ? 0u : a.x0;
+  int e = s1 ? 63 : 95;
+  if (hi == 0u) {  // rare: below 2^-38 of the scale
+    hi = mi;
+    mi = 0u;
+    e = 31;
+  }
+  const int z = __clz((int)hi);
+  const unsigned nh = __funnelshift_l(mi, hi, z), nl = __funnelshift_l(lo, mi, z);
+  const unsigned ml = __funnelshift_r(nl, nh, 11), up = nl >> 10 & 1u;
+  const unsigned mh = (nh >> 11) + ((unsigned)(e - z + sc - 70 + 1022) << 20);
+  unsigned rl, rh;
+  asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;" : "=r"(rl), "=r"(rh) : "r"(ml), "r"(up), "r"(mh));
+  rh = neg ? rh | 0x80000000u : rh;
+  return hi == 0u ? 0.0 : __hiloint2double((int)rh, (int)rl);
 }
 
 // MODE -1: C -= A B, 0: C = A B, 1: C += A B.
@@ -405,7 +543,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   la_pdl_wait();
   la_pdl_trigger();
   extern __shared__ __align__(1024) unsigned char split_raw[];
-  __shared__ __align__(8) uint64_t full[NST], empty[NST], acc_full, acc_empty, last;
+  __shared__ __align__(8) uint64_t full[NST], empty[NST], acc_full[2], acc_empty[2], last;
   __shared__ uint32_t tmem_holder;
   __shared__ volatile int s_fail;
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -419,8 +557,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(&acc_full, 1);
-    mbar_init(&acc_empty, EPI_WARPS);
+    for (int h = 0; h < 2; h++) {
+      mbar_init(&acc_full[h], 1);
+      mbar_init(&acc_empty[h], EPI_WARPS);
+    }
     mbar_init(&last, 1);
     s_fail = 0;
     la_tma::mbar_init_fence();
@@ -439,9 +579,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
     int n = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+      if (!__ldg(p.fits + t)) continue;
       int tm, tn;
       tile_at(p, t, tm, tn);
-      if (!tile_fits(p, tm, tn, lane)) continue;
+      // C's tile into L2 (its rows are 512 bytes; the epilogue's loads would wait for DRAM)
+      if (p.prefetch)
+        for (int q = lane; q < PM * 4; q += 32) {
+          const int r = tm * PM + q / 4, c = tn * PN + q % 4 * 16;
+          if (r < p.M && c < p.N)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.C + (size_t)r * p.ldc + c));
+        }
       if (lane == 0)
         for (int s = 0; s < nst; s++, n++) {
           const int b = n % NST;
@@ -464,41 +611,40 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
     int n = 0, chunk = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
-      int tm, tn;
-      tile_at(p, t, tm, tn);
-      if (!tile_fits(p, tm, tn, lane)) continue;
+      if (!__ldg(p.fits + t)) continue;
       if (lane == 0)
         for (int s = 0; s < nst && ok; s++, n++) {
           const int b = n % NST;
-          if (s % CHUNK_STAGES == 0 && chunk > 0 &&
-              !sw_wait(&acc_empty, (uint32_t)((chunk - 1) & 1), p.err))
-            ok = false;
-          if (ok && !sw_wait(&full[b], (uint32_t)((n / NST) & 1), p.err)) ok = false;
+          const bool first = s % CHUNK_STAGES == 0;
+          const bool end = s % CHUNK_STAGES == CHUNK_STAGES - 1 || s == nst - 1;
+          if (!sw_wait(&full[b], (uint32_t)((n / NST) & 1), p.err)) ok = false;
+          const uint32_t sa = smem_u32(smem + b * PST_BYTES), sb = sa + PA_BYTES;
+          // accumulators 0-3, then 4-7: digit d of A with the digits t of B, d + t in the half
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            if (ok && first && chunk > 0 &&
+                !sw_wait(&acc_empty[h], (uint32_t)((chunk - 1) & 1), p.err))
+              ok = false;
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll
+            for (int k = 0; k < PK / 16; k++)
+#pragma unroll
+              for (int d = 0; d < (h ? SL : HG); d++) {
+                const int t0 = h ? (d < HG ? HG - d : 0) : 0;
+                const int t1 = h ? SL - d : HG - d;
+                mma_f16(tmem + (d + t0) * PN, sdesc64(sa + d * (PM * PK * 2) + k * 32),
+                        sdesc64(sb + t0 * (PN * PK * 2) + k * 32), idesc_f16((t1 - t0) * PN),
+                        d == 0 && first && k == 0 ? 0u : 1u);
+              }
+            if (end) tc_commit(&acc_full[h]);
+          }
           if (!ok) {
             s_fail = 1;
             break;
           }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa = smem_u32(smem + b * PST_BYTES), sb = sa + PA_BYTES;
-#pragma unroll
-          for (int k = 0; k < PK / 16; k++) {
-            const uint32_t acc = s % CHUNK_STAGES == 0 && k == 0 ? 0u : 1u;
-#pragma unroll
-            for (int d = 0; d < SL; d++) {  // digit d of A with digits [0, 8 - d) of B
-              const uint64_t ad = sdesc64(sa + d * (PM * PK * 2) + k * 32);
-              const int n0 = SL - d < 4 ? SL - d : 4, n1 = SL - d - n0;
-              mma_f16(tmem + d * PN, ad, sdesc64(sb + k * 32), idesc_f16(n0 * PN),
-                      d == 0 ? acc : 1u);
-              if (n1 > 0)
-                mma_f16(tmem + (d + 4) * PN, ad, sdesc64(sb + 4 * (PN * PK * 2) + k * 32),
-                        idesc_f16(n1 * PN), d == 0 ? acc : 1u);
-            }
-          }
           tc_commit(&empty[b]);
-          if (s % CHUNK_STAGES == CHUNK_STAGES - 1 || s == nst - 1) {
-            tc_commit(&acc_full);
-            chunk++;
-          }
+          if (end) chunk++;
         }
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
     }
@@ -514,42 +660,43 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
     int chunk = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
+      if (!__ldg(p.fits + t)) continue;
       int tm, tn;
       tile_at(p, t, tm, tn);
-      if (!tile_fits(p, tm, tn, lane)) {
-        if (tid == 0) p.list[1 + atomicAdd(p.list, 1)] = t;
-        continue;
-      }
       const int m0 = tm * PM, n0 = tn * PN;
       const int sr = m0 + row < p.M ? __ldg(p.ea + m0 + row) : 0;
       const int sc = n0 + col + (lane & 15) < p.N ? __ldg(p.eb + n0 + col + (lane & 15)) : 0;
-      long long hi[16], lo[16];
+      long long hi[16], lo[16];  // d[0..3] 2^(24 - 8 g), d[4..7] 2^(56 - 8 g)
 #pragma unroll
       for (int j = 0; j < 16; j++) hi[j] = lo[j] = 0;
-      for (int c = 0; c < nchunk; c++, chunk++) {
-        // warp-uniform: every lane waits on the same phase
-        ok = __all_sync(0xffffffffu, sw_wait(&acc_full, (uint32_t)(chunk & 1), p.err));
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;");
+      for (int c = 0; c < nchunk && ok; c++, chunk++) {
 #pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-          uint32_t r[SL][2];
+        for (int h = 0; h < 2; h++) {
+          // warp-uniform: every lane waits on the same phase
+          ok = ok && __all_sync(0xffffffffu, sw_wait(&acc_full[h], (uint32_t)(chunk & 1), p.err));
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-          for (int g = 0; g < SL; g++) tmem_ld2(tbase + g * PN + j, r[g]);
-          tmem_wait(r);
+          for (int j = 0; j < 16; j += 4) {
+            uint32_t r[HG][4];
 #pragma unroll
-          for (int i = 0; i < 2; i++) {
-            int d[SL];
+            for (int g = 0; g < HG; g++) tmem_ld4(tbase + (h * HG + g) * PN + j, r[g]);
+            tmem_wait(r);
 #pragma unroll
-            for (int g = 0; g < SL; g++) d[g] = __float2int_rn(__uint_as_float(r[g][i]));
-            const int h0 = d[0] * 256 + d[1], h1 = d[2] * 256 + d[3];  // below 2^31
-            hi[j + i] += (long long)h0 * 65536 + h1;
-            lo[j + i] += (long long)d[4] * 16777216 + (long long)d[5] * 65536 +
-                         (long long)d[6] * 256 + d[7];
+            for (int i = 0; i < 4; i++) {
+              int d[HG];
+#pragma unroll
+              for (int g = 0; g < HG; g++) d[g] = __float2int_rn(__uint_as_float(r[g][i]));
+              if (h == 0)  // d[0] 256 + d[1] and d[2] 256 + d[3] are below 2^31
+                hi[j + i] += (long long)(d[0] * 256 + d[1]) * 65536 + (d[2] * 256 + d[3]);
+              else
+                lo[j + i] += (long long)d[0] * 16777216 + (long long)d[1] * 65536 +
+                             (long long)d[2] * 256 + d[3];
+            }
           }
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          if (lane == 0) mbar_arrive(&acc_empty[h]);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;");
-        if (lane == 0) mbar_arrive(&acc_empty);
       }
       if (!ok) break;
       // 8 columns at a time through shared memory: each lane rounds its row, then the warp reads
@@ -568,7 +715,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
         for (int j = 0; j < 8; j++) {
           const int eb = __shfl_sync(0xffffffffu, sc, g * 8 + j);
           wbuf[lane * 8 + (j ^ ((lane >> 1) & 7))] =
-              round_sum(hi[g * 8 + j], lo[g * 8 + j], sr + eb);
+              round_sum(sum96(hi[g * 8 + j], lo[g * 8 + j]), sr + eb);
         }
         __syncwarp();
 #pragma unroll
@@ -687,13 +834,16 @@ la_status launch_product(la_ctx ctx, cudaStream_t st, const CUtensorMap& ta, con
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SPLIT_SMEM);
   });
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaFuncSetAttribute(gemm_split)");
+  e = la_launch(ctx, guard_kernel, dim3((p.tiles + p.per_cta - 1) / p.per_cta), dim3(GUARD_T), 0, st,
+                p);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "guard_kernel launch");
   e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(std::min(p.tiles, ctx->sm_count)),
                 dim3(SPLIT_T), SPLIT_SMEM, st, ta, tb, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "gemm_split_kernel launch");
   const int halves = (int)std::min<long long>(2ll * p.tiles, (long long)FMA_PER_SM * ctx->sm_count);
   e = la_launch(ctx, fma_tiles_kernel<MODE>, dim3(halves), dim3(FMA_T), 0, st, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "fma_tiles_kernel launch");
-  ctx->launches += 2;
+  ctx->launches += 3;
   return la_check_launch(ctx, "gemm_split_kernel");
 }
 
@@ -714,40 +864,32 @@ struct Side {
 
 constexpr int COLS_ALL_K = 512;  // columns of up to this many k are split by one CTA per 32
 
-la_status split_rows(la_ctx ctx, cudaStream_t st, const double* X, size_t ldx, int R, int K, int kp,
-                     const Side& s, int* nlist) {
-  const cudaError_t e = la_launch(ctx, split_rows_kernel, dim3((R + 7) / 8), dim3(256), 0, st, X,
-                                  ldx, R, K, kp, s.dig, s.exps, s.cnt, nlist);
-  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "split_rows_kernel launch");
+la_status launch_splits(la_ctx ctx, cudaStream_t st, const SplitSide& a, const SplitSide& b, bool same,
+                        bool b_rows, int K, int kp, int* maxexp, int* list) {
+  const int ra = (a.n + 7) / 8;
+  const bool parts = !same && !b_rows && K > COLS_ALL_K;
+  const int rb = same || parts ? 0 : b_rows ? (b.n + 7) / 8 : (b.n + 31) / 32;
+  cudaError_t e = la_launch(ctx, split_kernel, dim3(ra + rb), dim3(256), 0, st, a, b, K, kp, ra,
+                            b_rows ? 1 : 0, list);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "split_kernel launch");
   ctx->launches++;
-  return la_check_launch(ctx, "split_rows_kernel");
-}
-
-la_status split_cols(la_ctx ctx, cudaStream_t st, const double* X, size_t ldx, int K, int N, int kp,
-                     const Side& s) {
-  cudaError_t e;
-  if (K <= COLS_ALL_K) {
-    e = la_launch(ctx, split_cols_kernel<true>, dim3((N + 31) / 32), dim3(256), 0, st, X, ldx, K, N,
-                  kp, K, (const int*)nullptr, s.dig, s.exps, s.cnt);
-  } else {
-    const int kper = 256, gy = (K + kper - 1) / kper;
-    LA_CUDA(ctx, cudaMemsetAsync(s.cnt, 0, (size_t)N * 3 * sizeof(int), st));  // cnt and me
-    col_exp_kernel<<<dim3((N + 31) / 32, gy), 256, 0, st>>>(X, ldx, K, N, kper, s.me);
-    ctx->launches++;
-    split_cols_kernel<false><<<dim3((N + 31) / 32, gy), 256, 0, st>>>(
-        X, ldx, K, N, kp, kper, s.me, s.dig, s.exps, s.cnt);
-    e = cudaGetLastError();
+  if (parts) {
+    const int kper = 256;
+    const dim3 grid((b.n + 31) / 32, (K + kper - 1) / kper);
+    // cnt and, right after it, the two words per column of col_exp_kernel
+    LA_CUDA(ctx, cudaMemsetAsync(b.cnt, 0, (size_t)b.n * 3 * sizeof(int), st));
+    col_exp_kernel<<<grid, 256, 0, st>>>(b.X, b.ldx, K, b.n, kper, maxexp);
+    split_cols_part_kernel<<<grid, 256, 0, st>>>(b, K, kp, kper, maxexp);
+    ctx->launches += 2;
   }
-  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "split_cols_kernel launch");
-  ctx->launches++;
-  return la_check_launch(ctx, "split_cols_kernel");
+  return la_check_launch(ctx, "split_kernel");
 }
 
 }  // namespace
 
 size_t gemm_split_ws(int M, int N, int K, bool same) {
   const size_t kp = up(K, 8), tiles = up(M, PM) / PM * (up(N, PN) / PN + 2);
-  return Side::bytes(M, kp) + (same ? 0 : Side::bytes(N, kp)) + up((tiles + 1) * 4, 256);
+  return Side::bytes(M, kp) + (same ? 0 : Side::bytes(N, kp)) + up((2 * tiles + 1) * 4, 256);
 }
 
 la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
@@ -788,13 +930,18 @@ la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N,
   p.ca = sa.cnt;
   p.eb = sb.exps;
   p.cb = sb.cnt;
+  p.prefetch = mode != 0;
+  // tiles per CTA of the guard: one while that leaves SMs free, up to eight
+  p.per_cta = std::min(GUARD_T / 32, 1 + p.tiles / (4 * ctx->sm_count));
+  p.da = sa.dig;
+  p.db = sb.dig;
+  p.kp = kp;
+  p.joint = (int)std::ceil(2.0 * std::sqrt((double)K));
   p.list = list;
+  p.fits = list + 1 + p.tiles;
   p.err = ctx->d_err;
-  LA_TRY(split_rows(ctx, st, A, lda, M, K, kp, sa, list));
-  if (!same) {
-    if (b_rows) LA_TRY(split_rows(ctx, st, B, ldb, N, K, kp, sb, nullptr));
-    else LA_TRY(split_cols(ctx, st, B, ldb, K, N, kp, sb));
-  }
+  const SplitSide xa{A, lda, M, sa.dig, sa.exps, sa.cnt}, xb{B, ldb, N, sb.dig, sb.exps, sb.cnt};
+  LA_TRY(launch_splits(ctx, st, xa, xb, same, b_rows, K, kp, sb.me, list));
   if (mode < 0) return launch_product<-1>(ctx, st, ta, tb, p);
   if (mode == 0) return launch_product<0>(ctx, st, ta, tb, p);
   return launch_product<1>(ctx, st, ta, tb, p);
