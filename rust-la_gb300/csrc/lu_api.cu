@@ -76,112 +76,159 @@ enum { PH_PANEL = 0, PH_SWAP = 1, PH_TRSM = 2, PH_GEMM = 3, PH_OTHER = 4 };
 // SM room for one CTA of the concurrent panel kernel.
 constexpr size_t GEMM_SMEM_WITH_PANEL = 78 * 1024;
 
-// FAST factorization of h->d_lu in place. Blocks of LU_NB = 64 columns, each factored in panels of
-// at most 32:
+// FAST factorization of h->d_lu in place. Blocks of LU_BASE = 64 columns are factored in panels of at
+// most 32:
 //   panel : cluster kernel (panel_cluster64.cu), the cooperative one (lu_panel.cu) beyond 8192 rows
 //   swaps of the panel on all other columns
 //   inner : triangular solve and FMA update of the block's remaining columns (32 x 32, K = 32)
-// then the block's triangular solve and its update A22 -= L21 U12 (K = 64) on all columns right of
-// it, by exact splitting on the tensor cores (gemm_split.cu). Every launch is a dependent one, so
-// that only their execution adds up. Measured, factor + solve: n = 8192, 16 right-hand sides 81 ms
-// (FP64 FMA updates beside a cooperative 64-column panel: 328 ms); n = 512 2.13 ms (3.86 ms). The
-// panels (30 ms of the 81) and the split updates (30 ms) bound it.
+// and a wider block is its left half, that half's triangular solve and update of the right half,
+// and the right half. After a block come its triangular solve and its update A22 -= L21 U12 on all
+// columns right of it. Updates run on the tensor cores by exact splitting (gemm_split.cu), whose
+// cost is the epilogue's per element of C, about the same for K = 64 and K = 256; so blocks are
+// wide where there are many rows (lu_block), and 64 columns where the launches of the wider
+// blocks' inner steps would cost more than they save. Every launch is a dependent one, so that only
+// their execution adds up. Measured, factor + solve with 16 right-hand sides at n = 8192: 54.9 ms
+// (64-column blocks throughout: 69.3 ms in the same build but for the guard of the split products;
+// FP64 FMA updates beside a cooperative panel: 328 ms).
 //
-// Every element's operations depend on the block's column and on the 128 x 64 tile grid that
-// starts at the block's end alone, so the allocation-free entry point, which updates in pieces of
-// whole tiles, gives the same bits.
-constexpr int LU_NB = 64;
+// Every element's operations depend on the blocks' columns and on the 128 x 64 tile grid that
+// starts at each update's corner alone, so the allocation-free entry point, which updates in
+// pieces of whole tiles, gives the same bits.
+constexpr int LU_BASE = 64;
+constexpr int LU_MAX_BLOCK = 256;
 constexpr int SPLIT_MIN_MN = 64 * 64;  // smaller updates: one FMA launch is no slower than four
 
-// C -= A B in pieces of whole tiles that the workspace takes.
-la_status split_update(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
-                       const double* B, size_t ldb, double* C, size_t ldc, void* ws, size_t bytes) {
-  int rb = M, cb = N;
-  while (gemm_split_ws(rb, cb, K, false) > bytes) {
-    if (rb <= 128 && cb <= 64) return LA_UNSUPPORTED;
-    if (rb > cb && rb > 128) rb = (rb + 1) / 2 > 128 ? ((rb + 1) / 2 + 127) / 128 * 128 : 128;
-    else if (cb > 64) cb = (cb + 1) / 2 > 64 ? ((cb + 1) / 2 + 63) / 64 * 64 : 64;
-    else rb = (rb + 1) / 2 > 128 ? ((rb + 1) / 2 + 127) / 128 * 128 : 128;
+// Block width for R remaining rows.
+int lu_block(int R) { return R > 3072 ? 256 : R > 1024 ? 128 : LU_BASE; }
+
+struct FastLu {
+  la_ctx ctx;
+  double* A;
+  size_t ld;
+  int m, n, W;
+  int* ipiv;
+  void* ws;
+  size_t ws_bytes;
+  unsigned bar_base = 0;
+  PhaseTimer t;
+
+  FastLu(la_ctx c, la_lu h)
+      : ctx(c), A(h->d_lu), ld(h->ld), m((int)h->m), n((int)h->n), W(std::min(32, c->panel_width)),
+        ipiv(h->d_ipiv), ws(c->split_ws), ws_bytes(c->split_ws_bytes), t(c) {}
+
+  double* at(int r, int c) { return A + (size_t)r * ld + c; }
+
+  // C[r0:r1, c0:c1] -= A[r0:r1, k0:k1] A[k0:k1, c0:c1], in pieces of whole tiles that the
+  // workspace takes.
+  la_status update(int r0, int r1, int k0, int k1, int c0, int c1) {
+    const int M = r1 - r0, N = c1 - c0, K = k1 - k0;
+    if (M <= 0 || N <= 0) return LA_OK;
+    if (ws && K >= 32 && (size_t)M * N >= SPLIT_MIN_MN) {
+      int rb = M, cb = N;
+      auto half = [](int x, int q) { return std::max(q, ((x + 1) / 2 + q - 1) / q * q); };
+      while (gemm_split_ws(rb, cb, K, false) > ws_bytes && (rb > 128 || cb > 64)) {
+        if (rb > 128 && rb >= cb) rb = half(rb, 128);
+        else if (cb > 64) cb = half(cb, 64);
+        else rb = half(rb, 128);
+      }
+      la_status s = LA_OK;
+      for (int r = r0; r < r1 && s == LA_OK; r += rb)
+        for (int c = c0; c < c1 && s == LA_OK; c += cb)
+          s = launch_gemm_split(ctx, ctx->stream, -1, std::min(rb, r1 - r), std::min(cb, c1 - c), K,
+                                at(r, k0), ld, at(k0, c), ld, false, at(r, c), ld, false, ws,
+                                ws_bytes);
+      if (s != LA_UNSUPPORTED) return s;
+    }
+    if (N <= 64 && K <= 64)
+      return launch_gemm_narrow(ctx, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld);
+    return launch_gemm(ctx, GM_FMA_SUB, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld);
   }
-  for (int r = 0; r < M; r += rb)
-    for (int c = 0; c < N; c += cb)
-      LA_TRY(launch_gemm_split(ctx, ctx->stream, -1, std::min(rb, M - r), std::min(cb, N - c), K,
-                               A + (size_t)r * lda, lda, B + c, ldb, false,
-                               C + (size_t)r * ldc + c, ldc, false, ws, bytes));
-  return LA_OK;
-}
+
+  // X = L11^-1 X, L11 the unit lower block of rows [r0, r1), X columns [c0, c1).
+  la_status solve(int r0, int r1, int c0, int c1) {
+    if (c1 <= c0) return LA_OK;
+    if (r1 - r0 <= LU_BASE) return launch_trsm_rowpanel(ctx, false, A, nullptr, ld, r0, r1 - r0, c0, c1);
+    const int mid = r0 + ((r1 - r0 + 1) / 2 + LU_BASE - 1) / LU_BASE * LU_BASE;
+    LA_TRY(solve(r0, mid, c0, c1));
+    LA_TRY(update(mid, r1, r0, mid, c0, c1));
+    return solve(mid, r1, c0, c1);
+  }
+
+  // Columns [b0, b1), rows [b0, m).
+  la_status factor(int b0, int b1) {
+    if (b1 - b0 > LU_BASE) {
+      const int mid = b0 + ((b1 - b0 + 1) / 2 + LU_BASE - 1) / LU_BASE * LU_BASE;
+      LA_TRY(factor(b0, mid));
+      size_t b = t.begin(ctx->stream);
+      LA_TRY(solve(b0, mid, mid, b1));
+      LA_TRY(update(mid, m, b0, mid, mid, b1));
+      t.end(ctx->stream, b, PH_OTHER);
+      return factor(mid, b1);
+    }
+    for (int j0 = b0; j0 < b1; j0 += W) {
+      const int jb = std::min(W, b1 - j0), j1 = j0 + jb;
+      size_t b = t.begin(ctx->stream);
+      la_status s = LA_UNSUPPORTED;
+      if (ctx->cluster_panels && (ctx->panel_ctas == 0 || ctx->split_ws))
+        s = launch_panel_cluster64(ctx, ctx->stream, A, ld, m, j0, jb, ipiv);
+      if (s == LA_UNSUPPORTED)
+        s = launch_panel(ctx, ctx->stream, false, A, nullptr, ld, m, j0, jb, ipiv, &bar_base);
+      LA_TRY(s);
+      t.end(ctx->stream, b, PH_PANEL);
+      b = t.begin(ctx->stream);
+      LA_TRY(launch_laswp(ctx, false, A, nullptr, ld, n, j0, jb));
+      t.end(ctx->stream, b, PH_SWAP);
+      if (j1 < b1) {
+        b = t.begin(ctx->stream);
+        LA_TRY(solve(j0, j1, j1, b1));
+        if (j1 < m)
+          LA_TRY(launch_gemm_narrow(ctx, m - j1, b1 - j1, jb, at(j1, j0), ld, at(j0, j1), ld,
+                                    at(j1, j1), ld));
+        t.end(ctx->stream, b, PH_OTHER);
+      }
+    }
+    return LA_OK;
+  }
+};
 
 la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
-  const int m = (int)h->m, n = (int)h->n, kmin = std::min(m, n);
-  const size_t ld = h->ld;
-  const int W = std::min(32, ctx->panel_width);
-  double* A = h->d_lu;
+  FastLu f(ctx, h);
+  const int m = f.m, n = f.n, kmin = std::min(m, n);
   cudaStream_t st = ctx->stream;
   LA_CUDA(ctx, cudaMemsetAsync(ctx->d_bar, 0, sizeof(unsigned), st));
-  unsigned bar_base = 0;
-  // Digits of one block's update, kept for the whole factorization. Without memory for them the
-  // updates are FMA products.
+  // Digits of one update, kept for the whole factorization. Without memory for them the updates are
+  // FMA products.
   DevBuf own(ctx);
-  void* ws = ctx->split_ws;
-  size_t ws_bytes = ctx->split_ws_bytes;
-  if (!ws && m > LU_NB && n > LU_NB && (size_t)(m - LU_NB) * (n - LU_NB) >= SPLIT_MIN_MN) {
-    ws_bytes = gemm_split_ws(m - LU_NB, n - LU_NB, LU_NB, false);
-    if (own.alloc(ws_bytes) == LA_OK) ws = own.p;
-    else ws_bytes = 0;
+  if (!f.ws && m > LU_BASE && n > LU_BASE) {
+    const int nb = std::min(lu_block(m), kmin);
+    f.ws_bytes = gemm_split_ws(m, n, nb, false);
+    if (own.alloc(f.ws_bytes) == LA_OK) f.ws = own.p;
   }
-  PhaseTimer t(ctx);
   struct PdlScope {
     la_ctx c;
     ~PdlScope() { c->pdl_now = false; }
   } scope{ctx};
-  ctx->pdl_now = ctx->pdl != 0 && !t.on;
-  for (int b0 = 0; b0 < kmin; b0 += LU_NB) {
-    const int b1 = std::min(b0 + LU_NB, kmin);
-    for (int j0 = b0; j0 < b1; j0 += W) {
-      const int jb = std::min(W, b1 - j0), j1 = j0 + jb;
-      size_t b = t.begin(st);
-      la_status s = LA_UNSUPPORTED;
-      if (ctx->cluster_panels && (ctx->panel_ctas == 0 || ctx->split_ws))
-        s = launch_panel_cluster64(ctx, st, A, ld, m, j0, jb, h->d_ipiv);
-      if (s == LA_UNSUPPORTED)
-        s = launch_panel(ctx, st, false, A, nullptr, ld, m, j0, jb, h->d_ipiv, &bar_base);
-      LA_TRY(s);
-      t.end(st, b, PH_PANEL);
-      b = t.begin(st);
-      LA_TRY(launch_laswp(ctx, false, A, nullptr, ld, n, j0, jb));
-      t.end(st, b, PH_SWAP);
-      if (j1 < b1) {
-        b = t.begin(st);
-        LA_TRY(launch_trsm_rowpanel(ctx, false, A, nullptr, ld, j0, jb, j1, b1));
-        LA_TRY(launch_gemm_narrow(ctx, m - j1, b1 - j1, jb, A + (size_t)j1 * ld + j0, ld,
-                                  A + (size_t)j0 * ld + j1, ld, A + (size_t)j1 * ld + j1, ld));
-        t.end(st, b, PH_OTHER);
-      }
+  ctx->pdl_now = ctx->pdl != 0 && !f.t.on;
+  for (int b0 = 0; b0 < kmin;) {
+    const int b1 = std::min(b0 + lu_block(m - b0), kmin);
+    LA_TRY(f.factor(b0, b1));
+    if (b1 < n) {
+      size_t b = f.t.begin(st);
+      LA_TRY(f.solve(b0, b1, b1, n));
+      f.t.end(st, b, PH_TRSM);
+      b = f.t.begin(st);
+      LA_TRY(f.update(b1, m, b0, b1, b1, n));
+      f.t.end(st, b, PH_GEMM);
     }
-    if (b1 >= n) continue;
-    size_t b = t.begin(st);
-    LA_TRY(launch_trsm_rowpanel(ctx, false, A, nullptr, ld, b0, b1 - b0, b1, n));
-    t.end(st, b, PH_TRSM);
-    if (b1 >= m) continue;
-    b = t.begin(st);
-    const double* L21 = A + (size_t)b1 * ld + b0;
-    const double* U12 = A + (size_t)b0 * ld + b1;
-    double* C = A + (size_t)b1 * ld + b1;
-    la_status s = LA_UNSUPPORTED;
-    if (ws && b1 - b0 >= 32 && (size_t)(m - b1) * (n - b1) >= SPLIT_MIN_MN)
-      s = split_update(ctx, m - b1, n - b1, b1 - b0, L21, ld, U12, ld, C, ld, ws, ws_bytes);
-    if (s == LA_UNSUPPORTED)
-      s = launch_gemm(ctx, GM_FMA_SUB, m - b1, n - b1, b1 - b0, L21, ld, U12, ld, C, ld);
-    LA_TRY(s);
-    t.end(st, b, PH_GEMM);
+    b0 = b1;
   }
   ctx->pdl_now = false;
-  size_t b = t.begin(st);
+  size_t b = f.t.begin(st);
   LA_TRY(launch_lu_finish(ctx, h, d_flags));
-  t.end(st, b, PH_OTHER);
-  if (t.on) {
+  f.t.end(st, b, PH_OTHER);
+  if (f.t.on) {
     LA_CUDA(ctx, cudaStreamSynchronize(st));
-    t.finish();
+    f.t.finish();
   } else {
     for (int i = 0; i < 5; i++) ctx->phase_ms[i] = 0;
   }
