@@ -8,22 +8,22 @@
 // returns None for a non-square matrix, at the first pair with
 // A[k][j] != A[j][k], or at the first d <= 0.
 //
-// Here the same values come from a blocked right-looking form in 64-column
-// panels (no pivoting, so every panel step is known in advance):
-//   1. chol_sym_check_kernel compares every strictly lower entry with its
-//      upper twin (the reference's '!=', so NaN fails), before anything is
-//      written;
-//   2. chol_diag_kernel factors the 64 x 64 diagonal block on one CTA, column
-//      by column;
-//   3. chol_panel_kernel computes the rows below it, one thread per row with
-//      the row's 64 values in registers;
-//   4. the trailing update A22 -= L21 L21' runs on the FP64 GEMM (TMA tiles in
-//      FAST) over row strips, each strip only up to its own diagonal, so about
-//      half of the square is skipped.
-// FAST accumulates A - sum with FMA in place. EXACT keeps, per element, the
-// running sum s in a second array S, adds products unfused in ascending i (the
-// GEMM's EXACT_ADD mode, then the panel kernels) and forms (A - s) / L[k][k]
-// and sqrt(A - d) exactly as the reference does, so L is bit-identical to it.
+// Here the same values come from blocked right-looking forms (no pivoting, so every panel step is
+// known in advance). chol_sym_check_kernel first compares every strictly lower entry with its
+// upper twin (the reference's '!=', so NaN fails), before anything is written.
+//
+// FAST (chol_fast_factor): panels of 32 columns. chol_panel32_kernel factors the 32 x 32 diagonal
+// block in every CTA (a 64 x 64 block would keep one SM's FP64 pipe busy for 22 us; 32 x 32 takes 3)
+// and solves the rows below; blocks of 64, 128 and 256 columns are a left half, its update of the
+// right half's columns, and the right half; the trailing update A22 -= L21 L21' covers the tiles at
+// or below the diagonal. Updates with K >= 64 run on the tensor cores by exact splitting
+// (gemm_split.cu; L21 is split once, as both operands), the K = 32 ones by FMA.
+//
+// EXACT: 64-column panels, chol_diag_kernel on one CTA, chol_panel_kernel for the rows below (a
+// thread per row), and the trailing update over row strips, each only up to its own diagonal. It
+// keeps, per element, the running sum s in a second array S, adds products unfused in ascending i
+// (the GEMM's EXACT_ADD mode, then the panel kernels) and forms (A - s) / L[k][k] and sqrt(A - d)
+// exactly as the reference does, so L is bit-identical to it.
 // A None result is reported after the whole factorization: the reference stops
 // at the first failing row, and every such row fails here too.
 #include "la_internal.cuh"
@@ -76,7 +76,6 @@ __global__ void chol_sym_check_kernel(const double* __restrict__ A, size_t ld, i
 
 // Diagonal block [j0, j0 + jb)^2 on one CTA (lower part, diagonal included).
 // flags[1] |= 1 at a non-positive d (cholesky.rs:97-100; NaN is not <= 0).
-template <bool EXACT>
 __global__ void __launch_bounds__(256)
 chol_diag_kernel(double* L, double* S, size_t ld, int j0, int jb, int* flags) {
   extern __shared__ __align__(16) double chd_raw[];
@@ -87,27 +86,26 @@ chol_diag_kernel(double* L, double* S, size_t ld, int j0, int jb, int* flags) {
     const int r = idx / jb, c = idx % jb;
     if (c <= r) {
       a[r][c] = L[(size_t)(j0 + r) * ld + j0 + c];
-      if (EXACT) s[r][c] = S[(size_t)(j0 + r) * ld + j0 + c];
+      s[r][c] = S[(size_t)(j0 + r) * ld + j0 + c];
     }
   }
   __syncthreads();
   for (int k = 0; k < jb; k++) {
     if (tid == 0) {
-      const double d = EXACT ? __dsub_rn(a[k][k], s[k][k]) : a[k][k];  // :96
+      const double d = __dsub_rn(a[k][k], s[k][k]);  // :96
       if (d <= 0.0) atomicOr(flags + 1, 1);
       a[k][k] = sqrt(d);  // :101
     }
     __syncthreads();
     const double dk = a[k][k];
     for (int r = k + 1 + tid; r < jb; r += 256)
-      a[r][k] = EXACT ? __dsub_rn(a[r][k], s[r][k]) / dk : a[r][k] / dk;  // :82
+      a[r][k] = __dsub_rn(a[r][k], s[r][k]) / dk;  // :82
     __syncthreads();
     const int m = jb - k - 1;
     for (int idx = tid; idx < m * m; idx += 256) {
       const int r = k + 1 + idx / m, c = k + 1 + idx % m;
       if (c > r) continue;
-      if (EXACT) s[r][c] = __dadd_rn(s[r][c], __dmul_rn(a[r][k], a[c][k]));  // :78, :86
-      else a[r][c] = fma(-a[r][k], a[c][k], a[r][c]);
+      s[r][c] = __dadd_rn(s[r][c], __dmul_rn(a[r][k], a[c][k]));  // :78, :86
     }
     __syncthreads();
   }
@@ -117,73 +115,155 @@ chol_diag_kernel(double* L, double* S, size_t ld, int j0, int jb, int* flags) {
   }
 }
 
-// FAST form of the diagonal block: warp 0 takes the square root and scales
-// the column by its reciprocal, then all threads apply the rank-1 update to
-// the lower triangle still open (rows and columns from a 16 x 16 thread
-// grid, no index division); two barriers per column.
-__global__ void __launch_bounds__(256)
-chol_diag_fast_kernel(double* L, size_t ld, int j0, int jb, int* flags) {
-  extern __shared__ __align__(16) double chd_raw[];
-  double(*a)[CHP] = reinterpret_cast<double(*)[CHP]>(chd_raw);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int idx = tid; idx < jb * jb; idx += 256) {
-    const int r = idx / jb, c = idx % jb;
-    if (c <= r) a[r][c] = L[(size_t)(j0 + r) * ld + j0 + c];
+// FAST panel: columns [j0, j0 + jb), jb <= 32, of rows [j0, n). Every CTA factors the diagonal block
+// (written to diag by CTA 0: other CTAs may still be reading the original, so it goes to L after
+// everything else), then solves its own rows below it.
+//   Diagonal block (warps 0-3): lane = row, warp w the columns c = w mod 4 in registers, so that all
+//   four FP64 pipes take part. Column k is scaled by 1/sqrt(d) in its warp and passed on through
+//   shared memory; the square roots themselves are taken at the end, all at once. The chain of 32
+//   reciprocal square roots (a dozen dependent FP64 instructions each) bounds the kernel.
+//   Rows (warps 4-7, 32 rows): 4 neighbouring lanes per row, lane q the columns c = q mod 4; x_k goes
+//   to the other three by a shuffle. An FMA instruction takes a sub-partition 64 clocks however few
+//   lanes it has, so a thread per row would need 496 x 64 clocks where this needs a quarter. They
+//   take column k while warps 0-3 work on column k + 1. Further rows of the CTA follow on all 8 warps.
+constexpr int CB = 32;
+constexpr int CB_T = 256;
+
+// One step of 4 lanes per row: v *= 1/L[k][k] in the lane of column k, then the columns after it.
+__device__ __forceinline__ void row_step(double (&v)[CB / 4], int k, int q, int lane,
+                                         const double (&dg)[CB][CB + 1], double rd) {
+  if (q == k % 4) v[k / 4] *= rd;
+  const double x = __shfl_sync(0xffffffffu, v[k / 4], lane / 4 * 4 + k % 4);
+#pragma unroll
+  for (int i = k / 4; i < CB / 4; i++)
+    if (4 * i + 3 > k && q + 4 * i > k) v[i] = fma(-x, dg[k][(q + 4 * i) % CB], v[i]);
+}
+
+__global__ void __launch_bounds__(CB_T)
+chol_panel32_kernel(double* L, size_t ld, int j0, int jb, int n, int rpc, double* diag,
+                    int* flags) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  __shared__ double dg[CB][CB + 1];  // the factored block, column by column: dg[k][r] = L[r][k]
+  __shared__ double rdg[CB], dd[CB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane & 3;
+  constexpr int NV = CB / 4;
+  const int rb = j0 + CB + blockIdx.x * rpc, re = min(n, rb + rpc);
+  double v[NV];
+  const int r1 = rb + (tid - CB_T / 2) / 4;  // warps 4-7: this thread's row
+  double* row = L + (size_t)(warp >= 4 && r1 < re ? r1 : j0) * ld + j0 + q;
+  if (warp < 4) {
+    const double* src = L + (size_t)(j0 + lane) * ld + j0 + warp;
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+      v[i] = lane < jb && warp + 4 * i <= lane ? src[4 * i] : 0.0;
+  } else {
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[i] = r1 < re ? row[4 * i] : 0.0;
   }
-  __syncthreads();
-  for (int k = 0; k < jb; k++) {
-    if (tid < 32) {
-      const double d = a[k][k];
-      const double q = sqrt(d);
-      const double rq = 1.0 / q;
-      if (tid == 0) {
-        if (d <= 0.0) atomicOr(flags + 1, 1);  // cholesky.rs:97-100
-        a[k][k] = q;
+#pragma unroll
+  for (int k = 0; k < CB; k++) {
+    if (k >= jb) break;
+    if (warp == k % 4) {
+      const double d = __shfl_sync(0xffffffffu, v[k / 4], k);
+      const double rq = rsqrt(d);
+      v[k / 4] *= rq;
+      dg[k][lane] = v[k / 4];
+      if (lane == k) {
+        rdg[k] = rq;
+        dd[k] = d;
       }
-      for (int r = k + 1 + tid; r < jb; r += 32) a[r][k] *= rq;
     }
     __syncthreads();
-    for (int r = k + 1 + ty; r < jb; r += 16) {
-      const double lr = a[r][k];
-      for (int c = k + 1 + tx; c <= r; c += 16) a[r][c] = fma(-lr, a[c][k], a[r][c]);
+    if (warp < 4) {
+      const double l = dg[k][lane];
+#pragma unroll
+      for (int i = k / 4; i < NV; i++)
+        if (4 * i + 3 > k && warp + 4 * i > k) v[i] = fma(-l, dg[k][(warp + 4 * i) % CB], v[i]);
+    } else {
+      row_step(v, k, q, lane, dg, rdg[k]);
     }
-    __syncthreads();
   }
-  for (int idx = tid; idx < jb * jb; idx += 256) {
-    const int r = idx / jb, c = idx % jb;
-    if (c <= r) L[(size_t)(j0 + r) * ld + j0 + c] = a[r][c];
+  if (warp >= 4) {
+    if (r1 < re)
+#pragma unroll
+      for (int i = 0; i < NV; i++) row[4 * i] = v[i];
+  } else if (blockIdx.x == 0) {
+    if (warp == 0 && lane < jb) {
+      if (dd[lane] <= 0.0) atomicOr(flags + 1, 1);  // cholesky.rs:97-100
+      diag[lane * (CB + 1)] = sqrt(dd[lane]);
+    }
+    for (int idx = tid; idx < CB * CB; idx += CB_T / 2)
+      if (idx / CB != idx % CB) diag[idx] = dg[idx % CB][idx / CB];  // [r][k]
+  }
+  for (int r0 = rb + CB; r0 < re; r0 += CB_T / 4) {
+    const int r = r0 + tid / 4;
+    row = L + (size_t)(r < re ? r : j0) * ld + j0 + q;
+#pragma unroll
+    for (int i = 0; i < NV; i++) v[i] = r < re ? row[4 * i] : 0.0;
+#pragma unroll
+    for (int k = 0; k < CB; k++) row_step(v, k, q, lane, dg, rdg[k]);
+    if (r < re)
+#pragma unroll
+      for (int i = 0; i < NV; i++) row[4 * i] = v[i];
   }
 }
 
-// Rows [r0, n) of the panel's columns [j0, j0 + 64): one thread per row, the
-// row's running values (FAST: A - sum; EXACT: the sums s) in registers, the
-// finished diagonal block broadcast from shared memory. Only a full-width
-// panel has rows below it (a narrower one is the last), so the width is fixed.
-template <bool EXACT>
+// C[r][c] -= sum_k L[r][j0 + k] L[c0 + c][j0 + k], k < 32, for rows [c0, n) and columns [c0, c0 + 32)
+// (the second half of a 64-column block): 16 rows per CTA, thread (column, 2 rows).
+constexpr int CU_T = 256, CU_R = 16;
+__global__ void __launch_bounds__(CU_T)
+chol_update32_kernel(double* L, size_t ld, int j0, int c0, int nc, int n) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  __shared__ double bt[CB][CB + 1], at[CB][CU_R + 1];
+  const int tid = threadIdx.x, c = tid & 31, g = tid >> 5;
+  const int rb = c0 + blockIdx.x * CU_R;
+  for (int idx = tid; idx < CB * CB; idx += CU_T) {
+    const int r = idx / CB, k = idx % CB;
+    bt[k][r] = r < nc ? L[(size_t)(c0 + r) * ld + j0 + k] : 0.0;
+  }
+  for (int idx = tid; idx < CU_R * CB; idx += CU_T) {
+    const int r = idx / CB, k = idx % CB;
+    at[k][r] = rb + r < n ? L[(size_t)(rb + r) * ld + j0 + k] : 0.0;
+  }
+  const int r0 = rb + g, r1 = rb + g + 8;
+  const bool in = c < nc;
+  double a0 = in && r0 < n ? L[(size_t)r0 * ld + c0 + c] : 0.0;
+  double a1 = in && r1 < n ? L[(size_t)r1 * ld + c0 + c] : 0.0;
+  __syncthreads();
+#pragma unroll 8
+  for (int k = 0; k < CB; k++) {
+    a0 = fma(-at[k][g], bt[k][c], a0);
+    a1 = fma(-at[k][g + 8], bt[k][c], a1);
+  }
+  if (in && r0 < n) L[(size_t)r0 * ld + c0 + c] = a0;
+  if (in && r1 < n) L[(size_t)r1 * ld + c0 + c] = a1;
+}
+
+// EXACT rows [r0, n) of the panel's columns [j0, j0 + 64): one thread per row, the row's sums s in
+// registers, the finished diagonal block broadcast from shared memory. Only a full-width panel has
+// rows below it (a narrower one is the last), so the width is fixed.
 __global__ void __launch_bounds__(PANEL_T)
 chol_panel_kernel(double* L, const double* S, size_t ld, int j0, int r0, int n) {
   __shared__ double dg[CHW][CHP];
-  __shared__ double rdg[CHW];
   for (int idx = threadIdx.x; idx < CHW * CHW; idx += PANEL_T) {
     const int r = idx / CHW, c = idx % CHW;
     if (c <= r) dg[r][c] = L[(size_t)(j0 + r) * ld + j0 + c];
   }
-  __syncthreads();
-  if (!EXACT && threadIdx.x < CHW) rdg[threadIdx.x] = 1.0 / dg[threadIdx.x][threadIdx.x];
   __syncthreads();
   const int r = r0 + blockIdx.x * PANEL_T + threadIdx.x;
   if (r >= n) return;
   double* row = L + (size_t)r * ld + j0;
   double v[CHW];
 #pragma unroll
-  for (int c = 0; c < CHW; c++) v[c] = EXACT ? S[(size_t)r * ld + j0 + c] : row[c];
+  for (int c = 0; c < CHW; c++) v[c] = S[(size_t)r * ld + j0 + c];
 #pragma unroll
   for (int k = 0; k < CHW; k++) {
-    const double x = EXACT ? __dsub_rn(row[k], v[k]) / dg[k][k] : v[k] * rdg[k];  // :82
+    const double x = __dsub_rn(row[k], v[k]) / dg[k][k];  // :82
     row[k] = x;
 #pragma unroll
-    for (int c = k + 1; c < CHW; c++)
-      v[c] = EXACT ? __dadd_rn(v[c], __dmul_rn(x, dg[c][k])) : fma(-x, dg[c][k], v[c]);
+    for (int c = k + 1; c < CHW; c++) v[c] = __dadd_rn(v[c], __dmul_rn(x, dg[c][k]));
   }
 }
 
@@ -205,10 +285,19 @@ __global__ void chol_transpose_kernel(const double* __restrict__ L, size_t ld, i
   }
 }
 
-// L[r][c] = 0 for c > r (cholesky.rs:104-106).
-__global__ void chol_zero_upper_kernel(double* L, size_t ld, int n) {
+// L[r][c] = 0 for c > r (cholesky.rs:104-106); in FAST the 32 x 32 diagonal blocks from diag.
+__global__ void chol_zero_upper_kernel(double* L, size_t ld, int n, const double* diag) {
+  la_pdl_wait();
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bj < bi) return;
+  if (diag && bi == bj) {
+    for (int r = threadIdx.y; r < 32 && bi * 32 + r < n; r += 8) {
+      const int c = threadIdx.x;
+      if (bi * 32 + c < n)
+        L[(size_t)(bi * 32 + r) * ld + bi * 32 + c] = c <= r ? diag[bi * 1024 + r * 32 + c] : 0.0;
+    }
+    return;
+  }
   for (int r = bi * 32 + threadIdx.y; r < min(n, bi * 32 + 32); r += 8) {
     const int c = bj * 32 + threadIdx.x;
     if (c < n && c > r) L[(size_t)r * ld + c] = 0.0;
@@ -234,13 +323,8 @@ __global__ void chol_back_exact_kernel(const double* __restrict__ L, size_t ld, 
 cudaError_t configure_chol() {
   static la_device_once once;
   return once.run([](int) {
-    cudaError_t e = cudaFuncSetAttribute(chol_diag_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(2 * CHW * CHP * sizeof(double)));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(chol_diag_fast_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(CHW * CHP * sizeof(double)));
-    return e;
+    return cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(2 * CHW * CHP * sizeof(double)));
   });
 }
 
@@ -251,26 +335,119 @@ la_status chol_check_ctx(la_ctx ctx) {
   return LA_OK;
 }
 
-// Factors h->d_l (a copy of A) in place; *none = the reference's None.
-la_status chol_factor(la_ctx ctx, la_chol h, int* none) {
+// FAST factorization of h->d_l (see the head of the file). Block widths as in the LU: an update's
+// cost is the split product's epilogue, so wide blocks where there are many rows. n = 4099 with 5
+// right-hand sides: 8.1 ms, of them 2.7 in the panels, 1.9 in the split products and 1.8 in the
+// solves (64-column panels with FP64 FMA updates beside them: 31.9 ms).
+struct FastChol {
+  la_ctx ctx;
+  double* L;
+  size_t ld;
+  int n;
+  double* diag;
+  int* flags;
+  void* ws;
+  size_t ws_bytes;
+  Buf T;  // a panel transposed, where the split product cannot be used
+
+  double* at(int r, int c) { return L + (size_t)r * ld + c; }
+
+  // Rows [c0, n), columns [c0, c1), -= L[.., k0:k1] L[c0:c1, k0:k1]'; lower: only at or below the
+  // diagonal (c1 = n then).
+  la_status update(int k0, int k1, int c0, int c1, bool lower) {
+    const int M = n - c0, N = c1 - c0, K = k1 - k0;
+    if (M <= 0 || N <= 0) return LA_OK;
+    if (N <= CB && K == CB) {
+      const cudaError_t e = la_launch(ctx, chol_update32_kernel, dim3((M + CU_R - 1) / CU_R),
+                                      dim3(CU_T), 0, ctx->stream, L, ld, k0, c0, N, n);
+      if (e != cudaSuccess) return la_cuda_fail(ctx, e, "chol_update32_kernel launch");
+      ctx->launches++;
+      return la_check_launch(ctx, "chol_update32_kernel");
+    }
+    if (ws) {
+      const la_status s = launch_gemm_split(ctx, ctx->stream, -1, M, N, K, at(c0, k0), ld,
+                                            at(c0, k0), ld, true, at(c0, c0), ld, lower, ws, ws_bytes);
+      if (s != LA_UNSUPPORTED) return s;
+    }
+    // by FMA, in steps of the transposed panel's 64 k
+    const size_t ldt = pad4c((size_t)n);
+    if (!T.p) LA_TRY(T.alloc((size_t)CHW * ldt * sizeof(double)));
+    for (int k = k0; k < k1; k += CHW) {
+      const int kb = std::min(CHW, k1 - k);
+      chol_transpose_kernel<<<dim3((N + 31) / 32, (kb + 31) / 32), dim3(32, 8), 0, ctx->stream>>>(
+          L, ld, k, kb, c0, N, T.d(), ldt);
+      ctx->launches++;
+      LA_TRY(la_check_launch(ctx, "chol_transpose_kernel"));
+      la_status s = LA_UNSUPPORTED;
+      if (lower) s = launch_gemm_lower(ctx, M, kb, at(c0, k), ld, T.d(), ldt, at(c0, c0), ld);
+      if (s == LA_UNSUPPORTED)
+        s = launch_gemm(ctx, GM_FMA_SUB, M, N, kb, at(c0, k), ld, T.d(), ldt, at(c0, c0), ld);
+      LA_TRY(s);
+    }
+    return LA_OK;
+  }
+
+  la_status factor(int b0, int b1) {
+    if (b1 - b0 > CB) {
+      const int mid = b0 + ((b1 - b0 + 1) / 2 + CB - 1) / CB * CB;
+      LA_TRY(factor(b0, mid));
+      LA_TRY(update(b0, mid, mid, b1, false));
+      return factor(mid, b1);
+    }
+    const int rows = n - b1;
+    // 32 rows per CTA while there are SMs for them (each CTA factors the diagonal block itself), then
+    // 64 more per pass
+    const int per = (rows + ctx->sm_count - 1) / ctx->sm_count;
+    const int rpc = CB + (std::max(0, per - CB) + 63) / 64 * 64;
+    const cudaError_t e =
+        la_launch(ctx, chol_panel32_kernel, dim3(std::max(1, (rows + rpc - 1) / rpc)), dim3(CB_T), 0,
+                  ctx->stream, L, ld, b0, b1 - b0, n, rpc, diag + (size_t)(b0 / CB) * CB * CB, flags);
+    if (e != cudaSuccess) return la_cuda_fail(ctx, e, "chol_panel32_kernel launch");
+    ctx->launches++;
+    return la_check_launch(ctx, "chol_panel32_kernel");
+  }
+};
+
+int chol_block(int R) { return R > 2048 ? 256 : R > 768 ? 128 : 64; }
+
+la_status chol_fast_factor(la_ctx ctx, la_chol h, int* d_flags) {
+  const int n = (int)h->n;
+  Buf diag(ctx), ws(ctx);
+  LA_TRY(diag.alloc((size_t)(n + CB - 1) / CB * CB * CB * sizeof(double)));
+  FastChol f{ctx, h->d_l, h->ld, n, diag.d(), d_flags, nullptr, 0, Buf(ctx)};
+  if (n > CHW) {
+    f.ws_bytes = gemm_split_ws(n, n, std::min(chol_block(n), n), true);
+    if (ws.alloc(f.ws_bytes) == LA_OK) f.ws = ws.p;
+  }
+  struct PdlScope {
+    la_ctx c;
+    ~PdlScope() { c->pdl_now = false; }
+  } scope{ctx};
+  ctx->pdl_now = ctx->pdl != 0;
+  for (int b0 = 0; b0 < n;) {
+    const int b1 = std::min(b0 + chol_block(n - b0), n);
+    LA_TRY(f.factor(b0, b1));
+    LA_TRY(f.update(b0, b1, b1, n, true));
+    b0 = b1;
+  }
+  const int nt = (n + 31) / 32;
+  const cudaError_t e = la_launch(ctx, chol_zero_upper_kernel, dim3(nt, nt), dim3(32, 8), 0,
+                                  ctx->stream, h->d_l, h->ld, n, (const double*)diag.d());
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "chol_zero_upper_kernel launch");
+  ctx->launches++;
+  return la_check_launch(ctx, "chol_zero_upper_kernel");
+}
+
+// EXACT factorization of h->d_l in place.
+la_status chol_exact_factor(la_ctx ctx, la_chol h, int* d_flags) {
   const int n = (int)h->n;
   const size_t ld = h->ld;
-  const bool exact = h->arith == LA_ARITH_EXACT;
   double* L = h->d_l;
   cudaStream_t st = ctx->stream;
   LA_CUDA(ctx, configure_chol());
-  int* d_flags = reinterpret_cast<int*>(ctx->d_small);
-  LA_CUDA(ctx, cudaMemsetAsync(d_flags, 0, 2 * sizeof(int), st));
-  const int nt = (n + 31) / 32;
-  chol_sym_check_kernel<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(L, ld, n, d_flags);
-  ctx->launches++;
-  LA_TRY(la_check_launch(ctx, "chol_sym_check_kernel"));
-
   Buf S(ctx), T0(ctx), T1(ctx);
-  if (exact) {
-    LA_TRY(S.alloc((size_t)n * ld * sizeof(double)));
-    LA_CUDA(ctx, cudaMemsetAsync(S.p, 0, (size_t)n * ld * sizeof(double), st));
-  }
+  LA_TRY(S.alloc((size_t)n * ld * sizeof(double)));
+  LA_CUDA(ctx, cudaMemsetAsync(S.p, 0, (size_t)n * ld * sizeof(double), st));
   // Transposed panels (the GEMM's K x N operand), two so that panel k + 1 can
   // be transposed while panel k's update still reads its own.
   const size_t ldt = pad4c((size_t)n);
@@ -279,25 +456,19 @@ la_status chol_factor(la_ctx ctx, la_chol h, int* none) {
     LA_TRY(T1.alloc((size_t)CHW * ldt * sizeof(double)));
   }
   double* Tbuf[2] = {T0.d(), T1.d()};
-  const size_t dsm = (exact ? 2 : 1) * CHW * CHP * sizeof(double);
+  const size_t dsm = 2 * CHW * CHP * sizeof(double);
   const bool look = ctx->lookahead != 0 && ctx->side_stream != nullptr;
 
   // Diagonal block, rows below and transpose of panel [j0, j0 + jb) on stream s.
   auto panel = [&](int j0, int jb, double* T, cudaStream_t s) -> la_status {
     const int j1 = j0 + jb;
-    if (exact)
-      chol_diag_kernel<true><<<1, 256, dsm, s>>>(L, S.d(), ld, j0, jb, d_flags);
-    else
-      chol_diag_fast_kernel<<<1, 256, dsm, s>>>(L, ld, j0, jb, d_flags);
+    chol_diag_kernel<<<1, 256, dsm, s>>>(L, S.d(), ld, j0, jb, d_flags);
     ctx->launches++;
     LA_TRY(la_check_launch(ctx, "chol_diag_kernel"));
     if (j1 >= n) return LA_OK;
     const int rows = n - j1;
     const int pg = (rows + PANEL_T - 1) / PANEL_T;
-    if (exact)
-      chol_panel_kernel<true><<<pg, PANEL_T, 0, s>>>(L, S.d(), ld, j0, j1, n);
-    else
-      chol_panel_kernel<false><<<pg, PANEL_T, 0, s>>>(L, nullptr, ld, j0, j1, n);
+    chol_panel_kernel<<<pg, PANEL_T, 0, s>>>(L, S.d(), ld, j0, j1, n);
     ctx->launches++;
     LA_TRY(la_check_launch(ctx, "chol_panel_kernel"));
     chol_transpose_kernel<<<dim3((rows + 31) / 32, (jb + 31) / 32), dim3(32, 8), 0, s>>>(
@@ -305,42 +476,30 @@ la_status chol_factor(la_ctx ctx, la_chol h, int* none) {
     ctx->launches++;
     return la_check_launch(ctx, "chol_transpose_kernel");
   };
-  // A22 -= L21 L21' (EXACT: S22 += ...) of panel [j0, j0 + jb) on rows and
-  // columns >= c0 (lower part): FAST as one launch over the tiles at or below
-  // the diagonal; EXACT (and FAST where TMA cannot take the operands) in up
-  // to 8 row strips [a, b) that each stop at their own diagonal block.
+  // S22 += L21 L21' of panel [j0, j0 + jb) on rows and columns >= c0 (lower part), in up to 8 row
+  // strips [a, b) that each stop at their own diagonal block.
   auto update = [&](int j0, int jb, const double* T, int c0) -> la_status {
     const int j1 = j0 + jb, rows = n - c0;
     if (rows <= 0) return LA_OK;
-    if (!exact) {
-      const la_status r = launch_gemm_lower(ctx, rows, jb, L + (size_t)c0 * ld + j0, ld,
-                                            T + (c0 - j1), ldt, L + (size_t)c0 * ld + c0, ld);
-      if (r != LA_UNSUPPORTED) return r;
-    }
     const int nstrip = std::max(1, std::min(8, rows / 512));
     const int hs = ((rows + nstrip - 1) / nstrip + CHW - 1) / CHW * CHW;
     for (int a = c0; a < n; a += hs) {
       const int b = std::min(n, a + hs);
-      double* C = (exact ? S.d() : L) + (size_t)a * ld + c0;
-      LA_TRY(launch_gemm(ctx, exact ? GM_EXACT_ADD : GM_FMA_SUB, b - a, b - c0, jb,
-                         L + (size_t)a * ld + j0, ld, T + (c0 - j1), ldt, C, ld));
+      LA_TRY(launch_gemm(ctx, GM_EXACT_ADD, b - a, b - c0, jb, L + (size_t)a * ld + j0, ld,
+                         T + (c0 - j1), ldt, S.d() + (size_t)a * ld + c0, ld));
     }
     return LA_OK;
   };
   // The next panel's columns [j1, j2) of rows >= j1 (a plain GEMM).
   auto update_next = [&](int j0, int jb, const double* T, int j1, int j2) -> la_status {
-    double* C = (exact ? S.d() : L) + (size_t)j1 * ld + j1;
-    return launch_gemm(ctx, exact ? GM_EXACT_ADD : GM_FMA_SUB, n - j1, j2 - j1, jb,
-                       L + (size_t)j1 * ld + j0, ld, T, ldt, C, ld);
+    return launch_gemm(ctx, GM_EXACT_ADD, n - j1, j2 - j1, jb, L + (size_t)j1 * ld + j0, ld, T, ldt,
+                       S.d() + (size_t)j1 * ld + j1, ld);
   };
 
-  // Lookahead, as in the LU: panel k's update of panel k + 1's columns first,
-  // then panel k + 1 on the high-priority side stream while the rest of panel
-  // k's update runs (rows and columns >= j2). They touch disjoint data: panel
-  // k + 1 owns columns [j1, j2) of rows >= j1, and the rest of the update reads
-  // panel k's finished columns and its transposed copy. The update keeps its
-  // full occupancy (an earlier form that capped it at two CTAs per SM to leave
-  // the panel room measured slower than no lookahead at all).
+  // Lookahead: panel k's update of panel k + 1's columns first, then panel k + 1 on the
+  // high-priority side stream while the rest of panel k's update runs (rows and columns >= j2).
+  // They touch disjoint data: panel k + 1 owns columns [j1, j2) of rows >= j1, and the rest of the
+  // update reads panel k's finished columns and its transposed copy.
   LA_TRY(panel(0, std::min(CHW, n), Tbuf[0], st));
   for (int j0 = 0, k = 0; j0 < n; j0 += CHW, k++) {
     const int jb = std::min(CHW, n - j0), j1 = j0 + jb;
@@ -361,9 +520,24 @@ la_status chol_factor(la_ctx ctx, la_chol h, int* none) {
       LA_TRY(panel(j1, jbn, Tn, st));
     }
   }
-  chol_zero_upper_kernel<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(L, ld, n);
+  const int nt = (n + 31) / 32;
+  chol_zero_upper_kernel<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(L, ld, n, nullptr);
   ctx->launches++;
-  LA_TRY(la_check_launch(ctx, "chol_zero_upper_kernel"));
+  return la_check_launch(ctx, "chol_zero_upper_kernel");
+}
+
+// Factors h->d_l (a copy of A) in place; *none = the reference's None.
+la_status chol_factor(la_ctx ctx, la_chol h, int* none) {
+  const int n = (int)h->n;
+  cudaStream_t st = ctx->stream;
+  int* d_flags = reinterpret_cast<int*>(ctx->d_small);
+  LA_CUDA(ctx, cudaMemsetAsync(d_flags, 0, 2 * sizeof(int), st));
+  const int nt = (n + 31) / 32;
+  chol_sym_check_kernel<<<dim3(nt, nt), dim3(32, 8), 0, st>>>(h->d_l, h->ld, n, d_flags);
+  ctx->launches++;
+  LA_TRY(la_check_launch(ctx, "chol_sym_check_kernel"));
+  LA_TRY(h->arith == LA_ARITH_EXACT ? chol_exact_factor(ctx, h, d_flags)
+                                    : chol_fast_factor(ctx, h, d_flags));
   int* flags = static_cast<int*>(ctx->h_pinned);
   LA_CUDA(ctx, cudaMemcpyAsync(flags, d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
   LA_TRY(la_sync_and_check(ctx, "cholesky factorization"));
