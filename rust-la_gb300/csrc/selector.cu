@@ -27,7 +27,6 @@ constexpr int OFF_B2 = OFF_W2 + H2 * H1;    // [H2]
 constexpr int OFF_W3 = OFF_B2 + H2;         // [NC][H2]
 constexpr int OFF_B3 = OFF_W3 + NC * H2;    // [NC]
 constexpr int NPARAM = OFF_B3 + NC;         // 5443
-constexpr int ACT = NF + H1 + H2 + NC;      // per-sample activations kept for backprop
 
 struct SysRec {
   long long a, b;
@@ -547,11 +546,7 @@ __device__ void mlp_fwd(const float* __restrict__ P, const float* x, float* h1, 
   for (int o = 0; o < NC; o++) pr[o] = lg3[o] / z;
 }
 
-// One thread per sample: normalise, forward, keep activations; with labels,
-// also the per-sample output delta and loss: the softmax cross-entropy, or,
-// with per-sample class costs (cost, NC per sample), the expected cost
-// sum_c p_c cost_c, whose gradient with respect to the logits is
-// p_c (cost_c - sum_j p_j cost_j).
+// Inference: one thread per sample.
 // Gate of the class output (inference): a linear score of the raw features
 // and the class probabilities, w[0..15] . x + w[16..18] . p + b; a system
 // whose score is >= 0 gets class 3 (no mixed attempt, straight to the FP64
@@ -565,9 +560,7 @@ struct Gate {
 
 __global__ void mlp_forward_kernel(const float* __restrict__ P, const float* __restrict__ mean,
                                    const float* __restrict__ stdv, const float* __restrict__ X,
-                                   int count, float* __restrict__ act, float* __restrict__ probs,
-                                   int* __restrict__ cls, const int* __restrict__ y,
-                                   const float* __restrict__ cost, float* __restrict__ loss,
+                                   int count, float* __restrict__ probs, int* __restrict__ cls,
                                    Gate gate) {
   __shared__ float Ps[NPARAM];
   for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) Ps[i] = P[i];
@@ -577,19 +570,6 @@ __global__ void mlp_forward_kernel(const float* __restrict__ P, const float* __r
   float x[NF], h1[H1], h2[H2], pr[NC];
   for (int k = 0; k < NF; k++) x[k] = (X[(size_t)s * NF + k] - mean[k]) / stdv[k];
   mlp_fwd(Ps, x, h1, h2, pr);
-  if (act) {
-    float* a = act + (size_t)s * ACT;
-    for (int k = 0; k < NF; k++) a[k] = x[k];
-    for (int k = 0; k < H1; k++) a[NF + k] = h1[k];
-    for (int k = 0; k < H2; k++) a[NF + H1 + k] = h2[k];
-    if (cost) {
-      float ec = 0.f;
-      for (int k = 0; k < NC; k++) ec = fmaf(pr[k], cost[(size_t)s * NC + k], ec);
-      for (int k = 0; k < NC; k++) a[NF + H1 + H2 + k] = pr[k] * (cost[(size_t)s * NC + k] - ec);
-    } else {
-      for (int k = 0; k < NC; k++) a[NF + H1 + H2 + k] = pr[k] - ((y && y[s] == k) ? 1.f : 0.f);
-    }
-  }
   if (probs)
     for (int k = 0; k < NC; k++) probs[(size_t)s * NC + k] = pr[k];
   if (cls) {
@@ -604,62 +584,161 @@ __global__ void mlp_forward_kernel(const float* __restrict__ P, const float* __r
     }
     cls[s] = best;
   }
-  if (loss && cost) {
-    float ec = 0.f;
-    for (int k = 0; k < NC; k++) ec = fmaf(pr[k], cost[(size_t)s * NC + k], ec);
-    loss[s] = ec;
-  } else if (loss && y) {
-    loss[s] = -logf(fmaxf(pr[y[s]], 1e-30f));
-  }
 }
 
-// Hidden-layer deltas per sample: d2 = (W3^T d3) . [h2 > 0], d1 = (W2^T d2) . [h1 > 0].
-__global__ void mlp_delta_kernel(const float* __restrict__ P, const float* __restrict__ act,
-                                 int count, float* __restrict__ delta) {
-  __shared__ float Ps[NPARAM];
-  for (int i = threadIdx.x; i < NPARAM; i += blockDim.x) Ps[i] = P[i];
+// Forward, backward and the summed gradient of a chunk of samples: 32 samples at a time with their
+// activations and deltas in shared memory, never in global memory. Each activation, output delta
+// and hidden delta is one thread's sum in ascending index, as in mlp_fwd. The gradient of every
+// parameter over the chunk stays in registers (a 4 x 4 tile of W2, 4 elements of W1, one or two of
+// the rest per thread) and goes to part[chunk][parameter]; mlp_reduce_kernel adds the chunks. One
+// thread per parameter walking all samples took 2.0 ms for 4096 of them (5,500 threads with
+// uncoalesced loads and one chain of additions each); this takes a few microseconds per 32 samples,
+// all chunks at once, and its sums of sums are more accurate.
+constexpr int BP_S = 32;         // samples at a time
+constexpr int BP_T = 256;
+constexpr int BP_CHUNKS = 608;   // most chunks: four CTAs on each of 152 SMs
+constexpr int BP_P = H1 + 1;     // padded row of a sample's 64 values
+constexpr size_t BP_SMEM = (size_t)(NPARAM + BP_S * (4 * BP_P + (NF + 1) + (NC + 1))) * sizeof(float);
+static_assert(H1 == 64 && H2 == 64 && NF == 16 && BP_T == 256, "the thread mapping of the gradient");
+
+__global__ void __launch_bounds__(BP_T)
+mlp_backprop_kernel(const float* __restrict__ P, const float* __restrict__ mean,
+                    const float* __restrict__ stdv, const float* __restrict__ X,
+                    const int* __restrict__ y, const float* __restrict__ cost, int count,
+                    int per_chunk, float* __restrict__ loss, float* __restrict__ part) {
+  extern __shared__ float bp[];
+  float* Ps = bp;
+  float* h1 = Ps + NPARAM;           // [BP_S][BP_P]
+  float* h2 = h1 + BP_S * BP_P;
+  float* d1 = h2 + BP_S * BP_P;
+  float* d2 = d1 + BP_S * BP_P;
+  float* x = d2 + BP_S * BP_P;       // [BP_S][NF + 1]
+  float* d3 = x + BP_S * (NF + 1);   // [BP_S][NC + 1]
+  const int tid = threadIdx.x, smp = tid & 31, grp = tid >> 5;  // a warp: 32 samples of one unit
+  for (int i = tid; i < NPARAM; i += BP_T) Ps[i] = P[i];
+  float g2[4][4] = {}, g1[4] = {}, gr[2] = {};
+  const int o2 = tid / 16 * 4, k2 = tid % 16 * 4;  // W2 tile
+  const int o1 = tid / 4, k1 = tid % 4 * 4;        // W1: four inputs of unit o1
+  const int s0 = blockIdx.x * per_chunk, s1 = min(count, s0 + per_chunk);
+  for (int sb = s0; sb < s1; sb += BP_S) {
+    const int ns = min(BP_S, s1 - sb);
+    __syncthreads();
+    for (int i = tid; i < BP_S * NF; i += BP_T) {
+      const int s = i / NF, k = i % NF;
+      x[s * (NF + 1) + k] = s < ns ? (X[(size_t)(sb + s) * NF + k] - mean[k]) / stdv[k] : 0.f;
+    }
+    __syncthreads();
+    for (int o = grp; o < H1; o += 8) {
+      float t = Ps[OFF_B1 + o];
+#pragma unroll
+      for (int k = 0; k < NF; k++) t = fmaf(Ps[OFF_W1 + o * NF + k], x[smp * (NF + 1) + k], t);
+      h1[smp * BP_P + o] = fmaxf(t, 0.f);
+    }
+    __syncthreads();
+    for (int o = grp; o < H2; o += 8) {
+      float t = Ps[OFF_B2 + o];
+#pragma unroll 16
+      for (int k = 0; k < H1; k++) t = fmaf(Ps[OFF_W2 + o * H1 + k], h1[smp * BP_P + k], t);
+      h2[smp * BP_P + o] = fmaxf(t, 0.f);
+    }
+    __syncthreads();
+    if (grp < NC) {
+      float t = Ps[OFF_B3 + grp];
+#pragma unroll 16
+      for (int k = 0; k < H2; k++) t = fmaf(Ps[OFF_W3 + grp * H2 + k], h2[smp * BP_P + k], t);
+      d3[smp * (NC + 1) + grp] = t;
+    }
+    __syncthreads();
+    // Softmax, loss and output delta: the cross-entropy of label y, or, with per-sample class
+    // costs, the expected cost sum_c p_c cost_c, whose gradient with respect to the logits is
+    // p_c (cost_c - sum_j p_j cost_j).
+    if (tid < BP_S) {
+      const int s = sb + tid;
+      float* l = d3 + tid * (NC + 1);
+      float pr[NC], mx = -INFINITY, z = 0.f;
+      for (int k = 0; k < NC; k++) mx = fmaxf(mx, l[k]);
+      for (int k = 0; k < NC; k++) { pr[k] = expf(l[k] - mx); z += pr[k]; }
+      for (int k = 0; k < NC; k++) pr[k] = pr[k] / z;
+      if (tid >= ns) {
+        for (int k = 0; k < NC; k++) l[k] = 0.f;
+      } else if (cost) {
+        float ec = 0.f;
+        for (int k = 0; k < NC; k++) ec = fmaf(pr[k], cost[(size_t)s * NC + k], ec);
+        for (int k = 0; k < NC; k++) l[k] = pr[k] * (cost[(size_t)s * NC + k] - ec);
+        loss[s] = ec;
+      } else {
+        const int c = y[s];
+        for (int k = 0; k < NC; k++) l[k] = pr[k] - (c == k ? 1.f : 0.f);
+        loss[s] = -logf(fmaxf(pr[c], 1e-30f));
+      }
+    }
+    __syncthreads();
+    for (int k = grp; k < H2; k += 8) {
+      float t = 0.f;
+#pragma unroll
+      for (int o = 0; o < NC; o++) t = fmaf(Ps[OFF_W3 + o * H2 + k], d3[smp * (NC + 1) + o], t);
+      d2[smp * BP_P + k] = h2[smp * BP_P + k] > 0.f ? t : 0.f;
+    }
+    __syncthreads();
+    for (int k = grp; k < H1; k += 8) {
+      float t = 0.f;
+#pragma unroll 16
+      for (int o = 0; o < H2; o++) t = fmaf(Ps[OFF_W2 + o * H1 + k], d2[smp * BP_P + o], t);
+      d1[smp * BP_P + k] = h1[smp * BP_P + k] > 0.f ? t : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int s = 0; s < BP_S; s++) {  // samples past ns have zero deltas
+      float a[4], d[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        a[i] = h1[s * BP_P + k2 + i];
+        d[i] = d2[s * BP_P + o2 + i];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) g2[i][j] = fmaf(d[i], a[j], g2[i][j]);
+      const float e = d1[s * BP_P + o1];
+#pragma unroll
+      for (int i = 0; i < 4; i++) g1[i] = fmaf(e, x[s * (NF + 1) + k1 + i], g1[i]);
+      // W3 (192), b1 and b2 on threads 192-255 and 0-63 more, b3
+      if (tid < NC * H2) gr[0] = fmaf(d3[s * (NC + 1) + tid / H2], h2[s * BP_P + tid % H2], gr[0]);
+      else gr[0] += d1[s * BP_P + tid - NC * H2];
+      if (tid < H2) gr[1] += d2[s * BP_P + tid];
+      else if (tid < H2 + NC) gr[1] += d3[s * (NC + 1) + tid - H2];
+    }
+  }
+  float* out = part + (size_t)blockIdx.x * NPARAM;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) out[OFF_W2 + (o2 + i) * H1 + k2 + j] = g2[i][j];
+#pragma unroll
+  for (int i = 0; i < 4; i++) out[OFF_W1 + o1 * NF + k1 + i] = g1[i];
+  if (tid < NC * H2) out[OFF_W3 + tid] = gr[0];
+  else out[OFF_B1 + tid - NC * H2] = gr[0];
+  if (tid < H2) out[OFF_B2 + tid] = gr[1];
+  else if (tid < H2 + NC) out[OFF_B3 + tid - H2] = gr[1];
+}
+
+// G[p] = (sum over chunks of part[chunk][p]) / count: 32 parameters per CTA, 8 threads each with
+// every eighth chunk, their sums added in order (deterministic).
+__global__ void __launch_bounds__(256)
+mlp_reduce_kernel(const float* __restrict__ part, int chunks, int count, float* __restrict__ G) {
+  __shared__ float t[8][32];
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31), g = threadIdx.x >> 5;
+  float v = 0.f;
+  if (p < NPARAM)
+    for (int c = g; c < chunks; c += 8) v += part[(size_t)c * NPARAM + p];
+  t[g][threadIdx.x & 31] = v;
   __syncthreads();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= count) return;
-  const float* a = act + (size_t)s * ACT;
-  const float* h1 = a + NF;
-  const float* h2 = a + NF + H1;
-  const float* d3 = a + NF + H1 + H2;
-  float d2[H2];
-  float* out = delta + (size_t)s * (H1 + H2);
-  for (int k = 0; k < H2; k++) {
-    float t = 0.f;
-    for (int o = 0; o < NC; o++) t = fmaf(Ps[OFF_W3 + o * H2 + k], d3[o], t);
-    d2[k] = h2[k] > 0.f ? t : 0.f;
-    out[H1 + k] = d2[k];
+  if (g == 0 && p < NPARAM) {
+    float r = t[0][threadIdx.x];
+#pragma unroll
+    for (int i = 1; i < 8; i++) r += t[i][threadIdx.x];
+    G[p] = r / (float)count;
   }
-  for (int k = 0; k < H1; k++) {
-    float t = 0.f;
-    for (int o = 0; o < H2; o++) t = fmaf(Ps[OFF_W2 + o * H1 + k], d2[o], t);
-    out[k] = h1[k] > 0.f ? t : 0.f;
-  }
-}
-
-// Mean gradient of the loss: one thread per parameter, samples summed in index
-// order (deterministic).
-__global__ void mlp_grad_kernel(const float* __restrict__ act, const float* __restrict__ delta,
-                                int count, float* __restrict__ G) {
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pidx >= NPARAM) return;
-  float g = 0.f;
-  for (int s = 0; s < count; s++) {
-    const float* a = act + (size_t)s * ACT;
-    const float* dl = delta + (size_t)s * (H1 + H2);
-    float v;
-    if (pidx < OFF_B1) { const int o = pidx / NF, k = pidx % NF; v = dl[o] * a[k]; }
-    else if (pidx < OFF_W2) { v = dl[pidx - OFF_B1]; }
-    else if (pidx < OFF_B2) { const int q = pidx - OFF_W2, o = q / H1, k = q % H1; v = dl[H1 + o] * a[NF + k]; }
-    else if (pidx < OFF_W3) { v = dl[H1 + pidx - OFF_B2]; }
-    else if (pidx < OFF_B3) { const int q = pidx - OFF_W3, o = q / H2, k = q % H2; v = a[NF + H1 + H2 + o] * a[NF + H1 + k]; }
-    else { v = a[NF + H1 + H2 + (pidx - OFF_B3)]; }
-    g += v;
-  }
-  G[pidx] = g / (float)count;
 }
 
 // Adam (beta1 0.9, beta2 0.999, eps 1e-8), t = step number from 1.
@@ -751,17 +830,25 @@ la_status la_mlp_set_params(la_mlp m, const float* params) {
 static la_status mlp_backprop(la_mlp m, const float* d_x, const int* d_y, const float* d_cost,
                               int count, float* loss) {
   la_ctx ctx = m->ctx;
-  float *act = nullptr, *delta = nullptr, *dl = nullptr;
-  la_status s = la_device_alloc(ctx, reinterpret_cast<void**>(&act), (size_t)count * ACT * 4);
-  if (s == LA_OK) s = la_device_alloc(ctx, reinterpret_cast<void**>(&delta), (size_t)count * (H1 + H2) * 4);
+  // Chunks of whole sets of 32 samples, at most BP_CHUNKS of them.
+  const int sets = (count + BP_S - 1) / BP_S;
+  const int per = (sets + BP_CHUNKS - 1) / BP_CHUNKS * BP_S, chunks = (count + per - 1) / per;
+  float *part = nullptr, *dl = nullptr;
+  la_status s = la_device_alloc(ctx, reinterpret_cast<void**>(&part), (size_t)chunks * NPARAM * 4);
   if (s == LA_OK) s = la_device_alloc(ctx, reinterpret_cast<void**>(&dl), (size_t)count * 4);
   if (s == LA_OK) {
-    const int g = (count + 127) / 128;
-    mlp_forward_kernel<<<g, 128, 0, ctx->stream>>>(m->P(), m->mean(), m->stdv(), d_x, count, act,
-                                                   nullptr, nullptr, d_y, d_cost, dl, Gate{});
-    mlp_delta_kernel<<<g, 128, 0, ctx->stream>>>(m->P(), act, count, delta);
-    mlp_grad_kernel<<<(NPARAM + 127) / 128, 128, 0, ctx->stream>>>(act, delta, count, m->grad());
-    ctx->launches += 3;
+    static la_device_once configured;
+    const cudaError_t e = configured.run([](int) {
+      return cudaFuncSetAttribute(mlp_backprop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)BP_SMEM);
+    });
+    if (e != cudaSuccess) s = la_cuda_fail(ctx, e, "cudaFuncSetAttribute(mlp_backprop)");
+  }
+  if (s == LA_OK) {
+    mlp_backprop_kernel<<<chunks, BP_T, BP_SMEM, ctx->stream>>>(
+        m->P(), m->mean(), m->stdv(), d_x, d_y, d_cost, count, per, dl, part);
+    mlp_reduce_kernel<<<(NPARAM + 31) / 32, 256, 0, ctx->stream>>>(part, chunks, count, m->grad());
+    ctx->launches += 2;
     s = la_check_launch(ctx, "mlp backprop");
   }
   if (s == LA_OK && loss) {
@@ -773,8 +860,7 @@ static la_status mlp_backprop(la_mlp m, const float* d_x, const int* d_y, const 
     for (float v : h) t += v;
     *loss = (float)(t / count);
   }
-  la_device_free(ctx, act);
-  la_device_free(ctx, delta);
+  la_device_free(ctx, part);
   la_device_free(ctx, dl);
   return s;
 }
@@ -847,8 +933,7 @@ la_status la_mlp_predict(la_mlp m, const float* d_x, int count, float* d_probs, 
   if (!m || !d_x || count <= 0) return LA_INVALID;
   LA_CUDA(m->ctx, cudaSetDevice(m->ctx->device));
   mlp_forward_kernel<<<(count + 127) / 128, 128, 0, m->ctx->stream>>>(
-      m->P(), m->mean(), m->stdv(), d_x, count, nullptr, d_probs, d_class, nullptr, nullptr,
-      nullptr, m->gate);
+      m->P(), m->mean(), m->stdv(), d_x, count, d_probs, d_class, m->gate);
   m->ctx->launches++;
   return la_check_launch(m->ctx, "mlp predict");
 }
