@@ -624,11 +624,10 @@ la_status la_chol_new(la_ctx ctx, const double* a, size_t m, size_t n, la_chol* 
   if (m != n) return LA_SINGULAR;           // cholesky.rs:57-59: None
   la_chol h = nullptr;
   LA_TRY(chol_alloc(ctx, n, &h));
-  cudaError_t e = cudaMemcpy2DAsync(h->d_l, h->ld * sizeof(double), a, n * sizeof(double),
-                                    n * sizeof(double), n, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) {
+  const la_status s = la_copy_to_device(ctx, h->d_l, h->ld, a, n, n);
+  if (s != LA_OK) {
     la_chol_free(h);
-    return la_cuda_fail(ctx, e, "copy A to device");
+    return s;
   }
   return chol_new_common(ctx, h, out);
 }
@@ -667,9 +666,7 @@ la_status la_chol_get_l(la_chol h, double* out) {
   if (!h || !out) return LA_INVALID;
   la_ctx ctx = h->ctx;
   LA_TRY(chol_check_ctx(ctx));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(out, h->n * sizeof(double), h->d_l, h->ld * sizeof(double),
-                                 h->n * sizeof(double), h->n, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_host(ctx, out, h->d_l, h->ld, h->n, h->n));
   return la_sync_and_check(ctx, "la_chol_get_l");
 }
 

@@ -43,6 +43,45 @@ void la_device_free(la_ctx ctx, void* p) {
   if (p) cudaFreeAsync(p, ctx->stream);
 }
 
+// Host matrices (rows x cols, dense) to and from device memory of pitch ld. Two-dimensional copies of
+// pageable memory go row by row inside the runtime: 50 MB (2500 rows) took 43 ms to the host, where
+// one contiguous copy takes 2 (3 into memory that was never touched). So a dense device side is
+// copied in one piece, and any other goes through a dense buffer and a copy on the device; without
+// memory for that, the two-dimensional copy.
+namespace {
+la_status copy_host_2d(la_ctx ctx, void* dev, size_t ld, void* host, size_t rows, size_t cols,
+                       bool to_host) {
+  const size_t w = cols * sizeof(double), pitch = ld * sizeof(double);
+  const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+  void* dense = ld == cols || rows == 1 ? dev : nullptr;
+  void* tmp = nullptr;
+  if (!dense && la_device_alloc(ctx, &tmp, rows * w) == LA_OK) dense = tmp;
+  cudaError_t e = cudaSuccess;
+  if (!dense) {
+    e = to_host ? cudaMemcpy2DAsync(host, w, dev, pitch, w, rows, kind, ctx->stream)
+                : cudaMemcpy2DAsync(dev, pitch, host, w, w, rows, kind, ctx->stream);
+  } else {
+    if (to_host && tmp)
+      e = cudaMemcpy2DAsync(tmp, w, dev, pitch, w, rows, cudaMemcpyDeviceToDevice, ctx->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(to_host ? host : dense, to_host ? dense : host, rows * w, kind, ctx->stream);
+    if (e == cudaSuccess && !to_host && tmp)
+      e = cudaMemcpy2DAsync(dev, pitch, tmp, w, w, rows, cudaMemcpyDeviceToDevice, ctx->stream);
+  }
+  la_device_free(ctx, tmp);
+  return e == cudaSuccess ? LA_OK : la_cuda_fail(ctx, e, to_host ? "copy to host" : "copy to device");
+}
+}  // namespace
+
+la_status la_copy_to_device(la_ctx ctx, double* dev, size_t ld, const double* host, size_t rows,
+                            size_t cols) {
+  return copy_host_2d(ctx, dev, ld, const_cast<double*>(host), rows, cols, false);
+}
+la_status la_copy_to_host(la_ctx ctx, double* host, const double* dev, size_t ld, size_t rows,
+                          size_t cols) {
+  return copy_host_2d(ctx, const_cast<double*>(dev), ld, host, rows, cols, true);
+}
+
 // Synchronizes the context's stream and turns a device-side error word into a status.
 la_status la_sync_and_check(la_ctx ctx, const char* what) {
   cudaError_t e = cudaStreamSynchronize(ctx->stream);

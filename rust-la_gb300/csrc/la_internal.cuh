@@ -198,6 +198,11 @@ la_status la_cuda_fail(la_ctx ctx, cudaError_t e, const char* what);
 la_status la_check_launch(la_ctx ctx, const char* what);
 la_status la_device_alloc(la_ctx ctx, void** p, size_t bytes);
 void la_device_free(la_ctx ctx, void* p);
+// Dense host matrix (rows x cols) <-> device memory of pitch ld, on the context's stream.
+la_status la_copy_to_device(la_ctx ctx, double* dev, size_t ld, const double* host, size_t rows,
+                            size_t cols);
+la_status la_copy_to_host(la_ctx ctx, double* host, const double* dev, size_t ld, size_t rows,
+                          size_t cols);
 la_status la_sync_and_check(la_ctx ctx, const char* what);
 
 #define LA_TRY(expr)                       \

@@ -478,9 +478,7 @@ la_status la_lu_new(la_ctx ctx, const double* a, size_t m, size_t n, la_lu* out)
   la_lu h = nullptr;
   LA_TRY(lu_alloc(ctx, m, n, &h));
   la_status s = LA_OK;
-  cudaError_t e = cudaMemcpy2DAsync(h->d_lu, h->ld * sizeof(double), a, n * sizeof(double),
-                                    n * sizeof(double), m, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) s = la_cuda_fail(ctx, e, "copy A to device");
+  s = la_copy_to_device(ctx, h->d_lu, h->ld, a, m, n);
   if (s == LA_OK) s = lu_factor(ctx, h);
   if (s != LA_OK) { la_lu_free(h); return s; }
   *out = h;
@@ -592,9 +590,7 @@ la_status la_lu_solve(la_lu h, const double* b, size_t brows, size_t nrhs, doubl
                                ctx->stream));
   LA_TRY(launch_permute_rows(ctx, h->d_piv, Bd.d(), nrhs, Xw.d(), ldw, (int)h->m, (int)nrhs));
   LA_TRY(lu_solve_inplace(ctx, h, Xw.d(), ldw, (int)nrhs));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(x, nrhs * sizeof(double), Xw.p, ldw * sizeof(double),
-                                 nrhs * sizeof(double), h->m, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_host(ctx, x, Xw.d(), ldw, h->m, nrhs));
   return la_sync_and_check(ctx, "lu solve");
 }
 
@@ -640,12 +636,7 @@ la_status la_matrix_inverse(la_ctx ctx, const double* a, size_t m, size_t n, dou
     s = Xw.alloc(n * ldw * sizeof(double));
     if (s == LA_OK) s = launch_identity_permuted(ctx, h->d_piv, Xw.d(), ldw, (int)n);
     if (s == LA_OK) s = lu_solve_inplace(ctx, h, Xw.d(), ldw, (int)n);
-    if (s == LA_OK) {
-      cudaError_t e = cudaMemcpy2DAsync(out, n * sizeof(double), Xw.p, ldw * sizeof(double),
-                                        n * sizeof(double), n, cudaMemcpyDeviceToHost,
-                                        ctx->stream);
-      if (e != cudaSuccess) s = la_cuda_fail(ctx, e, "copy inverse");
-    }
+    if (s == LA_OK) s = la_copy_to_host(ctx, out, Xw.d(), ldw, n, n);
     if (s == LA_OK) s = la_sync_and_check(ctx, "inverse");
   }
   la_lu_free(h);
@@ -674,13 +665,10 @@ la_status la_matrix_mul(la_ctx ctx, const double* a, size_t m, size_t k, const d
   LA_TRY(A.alloc(m * la * sizeof(double)));
   LA_TRY(B.alloc(k * lb * sizeof(double)));
   LA_TRY(C.alloc(m * lc * sizeof(double)));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(A.p, la * 8, a, k * 8, k * 8, m, cudaMemcpyHostToDevice,
-                                 ctx->stream));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(B.p, lb * 8, b, n * 8, n * 8, k, cudaMemcpyHostToDevice,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_device(ctx, A.d(), la, a, m, k));
+  LA_TRY(la_copy_to_device(ctx, B.d(), lb, b, k, n));
   LA_TRY(gemm_device_common(ctx, A.d(), la, B.d(), lb, C.d(), lc, m, k, n));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(c, n * 8, C.p, lc * 8, n * 8, m, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_host(ctx, c, C.d(), lc, m, n));
   return la_sync_and_check(ctx, "matrix mul");
 }
 

@@ -407,11 +407,10 @@ la_status la_qr_new(la_ctx ctx, const double* a, size_t m, size_t n, la_qr* out)
   *out = nullptr;
   la_qr h = nullptr;
   LA_TRY(qr_alloc(ctx, m, n, &h));
-  cudaError_t e = cudaMemcpy2DAsync(h->d_qr, h->ld * sizeof(double), a, n * sizeof(double),
-                                    n * sizeof(double), m, cudaMemcpyHostToDevice, ctx->stream);
-  if (e != cudaSuccess) {
+  const la_status s = la_copy_to_device(ctx, h->d_qr, h->ld, a, m, n);
+  if (s != LA_OK) {
     la_qr_free(h);
-    return la_cuda_fail(ctx, e, "copy A to device");
+    return s;
   }
   return qr_new_common(ctx, h, out);
 }
@@ -473,9 +472,7 @@ la_status la_qr_get_q(la_qr h, double* out) {
   else
     for (int k = dc - 1; k >= 0; k--)  // qr.rs:163-191
       LA_TRY(reflect(ctx, exact, h->d_qr, h->ld, k, k, m, h->d_rdiag, Qm.d(), ldq, k, m, 1));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(out, h->m * sizeof(double), Qm.p, ldq * sizeof(double),
-                                 h->m * sizeof(double), h->m, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_host(ctx, out, Qm.d(), ldq, h->m, h->m));
   return la_sync_and_check(ctx, "la_qr_get_q");
 }
 
@@ -494,9 +491,7 @@ la_status la_qr_solve(la_qr h, const double* b, size_t brows, size_t nrhs, doubl
   QBuf X(ctx), R(ctx);
   LA_TRY(X.alloc(h->n * ldw * sizeof(double)));
   LA_TRY(R.alloc(h->n * ldr * sizeof(double)));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(X.p, ldw * sizeof(double), b, nrhs * sizeof(double),
-                                 nrhs * sizeof(double), h->n, cudaMemcpyHostToDevice,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_device(ctx, X.d(), ldw, b, h->n, nrhs));
   if (h->d_gram)  // Y = Q' B (qr.rs:211-223), block by block
     LA_TRY(qr_blocked_apply(ctx, h->d_qr, h->ld, n, n, h->d_rdiag, h->d_gram, 2, X.d(), ldw, nx));
   else
@@ -508,9 +503,7 @@ la_status la_qr_solve(la_qr h, const double* b, size_t brows, size_t nrhs, doubl
   LA_TRY(la_check_launch(ctx, "qr_extract_kernel"));
   // R X = Y (qr.rs:225-235): descending terms, then the division by rdiag
   LA_TRY(launch_tri_wave(ctx, exact, true, true, R.d(), ldr, X.d(), ldw, n, nx));
-  LA_CUDA(ctx, cudaMemcpy2DAsync(x, nrhs * sizeof(double), X.p, ldw * sizeof(double),
-                                 nrhs * sizeof(double), h->n, cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+  LA_TRY(la_copy_to_host(ctx, x, X.d(), ldw, h->n, nrhs));
   return la_sync_and_check(ctx, "la_qr_solve");
 }
 
