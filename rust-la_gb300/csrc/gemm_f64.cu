@@ -388,12 +388,12 @@ la_status launch_gemm(la_ctx ctx, int mode, int M, int N, int K, const double* A
   return launch_bn<64>(ctx, mode, M, N, K, A, lda, B, ldb, C, ldc, min_smem);
 }
 
-// C -= A B by tiles of 64 x 16: an SM needs 33 us for a 64 x 64 tile of 32 k, whatever part of it
-// exists, and 8 us for one of these.
-la_status launch_gemm_narrow(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
+// C -= A B (GM_FMA_SUB) or C = A B (GM_FMA_ZERO) by tiles of 64 x 16: an SM needs 33 us for a
+// 64 x 64 tile of 32 k, whatever part of it exists, and 8 us for one of these.
+la_status launch_gemm_narrow(la_ctx ctx, int mode, int M, int N, int K, const double* A, size_t lda,
                              const double* B, size_t ldb, double* C, size_t ldc) {
   if (M <= 0 || N <= 0 || K <= 0) return LA_OK;
-  return launch_bn<16>(ctx, GM_FMA_SUB, M, N, K, A, lda, B, ldb, C, ldc, 0);
+  return launch_bn<16>(ctx, mode, M, N, K, A, lda, B, ldb, C, ldc, 0);
 }
 
 // Split-K product for tall-skinny inner products (C = A B with K >> M): the

@@ -29,11 +29,12 @@
 // where the error left out is no larger than the chain's. guard_kernel decides it per tile, in two
 // steps. The split kernels count, per row and column, the entries within 2^-5 of the scale; if the
 // smallest row count and the smallest column count exceed K by 2 sqrt(K) together, that many k have
-// both entries large, and the sum is at least 2 sqrt(K) 2^-10. Else the sums are formed, in FP32
-// from the leading two digits (8 us for 128 x 64 x 256, where the FMA tile takes 1 ms). Every other
+// both entries large, and the sum is at least 2 sqrt(K) 2^-10. Else the sums are formed from the
+// leading two digits by mma.sync (a few microseconds, where the FMA tile of K = 256 takes 1 ms; as
+// FP32 FMAs they took 65 us for K = 700, a tenth of the FMA tiles that may follow). Every other
 // tile (graded or sparse operands, values that are not finite or beyond 2^+-400) goes on a list that
-// fma_tiles_kernel, launched after the product, works off with FMA chains in ascending k, 64 x 64
-// tiles as in gemm_f64.cu (it ends at once where the list is empty).
+// the epilogue warps work off at the end of the product (fma_tiles), with FMA chains in ascending k
+// and 64 x 64 tiles as in gemm_f64.cu.
 //
 // Measured on 8192^3 (A and B N(0,1)): 24.0 ms against 876.6 ms by FMA, 36 x 2 x 8192^3 FP16
 // operations in all, 1.65 PFLOP/s; rms error against quadruple precision 5 to 17 times smaller than
@@ -80,7 +81,7 @@ constexpr int LARGE_BITS = 4;         // "large": exponent within 4 of the large
 constexpr float GUARD = 0.0021f;      // 2^-8.9
 constexpr int CNT_BAD = -(1 << 29);   // count of a row the digits cannot represent
 constexpr int FT = 64, FK = 16;       // FMA tiles: 64 x 64 in slabs of 16 k
-constexpr int FMA_T = 256, FMA_PER_SM = 3;
+static_assert(2 * 2 * FK * FT * 8 <= EPI_BYTES, "the FMA slabs reuse the epilogue's buffer");
 
 using la_tma::mbar_init;
 using la_tma::smem_u32;
@@ -230,15 +231,16 @@ __device__ __forceinline__ void split_rows(int block, const double* __restrict__
   }
 }
 
-// Largest biased exponent of each column of X (K x N) over k [blockIdx.y * kper, ...), and a
-// denormal's presence as bit 11, into maxexp (zeroed before).
-__global__ void __launch_bounds__(256)
-col_exp_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kper,
-               int* __restrict__ maxexp) {
-  const int c = blockIdx.x * 32 + (threadIdx.x & 31), ty = threadIdx.x >> 5;
-  const int k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
+// Largest biased exponent of each column of X (K x N) over k [yblock * kper, ...), and a denormal's
+// presence as a flag, into maxexp (zeroed before).
+__device__ __forceinline__ void col_exps(int block, int yblock, const double* __restrict__ X,
+                                         size_t ldx, int K, int N, int kper,
+                                         int* __restrict__ maxexp) {
+  const int c = block * 32 + (threadIdx.x & 31), ty = threadIdx.x >> 5;
+  const int k0 = yblock * kper, k1 = min(K, k0 + kper);
   if (c >= N) return;
   int me = 0, den = 0;
+#pragma unroll 8
   for (int k = k0 + ty; k < k1; k += 8) {
     const double v = X[(size_t)k * ldx + c];
     me = max(me, exp_bits(v));
@@ -248,10 +250,10 @@ col_exp_kernel(const double* __restrict__ X, size_t ldx, int K, int N, int kper,
   if (den) atomicOr(maxexp + N + c, 1);
 }
 
-// Columns of X (K x N, pitch ldx), k [blockIdx.y * kper, ...), into digits [SL][N][kp]. 32 columns
+// Columns of X (K x N, pitch ldx), k [yblock * kper, ...), into digits [SL][N][kp]. 32 columns
 // per CTA: 64 k at a time go through shared memory, so that global rows are read 256 bytes at a
 // time and a digit's k are written 128 bytes at a time. ALL: the CTA sees every k of its columns
-// and finds their exponents itself; else they come from col_exp_kernel and counts are added up.
+// and finds their exponents itself; else they come from col_exps and counts are added up.
 template <bool ALL>
 __device__ __forceinline__ void split_cols(int block, int yblock, const double* __restrict__ X,
                                            size_t ldx, int K, int N, int kp, int kper,
@@ -324,8 +326,10 @@ __device__ __forceinline__ void split_cols(int block, int yblock, const double* 
   }
 }
 
-// Rows of A and columns of B in one launch: the first ra CTAs take 8 rows of A each, the next rb 8
-// rows of B' (b_rows) or 32 columns of B. list[0] is zeroed for the guard.
+// Rows of A and columns of B in one launch: the first ra CTAs take 8 rows of A each, the others 8
+// rows of B' (b_rows), 32 columns of B, or (kper > 0: the columns are split afterwards, in pieces of
+// K) the exponents of 32 columns over one piece. list[0] is zeroed for the guard and b.cnt for the
+// pieces.
 struct SplitSide {
   const double* X;
   size_t ldx;
@@ -334,17 +338,29 @@ struct SplitSide {
   int *exps, *cnt;
 };
 __global__ void __launch_bounds__(256)
-split_kernel(const SplitSide a, const SplitSide b, int K, int kp, int ra, int b_rows, int* list) {
+split_kernel(const SplitSide a, const SplitSide b, int K, int kp, int ra, int b_rows, int kper,
+             int* list, int* maxexp) {
   la_pdl_wait();
   la_pdl_trigger();
   const int block = blockIdx.x;
   if (block == 0 && threadIdx.x == 0) *list = 0;
-  if (block < ra) split_rows(block, a.X, a.ldx, a.n, K, kp, a.dig, a.exps, a.cnt);
-  else if (b_rows) split_rows(block - ra, b.X, b.ldx, b.n, K, kp, b.dig, b.exps, b.cnt);
-  else split_cols<true>(block - ra, 0, b.X, b.ldx, K, b.n, kp, K, nullptr, b.dig, b.exps, b.cnt);
+  if (kper)
+    for (int i = block * 256 + threadIdx.x; i < b.n; i += gridDim.x * 256) b.cnt[i] = 0;
+  if (block < ra) {
+    split_rows(block, a.X, a.ldx, a.n, K, kp, a.dig, a.exps, a.cnt);
+  } else if (b_rows) {
+    split_rows(block - ra, b.X, b.ldx, b.n, K, kp, b.dig, b.exps, b.cnt);
+  } else if (kper) {
+    const int gx = (b.n + 31) / 32;
+    col_exps((block - ra) % gx, (block - ra) / gx, b.X, b.ldx, K, b.n, kper, maxexp);
+  } else {
+    split_cols<true>(block - ra, 0, b.X, b.ldx, K, b.n, kp, K, nullptr, b.dig, b.exps, b.cnt);
+  }
 }
 __global__ void __launch_bounds__(256)
 split_cols_part_kernel(const SplitSide b, int K, int kp, int kper, const int* __restrict__ maxexp) {
+  la_pdl_wait();
+  la_pdl_trigger();
   split_cols<false>(blockIdx.x, blockIdx.y, b.X, b.ldx, K, b.n, kp, kper, maxexp, b.dig, b.exps,
                     b.cnt);
 }
@@ -353,6 +369,8 @@ split_cols_part_kernel(const SplitSide b, int K, int kp, int kper, const int* __
 
 struct SplitArgs {
   int M, N, K, tri, tiles_m, tiles_n, tiles, prefetch, per_cta;
+  int splits, kper;  // K in `splits` pieces of kper (a multiple of 128), piece z into C + z czs
+  size_t czs;
   const double* A;   // the operands themselves, for the FMA tiles
   size_t lda;
   const double* B;
@@ -364,7 +382,7 @@ struct SplitArgs {
   const __half *da, *db;  // the digits [SL][rows][kp]
   int kp, joint;     // joint: 2 sqrt(K), rounded up
   int* fits;         // per tile: 1 where the digits hold what it needs
-  int* list;         // [0] count, then the tiles left to fma_tiles_kernel
+  int* list;         // [0] count, then the tiles left to fma_tiles
   int* err;
 };
 
@@ -386,16 +404,43 @@ __device__ __forceinline__ void tile_at(const SplitArgs& p, int t, int& tm, int&
   tn = r / rows;
 }
 
+// Leading two digits of 8 neighbouring k of a row, as |a| in units of 2^ea, FP16 (11 bits are plenty
+// for a sum that decides within a factor).
+__device__ __forceinline__ uint4 abs8(const __half* d, size_t ss, int k, int K, int kp, bool in) {
+  uint4 x = make_uint4(0u, 0u, 0u, 0u), y = x;
+  if (in && k < kp) {  // rows are kp values, a multiple of 8
+    x = *reinterpret_cast<const uint4*>(d + k);
+    y = *reinterpret_cast<const uint4*>(d + ss + k);
+  }
+  const __half2 c0 = __float2half2_rn(0.0078125f), c1 = __float2half2_rn(3.0517578125e-5f);
+  __half2* xs = reinterpret_cast<__half2*>(&x);
+  const __half2* ys = reinterpret_cast<const __half2*>(&y);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    xs[i] = __habs2(__hfma2(xs[i], c0, __hmul2(ys[i], c1)));
+    // what lies between K and kp is not set
+    if (k + 2 * i >= K) xs[i] = __float2half2_rn(0.f);
+    else if (k + 2 * i + 1 >= K) xs[i] = __halves2half2(__low2half(xs[i]), __ushort_as_half(0));
+  }
+  return x;
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
+                                          uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // fits[tile] (see the head of the file), and the list of the others. A warp per tile compares the
 // counts; the tiles they do not decide are summed by the whole CTA, one after the other.
-constexpr int GK = 32;        // k per slab of the FP32 sums
 constexpr int GUARD_T = 256;
 __global__ void __launch_bounds__(GUARD_T)
 guard_kernel(const __grid_constant__ SplitArgs p) {
   la_pdl_wait();
   la_pdl_trigger();
   __shared__ int s_sum[GUARD_T / 32];
-  __shared__ __align__(16) float as[GK][PM + 4], bs[GK][PN + 4];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   {
     const int t = blockIdx.x * p.per_cta + warp;
@@ -431,66 +476,41 @@ guard_kernel(const __grid_constant__ SplitArgs p) {
     const int t = blockIdx.x * p.per_cta + w;
     int tm, tn;
     tile_at(p, t, tm, tn);
-    // sum_k |a_ik| |b_kj| in units of 2^(ea + eb), every element of the tile: rows 8 ty.., columns
-    // 4 tx..
-    const int tx = tid & 15, ty = tid >> 4;
+    // sum_k |a_ik| |b_kj| in units of 2^(ea + eb), every element of the tile: warp w the rows
+    // 32 (w / 2).. and columns 32 (w % 2)... Each thread takes 8 neighbouring k of its rows at a time
+    // for two mma.sync; which k an operand register holds does not matter to the sum as long as A
+    // and B agree.
+    const int g = lane >> 2, kq = (lane & 3) * 8;
+    const int row0 = tm * PM + warp / 2 * 32 + g, col0 = tn * PN + warp % 2 * 32 + g;
     const size_t sa = (size_t)p.M * p.kp, sb = (size_t)p.N * p.kp;
-    constexpr int LOADS = (PM + PN) * (GK / 4) / GUARD_T;  // 4 k of one row per load
-    uint2 d0[LOADS], d1[LOADS];
-    auto fetch = [&](int k0) {
+    float acc[2][4][4] = {};
+    for (int k0 = 0; k0 < p.K; k0 += 32) {
+      uint4 a[4], b[4];
 #pragma unroll
-      for (int q = 0; q < LOADS; q++) {
-        const int e = tid + q * GUARD_T, row = e / (GK / 4), k = k0 + e % (GK / 4) * 4;
-        const bool ina = row < PM;
-        const int g = ina ? tm * PM + row : tn * PN + row - PM;
-        d0[q] = d1[q] = make_uint2(0u, 0u);
-        if (g < (ina ? p.M : p.N) && k < p.K) {  // rows are kp values, a multiple of 8
-          const __half* d = (ina ? p.da : p.db) + (size_t)g * p.kp + k;
-          d0[q] = *reinterpret_cast<const uint2*>(d);
-          d1[q] = *reinterpret_cast<const uint2*>(d + (ina ? sa : sb));
+      for (int i = 0; i < 4; i++) {
+        a[i] = abs8(p.da + (size_t)(row0 + 8 * i) * p.kp, sa, k0 + kq, p.K, p.kp, row0 + 8 * i < p.M);
+        b[i] = abs8(p.db + (size_t)(col0 + 8 * i) * p.kp, sb, k0 + kq, p.K, p.kp, col0 + 8 * i < p.N);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          mma_16816(acc[i][j], a[2 * i].x, a[2 * i + 1].x, a[2 * i].y, a[2 * i + 1].y, b[j].x, b[j].y);
+          mma_16816(acc[i][j], a[2 * i].z, a[2 * i + 1].z, a[2 * i].w, a[2 * i + 1].w, b[j].z, b[j].w);
         }
-      }
-    };
-    float acc[8][4] = {};
-    fetch(0);
-    for (int k0 = 0; k0 < p.K; k0 += GK) {
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < LOADS; q++) {
-        const int e = tid + q * GUARD_T, row = e / (GK / 4), k = e % (GK / 4) * 4;
-        const __half* x = reinterpret_cast<const __half*>(&d0[q]);
-        const __half* y = reinterpret_cast<const __half*>(&d1[q]);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const float v = k0 + k + i < p.K ? fabsf(__half2float(x[i]) * 0.0078125f +
-                                                   __half2float(y[i]) * 3.0517578125e-5f)
-                                           : 0.f;  // what lies between K and kp is not set
-          if (row < PM) as[k + i][row] = v;
-          else bs[k + i][row - PM] = v;
-        }
-      }
-      __syncthreads();
-      if (k0 + GK < p.K) fetch(k0 + GK);
-#pragma unroll 8
-      for (int k = 0; k < GK; k++) {
-        const float4 x0 = *reinterpret_cast<const float4*>(&as[k][8 * ty]);
-        const float4 x1 = *reinterpret_cast<const float4*>(&as[k][8 * ty + 4]);
-        const float4 y0 = *reinterpret_cast<const float4*>(&bs[k][4 * tx]);
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-        const float y[4] = {y0.x, y0.y, y0.z, y0.w};
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
-      }
     }
     const float need = GUARD * sqrtf((float)p.K);
     bool ok = true;
 #pragma unroll
-    for (int i = 0; i < 8; i++)
+    for (int i = 0; i < 2; i++)
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (tm * PM + 8 * ty + i < p.M && tn * PN + 4 * tx + j < p.N) ok = ok && acc[i][j] >= need;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int r = row0 + 16 * i + 8 * (e >> 1);
+          const int c = col0 - g + 8 * j + 2 * (lane & 3) + (e & 1);
+          if (r < p.M && c < p.N) ok = ok && acc[i][j][e] >= need;
+        }
     const bool fit = __syncthreads_and(ok ? 1 : 0) != 0;
     if (tid == 0) {
       p.fits[t] = fit ? 1 : 0;
@@ -535,6 +555,82 @@ __device__ __forceinline__ double round_sum(Sum96 a, int sc) {
   return hi == 0u ? 0.0 : __hiloint2double((int)rh, (int)rl);
 }
 
+__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_T) : "memory"); }
+
+// The listed tiles by FMA chains in ascending k, in halves of 64 x 64, by the epilogue's 512
+// threads: thread (tx, ty) owns rows ty + 32 i and columns tx + 16 j. The next slab's values wait in
+// registers while the present one is used; the FP64 pipe (two FMAs per clock) hides the rest. buf:
+// two slabs of A and of B.
+template <int MODE>
+__device__ __noinline__ void fma_tiles(const SplitArgs& p, double* buf, int tid) {
+  double(*as)[FK][FT] = reinterpret_cast<double(*)[FK][FT]>(buf);
+  double(*bs)[FK][FT] = reinterpret_cast<double(*)[FK][FT]>(buf + 2 * FK * FT);
+  const int items = 2 * p.splits * *reinterpret_cast<volatile int*>(p.list);
+  const int tx = tid & 15, ty = tid >> 4;
+  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+    int tm, tn;
+    tile_at(p, p.list[1 + it / (2 * p.splits)], tm, tn);
+    const int z = it / 2 % p.splits;
+    const int kb = z * p.kper, ke = min(p.K, kb + p.kper);
+    double* C = p.C + z * p.czs;
+    const int m0 = tm * PM + (it & 1) * FT, n0 = tn * PN;
+    double acc[2][4], ra[2], rb[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int r = m0 + ty + 32 * i, c = n0 + tx + 16 * j;
+        acc[i][j] = MODE != 0 && r < p.M && c < p.N ? C[(size_t)r * p.ldc + c] : 0.0;
+      }
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int e = tid + q * EPI_T;
+        const int r = e / FK, k = e % FK;
+        ra[q] = m0 + r < p.M && k0 + k < ke ? p.A[(size_t)(m0 + r) * p.lda + k0 + k] : 0.0;
+        if (p.b_rows)
+          rb[q] = n0 + r < p.N && k0 + k < ke ? p.B[(size_t)(n0 + r) * p.ldb + k0 + k] : 0.0;
+        else
+          rb[q] = n0 + e % FT < p.N && k0 + e / FT < ke
+                      ? p.B[(size_t)(k0 + e / FT) * p.ldb + n0 + e % FT] : 0.0;
+      }
+    };
+    epi_sync();  // the buffer's last users are done
+    fetch(kb);
+    for (int k0 = kb, b = 0; k0 < ke; k0 += FK, b ^= 1) {
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int e = tid + q * EPI_T;
+        as[b][e % FK][(e / FK) ^ (e % FK)] = ra[q];
+        const int k = p.b_rows ? e % FK : e / FT, c = p.b_rows ? e / FK : e % FT;
+        bs[b][k][c ^ k] = rb[q];
+      }
+      epi_sync();  // the other buffer's readers of two slabs ago are done, too
+      if (k0 + FK < ke) fetch(k0 + FK);
+      const int kn = min(FK, ke - k0);
+#pragma unroll 4
+      for (int k = 0; k < kn; k++) {
+        double a[2], v[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) a[i] = as[b][k][(ty + 32 * i) ^ k];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = bs[b][k][(tx + 16 * j) ^ k];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = fma(MODE < 0 ? -a[i] : a[i], v[j], acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int r = m0 + ty + 32 * i, c = n0 + tx + 16 * j;
+        if (r < p.M && c < p.N) C[(size_t)r * p.ldc + c] = acc[i][j];
+      }
+  }
+}
+
 // MODE -1: C -= A B, 0: C = A B, 1: C += A B.
 template <int MODE>
 __global__ void __launch_bounds__(SPLIT_T, 1)
@@ -549,8 +645,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(split_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int nst = (p.K + PK - 1) / PK;                           // stages per tile
-  const int nchunk = (nst + CHUNK_STAGES - 1) / CHUNK_STAGES;
+  const int total = p.tiles * p.splits;
+  // The grid has a CTA for every FMA half of small products; without FMA tiles they are done here.
+  if (blockIdx.x >= total && *reinterpret_cast<volatile int*>(p.list) == 0) return;
+  // Item t: tile t % tiles of piece t / tiles, whose stages are s0, s0 + 1, ... (nst of them).
+  auto item = [&](int t, int& tile, int& z, int& s0) {
+    z = t / p.tiles;
+    tile = t - z * p.tiles;
+    s0 = z * (p.kper / PK);
+    return (min(p.kper, p.K - z * p.kper) + PK - 1) / PK;
+  };
 
   if (tid == 0) {
     for (int s = 0; s < NST; s++) {
@@ -578,10 +682,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   if (warp == EPI_WARPS) {  // TMA producer
     int n = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
-      if (!__ldg(p.fits + t)) continue;
-      int tm, tn;
-      tile_at(p, t, tm, tn);
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int tile, z, s0, tm, tn;
+      const int nst = item(t, tile, z, s0);
+      if (!__ldg(p.fits + tile)) continue;
+      tile_at(p, tile, tm, tn);
       // C's tile into L2 (its rows are 512 bytes; the epilogue's loads would wait for DRAM)
       if (p.prefetch)
         for (int q = lane; q < PM * 4; q += 32) {
@@ -599,8 +704,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
           }
           unsigned char* st = smem + b * PST_BYTES;
           la_tma::mbar_expect_tx(&full[b], PST_BYTES);
-          tma_load_3d(st, &ta, s * PK, tm * PM, 0, &full[b]);
-          tma_load_3d(st + PA_BYTES, &tb, s * PK, tn * PN, 0, &full[b]);
+          tma_load_3d(st, &ta, (s0 + s) * PK, tm * PM, 0, &full[b]);
+          tma_load_3d(st + PA_BYTES, &tb, (s0 + s) * PK, tn * PN, 0, &full[b]);
         }
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
     }
@@ -610,8 +715,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   } else if (warp == EPI_WARPS + 1) {  // MMA issuer
     int n = 0, chunk = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
-      if (!__ldg(p.fits + t)) continue;
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int tile, z, s0;
+      const int nst = item(t, tile, z, s0);
+      if (!__ldg(p.fits + tile)) continue;
       if (lane == 0)
         for (int s = 0; s < nst && ok; s++, n++) {
           const int b = n % NST;
@@ -659,10 +766,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
     double* wbuf = reinterpret_cast<double*>(smem + NST * PST_BYTES) + warp * (32 * 8);
     int chunk = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < p.tiles && ok; t += gridDim.x) {
-      if (!__ldg(p.fits + t)) continue;
-      int tm, tn;
-      tile_at(p, t, tm, tn);
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int tile, z, s0, tm, tn;
+      const int nchunk = (item(t, tile, z, s0) + CHUNK_STAGES - 1) / CHUNK_STAGES;
+      if (!__ldg(p.fits + tile)) continue;
+      tile_at(p, tile, tm, tn);
+      double* C = p.C + z * p.czs;
       const int m0 = tm * PM, n0 = tn * PN;
       const int sr = m0 + row < p.M ? __ldg(p.ea + m0 + row) : 0;
       const int sc = n0 + col + (lane & 15) < p.N ? __ldg(p.eb + n0 + col + (lane & 15)) : 0;
@@ -709,7 +818,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const int gr = m0 + (warp & 3) * 32 + 4 * i + (lane >> 3);
-          if (MODE != 0) old[i] = gr < p.M && c < p.N ? p.C[(size_t)gr * p.ldc + c] : 0.0;
+          if (MODE != 0) old[i] = gr < p.M && c < p.N ? C[(size_t)gr * p.ldc + c] : 0.0;
         }
 #pragma unroll
         for (int j = 0; j < 8; j++) {
@@ -723,90 +832,20 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
           const int r = 4 * i + (lane >> 3), gr = m0 + (warp & 3) * 32 + r;
           const double v = wbuf[r * 8 + (cc ^ ((r >> 1) & 7))];
           if (gr < p.M && c < p.N)
-            p.C[(size_t)gr * p.ldc + c] = MODE == 0 ? v : MODE < 0 ? old[i] - v : old[i] + v;
+            C[(size_t)gr * p.ldc + c] = MODE == 0 ? v : MODE < 0 ? old[i] - v : old[i] + v;
         }
         __syncwarp();
       }
     }
     if (!ok) s_fail = 1;
+    // every epilogue warp comes here, whatever its waits gave, and the list is the same for all
+    if (*reinterpret_cast<volatile int*>(p.list) != 0)
+      fma_tiles<MODE>(p, reinterpret_cast<double*>(smem + NST * PST_BYTES), tid);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
-}
-
-// The listed tiles by FMA chains in ascending k, in halves of 64 x 64: thread (tx, ty) owns rows
-// ty + 16 i and columns tx + 16 j. The next slab's values wait in registers while the present one
-// is used; the FP64 pipe (two FMAs per clock) hides the rest.
-template <int MODE>
-__global__ void __launch_bounds__(FMA_T, FMA_PER_SM)
-fma_tiles_kernel(const __grid_constant__ SplitArgs p) {
-  la_pdl_wait();
-  la_pdl_trigger();
-  __shared__ double as[2][FK][FT], bs[2][FK][FT];
-  if (*reinterpret_cast<volatile int*>(p.err) != 0) return;
-  const int items = 2 * *reinterpret_cast<volatile int*>(p.list);
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    int tm, tn;
-    tile_at(p, p.list[1 + it / 2], tm, tn);
-    const int m0 = tm * PM + (it & 1) * FT, n0 = tn * PN;
-    double acc[4][4], ra[4], rb[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int r = m0 + ty + 16 * i, c = n0 + tx + 16 * j;
-        acc[i][j] = MODE != 0 && r < p.M && c < p.N ? p.C[(size_t)r * p.ldc + c] : 0.0;
-      }
-    auto fetch = [&](int k0) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int e = tid + q * FMA_T;
-        const int r = e / FK, k = e % FK;
-        ra[q] = m0 + r < p.M && k0 + k < p.K ? p.A[(size_t)(m0 + r) * p.lda + k0 + k] : 0.0;
-        if (p.b_rows)
-          rb[q] = n0 + r < p.N && k0 + k < p.K ? p.B[(size_t)(n0 + r) * p.ldb + k0 + k] : 0.0;
-        else
-          rb[q] = n0 + e % FT < p.N && k0 + e / FT < p.K
-                      ? p.B[(size_t)(k0 + e / FT) * p.ldb + n0 + e % FT] : 0.0;
-      }
-    };
-    fetch(0);
-    for (int k0 = 0, b = 0; k0 < p.K; k0 += FK, b ^= 1) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int e = tid + q * FMA_T;
-        as[b][e % FK][(e / FK) ^ (e % FK)] = ra[q];
-        const int k = p.b_rows ? e % FK : e / FT, c = p.b_rows ? e / FK : e % FT;
-        bs[b][k][c ^ k] = rb[q];
-      }
-      __syncthreads();  // the other buffer's readers of two slabs ago are done, too
-      if (k0 + FK < p.K) fetch(k0 + FK);
-      const int kn = min(FK, p.K - k0);
-#pragma unroll 4
-      for (int k = 0; k < kn; k++) {
-        double a[4], v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) a[i] = as[b][k][(ty + 16 * i) ^ k];
-#pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = bs[b][k][(tx + 16 * j) ^ k];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fma(MODE < 0 ? -a[i] : a[i], v[j], acc[i][j]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int r = m0 + ty + 16 * i, c = n0 + tx + 16 * j;
-        if (r < p.M && c < p.N) p.C[(size_t)r * p.ldc + c] = acc[i][j];
-      }
-  }
 }
 
 size_t up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -837,13 +876,10 @@ la_status launch_product(la_ctx ctx, cudaStream_t st, const CUtensorMap& ta, con
   e = la_launch(ctx, guard_kernel, dim3((p.tiles + p.per_cta - 1) / p.per_cta), dim3(GUARD_T), 0, st,
                 p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "guard_kernel launch");
-  e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(std::min(p.tiles, ctx->sm_count)),
+  e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(std::min(2 * p.tiles * p.splits, ctx->sm_count)),
                 dim3(SPLIT_T), SPLIT_SMEM, st, ta, tb, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "gemm_split_kernel launch");
-  const int halves = (int)std::min<long long>(2ll * p.tiles, (long long)FMA_PER_SM * ctx->sm_count);
-  e = la_launch(ctx, fma_tiles_kernel<MODE>, dim3(halves), dim3(FMA_T), 0, st, p);
-  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "fma_tiles_kernel launch");
-  ctx->launches += 3;
+  ctx->launches += 2;
   return la_check_launch(ctx, "gemm_split_kernel");
 }
 
@@ -868,19 +904,19 @@ la_status launch_splits(la_ctx ctx, cudaStream_t st, const SplitSide& a, const S
                         bool b_rows, int K, int kp, int* maxexp, int* list) {
   const int ra = (a.n + 7) / 8;
   const bool parts = !same && !b_rows && K > COLS_ALL_K;
-  const int rb = same || parts ? 0 : b_rows ? (b.n + 7) / 8 : (b.n + 31) / 32;
+  const int kper = parts ? 256 : 0, pieces = parts ? (K + kper - 1) / kper : 1;
+  const int gx = (b.n + 31) / 32;
+  const int rb = same ? 0 : b_rows ? (b.n + 7) / 8 : gx * pieces;
+  if (parts) LA_CUDA(ctx, cudaMemsetAsync(maxexp, 0, (size_t)b.n * 2 * sizeof(int), st));
   cudaError_t e = la_launch(ctx, split_kernel, dim3(ra + rb), dim3(256), 0, st, a, b, K, kp, ra,
-                            b_rows ? 1 : 0, list);
+                            b_rows ? 1 : 0, kper, list, maxexp);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "split_kernel launch");
   ctx->launches++;
   if (parts) {
-    const int kper = 256;
-    const dim3 grid((b.n + 31) / 32, (K + kper - 1) / kper);
-    // cnt and, right after it, the two words per column of col_exp_kernel
-    LA_CUDA(ctx, cudaMemsetAsync(b.cnt, 0, (size_t)b.n * 3 * sizeof(int), st));
-    col_exp_kernel<<<grid, 256, 0, st>>>(b.X, b.ldx, K, b.n, kper, maxexp);
-    split_cols_part_kernel<<<grid, 256, 0, st>>>(b, K, kp, kper, maxexp);
-    ctx->launches += 2;
+    e = la_launch(ctx, split_cols_part_kernel, dim3(gx, pieces), dim3(256), 0, st, b, K, kp, kper,
+                  (const int*)maxexp);
+    if (e != cudaSuccess) return la_cuda_fail(ctx, e, "split_cols_part_kernel launch");
+    ctx->launches++;
   }
   return la_check_launch(ctx, "split_kernel");
 }
@@ -894,9 +930,13 @@ size_t gemm_split_ws(int M, int N, int K, bool same) {
 
 la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
                             const double* A, size_t lda, const double* B, size_t ldb, bool b_rows,
-                            double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes) {
+                            double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes, int splits,
+                            int kper, size_t czs) {
   if (M <= 0 || N <= 0) return LA_OK;
   if (K <= 0 || K > (1 << 20) || (tri && M != N)) return LA_UNSUPPORTED;
+  if (splits > 1 && (mode != 0 || kper % (CHUNK_STAGES * PK) || (long long)(splits - 1) * kper >= K ||
+                     (long long)splits * kper < K))
+    return LA_UNSUPPORTED;
   const bool same = b_rows && A == B && lda == ldb && M == N;
   const int kp = (int)up(K, 8);
   if (!ws || ws_bytes < gemm_split_ws(M, N, K, same)) return LA_UNSUPPORTED;
@@ -917,7 +957,10 @@ la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N,
   p.tiles_n = (N + PN - 1) / PN;
   const long long lower = (long long)p.tiles_m * (p.tiles_m + 1);
   const long long tiles = tri ? lower : (long long)p.tiles_m * p.tiles_n;
-  if (tiles > (1 << 24)) return LA_UNSUPPORTED;
+  if (tiles * splits > (1 << 24)) return LA_UNSUPPORTED;
+  p.splits = splits;
+  p.kper = splits > 1 ? kper : (int)up(K, PK);
+  p.czs = czs;
   p.tiles = (int)tiles;
   p.A = A;
   p.lda = lda;

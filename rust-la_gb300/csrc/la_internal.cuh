@@ -233,11 +233,13 @@ la_status launch_gemm_lower(la_ctx ctx, int M, int K, const double* A, size_t ld
 // Products on the tensor cores by exact splitting (gemm_split.cu): C (M x N) -= A B (mode -1), = A B
 // (0) or += A B (1); A M x K, B K x N, or N x K rows of B' when b_rows; any alignment. tri: the
 // square C's part at or below the diagonal, in tiles. ws: gemm_split_ws bytes of device memory,
-// used until the product is done (same: B' is A). LA_UNSUPPORTED: nothing launched.
+// used until the product is done (same: B' is A). splits > 1 (mode 0): K in pieces of kper, a
+// multiple of 128, piece z's product to C + z czs. LA_UNSUPPORTED: nothing launched.
 size_t gemm_split_ws(int M, int N, int K, bool same);
 la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
                             const double* A, size_t lda, const double* B, size_t ldb, bool b_rows,
-                            double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes);
+                            double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes,
+                            int splits = 1, int kper = 0, size_t czs = 0);
 // C + z * czs = A[:, z kper : (z + 1) kper] B[z kper : (z + 1) kper, :] for z < splits
 // (fused, from zero); kper a multiple of 32, splits * kper >= K > (splits - 1) kper.
 la_status launch_gemm_splitk(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
@@ -261,8 +263,8 @@ la_status launch_panel(la_ctx ctx, cudaStream_t stream, bool exact, double* A, d
                        size_t ld, int m, int j0, int jb, int* d_ipiv, unsigned* bar_base);
 la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t stream, double* A, size_t ld, int m, int j0,
                                  int jb, int* d_ipiv);
-// C -= A B with tiles of 16 columns (N <= 64), for narrow updates.
-la_status launch_gemm_narrow(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,
+// C -= A B or C = A B (mode GM_FMA_SUB, GM_FMA_ZERO) with tiles of 16 columns.
+la_status launch_gemm_narrow(la_ctx ctx, int mode, int M, int N, int K, const double* A, size_t lda,
                              const double* B, size_t ldb, double* C, size_t ldc);
 la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int n, int j0,
                        int jb);

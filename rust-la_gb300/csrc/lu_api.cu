@@ -96,7 +96,7 @@ constexpr size_t GEMM_SMEM_WITH_PANEL = 78 * 1024;
 // pieces of whole tiles, gives the same bits.
 constexpr int LU_BASE = 64;
 constexpr int LU_MAX_BLOCK = 256;
-constexpr int SPLIT_MIN_MN = 64 * 64;  // smaller updates: one FMA launch is no slower than four
+constexpr int SPLIT_MIN_MN = 64 * 64;  // smaller updates: one FMA launch is no slower than three
 
 // Block width for R remaining rows.
 int lu_block(int R) { return R > 3072 ? 256 : R > 1024 ? 128 : LU_BASE; }
@@ -140,7 +140,7 @@ struct FastLu {
       if (s != LA_UNSUPPORTED) return s;
     }
     if (N <= 64 && K <= 64)
-      return launch_gemm_narrow(ctx, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld);
+      return launch_gemm_narrow(ctx, GM_FMA_SUB, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld);
     return launch_gemm(ctx, GM_FMA_SUB, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld);
   }
 
@@ -182,8 +182,8 @@ struct FastLu {
         b = t.begin(ctx->stream);
         LA_TRY(solve(j0, j1, j1, b1));
         if (j1 < m)
-          LA_TRY(launch_gemm_narrow(ctx, m - j1, b1 - j1, jb, at(j1, j0), ld, at(j0, j1), ld,
-                                    at(j1, j1), ld));
+          LA_TRY(launch_gemm_narrow(ctx, GM_FMA_SUB, m - j1, b1 - j1, jb, at(j1, j0), ld, at(j0, j1),
+                                    ld, at(j1, j1), ld));
         t.end(ctx->stream, b, PH_OTHER);
       }
     }
@@ -417,7 +417,7 @@ la_status gemm_device_common(la_ctx ctx, const double* d_a, size_t lda, const do
   const int mode = ctx->arith == LA_ARITH_EXACT ? GM_EXACT_ZERO : GM_FMA_ZERO;
   if (mode == GM_FMA_ZERO && n > 16 && k >= 32) {
     // On the tensor cores from 32 k and 17 columns on: one FMA tile of 64 x 64 x 32 keeps an SM busy
-    // for 33 us, while the split product's four launches of one tile take about 15 us in all
+    // for 33 us, while the split product's three launches of one tile take about 15 us in all
     // (8192^3: 27.9 ms against 876 ms). In slabs of K whose digits fit the workspace.
     const size_t kc = std::max<size_t>(128, SPLIT_WS_MAX / (16 * (m + n)) / 128 * 128);
     DevBuf ws(ctx);

@@ -31,10 +31,15 @@
 //                      block goes back to A with zeros above the diagonal of
 //                      its top square (whose final content is kept in rsave),
 //                      V' to its own buffer, a to rdiag and tau.
-//   W = V' A[j:, j:]   split-K FP64 GEMM (gemm_f64) and a reduction of the
-//                      partial products; W's first nb columns are G.
+//   W = V' A[j:, j:]   split-K product and a reduction of the partial products; W's first nb
+//                      columns are G.
 //   W2 = T' W          qr_tsolve_kernel (one warp per column).
 //   A[j:, j+nb:] -= V W2, then the top square restored from rsave.
+// Where there are rows enough below the block's top square (tc_block), both products take those rows
+// on the tensor cores by exact splitting (gemm_split.cu). The top square, which holds V's zeros and
+// its large diagonal, does not suit the digits' scaling; its part of W is added where the partial
+// products are summed (qr_wsum_top_kernel), its part of the update where W2 is formed
+// (qr_tsolve_kernel), from V', and the panel writes its final content to A at once.
 // G of every block is kept for get_q and solve.
 //
 // The blocked and the column-by-column FAST forms perform the same reflections
@@ -42,6 +47,7 @@
 #include <algorithm>
 
 #include "la_internal.cuh"
+#include "tma_util.cuh"
 
 namespace {
 
@@ -77,7 +83,7 @@ struct QrPanelArgs {
   double* tau;        // [nb]
   double* vt;         // V' (nb x rows, pitch ldv)
   size_t ldv;
-  double* rsave;      // the top square's final content (nb x QB)
+  double* rsave;      // the top square's final content (nb x QB); null: straight to A
 };
 
 __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
@@ -86,6 +92,8 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
   __shared__ double own[2][QB];                // the diagonal row: q, then t_c
   __shared__ double red[QPT];
   __shared__ double mine[QB], tot[QB], fac[QB];
+  la_pdl_wait();
+  la_pdl_trigger();
   const int tid = threadIdx.x;
   const uint32_t rank = cta_rank();
   const int CL = (int)gridDim.x;  // one cluster per launch
@@ -168,8 +176,8 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
     const int lr = idx / nb, c = idx % nb;
     const int i = r0 + lr - p.j;
     const double v = P[lr * QNBP + c];
-    if (i < nb) p.rsave[i * QB + c] = v;
-    p.A[(size_t)(r0 + lr) * p.ld + p.j + c] = c > i ? 0.0 : v;
+    if (i < nb && p.rsave) p.rsave[i * QB + c] = v;
+    p.A[(size_t)(r0 + lr) * p.ld + p.j + c] = c > i && p.rsave ? 0.0 : v;
   }
   for (int idx = tid; idx < nr * nb; idx += QPT) {
     const int c = idx / nr, lr = idx % nr;
@@ -181,6 +189,8 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
 // out[r][c] = sum over z < splits of part[z][r][c] (ascending z).
 __global__ void qr_wsum_kernel(const double* __restrict__ part, size_t ldp, size_t pzs, int splits,
                                int rows, int cols, double* __restrict__ out, size_t ldo) {
+  la_pdl_wait();
+  la_pdl_trigger();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)rows * cols) return;
   const int r = (int)(idx / cols), c = (int)(idx % cols);
@@ -190,17 +200,61 @@ __global__ void qr_wsum_kernel(const double* __restrict__ part, size_t ldp, size
   out[(size_t)r * ldo + c] = s;
 }
 
+// out = sum over z < splits of part[z] + V_top' T_top, QB x cols: the partial products of the rows
+// below the top square and the square's own QB k by FMA. 8 columns per CTA (an SM needs 8 us for
+// them), thread (column, rows r, r + 32). T_top's first nvc columns are V's own, which A does not
+// hold explicitly: they come from V'.
+constexpr int WT_C = 8;
+__global__ void __launch_bounds__(256)
+qr_wsum_top_kernel(const double* __restrict__ part, size_t ldp, size_t pzs, int splits,
+                   const double* __restrict__ vt, size_t ldv, const double* __restrict__ T,
+                   size_t ldt, int cols, int nvc, double* __restrict__ out, size_t ldo) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  __shared__ double v[QB][QNBP], t[QB][WT_C + 1];
+  const int tid = threadIdx.x, cl = tid % WT_C, r = tid / WT_C;  // r 0..31
+  const int c0 = blockIdx.x * WT_C, c = c0 + cl;
+  for (int idx = tid; idx < QB * QB; idx += 256)
+    v[idx / QB][idx % QB] = vt[(size_t)(idx / QB) * ldv + idx % QB];
+  for (int k = r; k < QB; k += 32)
+    t[k][cl] = c >= cols ? 0.0 : c < nvc ? vt[(size_t)c * ldv + k] : T[(size_t)k * ldt + c];
+  double a0 = 0.0, a1 = 0.0;
+  if (c < cols)
+    for (int z = 0; z < splits; z++) {
+      a0 += part[z * pzs + (size_t)r * ldp + c];
+      a1 += part[z * pzs + (size_t)(r + 32) * ldp + c];
+    }
+  __syncthreads();
+#pragma unroll 8
+  for (int k = 0; k < QB; k++) {
+    a0 = fma(v[r][k], t[k][cl], a0);
+    a1 = fma(v[r + 32][k], t[k][cl], a1);
+  }
+  if (c < cols) {
+    out[(size_t)r * ldo + c] = a0;
+    out[(size_t)(r + 32) * ldo + c] = a1;
+  }
+}
+
 // W2[:, c] = T' W[:, c] (forward) or T W[:, c] (backward) for c < ncols, with
 // T^-1 = diag(1/tau) + strictly_upper(G) (nb x nb, pitch ldg): one warp per
 // column, lane l holding rows l and l + 32. Each step takes W2_i from its
 // lane (a shuffle) and applies it to the rows still open (right-looking), so
 // the chain per column is nb shuffles, with the FMAs of a step independent.
-// gsave (when not null) receives G (pitch QB) from CTA 0.
+// gsave (when not null) receives G (pitch QB) from CTA 0. TOP: also C[0:QB, c] -= V_top W2[:, c], the
+// update of the block's top rows (nb = QB; V' in vt).
+constexpr size_t QTS_SMEM = (size_t)2 * QB * QNBP * sizeof(double);
+template <bool TOP>
 __global__ void __launch_bounds__(QTS_W * 32)
 qr_tsolve_kernel(const double* __restrict__ G, size_t ldg, const double* __restrict__ tau, int nb,
                  const double* __restrict__ W, size_t ldw, int ncols, double* __restrict__ W2,
-                 size_t ldw2, int forward, double* __restrict__ gsave) {
-  __shared__ double Gs[QB][QNBP];
+                 size_t ldw2, int forward, double* __restrict__ gsave,
+                 const double* __restrict__ vt, size_t ldv, double* __restrict__ C, size_t ldc) {
+  la_pdl_wait();
+  la_pdl_trigger();
+  extern __shared__ __align__(16) double qts[];
+  double(*Gs)[QNBP] = reinterpret_cast<double(*)[QNBP]>(qts);
+  double(*Vs)[QNBP] = reinterpret_cast<double(*)[QNBP]>(qts + QB * QNBP);  // Vs[k][i] = V[i][k]
   __shared__ double ts[QB];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int idx = tid; idx < nb * nb; idx += QTS_W * 32) {
@@ -209,6 +263,9 @@ qr_tsolve_kernel(const double* __restrict__ G, size_t ldg, const double* __restr
     Gs[r][q] = g;
     if (gsave && blockIdx.x == 0) gsave[r * QB + q] = g;
   }
+  if (TOP)
+    for (int idx = tid; idx < QB * QB; idx += QTS_W * 32)
+      Vs[idx / QB][idx % QB] = vt[(size_t)(idx / QB) * ldv + idx % QB];
   if (tid < QB) ts[tid] = tid < nb ? tau[tid] : 0.0;
   __syncthreads();
   const int c = blockIdx.x * QTS_W + warp;
@@ -237,6 +294,22 @@ qr_tsolve_kernel(const double* __restrict__ G, size_t ldg, const double* __restr
   }
   if (r0 < nb) W2[(size_t)r0 * ldw2 + c] = a0;
   if (r1 < nb) W2[(size_t)r1 * ldw2 + c] = a1;
+  if (TOP) {
+    double x0 = C[(size_t)r0 * ldc + c], x1 = C[(size_t)r1 * ldc + c];
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {  // V's zeros above its diagonal are terms like any other
+      const double w = __shfl_sync(0xffffffffu, a0, k);
+      x0 = fma(-Vs[k][r0], w, x0);
+      x1 = fma(-Vs[k][r1], w, x1);
+    }
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {  // rows below 32 have none of these columns
+      const double w = __shfl_sync(0xffffffffu, a1, k);
+      x1 = fma(-Vs[k + 32][r1], w, x1);
+    }
+    C[(size_t)r0 * ldc + c] = x0;
+    C[(size_t)r1 * ldc + c] = x1;
+  }
 }
 
 // V of a factored block (rows [j, m), columns [j, j + nb)) in explicit form:
@@ -246,6 +319,8 @@ __global__ void qr_build_v_kernel(const double* __restrict__ A, size_t ld, int m
                                   const double* __restrict__ rdiag, int mode,
                                   double* __restrict__ vx, double* __restrict__ vt, size_t ldv,
                                   double* __restrict__ tau) {
+  la_pdl_wait();
+  la_pdl_trigger();
   const int rows = m - j;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < (size_t)nb) {
@@ -318,13 +393,15 @@ la_status launch_qr_panel(la_ctx ctx, const QrPanelArgs& a, int cluster, cudaStr
   cfg.blockDim = dim3(QPT);
   cfg.dynamicSmemBytes = (size_t)a.rpc * QNBP * sizeof(double);
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = ctx->pdl_now ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, qr_panel_kernel, a);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaLaunchKernelEx(qr_panel)");
   ctx->launches++;
@@ -353,8 +430,52 @@ struct DevBuf {
   double* d() const { return static_cast<double*>(p); }
 };
 
-// W = V' T[j:, cols] (nb x ncols) by split-K GEMM and reduction into wf
-// (pitch ldw), from vt (nb x rows, pitch ldv) and T (pitch ldt).
+// Workspace of the split products (null: FMA products throughout).
+struct SplitWs {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+// Whether a block of `rows` rows uses them against `right` columns (get_q: all of them; else those
+// right of the block): a whole 64-row square on top, and enough below and beside it that their
+// launches are no slower than one FMA product (a 64 x 64 x 64 FMA tile alone takes 66 us).
+bool tc_block(const SplitWs& ws, int nb, int rows, int right) {
+  return ws.p && nb == QB && rows >= 3 * QB && right > 32;
+}
+// Pieces of the K = rows below the top square: about one tile per SM, at least 256 k each.
+void split_plan_tc(la_ctx ctx, int tiles, int K, int* splits, int* kper) {
+  const int s = std::max(1, std::min(K / 256, ctx->sm_count / std::max(1, tiles)));
+  *kper = ((K + s - 1) / s + 127) / 128 * 128;
+  *splits = (K + *kper - 1) / *kper;
+}
+// Digits for products against up to n columns of m rows; without the memory: FMA products.
+la_status alloc_split(la_ctx ctx, DevBuf& buf, int m, int n, SplitWs* ws) {
+  ws->bytes = std::max(gemm_split_ws(QB, n, m, false), gemm_split_ws(m, n, QB, false));
+  if (la_tma::get_encoder(ctx) && buf.alloc((ws->bytes + 7) / 8) == LA_OK) ws->p = buf.p;
+  return LA_OK;
+}
+
+// The block's [G | W] = V' T[j:, cols] on the tensor cores: rows below the top square by split
+// products, the square in the sum. vt: V' (QB x rows, pitch ldv), T (pitch ldt), wf (pitch ldw).
+la_status apply_vt_tc(la_ctx ctx, const SplitWs& ws, const double* vt, size_t ldv, int rows,
+                      const double* T, size_t ldt, int ncols, int nvc, double* part, size_t part_cap,
+                      double* wf, size_t ldw) {
+  const size_t ldp = pad4b((size_t)ncols), pzs = (size_t)QB * ldp;
+  int splits, kper;
+  split_plan_tc(ctx, (ncols + 63) / 64, rows - QB, &splits, &kper);
+  if ((size_t)splits * pzs > part_cap) return LA_INVALID;
+  LA_TRY(launch_gemm_split(ctx, ctx->stream, 0, QB, ncols, rows - QB, vt + QB, ldv,
+                           T + (size_t)QB * ldt, ldt, false, part, ldp, false, ws.p, ws.bytes, splits,
+                           kper, pzs));
+  const cudaError_t e = la_launch(ctx, qr_wsum_top_kernel, dim3((ncols + WT_C - 1) / WT_C), dim3(256),
+                                  0, ctx->stream, (const double*)part, ldp, pzs, splits, vt, ldv, T,
+                                  ldt, ncols, nvc, wf, ldw);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "qr_wsum_top_kernel launch");
+  ctx->launches++;
+  return la_check_launch(ctx, "qr_wsum_top_kernel");
+}
+
+// W = V' T[j:, cols] (nb x ncols) by split-K GEMM and reduction into wf (pitch ldw), from vt
+// (nb x rows, pitch ldv) and T (pitch ldt).
 la_status apply_vt(la_ctx ctx, const double* vt, size_t ldv, int nb, int rows, const double* T,
                    size_t ldt, int ncols, double* part, size_t part_cap, double* wf, size_t ldw) {
   int splits, kper;
@@ -363,24 +484,37 @@ la_status apply_vt(la_ctx ctx, const double* vt, size_t ldv, int nb, int rows, c
   if ((size_t)splits * pzs > part_cap) return LA_INVALID;
   LA_TRY(launch_gemm_splitk(ctx, nb, ncols, rows, vt, ldv, T, ldt, part, ldp, pzs, splits, kper));
   const size_t total = (size_t)nb * ncols;
-  qr_wsum_kernel<<<blocks_of(total, 256), 256, 0, ctx->stream>>>(part, ldp, pzs, splits, nb, ncols,
-                                                                wf, ldw);
+  const cudaError_t e =
+      la_launch(ctx, qr_wsum_kernel, dim3(blocks_of(total, 256)), dim3(256), 0, ctx->stream,
+                (const double*)part, ldp, pzs, splits, nb, ncols, wf, ldw);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "qr_wsum_kernel launch");
   ctx->launches++;
   return la_check_launch(ctx, "qr_wsum_kernel");
 }
 
+// top: C[0:QB] -= V_top W2 too (vt, C).
 la_status launch_tsolve(la_ctx ctx, const double* G, size_t ldg, const double* tau, int nb,
                         const double* W, size_t ldw, int ncols, double* W2, size_t ldw2,
-                        bool forward, double* gsave) {
+                        bool forward, double* gsave, bool top = false, const double* vt = nullptr,
+                        size_t ldv = 0, double* C = nullptr, size_t ldc = 0) {
   if (ncols <= 0 && !gsave) return LA_OK;
-  qr_tsolve_kernel<<<std::max(1, blocks_of((size_t)std::max(ncols, 0), QTS_W)), QTS_W * 32, 0,
-                     ctx->stream>>>(G, ldg, tau, nb, W, ldw, std::max(ncols, 0), W2, ldw2,
-                                    forward ? 1 : 0, gsave);
+  static la_device_once configured;
+  LA_CUDA(ctx, configured.run([](int) {
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const cudaError_t r = cudaFuncSetAttribute(qr_tsolve_kernel<true>, at, (int)QTS_SMEM);
+    return r == cudaSuccess ? cudaFuncSetAttribute(qr_tsolve_kernel<false>, at, (int)QTS_SMEM) : r;
+  }));
+  const int n = std::max(ncols, 0);
+  const cudaError_t e = la_launch(
+      ctx, top ? qr_tsolve_kernel<true> : qr_tsolve_kernel<false>,
+      dim3(std::max(1, blocks_of((size_t)n, QTS_W))), dim3(QTS_W * 32), top ? QTS_SMEM : QTS_SMEM / 2,
+      ctx->stream, G, ldg, tau, nb, W, ldw, n, W2, ldw2, forward ? 1 : 0, gsave, vt, ldv, C, ldc);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "qr_tsolve_kernel launch");
   ctx->launches++;
   return la_check_launch(ctx, "qr_tsolve_kernel");
 }
 
-// The largest partial-product buffer over the blocks: splits x nb x pitch.
+// The largest partial-product buffer over the blocks: splits x nb x pitch (of either plan).
 size_t part_doubles(la_ctx ctx, int m, int dc, int cols_total, bool cols_from_j) {
   size_t cap = 0;
   for (int j = 0; j < dc; j += QB) {
@@ -389,6 +523,10 @@ size_t part_doubles(la_ctx ctx, int m, int dc, int cols_total, bool cols_from_j)
     int splits, kper;
     split_plan(ctx, (ncols + 63) / 64, m - j, &splits, &kper);
     cap = std::max(cap, (size_t)splits * QB * pad4b((size_t)ncols));
+    if (m - j > QB) {
+      split_plan_tc(ctx, (ncols + 63) / 64, m - j - QB, &splits, &kper);
+      cap = std::max(cap, (size_t)splits * QB * pad4b((size_t)ncols));
+    }
   }
   return cap;
 }
@@ -413,68 +551,55 @@ la_status qr_blocked_factor(la_ctx ctx, double* A, size_t ld, int m, int n, doub
   const size_t pcap = part_doubles(ctx, m, dc, n, true);
   DevBuf vt(ctx), rsave(ctx), tau(ctx), part(ctx), wf(ctx), w2(ctx);
   LA_TRY(vt.alloc((size_t)QB * ldv));
-  LA_TRY(rsave.alloc((size_t)2 * QB * QB));  // alternating by block parity
+  LA_TRY(rsave.alloc((size_t)QB * QB));
   LA_TRY(tau.alloc(QB));
   LA_TRY(part.alloc(std::max<size_t>(pcap, 1)));
   LA_TRY(wf.alloc((size_t)QB * ldw));
   LA_TRY(w2.alloc((size_t)QB * ldw));
-  cudaStream_t ms = ctx->stream;
-  const bool look = ctx->lookahead != 0 && ctx->side_stream != nullptr;
-  auto panel = [&](int b, cudaStream_t s) {
-    const int j = b * QB;
+  DevBuf dig(ctx);
+  SplitWs ws;
+  LA_TRY(alloc_split(ctx, dig, m, n, &ws));
+  struct PdlScope {
+    la_ctx c;
+    ~PdlScope() { c->pdl_now = false; }
+  } scope{ctx};
+  ctx->pdl_now = ctx->pdl != 0;
+  for (int j = 0, b = 0; j < dc; j += QB, b++) {
+    const int nb = std::min(QB, dc - j), rows = m - j, ncols = n - j;
+    double* Aj = A + (size_t)j * ld + j;
     QrPanelArgs a;
     a.A = A;
     a.ld = ld;
     a.m = m;
     a.j = j;
-    a.nb = std::min(QB, dc - j);
-    a.rpc = (m - j + caps.cluster - 1) / caps.cluster;
+    a.nb = nb;
+    a.rpc = (rows + caps.cluster - 1) / caps.cluster;
     a.rdiag = rdiag;
     a.tau = tau.d();
     a.vt = vt.d();
     a.ldv = ldv;
-    a.rsave = rsave.d() + (size_t)(b & 1) * QB * QB;
-    return launch_qr_panel(ctx, a, caps.cluster, s);
-  };
-  // Lookahead (as in the mixed LU): once the next block's columns are
-  // updated, its panel runs on the side stream beside the update of the rest.
-  // The two touch disjoint columns; tau and V' are consumed before the fork
-  // and the top squares' saved content alternates between two buffers.
-  LA_TRY(panel(0, ms));
-  bool forked = false;
-  for (int j = 0, b = 0; j < dc; j += QB, b++) {
-    const int nb = std::min(QB, dc - j), rows = m - j, ncols = n - j;
-    const int nbn = j + nb < dc ? std::min(QB, dc - j - nb) : 0;  // the next block's width
-    double* Aj = A + (size_t)j * ld + j;
-    if (forked) {
-      LA_CUDA(ctx, cudaStreamWaitEvent(ms, ctx->ev_join, 0));
-      forked = false;
+    const bool tc = tc_block(ws, nb, rows, ncols - nb);
+    a.rsave = tc ? nullptr : rsave.d();
+    LA_TRY(launch_qr_panel(ctx, a, caps.cluster, ctx->stream));
+    double* gj = gram + (size_t)b * QB * QB;
+    // [G | W] = V' A[j:, j:]; W2 = T' W for the columns right of the block (G kept for get_q and
+    // solve); A[j:, j+nb:] -= V W2
+    if (tc) {
+      LA_TRY(apply_vt_tc(ctx, ws, vt.d(), ldv, rows, Aj, ld, ncols, QB, part.d(), pcap, wf.d(), ldw));
+      LA_TRY(launch_tsolve(ctx, wf.d(), ldw, tau.d(), nb, wf.d() + nb, ldw, ncols - nb, w2.d(), ldw,
+                           true, gj, true, vt.d(), ldv, Aj + nb, ld));
+      LA_TRY(launch_gemm_split(ctx, ctx->stream, -1, rows - QB, ncols - nb, nb, Aj + (size_t)QB * ld,
+                               ld, w2.d(), ldw, false, Aj + (size_t)QB * ld + nb, ld, false, ws.p,
+                               ws.bytes));
+      continue;
     }
-    // [G | W] = V' A[j:, j:]
     LA_TRY(apply_vt(ctx, vt.d(), ldv, nb, rows, Aj, ld, ncols, part.d(), pcap, wf.d(), ldw));
-    // W2 = T' W for the columns right of the block; G kept for get_q and solve
     LA_TRY(launch_tsolve(ctx, wf.d(), ldw, tau.d(), nb, wf.d() + nb, ldw, ncols - nb, w2.d(), ldw,
-                         true, gram + (size_t)b * QB * QB));
-    // A[j:, j+nb:] -= V W2: the next block's columns first when it runs ahead
-    // (an odd width would misalign the rest's operand: no split then)
-    const bool split = look && nbn > 0 && nbn % 2 == 0 && ncols - nb > nbn;
-    if (split) {
-      LA_TRY(launch_gemm(ctx, GM_FMA_SUB, rows, nbn, nb, Aj, ld, w2.d(), ldw, Aj + nb, ld));
-      LA_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ms));
-      LA_CUDA(ctx, cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0));
-      LA_TRY(panel(b + 1, ctx->side_stream));
-      LA_CUDA(ctx, cudaEventRecord(ctx->ev_join, ctx->side_stream));
-      forked = true;
-      LA_TRY(launch_gemm(ctx, GM_FMA_SUB, rows, ncols - nb - nbn, nb, Aj, ld, w2.d() + nbn, ldw,
-                         Aj + nb + nbn, ld));
-    } else {
-      if (ncols > nb)
-        LA_TRY(launch_gemm(ctx, GM_FMA_SUB, rows, ncols - nb, nb, Aj, ld, w2.d(), ldw, Aj + nb, ld));
-    }
-    LA_TRY(launch_copy2d(ctx, rsave.d() + (size_t)(b & 1) * QB * QB, QB, Aj, ld, nb, nb));
-    if (!split && nbn > 0) LA_TRY(panel(b + 1, ms));
+                         true, gj));
+    if (ncols > nb)
+      LA_TRY(launch_gemm(ctx, GM_FMA_SUB, rows, ncols - nb, nb, Aj, ld, w2.d(), ldw, Aj + nb, ld));
+    LA_TRY(launch_copy2d(ctx, rsave.d(), QB, Aj, ld, nb, nb));
   }
-  if (forked) LA_CUDA(ctx, cudaStreamWaitEvent(ms, ctx->ev_join, 0));
   return LA_OK;
 }
 
@@ -491,19 +616,39 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
   LA_TRY(part.alloc(std::max<size_t>(pcap, 1)));
   LA_TRY(wf.alloc((size_t)QB * ldw));
   LA_TRY(w2.alloc((size_t)QB * ldw));
+  // Digits of the products, where the columns are many (get_q).
+  DevBuf dig(ctx);
+  SplitWs ws;
+  if (cols >= 2 * QB) LA_TRY(alloc_split(ctx, dig, m, cols, &ws));
+  struct PdlScope {
+    la_ctx c;
+    ~PdlScope() { c->pdl_now = false; }
+  } scope{ctx};
+  ctx->pdl_now = ctx->pdl != 0;
   const int nblocks = (dc + QB - 1) / QB;
   for (int s = 0; s < nblocks; s++) {
     const int b = getq ? nblocks - 1 - s : s;
     const int j = b * QB, nb = std::min(QB, dc - j), rows = m - j;
     const int c0 = getq ? j : 0, ncols = cols - c0;
-    qr_build_v_kernel<<<blocks_of((size_t)rows * nb, 256), 256, 0, ctx->stream>>>(
-        A, ld, m, j, nb, rdiag, mode, vx.d(), vt.d(), ldv, tau.d());
+    const cudaError_t e =
+        la_launch(ctx, qr_build_v_kernel, dim3(blocks_of((size_t)rows * nb, 256)), dim3(256), 0,
+                  ctx->stream, A, ld, m, j, nb, rdiag, mode, vx.d(), vt.d(), ldv, tau.d());
+    if (e != cudaSuccess) return la_cuda_fail(ctx, e, "qr_build_v_kernel launch");
     ctx->launches++;
     LA_TRY(la_check_launch(ctx, "qr_build_v_kernel"));
     double* Tj = T + (size_t)j * ldt + c0;
+    const double* gj = gram + (size_t)b * QB * QB;
+    if (tc_block(ws, nb, rows, ncols)) {
+      LA_TRY(apply_vt_tc(ctx, ws, vt.d(), ldv, rows, Tj, ldt, ncols, 0, part.d(), pcap, wf.d(), ldw));
+      LA_TRY(launch_tsolve(ctx, gj, QB, tau.d(), nb, wf.d(), ldw, ncols, w2.d(), ldw, !getq, nullptr,
+                           true, vt.d(), ldv, Tj, ldt));
+      LA_TRY(launch_gemm_split(ctx, ctx->stream, -1, rows - QB, ncols, nb, vx.d() + (size_t)QB * QB,
+                               QB, w2.d(), ldw, false, Tj + (size_t)QB * ldt, ldt, false, ws.p,
+                               ws.bytes));
+      continue;
+    }
     LA_TRY(apply_vt(ctx, vt.d(), ldv, nb, rows, Tj, ldt, ncols, part.d(), pcap, wf.d(), ldw));
-    LA_TRY(launch_tsolve(ctx, gram + (size_t)b * QB * QB, QB, tau.d(), nb, wf.d(), ldw, ncols,
-                         w2.d(), ldw, !getq, nullptr));
+    LA_TRY(launch_tsolve(ctx, gj, QB, tau.d(), nb, wf.d(), ldw, ncols, w2.d(), ldw, !getq, nullptr));
     LA_TRY(launch_gemm(ctx, GM_FMA_SUB, rows, ncols, nb, vx.d(), QB, w2.d(), ldw, Tj, ldt));
   }
   return LA_OK;
