@@ -184,7 +184,7 @@ la_status la_ctx_create(int device, la_ctx* out) {
   off = align_up(off + (size_t)2 * MAX_PANEL_CTAS * MAX_PANEL_W * sizeof(double), 256);
   const size_t o_da = off; off = align_up(off + 2 * MAX_PANEL_W * sizeof(double), 256);
   const size_t o_ds = off; off = align_up(off + 2 * MAX_PANEL_W * sizeof(double), 256);
-  const size_t o_sw = off; off = align_up(off + (1 + 4 * MAX_PANEL_W) * sizeof(int), 256);
+  const size_t o_sw = off; off = align_up(off + SWAP_LISTS * SWAP_STRIDE * sizeof(int), 256);
   const size_t o_sm = off; off = align_up(off + 8 * sizeof(double), 256);
   const size_t o_sv = off; off = align_up(off + (2 + 2 * SOLVE_WAVE_MAX_GROUPS) * sizeof(int), 256);
   e = cudaMalloc(&ctx->d_scratch, off);

@@ -71,6 +71,10 @@ enum GemmMode : int {
 
 constexpr int MAX_PANEL_CTAS = 1024;
 constexpr int MAX_PANEL_W = 64;
+// Composed row moves of a panel: words of one list, and lists kept (the panels of one block of
+// columns and of the block before it, whose moves reach the columns outside the block later).
+constexpr int SWAP_STRIDE = 260;
+constexpr int SWAP_LISTS = 32;
 // Column groups (4 right-hand sides each) of the wavefront triangular solve;
 // more right-hand sides take the block-step solve.
 constexpr int SOLVE_WAVE_MAX_GROUPS = 1024;
@@ -130,7 +134,9 @@ struct la_context {
   double* d_cand_row = nullptr;  // [2][MAX_PANEL_CTAS][64]
   double* d_diag_a = nullptr;    // [2][64]
   double* d_diag_s = nullptr;    // [2][64]
-  int* d_swaps = nullptr;        // [1 + 2*128] composed row moves of one panel
+  int* d_swaps = nullptr;        // [SWAP_LISTS][SWAP_STRIDE] composed row moves of a panel each
+  int swap_list = 0;             // the list that panels write and launch_laswp* read next
+  int* swaps() const { return d_swaps + swap_list * SWAP_STRIDE; }
   double* d_small = nullptr;     // [8] small device results (det, flags)
   int* d_solve_sync = nullptr;   // [2 + 2*SOLVE_WAVE_MAX_GROUPS] wavefront solve tickets, progress
   // Workspace of the split products where nothing may be allocated (noalloc.cu); null: allocate.
@@ -266,15 +272,18 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t stream, double* A, siz
 // C -= A B or C = A B (mode GM_FMA_SUB, GM_FMA_ZERO) with tiles of 16 columns.
 la_status launch_gemm_narrow(la_ctx ctx, int mode, int M, int N, int K, const double* A, size_t lda,
                              const double* B, size_t ldb, double* C, size_t ldc);
-la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int n, int j0,
-                       int jb);
+// The row moves of panel [j0, j0 + jb) (the current list) on columns [c0, j0) and [j0 + jb, c1).
+la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int c0, int c1,
+                       int j0, int jb);
+// The row moves of `lists` panels, one after the other, starting with list first, on columns
+// [c0, c1).
+la_status launch_laswp_lists_f32(la_ctx ctx, float* A, size_t ld, int first, int lists, int c0,
+                                 int c1);
 la_status launch_trsm_rowpanel(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int j0,
                                int jb, int c_begin, int c_end);
 la_status launch_panel_f32(la_ctx ctx, cudaStream_t stream, float* A, size_t ld, int m, int j0,
                            int jb, int* d_ipiv, unsigned* bar_base);
-la_status launch_laswp_f32(la_ctx ctx, float* A, size_t ld, int n, int j0, int jb);
-la_status launch_laswp_seq_f32(la_ctx ctx, float* A, size_t ld, const int* ipiv, int k0, int k1,
-                               int c0, int c1);
+la_status launch_laswp_f32(la_ctx ctx, float* A, size_t ld, int c0, int c1, int j0, int jb);
 la_status launch_panel_cluster_f32(la_ctx ctx, float* A, size_t ld, int m, int j0, int jb,
                                    int* d_ipiv);
 la_status launch_trsm_rowpanel_f32(la_ctx ctx, float* A, size_t ld, int j0, int jb, int c_begin,

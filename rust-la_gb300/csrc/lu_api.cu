@@ -176,7 +176,7 @@ struct FastLu {
       LA_TRY(s);
       t.end(ctx->stream, b, PH_PANEL);
       b = t.begin(ctx->stream);
-      LA_TRY(launch_laswp(ctx, false, A, nullptr, ld, n, j0, jb));
+      LA_TRY(launch_laswp(ctx, false, A, nullptr, ld, 0, n, j0, jb));
       t.end(ctx->stream, b, PH_SWAP);
       if (j1 < b1) {
         b = t.begin(ctx->stream);
@@ -287,7 +287,7 @@ la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
     const int jb = std::min(W, kmin - j0);
     const int j1 = j0 + jb;
     size_t b = t.begin(ms);
-    LA_TRY(launch_laswp(ctx, exact, A, S.d(), ld, n, j0, jb));
+    LA_TRY(launch_laswp(ctx, exact, A, S.d(), ld, 0, n, j0, jb));
     t.end(ms, b, PH_SWAP);
     if (j1 < n) {
       b = t.begin(ms);

@@ -49,26 +49,33 @@ laswp_kernel(T* M0, T* M1, T* M2, size_t ld, int b0, int e0, int b1, int e1,
     if (ok) M[(size_t)dst[q] * ld + c] = tmp[q][threadIdx.x % SW_COLS];
 }
 
-// Row interchanges of pivot positions [k0, k1) (ipiv[k] = the row swapped with
-// row k, in order) on columns [c0, c1): one thread per column applies the swaps
-// in sequence (the panel's own composed moves are for the columns next to the
-// panel; this form serves columns whose swaps were deferred).
+// The moves of `lists` panels, one list after the other, on columns [c0, c1), whose swaps were
+// deferred to the end of their block: a list's sources are all in registers before its first
+// destination is written. Lists go through L2 one after the other, about a microsecond each; one
+// thread per column replaying the interchanges themselves took 141 us for 256 of them (n = 16384,
+// every pivot off the diagonal), each a dependent round trip. (In the FP64 LU, whose chain leaves
+// nothing to run beside it, deferring the swaps this way measured 2 to 3 % slower.)
 template <typename T>
-__global__ void laswp_seq_kernel(T* A, size_t ld, const int* __restrict__ ipiv, int k0, int k1,
-                                 int c0, int c1, const int* err) {
+__global__ void __launch_bounds__(256)
+laswp_lists_kernel(T* A, size_t ld, const int* __restrict__ swaps, int lists, int c0, int c1,
+                   const int* err) {
   la_pdl_wait();
   la_pdl_trigger();
-  const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= c1 || aborted(err)) return;  // no barrier in this kernel
-  for (int k = k0; k < k1; k++) {
-    const int p = ipiv[k];
-    if (p != k) {
-      T* a = A + (size_t)k * ld + c;
-      T* b = A + (size_t)p * ld + c;
-      const T t = *a;
-      *a = *b;
-      *b = t;
-    }
+  constexpr int G = 256 / SW_COLS, PER = 2 * MAX_PANEL_W / G;  // move groups, moves per thread
+  const int c = c0 + blockIdx.x * SW_COLS + threadIdx.x % SW_COLS;
+  const int g = threadIdx.x / SW_COLS;
+  const bool ok = c < c1 && !aborted(err);
+  for (int s = 0; s < lists; s++, swaps += SWAP_STRIDE) {
+    const int cnt = swaps[0];
+    T v[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+      if (ok && g + i * G < cnt) v[i] = A[(size_t)swaps[1 + 2 * MAX_PANEL_W + g + i * G] * ld + c];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+      if (ok && g + i * G < cnt) A[(size_t)swaps[1 + g + i * G] * ld + c] = v[i];
+    __syncthreads();
   }
 }
 
@@ -406,26 +413,37 @@ int grid_for(la_ctx ctx, size_t total) {
 
 template <typename T>
 la_status launch_laswp_t(la_ctx ctx, cudaStream_t stream, bool exact, T* A, T* S, size_t ld,
-                         int n, int j0, int jb) {
+                         int c0, int c1, int j0, int jb) {
   const int j1 = j0 + jb;
-  const int left = j0, right = n - j1;
+  const int left = j0 - c0, right = c1 - j1;
   const int gx = std::max((left + SW_COLS - 1) / SW_COLS, (right + SW_COLS - 1) / SW_COLS);
-  if (gx == 0) return LA_OK;
+  if (gx <= 0) return LA_OK;
   dim3 grid(gx, exact ? 3 : 2);
   const cudaError_t e = la_launch(ctx, laswp_kernel<T>, grid, dim3(256), 0, stream, A, A,
-                                  exact ? S : nullptr, ld, 0, j0, j1, n, j1, n,
-                                  (const int*)ctx->d_swaps, (const int*)ctx->d_err);
+                                  exact ? S : nullptr, ld, c0, j0, j1, c1, j1, c1,
+                                  (const int*)ctx->swaps(), (const int*)ctx->d_err);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "laswp_kernel launch");
   ctx->launches++;
   return la_check_launch(ctx, "laswp_kernel");
 }
 
-la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int n, int j0,
-                       int jb) {
-  return launch_laswp_t<double>(ctx, ctx->stream, exact, A, S, ld, n, j0, jb);
+la_status launch_laswp(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int c0, int c1,
+                       int j0, int jb) {
+  return launch_laswp_t<double>(ctx, ctx->stream, exact, A, S, ld, c0, c1, j0, jb);
 }
-la_status launch_laswp_f32(la_ctx ctx, float* A, size_t ld, int n, int j0, int jb) {
-  return launch_laswp_t<float>(ctx, ctx->stream, false, A, nullptr, ld, n, j0, jb);
+la_status launch_laswp_f32(la_ctx ctx, float* A, size_t ld, int c0, int c1, int j0, int jb) {
+  return launch_laswp_t<float>(ctx, ctx->stream, false, A, nullptr, ld, c0, c1, j0, jb);
+}
+la_status launch_laswp_lists_f32(la_ctx ctx, float* A, size_t ld, int first, int lists, int c0,
+                                 int c1) {
+  if (c1 <= c0 || lists <= 0) return LA_OK;
+  const cudaError_t e =
+      la_launch(ctx, laswp_lists_kernel<float>, dim3((c1 - c0 + SW_COLS - 1) / SW_COLS), dim3(256), 0,
+                ctx->stream, A, ld, (const int*)(ctx->d_swaps + first * SWAP_STRIDE), lists, c0, c1,
+                (const int*)ctx->d_err);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "laswp_lists_kernel launch");
+  ctx->launches++;
+  return la_check_launch(ctx, "laswp_lists_kernel");
 }
 la_status launch_trsm_block_f32(la_ctx ctx, float* A, size_t ld, int j0, int jbo, int c_begin,
                                 int c_end) {
@@ -442,17 +460,6 @@ la_status launch_trsm_block_f32(la_ctx ctx, float* A, size_t ld, int j0, int jbo
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "trsm_block_kernel launch");
   ctx->launches++;
   return la_check_launch(ctx, "trsm_block_kernel");
-}
-
-la_status launch_laswp_seq_f32(la_ctx ctx, float* A, size_t ld, const int* ipiv, int k0, int k1,
-                               int c0, int c1) {
-  if (k1 <= k0 || c1 <= c0) return LA_OK;
-  const cudaError_t e = la_launch(ctx, laswp_seq_kernel<float>, dim3((c1 - c0 + 255) / 256),
-                                  dim3(256), 0, ctx->stream, A, ld, ipiv, k0, k1, c0, c1,
-                                  (const int*)ctx->d_err);
-  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "laswp_seq_kernel launch");
-  ctx->launches++;
-  return la_check_launch(ctx, "laswp_seq_kernel");
 }
 
 template <typename T>

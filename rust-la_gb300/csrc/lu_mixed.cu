@@ -425,8 +425,11 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
   LA_CUDA(ctx, cudaMemsetAsync(d_stat, 0, 256, ms));
 
   // Inner panels of the outer panel [j0, j1o) on stream s; row swaps on the
-  // columns < climit only.
-  auto inner = [&](int j0, int j1o, int climit, cudaStream_t s) -> la_status {
+  // outer panel's own columns only (the others take them from the panel's
+  // lists, which alternate between two sets: the columns left of the panel
+  // take their swaps beside the next panel's chain).
+  auto lists_of = [&](int j0) { return j0 / WO % 2 * (SWAP_LISTS / 2); };
+  auto inner = [&](int j0, int j1o, cudaStream_t s) -> la_status {
     cudaStream_t saved = ctx->stream;
     ctx->stream = s;
     // panel, row swaps, triangular solve and rank-32 update follow one
@@ -436,12 +439,13 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
     for (int i0 = j0; i0 < j1o && st == LA_OK; i0 += WI) {
       const int ib = std::min(WI, j1o - i0);
       const int i1 = i0 + ib;
+      ctx->swap_list = lists_of(j0) + (i0 - j0) / WI;
       // One thread-block cluster holds the panel when it fits; else the
       // cooperative multi-CTA kernel.
       st = ctx->cluster_panels ? launch_panel_cluster_f32(ctx, A, ld, m, i0, ib, h->d_ipiv)
                                : LA_UNSUPPORTED;
       if (st == LA_UNSUPPORTED) st = launch_panel_f32(ctx, s, A, ld, m, i0, ib, h->d_ipiv, &bar_base);
-      if (st == LA_OK) st = launch_laswp_f32(ctx, A, ld, climit, i0, ib);
+      if (st == LA_OK) st = launch_laswp_f32(ctx, A, ld, j0, j1o, i0, ib);
       if (st == LA_OK && i1 < j1o) {
         // Two launches: fusing them into one (every CTA solving the small
         // triangle, then updating its rows from shared memory) measured 12.6 ms
@@ -554,19 +558,26 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
   // on an early return.
   struct PdlReset {
     la_ctx c;
-    ~PdlReset() { c->pdl_now = false; }
+    ~PdlReset() {
+      c->pdl_now = false;
+      c->swap_list = 0;
+    }
   } pdl_reset{ctx};
   // The first outer panel on the main stream.
-  LA_TRY(inner(0, std::min(WO, kmin), std::min(WO, kmin), ms));
+  LA_TRY(inner(0, std::min(WO, kmin), ms));
   for (int j0 = 0; j0 < kmin; j0 += WO) {
     const int j1o = std::min(j0 + WO, kmin);
-    if (j1o >= n) break;
+    const int lists = (j1o - j0 + WI - 1) / WI;
+    if (j1o >= n) {
+      LA_TRY(launch_laswp_lists_f32(ctx, A, ld, lists_of(j0), lists, 0, j0));
+      break;
+    }
     const int j2o = std::min(j1o + WO, kmin);  // the next outer panel [j1o, j2o)
     // This panel's swaps on the columns its inner panels left out, then the
     // next panel's columns: the serial part between the two chains, as
     // dependent launches (the rest of the update, after the fork, is not).
     ctx->pdl_now = ctx->pdl != 0;
-    LA_TRY(launch_laswp_seq_f32(ctx, A, ld, h->d_ipiv, j0, j1o, j1o, n));
+    LA_TRY(launch_laswp_lists_f32(ctx, A, ld, lists_of(j0), lists, j1o, n));
     LA_TRY(outer_trsm(j0, j1o, j1o, j2o));
     LA_TRY(update(j0, j1o, j1o, j2o, true));
     ctx->pdl_now = false;
@@ -576,7 +587,7 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
         LA_CUDA(ctx, cudaEventRecord(ctx->ev_fork, ms));
         LA_CUDA(ctx, cudaStreamWaitEvent(ss, ctx->ev_fork, 0));
       }
-      LA_TRY(inner(j1o, j2o, j2o, ss));
+      LA_TRY(inner(j1o, j2o, ss));
       forked = look;
     }
     if (j2o < n) {
@@ -585,6 +596,7 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
       LA_TRY(outer_trsm(j0, j1o, j2o, n));
       LA_TRY(update(j0, j1o, j2o, n, false));
     }
+    LA_TRY(launch_laswp_lists_f32(ctx, A, ld, lists_of(j0), lists, 0, j0));
     if (forked) {
       LA_CUDA(ctx, cudaEventRecord(ctx->ev_join, ss));
       LA_CUDA(ctx, cudaStreamWaitEvent(ms, ctx->ev_join, 0));

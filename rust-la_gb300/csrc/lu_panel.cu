@@ -382,7 +382,7 @@ la_status launch_panel_t(la_ctx ctx, cudaStream_t stream, bool exact, T* A, T* S
   p.cand_row = ctx->d_cand_row;
   p.diag_a = ctx->d_diag_a;
   p.diag_s = ctx->d_diag_s;
-  p.swaps = ctx->d_swaps;
+  p.swaps = ctx->swaps();
   p.cstride = ctx->cand_stride;
 
   void* args[] = {&p};

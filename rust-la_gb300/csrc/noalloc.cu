@@ -33,7 +33,7 @@ constexpr size_t NA_OFF_DIAGA = NA_OFF_CROW + (size_t)2 * NA_CTAS * MAX_PANEL_W 
 constexpr size_t NA_OFF_DIAGS = NA_OFF_DIAGA + 2 * MAX_PANEL_W * sizeof(double);
 constexpr size_t NA_OFF_SWAPS = NA_OFF_DIAGS + 2 * MAX_PANEL_W * sizeof(double);
 // Digits of an update of 2048 x 1024 elements (K = 64); larger ones go in pieces of whole tiles.
-constexpr size_t NA_OFF_SPLIT = NA_OFF_SWAPS + 4096;
+constexpr size_t NA_OFF_SPLIT = NA_OFF_SWAPS + (SWAP_LISTS * SWAP_STRIDE * sizeof(int) + 255) / 256 * 256;
 constexpr size_t NA_SPLIT_BYTES = (size_t)(2048 + 1024) * (64 * 16 + 16) + 16384;
 constexpr size_t NA_BYTES = NA_OFF_SPLIT + NA_SPLIT_BYTES;  // about 3.3 MB in total
 

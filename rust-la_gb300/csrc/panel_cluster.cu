@@ -557,7 +557,7 @@ la_status launch_reg(la_ctx ctx, float* A, size_t ld, int m, int j0, int jb, int
   a.jb = jb;
   a.rpc = rpc;
   a.ipiv = d_ipiv;
-  a.swaps = ctx->d_swaps;
+  a.swaps = ctx->swaps();
   a.err = ctx->d_err;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cluster);
@@ -654,7 +654,7 @@ la_status launch_panel_cluster_f32(la_ctx ctx, float* A, size_t ld, int m, int j
   a.jb = jb;
   a.rpc = rpc;
   a.ipiv = d_ipiv;
-  a.swaps = ctx->d_swaps;
+  a.swaps = ctx->swaps();
   a.err = ctx->d_err;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cluster);

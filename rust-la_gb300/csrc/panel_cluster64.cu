@@ -421,7 +421,7 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, size_t 
   a.stall = 0;
   if (ctx->inject_panel_stall > 0 && --ctx->inject_panel_stall == 0) a.stall = 1;
   a.ipiv = d_ipiv;
-  a.swaps = ctx->d_swaps;
+  a.swaps = ctx->swaps();
   a.err = ctx->d_err;
   a.wait_ns = ctx->wait_limit_us > 0 ? (unsigned long long)ctx->wait_limit_us * 1000ull : WAIT_NS;
   if (a.rpc <= 64) return launch_t<256, 4>(ctx, st, C, a);
