@@ -82,7 +82,7 @@ typedef enum la_option {
   LA_OPT_LOOKAHEAD = 5,
   /* 1 (default): the FP32 panels of the mixed LU and the panels of the FAST LU
    * run on one thread-block cluster (distributed shared memory); 0: the
-   * cooperative multi-CTA kernel. The FAST LU's results are the same bits. */
+   * cooperative multi-CTA kernel. The LU's results are the same bits. */
   LA_OPT_CLUSTER_PANEL = 6,
   /* Batch plans (read when a plan is built): largest Krylov basis (0-20) of
    * the GMRES-IR stage that a LA_BATCH_MIXED plan runs on a system whose

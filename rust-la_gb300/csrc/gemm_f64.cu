@@ -385,6 +385,11 @@ la_status launch_gemm(la_ctx ctx, int mode, int M, int N, int K, const double* A
             : launch_tma<GM_FMA_ZERO>(ctx, M, N, K, A, lda, B, ldb, C, ldc, min_smem);
     if (s != LA_UNSUPPORTED) return s;
   }
+  // The carry of the EXACT LU (two FP64 instructions per term): a 64 x 64 tile of 64 k keeps an SM
+  // busy for 132 us, so while there are few of them, tiles of 16 columns (33 us) share the work
+  // evenly (n = 1000: 54 us per update on average, one wide tile alone takes 132).
+  if (mode == GM_EXACT_ADD && (long long)((M + 63) / 64) * ((N + 63) / 64) < 6ll * ctx->sm_count)
+    return launch_bn<16>(ctx, mode, M, N, K, A, lda, B, ldb, C, ldc, min_smem);
   return launch_bn<64>(ctx, mode, M, N, K, A, lda, B, ldb, C, ldc, min_smem);
 }
 

@@ -80,26 +80,24 @@ laswp_lists_kernel(T* A, size_t ld, const int* __restrict__ swaps, int lists, in
 }
 
 // ---- row-panel triangular update: U12 = L11^{-1} A12 ----------------------
-// Rows [j0, j0+jb), columns [c_begin, c_end), one 32-column strip per CTA.
-// Column sweep over k (one barrier per k): row k is finished, then every row
-// i > k of the block takes its k-th term, i.e. each element receives its terms
-// in ascending k, like lu.rs:124-128 (EXACT: s += l*u, u = a - s) or with FMA.
+// Rows [j0, j0+jb), columns [c_begin, c_end), one 32-column strip per CTA (FP32
+// blocks wider than 32 rows). Column sweep over k (one barrier per k): row k is
+// finished, then every row i > k of the block takes its k-th term by FMA, i.e.
+// each element receives its terms in ascending k, like lu.rs:124-128.
 constexpr int TR_COLS = 32;
 constexpr int LP = MAX_PANEL_W + 1;  // padded row of the triangular block in shared memory
 template <typename T>
-constexpr size_t trsm_smem(bool exact) {
-  return (size_t)(MAX_PANEL_W * LP + MAX_PANEL_W * TR_COLS * (exact ? 2 : 1)) * sizeof(T);
+constexpr size_t trsm_smem() {
+  return (size_t)(MAX_PANEL_W * LP + MAX_PANEL_W * TR_COLS) * sizeof(T);
 }
 
-template <typename T, bool EXACT>
+template <typename T>
 __global__ void __launch_bounds__(256)
-trsm_rowpanel_kernel(T* A, const T* S, size_t ld, int j0, int jb, int c_begin, int c_end) {
+trsm_rowpanel_kernel(T* A, size_t ld, int j0, int jb, int c_begin, int c_end) {
   extern __shared__ __align__(16) double dsm_raw[];
   T* dsm = reinterpret_cast<T*>(dsm_raw);
   T(*L)[LP] = reinterpret_cast<T(*)[LP]>(dsm);
   T(*xa)[TR_COLS] = reinterpret_cast<T(*)[TR_COLS]>(dsm + MAX_PANEL_W * LP);
-  T(*xs)[TR_COLS] =
-      reinterpret_cast<T(*)[TR_COLS]>(dsm + MAX_PANEL_W * LP + MAX_PANEL_W * TR_COLS);
   const int tx = threadIdx.x % TR_COLS, ty = threadIdx.x / TR_COLS;  // ty 0..7
   const int c = c_begin + blockIdx.x * TR_COLS + tx;
   const bool ok = c < c_end;
@@ -110,43 +108,35 @@ trsm_rowpanel_kernel(T* A, const T* S, size_t ld, int j0, int jb, int c_begin, i
   for (int i = ty; i < jb; i += 8) {
     size_t off = (size_t)(j0 + i) * ld + c;
     xa[i][tx] = ok ? A[off] : T(0);
-    if (EXACT) xs[i][tx] = ok ? S[off] : T(0);
   }
   __syncthreads();
   for (int k = 0; k < jb; k++) {
-    if (EXACT && ty == (k & 7)) {
-      // Row k is complete (this thread applied all its earlier terms): u = a - s.
-      xa[k][tx] = __dsub_rn(xa[k][tx], xs[k][tx]);
-    }
     __syncthreads();
     const T uk = xa[k][tx];
-    for (int i = ty; i < jb; i += 8) {
-      if (i <= k) continue;
-      if (EXACT)
-        xs[i][tx] = __dadd_rn(xs[i][tx], __dmul_rn(L[i][k], uk));
-      else
-        xa[i][tx] = fma(-L[i][k], uk, xa[i][tx]);
-    }
+    for (int i = ty; i < jb; i += 8)
+      if (i > k) xa[i][tx] = fma(-L[i][k], uk, xa[i][tx]);
   }
   __syncthreads();
   if (ok)
     for (int i = ty; i < jb; i += 8) A[(size_t)(j0 + i) * ld + c] = xa[i][tx];
 }
 
-// FAST FP64 form, jb <= 64: 8 columns per CTA. With two FP64 FMAs per clock an SM needs 16 clocks
+// FP64 form, jb <= 64: 8 columns per CTA. With two FP64 FMAs per clock an SM needs 16 clocks
 // for one warp's FMA, so the 64 x 64 triangle costs 0.5 us a column and the strip's width sets the
 // latency: the 32-column CTAs of the kernel above took 49 us however few columns there were. Row k
 // is final when step k starts; the rows below take its term, neighbouring items (row, column) on
 // neighbouring threads, so that no lane idles but in the last warp. The same FMAs in the same
 // order as above, so the same bits.
+// EXACT: the running sums s from S, row k formed as a - s at its step, terms added unfused.
 constexpr int TC8 = 8;
 constexpr int TC8_T = 256;
+template <bool EXACT>
 __global__ void __launch_bounds__(TC8_T)
-trsm_cols8_kernel(double* A, size_t ld, int j0, int jb, int c_begin, int c_end) {
+trsm_cols8_kernel(double* A, const double* S, size_t ld, int j0, int jb, int c_begin, int c_end) {
   la_pdl_wait();
   la_pdl_trigger();
   __shared__ double L[MAX_PANEL_W][MAX_PANEL_W + 1];
-  __shared__ double x[MAX_PANEL_W][TC8];
+  __shared__ double x[MAX_PANEL_W][TC8], xs[EXACT ? MAX_PANEL_W : 1][TC8];
   const int tid = threadIdx.x, col = tid % TC8, r0 = tid / TC8;  // r0 0..31
   const int c = c_begin + blockIdx.x * TC8 + col;
   const bool ok = c < c_end;
@@ -154,11 +144,26 @@ trsm_cols8_kernel(double* A, size_t ld, int j0, int jb, int c_begin, int c_end) 
     const int i = idx / MAX_PANEL_W, k = idx % MAX_PANEL_W;
     if (k < i) L[i][k] = A[(size_t)(j0 + i) * ld + j0 + k];
   }
-  for (int i = r0; i < jb; i += TC8_T / TC8) x[i][col] = ok ? A[(size_t)(j0 + i) * ld + c] : 0.0;
+  for (int i = r0; i < jb; i += TC8_T / TC8) {
+    x[i][col] = ok ? A[(size_t)(j0 + i) * ld + c] : 0.0;
+    if (EXACT) xs[i][col] = ok ? S[(size_t)(j0 + i) * ld + c] : 0.0;
+  }
   __syncthreads();
+  if (EXACT) {
+    if (r0 == 0) x[0][col] = __dsub_rn(x[0][col], xs[0][col]);
+    __syncthreads();
+  }
   for (int k = 0; k + 1 < jb; k++) {
     const double u = x[k][col];
-    for (int i = k + 1 + r0; i < jb; i += TC8_T / TC8) x[i][col] = fma(-L[i][k], u, x[i][col]);
+    for (int i = k + 1 + r0; i < jb; i += TC8_T / TC8) {
+      if (EXACT) {
+        const double s = __dadd_rn(xs[i][col], __dmul_rn(L[i][k], u));
+        xs[i][col] = s;
+        if (i == k + 1) x[i][col] = __dsub_rn(x[i][col], s);  // its last term
+      } else {
+        x[i][col] = fma(-L[i][k], u, x[i][col]);
+      }
+    }
     __syncthreads();
   }
   if (ok)
@@ -388,21 +393,6 @@ __global__ void copy2d_kernel(const double* __restrict__ src, size_t lds, double
   }
 }
 
-// Dynamic shared memory above 48 KB needs an opt-in per kernel.
-cudaError_t configure_smem_attrs() {
-  static la_device_once once;
-  return once.run([](int) {
-    cudaError_t e = cudaFuncSetAttribute(trsm_rowpanel_kernel<double, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)trsm_smem<double>(true));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(trsm_rowpanel_kernel<float, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)trsm_smem<float>(false));
-    return e;
-  });
-}
-
 int grid_for(la_ctx ctx, size_t total) {
   size_t g = (total + 255) / 256;
   size_t cap = (size_t)ctx->sm_count * 8;
@@ -466,22 +456,19 @@ template <typename T>
 la_status launch_trsm_t(la_ctx ctx, bool exact, T* A, T* S, size_t ld, int j0, int jb,
                         int c_begin, int c_end) {
   if (c_end <= c_begin) return LA_OK;
-  if (sizeof(T) == 8 && !exact) {
+  if (sizeof(T) == 8) {
     const cudaError_t e =
-        la_launch(ctx, trsm_cols8_kernel, dim3((c_end - c_begin + TC8 - 1) / TC8), dim3(TC8_T), 0,
-                  ctx->stream, reinterpret_cast<double*>(A), ld, j0, jb, c_begin, c_end);
+        la_launch(ctx, exact ? trsm_cols8_kernel<true> : trsm_cols8_kernel<false>,
+                  dim3((c_end - c_begin + TC8 - 1) / TC8), dim3(TC8_T), 0, ctx->stream,
+                  reinterpret_cast<double*>(A), reinterpret_cast<const double*>(S), ld, j0, jb,
+                  c_begin, c_end);
     if (e != cudaSuccess) return la_cuda_fail(ctx, e, "trsm_cols8_kernel launch");
     ctx->launches++;
     return la_check_launch(ctx, "trsm_cols8_kernel");
   }
-  LA_CUDA(ctx, configure_smem_attrs());
   dim3 grid((c_end - c_begin + TR_COLS - 1) / TR_COLS);
-  if (exact)
-    trsm_rowpanel_kernel<T, true><<<grid, 256, trsm_smem<T>(true), ctx->stream>>>(A, S, ld, j0, jb,
-                                                                               c_begin, c_end);
-  else
-    trsm_rowpanel_kernel<T, false><<<grid, 256, trsm_smem<T>(false), ctx->stream>>>(
-        A, S, ld, j0, jb, c_begin, c_end);
+  trsm_rowpanel_kernel<float><<<grid, 256, trsm_smem<float>(), ctx->stream>>>(
+      reinterpret_cast<float*>(A), ld, j0, jb, c_begin, c_end);
   ctx->launches++;
   return la_check_launch(ctx, "trsm_rowpanel_kernel");
 }

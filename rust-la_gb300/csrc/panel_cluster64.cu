@@ -1,4 +1,4 @@
-// FP64 panel factorization (FAST arithmetic) on one thread-block cluster: columns
+// FP64 panel factorization on one thread-block cluster: columns
 // [j0, j0 + jb), jb <= 32, over rows [j0, m), with partial pivoting by the reference's
 // rule (src/decomp/lu.rs:132-160: the first row of maximal |v|, a NaN below the
 // diagonal never chosen, one on it never displaced).
@@ -17,6 +17,9 @@
 //   * An element takes its updates in ascending k by FMA and its multiplier as
 //     v * (1 / pivot), exactly the operations of lu_panel.cu's FAST form: the two
 //     kernels give the same bits.
+//   * EXACT keeps, per element, the original a and the running sum s of l_ik u_kj (unfused,
+//     ascending k, lu.rs:124-126), forms a - s when a column or a pivot row is reached, and
+//     divides by the pivot: the operations of lu_panel.cu's EXACT form.
 //   * Column c's updates are split: column c + 1 first, then the candidates of c + 1
 //     are found and pushed, and the other columns take their update while the push
 //     travels. A candidate row is therefore published one update behind, together
@@ -35,6 +38,7 @@
 // find and publish the candidate, 650 to push it, 250 to pick the winner, 350 to scale and
 // form the next column, and the update (64 clocks per FMA and warp of a sub-partition:
 // from 512 rows per CTA on it is half of the time).
+// EXACT, 24 to 1000 rows: 69 on average, against 188 for 32 columns of the cooperative kernel.
 //
 // Waits are bounded (2 s or LA_OPT_WAIT_LIMIT_US): a thread whose wait gives up
 // records DERR_PANEL_TIMEOUT, waits for nothing more and pushes nothing more, but
@@ -115,6 +119,7 @@ __device__ __forceinline__ int warp_best(unsigned long long key, int pos) {
 
 struct Panel64Args {
   double* A;
+  const double* S;  // EXACT: the running sums
   size_t ld;
   int m, j0, jb, rpc, vec, stall;
   int* ipiv;
@@ -130,13 +135,18 @@ struct __align__(16) PushSlot {
   double rcp, pad2;
 };
 
-// v[i] = fma(l, u[Q i], v[i]) for 1 <= i < n. A switch into the unrolled sequence: an FMA that a
+// FAST: v is the element, v - l u; EXACT: v is its running sum, v + l u.
+template <bool EXACT>
+__device__ __forceinline__ double term(double v, double l, double u) {
+  return EXACT ? __dadd_rn(v, __dmul_rn(l, u)) : fma(-l, u, v);
+}
+// v[i] = term(v[i], l, u[Q i]) for 1 <= i < n. A switch into the unrolled sequence: an FMA that a
 // predicate switches off takes the FP64 pipe as long as any other.
-template <int Q, int NV>
+template <int Q, int NV, bool EXACT>
 __device__ __forceinline__ void update_tail(double (&v)[NV], double l, const double* u, int n) {
 #define LA_U(i) \
   case (i) + 1: \
-    if ((i) < NV) v[(i) % NV] = fma(l, u[Q * (i)], v[(i) % NV]); \
+    if ((i) < NV) v[(i) % NV] = term<EXACT>(v[(i) % NV], l, u[Q * (i)]); \
     [[fallthrough]];
   switch (n) {
     LA_U(31) LA_U(30) LA_U(29) LA_U(28) LA_U(27) LA_U(26) LA_U(25) LA_U(24)
@@ -149,12 +159,13 @@ __device__ __forceinline__ void update_tail(double (&v)[NV], double l, const dou
 }
 
 // T threads with rows and one more warp, for the reciprocals.
-template <int T, int Q>
+template <int T, int Q, bool EXACT>
 __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel64Args p) {
   constexpr int NW = T / 32;
   constexpr int NV = PW / Q;  // values per thread: columns q, q + Q, ...
   __shared__ PushSlot recv[3][PMAXC];
-  __shared__ double wrow[2][NW][PW];
+  constexpr int NS = EXACT ? NV : 1;
+  __shared__ double wrow[2][NW][PW], wsum[EXACT ? 2 : 1][NW][EXACT ? PW : 1];
   __shared__ double wl[2][NW];  // the published row's multiplier of the previous column
   __shared__ unsigned long long wkey[2][NW];
   __shared__ int wpos[2][NW];
@@ -179,7 +190,7 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
   la_pdl_wait();
   la_pdl_trigger();
   bool live = *reinterpret_cast<volatile int*>(p.err) == 0;
-  double v[NV];
+  double v[NV], sm[NS];  // EXACT: a and s
   const int q = lane % Q, lr = tid / Q;
   int pos = tid < T && lr < nrows ? row0 + lr : -1;
   {
@@ -194,6 +205,11 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
     } else {
 #pragma unroll
       for (int i = 0; i < NV; i++) v[i] = pos >= 0 && q + Q * i < jb ? src[q + Q * i] : 0.0;
+    }
+    if (EXACT) {
+      const double* ssrc = p.S + (size_t)(pos >= 0 ? pos : p.j0) * p.ld + p.j0;
+#pragma unroll
+      for (int i = 0; i < NS; i++) sm[i] = pos >= 0 && q + Q * i < jb ? ssrc[q + Q * i] : 0.0;
     }
   }
 
@@ -217,13 +233,19 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
       // this warp's candidate of column c, its row one update behind
       if (warp < NW) {
         const bool mine = q == s && pos >= j;
-        const unsigned long long key = key_of(v[0], pos == j);
+        const unsigned long long key = key_of(EXACT ? __dsub_rn(v[0], sm[0]) : v[0], pos == j);
         const int src = warp_best(key, mine ? pos : -1);
         if (src >= 0 && lane / Q == src / Q) {
           double* dst = wrow[par][warp] + cb + q;
 #pragma unroll
           for (int i = 0; i < NV; i++)
             if (cb + Q * i < jb) dst[Q * i] = v[i];
+          if (EXACT) {
+            double* sdst = wsum[par % (EXACT ? 2 : 1)][warp] + cb + q;
+#pragma unroll
+            for (int i = 0; i < NS; i++)
+              if (cb + Q * i < jb) sdst[Q * i] = sm[i];
+          }
           if (lane == src) {
             wl[par][warp] = lp;
             wkey[par][warp] = key;
@@ -244,7 +266,13 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
         double t = 0.0;
         if (w >= 0 && lane >= c) {
           t = wrow[par][w][lane];
-          if (c > 0 && lane > c) t = fma(-wl[par][w], uprev[lane], t);
+          if (EXACT) {
+            double sl = wsum[par % (EXACT ? 2 : 1)][w][lane % (EXACT ? PW : 1)];
+            if (c > 0 && lane > c) sl = term<true>(sl, wl[par][w], uprev[lane]);
+            t = __dsub_rn(t, sl);
+          } else if (c > 0 && lane > c) {
+            t = term<false>(t, wl[par][w], uprev[lane]);
+          }
         }
         for (int to = warp; to < C; to += NW) {
           uint32_t bar = bar0 + slot * 8, dst = dst0 + slot * (uint32_t)sizeof(recv[0]);
@@ -265,7 +293,7 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
                 : "memory");
         }
       } else if (live) {
-        const double rcp = 1.0 / (w >= 0 ? wrow[par][w][c] : 1.0);
+        const double rcp = EXACT ? 1.0 : 1.0 / (w >= 0 ? wrow[par][w][c] : 1.0);
         if (lane < C)
           asm volatile(
               "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
@@ -280,10 +308,15 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
       }
       // the previous column's update of the columns after c, while the pushes travel
       if (act) {
-        const double l = -lp;
         const double* u = uprev + cb + q;
-        if (Q > 1 && s < Q - 1 && q > s) v[0] = fma(l, u[0], v[0]);
-        update_tail<Q, NV>(v, l, u, (jb - cb + Q - 1) / Q);  // slots with cb + Q i < jb
+        const int nt = (jb - cb + Q - 1) / Q;  // slots with cb + Q i < jb
+        if (EXACT) {
+          if (Q > 1 && s < Q - 1 && q > s) sm[0] = term<true>(sm[0], lp, u[0]);
+          update_tail<Q, NS, true>(sm, lp, u, nt);
+        } else {
+          if (Q > 1 && s < Q - 1 && q > s) v[0] = term<false>(v[0], lp, u[0]);
+          update_tail<Q, NV, false>(v, lp, u, nt);
+        }
       }
       if (live) live = wait_pushes(&rbar[slot], (uint32_t)((c / 3) & 1), p.err, p.wait_ns);
       live = __all_sync(0xffffffffu, live);
@@ -304,13 +337,25 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
       }
       // the multiplier, from the row's thread of column c to its others; a zero pivot (key 1)
       // leaves the column as it is
-      if (act && q == s && win.key != 1ull) v[0] = v[0] * win.rcp;
+      if (EXACT) {
+        if (act && q == s) {
+          const double x = __dsub_rn(v[0], sm[0]);
+          v[0] = win.key != 1ull ? x / u[c] : x;
+          sm[0] = 0.0;
+        }
+      } else if (act && q == s && win.key != 1ull) {
+        v[0] = v[0] * win.rcp;
+      }
       lp = Q == 1 ? v[0] : __shfl_sync(0xffffffffu, v[0], lane / Q * Q + s);
       if (act && c + 1 < jb) {
+        double(&x)[EXACT ? NS : NV] = [&]() -> double(&)[EXACT ? NS : NV] {
+          if constexpr (EXACT) return sm;
+          else return v;
+        }();
         if (s + 1 < Q) {
-          if (q == s + 1) v[0] = fma(-lp, u[c + 1], v[0]);
+          if (q == s + 1) x[0] = term<EXACT>(x[0], lp, u[c + 1]);
         } else if (q == 0) {
-          v[NV > 1 ? 1 : 0] = fma(-lp, u[c + 1], v[NV > 1 ? 1 : 0]);
+          x[1] = term<EXACT>(x[1], lp, u[c + 1]);
         }
       }
       uprev = u;
@@ -323,6 +368,12 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
 #pragma unroll
     for (int i = 0; i < NV - 1; i++) v[i] = v[i + 1];
     v[NV - 1] = t;
+    if (EXACT) {
+      const double ts = sm[0];
+#pragma unroll
+      for (int i = 0; i < NS - 1; i++) sm[i] = sm[i + 1];
+      sm[NS - 1] = ts;
+    }
   }
   const bool ok = __syncthreads_and(live ? 1 : 0) != 0;
   cluster_barrier();  // no CTA leaves while pushes into its shared memory may be in flight
@@ -333,7 +384,16 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
 #pragma unroll
     for (int i = 0; i < NV - 1; i++) v[i] = v[i + 1];
     v[NV - 1] = t;
+    if (EXACT) {
+      const double ts = sm[0];
+#pragma unroll
+      for (int i = 0; i < NS - 1; i++) sm[i] = sm[i + 1];
+      sm[NS - 1] = ts;
+    }
   }
+  if (EXACT)
+#pragma unroll
+    for (int i = 0; i < NS; i++) v[i] = __dsub_rn(v[i], sm[i]);
   if (pos >= 0) {
     double* dst = p.A + (size_t)pos * p.ld + p.j0;
     if (Q == 1 && p.vec && jb == PW) {
@@ -350,7 +410,7 @@ __global__ void __launch_bounds__(T + 32, 1) panel_cluster64_kernel(const Panel6
 }
 
 // CTAs per cluster: LA_UNSUPPORTED (nothing launched) where such a cluster cannot be resident.
-template <int T, int Q>
+template <int T, int Q, bool EXACT>
 la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   static unsigned ok_for[LA_MAX_DEVICES];  // bit C: a cluster of C CTAs can be resident
   static la_device_once once;
@@ -370,7 +430,7 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   cfg.attrs = at;
   once.run([](int d) {
     ok_for[d] = 0;
-    if (cudaFuncSetAttribute(panel_cluster64_kernel<T, Q>,
+    if (cudaFuncSetAttribute(panel_cluster64_kernel<T, Q, EXACT>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
       for (int c = 1; c <= PMAXC; c *= 2) {
         cudaLaunchAttribute ca;
@@ -384,7 +444,7 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
         q.attrs = &ca;
         q.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, panel_cluster64_kernel<T, Q>, &q) == cudaSuccess && n > 0)
+        if (cudaOccupancyMaxActiveClusters(&n, panel_cluster64_kernel<T, Q, EXACT>, &q) == cudaSuccess && n > 0)
           ok_for[d] |= 1u << c;
       }
     cudaGetLastError();
@@ -392,7 +452,7 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
   });
   if (!(ok_for[dev] >> C & 1u)) return LA_UNSUPPORTED;
   cfg.numAttrs = ctx->pdl_now ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, panel_cluster64_kernel<T, Q>, a);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, panel_cluster64_kernel<T, Q, EXACT>, a);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaLaunchKernelEx(panel_cluster64)");
   ctx->launches++;
   return LA_OK;
@@ -401,17 +461,19 @@ la_status launch_t(la_ctx ctx, cudaStream_t st, int C, const Panel64Args& a) {
 }  // namespace
 
 // Returns LA_UNSUPPORTED (nothing launched) when the panel does not fit one cluster: more than 32
-// columns or 8192 rows, or no such cluster on this device; the cooperative kernel takes it then.
-la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, size_t ld, int m, int j0,
-                                 int jb, int* d_ipiv) {
+// columns, 8192 rows or (EXACT, with twice the registers per element) 4096, or no such cluster on
+// this device; the cooperative kernel takes it then. S: the running sums of EXACT, else null.
+la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, const double* S, size_t ld,
+                                 int m, int j0, int jb, int* d_ipiv) {
   const int R = m - j0;
   if (R <= 0 || jb <= 0) return LA_OK;
-  if (jb > PW || R > PMAXC * 512) return LA_UNSUPPORTED;
+  if (jb > PW || R > PMAXC * (S ? 256 : 512)) return LA_UNSUPPORTED;
   // 32 rows per CTA until the cluster is full (R = 256: 51 us, with 128 rows per CTA 82)
   int C = 1;
   while (C < PMAXC && R > C * 32) C *= 2;
   Panel64Args a;
   a.A = A;
+  a.S = S;
   a.ld = ld;
   a.m = m;
   a.j0 = j0;
@@ -424,8 +486,13 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, size_t 
   a.swaps = ctx->swaps();
   a.err = ctx->d_err;
   a.wait_ns = ctx->wait_limit_us > 0 ? (unsigned long long)ctx->wait_limit_us * 1000ull : WAIT_NS;
-  if (a.rpc <= 64) return launch_t<256, 4>(ctx, st, C, a);
-  if (a.rpc <= 128) return launch_t<256, 2>(ctx, st, C, a);
-  if (a.rpc <= 256) return launch_t<256, 1>(ctx, st, C, a);
-  return launch_t<512, 1>(ctx, st, C, a);
+  if (S) {
+    if (a.rpc <= 64) return launch_t<256, 4, true>(ctx, st, C, a);
+    if (a.rpc <= 128) return launch_t<256, 2, true>(ctx, st, C, a);
+    return launch_t<512, 2, true>(ctx, st, C, a);
+  }
+  if (a.rpc <= 64) return launch_t<256, 4, false>(ctx, st, C, a);
+  if (a.rpc <= 128) return launch_t<256, 2, false>(ctx, st, C, a);
+  if (a.rpc <= 256) return launch_t<256, 1, false>(ctx, st, C, a);
+  return launch_t<512, 1, false>(ctx, st, C, a);
 }
