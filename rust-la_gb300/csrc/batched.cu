@@ -13,8 +13,7 @@
 //   integers and the final map is the permutation P (lu.rs:245-254);
 //   solves for B_i and writes X_i.
 // Per 16-column panel: the panel is staged in shared memory in the arithmetic
-// type, factored column by column (each thread owns rows, two barriers per
-// column), written back; U12 = L11^-1 A12 is solved with each column in
+// type, factored column by column in registers (panel_regs), written back; U12 = L11^-1 A12 is solved with each column in
 // registers; A22 -= L21 U12 is register-tiled (a thread holds 4x4 of A22 and
 // its rows of L21, all loads of a tile are issued before its FMAs).
 // The working matrix is stored in the system's factor precision: FP64 (plain
@@ -203,6 +202,147 @@ __device__ __forceinline__ void trailing_update(typename P::S* M, int p, const i
   }
 }
 
+// The best (largest key, then lowest position) of a warp's lanes with pos >= 0: its lane (some lane
+// has one). Keys of FP32 values fit 32 bits: one warp reduction, a second one only on ties.
+template <typename R>
+__device__ __forceinline__ int panel_best(unsigned long long key, int pos) {
+  const unsigned full = 0xffffffffu;
+  const bool in = pos >= 0;
+  const unsigned hi = in ? (sizeof(R) == 8 ? (unsigned)(key >> 32) : (unsigned)key) : 0u;
+  const unsigned mh = __reduce_max_sync(full, hi);
+  bool e = in && hi == mh;
+  unsigned who = __ballot_sync(full, e);
+  if (who & (who - 1)) {
+    if (sizeof(R) == 8) {
+      const unsigned lo = e ? (unsigned)key : 0u;
+      const unsigned ml = __reduce_max_sync(full, lo);
+      e = e && lo == ml;
+    }
+    const unsigned p = e ? (unsigned)pos : ~0u;
+    const unsigned mp = __reduce_min_sync(full, p);
+    who = __ballot_sync(full, e && p == mp);
+  }
+  return who ? __ffs(who) - 1 : 0;
+}
+
+// Factors the staged panel (prow rows, jb columns, staged row s of logical position s) with each
+// thread's RPT rows in registers, on the CTA's first W warps; staged rows hold the factors on return, perm the row at each
+// position, and rmap[0..jb) takes the row interchanges (prow <= 32 RPT W). The other warps skip it:
+// fewer warps with more rows each repeat less of a column's search, and one warp needs no barrier.
+//   Column jj sits in register slot 0 (the window moves by one slot per column, so there is one copy
+//   of the loop body and every register index is static). Each warp's best candidate writes its row
+//   to its place in st, one barrier, then every warp picks the winner from the warps' candidates and
+//   takes the pivot row from st. A row's multiplier goes to st as it is formed. Written as in the
+//   loop of block_lu that this replaces: the same operations on every value.
+//   What bounds it: the chain of one column (two warp reductions, a barrier, the reciprocal, the next
+//   column). With the rows in shared memory, a 64-bit shuffle tree and a serial scan of the warps'
+//   candidates, a column took 3700 clocks in FP32 (n up to 512, two CTAs per SM) and 4500 in FP64 (n up
+//   to 256); now 1900 and 2800, at four to five clocks per instruction of a warp.
+template <typename R, int RPT>
+__device__ __forceinline__ void panel_regs(R* st, int prow, int jb, int W, int* perm, int* rmap,
+                                        Shared* shp) {
+  Shared& sh = *shp;
+  const unsigned full = 0xffffffffu;
+  const int BT = 32 * W;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  R v[RPT][PBW];
+  int pos[RPT];  // logical position relative to the panel's first row; -1: no row
+#pragma unroll
+  for (int t = 0; t < RPT; t++) {
+    const int s = tid + BT * t;
+    pos[t] = s < prow ? s : -1;
+#pragma unroll
+    for (int c = 0; c < PBW; c++) v[t][c] = s < prow && c < jb ? st[s * SP + c] : R(0);
+  }
+#pragma unroll 1
+  for (int jj = 0; jj < jb; jj++) {
+    const int par = jj & 1, left = jb - jj;
+    unsigned long long bk = 0ull;
+    int bp = -1, bt = 0;
+#pragma unroll
+    for (int t = 0; t < RPT; t++)
+      if (pos[t] >= jj) {
+        const unsigned long long k = bkey<R>(v[t][0], pos[t], jj);
+        if (bbetter(k, pos[t], bk, bp)) { bk = k; bp = pos[t]; bt = t; }
+      }
+    const int src = panel_best<R>(bk, bp);
+    const int sbt = __shfl_sync(full, bt, src), sbp = __shfl_sync(full, bp, src);
+    int bs = 32 * warp + src + BT * sbt;
+    if (lane == src) {
+      sh.rk[par][warp] = bk;
+      sh.rp[par][warp] = bp;
+      sh.rs[par][warp] = bs;
+    }
+#pragma unroll
+    for (int t = 0; t < RPT; t++)
+      if (sbp >= 0 && sbt == t && lane == src) {
+        R* row = st + bs * SP + jj;
+#pragma unroll
+        for (int i = 0; i < PBW; i++)
+          if (i < left) row[i] = v[t][i];
+      }
+    bp = sbp;  // >= jj with one warp: the row at position jj always has a key
+    if (W > 1) {
+      asm volatile("bar.sync 1, %0;" ::"r"(BT) : "memory");
+      const unsigned long long wk = lane < W ? sh.rk[par][lane] : 0ull;
+      const int wp = lane < W ? sh.rp[par][lane] : -1;
+      const int w = panel_best<R>(wk, wp);
+      bp = __shfl_sync(full, wp, w);
+      bs = sh.rs[par][w];
+    } else {
+      __syncwarp();
+    }
+    const R* prow_v = st + bs * SP;
+    R u[PBW];
+#pragma unroll
+    for (int i = 0; i < PBW; i++) u[i] = prow_v[min(jj + i, PBW - 1)];
+    const R d = u[0];
+    const R sc = d != R(0) ? R(1) / d : R(1);
+    R l[RPT];
+    bool any = false;
+#pragma unroll
+    for (int t = 0; t < RPT; t++) {
+      const int s = tid + BT * t;
+      if (pos[t] == jj) pos[t] = bp;  // the row displaced from position jj goes to bp
+      if (s == bs) pos[t] = jj;
+      l[t] = R(0);
+      if (pos[t] > jj) {
+        l[t] = d != R(0) ? v[t][0] * sc : v[t][0];
+        st[s * SP + jj] = l[t];
+        any = true;
+      }
+    }
+    // Rows without a place below the pivot (finished ones) take no update that is read again.
+    // FP64: a switch into the unrolled sequence, since an FMA of columns beyond the panel would take
+    // the FP64 pipe like any other.
+#define LA_U(i)                                                                       \
+  case (i) + 1:                                                                       \
+    _Pragma("unroll") for (int t = 0; t < RPT; t++) v[t][i] = fma(-l[t], u[i], v[t][i]); \
+    [[fallthrough]];
+    if (any) {
+      switch (sizeof(R) == 8 ? left : PBW) {
+        LA_U(15) LA_U(14) LA_U(13) LA_U(12) LA_U(11) LA_U(10) LA_U(9) LA_U(8)
+        LA_U(7) LA_U(6) LA_U(5) LA_U(4) LA_U(3) LA_U(2) LA_U(1)
+        default: break;
+      }
+    }
+#undef LA_U
+#pragma unroll
+    for (int t = 0; t < RPT; t++)
+#pragma unroll
+      for (int i = 0; i + 1 < PBW; i++) v[t][i] = v[t][i + 1];
+    if (tid == 0 && bp != jj) {
+      const int t = perm[jj];
+      perm[jj] = perm[bp];
+      perm[bp] = t;
+      const int r = rmap[jj];
+      rmap[jj] = rmap[bp];
+      rmap[bp] = r;
+    }
+    if (W == 1) __syncwarp();  // the next candidate's row is written after every lane has read this one
+  }
+}
+
 // Blocked right-looking LU with partial pivoting of M (n x n, pitch p, rows
 // addressed through rmap: logical row i is physical row rmap[i]). On return
 // rmap[i] = the original row now at position i (the reference's piv).
@@ -237,94 +377,110 @@ __device__ void block_lu(typename P::S* M, int p, int n, int* rmap, typename P::
   __syncthreads();
   for (int j0 = 0; j0 < n; j0 += PBW) {
     const int jb = min(PBW, n - j0), j1 = j0 + jb, prow = n - j0;
-    for (int idx = tid; idx < prow * jb; idx += BT) {
-      const int r = idx / jb, c = idx - r * jb;
-      st[r * SP + c] = P::ld(&M[(size_t)rmap[j0 + r] * p + j0 + c]);
+    S* const Mp = M + j0;  // the panel
+    for (int idx = tid; idx < prow * PBW; idx += BT) {
+      const int r = idx / PBW, c = idx % PBW;
+      if (c < jb) st[r * SP + c] = P::ld(&Mp[(size_t)rmap[j0 + r] * p + c]);
     }
     for (int r = tid; r < prow; r += BT) {
       perm[r] = r;
       spos[r] = r;
     }
     __syncthreads();
-    for (int jj = 0; jj < jb; jj++) {
-      const int par = jj & 1;
-      unsigned long long bk = 0ull;
-      int bp = -1, bs = -1;
-      for (int s = tid; s < prow; s += BT) {
-        const int ps = spos[s];
-        if (ps >= jj) {
-          const unsigned long long k = bkey<R>(st[s * SP + jj], ps, jj);
-          if (bbetter(k, ps, bk, bp)) { bk = k; bp = ps; bs = s; }
-        }
+    // Warps and rows per thread of the panel. FP32: four rows per thread from 65 rows on. FP64: the
+    // updates take the FP64 pipes, so the rows go over as many warps as there are. Beyond four rows per
+    // thread (two-warp CTAs with n > 256) they stay in st.
+    const int rpt = sizeof(R) == 8 ? (prow + BT - 1) / BT : (prow + 31) / 32;
+    const int PR = rpt <= 1 ? 1 : 2, W = (prow + 32 * PR - 1) / (32 * PR);
+    if (W <= NW) {
+      if (warp >= W) {
+        // at the barrier below
+      } else if (PR == 1) {
+        panel_regs<R, 1>(st, prow, jb, W, perm, rmap + j0, &sh);
+      } else {
+        panel_regs<R, 2>(st, prow, jb, W, perm, rmap + j0, &sh);
       }
-      for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long ok = __shfl_down_sync(0xffffffffu, bk, off);
-        const int op = __shfl_down_sync(0xffffffffu, bp, off);
-        const int os = __shfl_down_sync(0xffffffffu, bs, off);
-        if (bbetter(ok, op, bk, bp)) { bk = ok; bp = op; bs = os; }
-      }
-      if (lane == 0) { sh.rk[par][warp] = bk; sh.rp[par][warp] = bp; sh.rs[par][warp] = bs; }
       __syncthreads();
-      bk = sh.rk[par][0];
-      bp = sh.rp[par][0];
-      bs = sh.rs[par][0];
-      for (int w = 1; w < NW; w++)
-        if (bbetter(sh.rk[par][w], sh.rp[par][w], bk, bp)) {
-          bk = sh.rk[par][w]; bp = sh.rp[par][w]; bs = sh.rs[par][w];
+    } else {
+      for (int jj = 0; jj < jb; jj++) {
+        const int par = jj & 1;
+        unsigned long long bk = 0ull;
+        int bp = -1, bs = -1;
+        for (int s = tid; s < prow; s += BT) {
+          const int ps = spos[s];
+          if (ps >= jj) {
+            const unsigned long long k = bkey<R>(st[s * SP + jj], ps, jj);
+            if (bbetter(k, ps, bk, bp)) { bk = k; bp = ps; bs = s; }
+          }
         }
-      // bp >= jj: the row at position jj always has a key.
-      const R* prow_v = st + bs * SP;
-      const R d = prow_v[jj];
-      const R sc = d != R(0) ? R(1) / d : R(1);
-      for (int s = tid; s < prow; s += BT) {
-        int ps = spos[s];
-        if (s == bs) {
-          spos[s] = jj;
-          continue;
+        for (int off = 16; off > 0; off >>= 1) {
+          const unsigned long long ok = __shfl_down_sync(0xffffffffu, bk, off);
+          const int op = __shfl_down_sync(0xffffffffu, bp, off);
+          const int os = __shfl_down_sync(0xffffffffu, bs, off);
+          if (bbetter(ok, op, bk, bp)) { bk = ok; bp = op; bs = os; }
         }
-        if (ps == jj) {  // the row displaced from position jj goes to bp
-          ps = bp;
-          spos[s] = bp;
+        if (lane == 0) { sh.rk[par][warp] = bk; sh.rp[par][warp] = bp; sh.rs[par][warp] = bs; }
+        __syncthreads();
+        bk = sh.rk[par][0];
+        bp = sh.rp[par][0];
+        bs = sh.rs[par][0];
+        for (int w = 1; w < NW; w++)
+          if (bbetter(sh.rk[par][w], sh.rp[par][w], bk, bp)) {
+            bk = sh.rk[par][w]; bp = sh.rp[par][w]; bs = sh.rs[par][w];
+          }
+        // bp >= jj: the row at position jj always has a key.
+        const R* prow_v = st + bs * SP;
+        const R d = prow_v[jj];
+        const R sc = d != R(0) ? R(1) / d : R(1);
+        for (int s = tid; s < prow; s += BT) {
+          int ps = spos[s];
+          if (s == bs) {
+            spos[s] = jj;
+            continue;
+          }
+          if (ps == jj) {  // the row displaced from position jj goes to bp
+            ps = bp;
+            spos[s] = bp;
+          }
+          if (ps > jj) {
+            R* row = st + s * SP;
+            const R l = d != R(0) ? row[jj] * sc : row[jj];
+            row[jj] = l;
+            for (int c = jj + 1; c < jb; c++) row[c] = fma(-l, prow_v[c], row[c]);
+          }
         }
-        if (ps > jj) {
-          R* row = st + s * SP;
-          const R l = d != R(0) ? row[jj] * sc : row[jj];
-          row[jj] = l;
-          for (int c = jj + 1; c < jb; c++) row[c] = fma(-l, prow_v[c], row[c]);
+        if (tid == 0 && bp != jj) {
+          const int t = perm[jj];
+          perm[jj] = perm[bp];
+          perm[bp] = t;
+          const int u = rmap[j0 + jj];
+          rmap[j0 + jj] = rmap[j0 + bp];
+          rmap[j0 + bp] = u;
         }
       }
-      if (tid == 0 && bp != jj) {
-        const int t = perm[jj];
-        perm[jj] = perm[bp];
-        perm[bp] = t;
-        const int u = rmap[j0 + jj];
-        rmap[j0 + jj] = rmap[j0 + bp];
-        rmap[j0 + bp] = u;
-      }
+      __syncthreads();
     }
-    __syncthreads();
-    for (int idx = tid; idx < prow * jb; idx += BT) {
-      const int r = idx / jb, c = idx - r * jb;
-      R* sv = st + perm[r] * SP + c;
-      const S v = P::cv(*sv);
-      M[(size_t)rmap[j0 + r] * p + j0 + c] = v;
-      *sv = P::up(v);
+    for (int idx = tid; idx < prow * PBW; idx += BT) {
+      const int r = idx / PBW, c = idx % PBW;
+      if (c < jb) {
+        R* sv = st + perm[r] * SP + c;
+        const S v = P::cv(*sv);
+        Mp[(size_t)rmap[j0 + r] * p + c] = v;
+        *sv = P::up(v);
+      }
     }
     if (j1 >= n) break;  // uniform; jb == PBW below
     const int nr = n - j1;
-    for (int idx = tid; idx < PBW * nr; idx += BT) {
-      const int k = idx / nr, c = idx - k * nr;
-      us[k * nr + c] = P::ld(&M[(size_t)rmap[j0 + k] * p + j1 + c]);
-    }
     __syncthreads();
     {
       const R* l11[PBW];
 #pragma unroll
       for (int i = 0; i < PBW; i++) l11[i] = st + perm[i] * SP;
       for (int c = tid; c < nr; c += BT) {
+        S* const mc = M + j1 + c;
         R u[PBW];
 #pragma unroll
-        for (int k = 0; k < PBW; k++) u[k] = us[k * nr + c];
+        for (int k = 0; k < PBW; k++) u[k] = P::ld(&mc[(size_t)rmap[j0 + k] * p]);
 #pragma unroll
         for (int k = 0; k < PBW; k++)
 #pragma unroll
@@ -332,7 +488,7 @@ __device__ void block_lu(typename P::S* M, int p, int n, int* rmap, typename P::
 #pragma unroll
         for (int k = 0; k < PBW; k++) {
           const S v = P::cv(u[k]);
-          M[(size_t)rmap[j0 + k] * p + j1 + c] = v;
+          mc[(size_t)rmap[j0 + k] * p] = v;
           us[k * nr + c] = P::up(v);
         }
       }
@@ -349,95 +505,242 @@ __device__ void block_lu(typename P::S* M, int p, int n, int* rmap, typename P::
   __syncthreads();
 }
 
-// One row of a block step of the triangular solves: x_i -= f * X_blk over all
-// nrhs right-hand sides, with the row's kbn (<= 16) factor entries f loaded
-// once (16 independent loads in flight) and the block's solved values X_blk
-// read from shared memory (the same address across the warp: a broadcast).
-template <typename P, typename TX>
-__device__ __forceinline__ void solve_row_update(const typename P::S* frow, int kbn, TX* xi,
-                                                 const TX* xblk, int nrhs) {
-  TX f[16];
-#pragma unroll
-  for (int k = 0; k < 16; k++) f[k] = k < kbn ? (TX)P::ld(&frow[k]) : TX(0);
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    if (c < nrhs) {
-      TX s = xi[c];
-#pragma unroll
-      for (int k = 0; k < 16; k++)
-        if (k < kbn) s = fma(-f[k], xblk[k * nrhs + c], s);
-      xi[c] = s;
-    }
+// Whether |v| is far from both ends of the range, so that products with another such value and the
+// remainders below are exact where they have to be.
+template <typename T>
+__device__ __forceinline__ bool mid_range(T v) {
+  if constexpr (sizeof(T) == 8) {
+    const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+    return e - 523u < 1000u;  // 2^-500 .. 2^500
+  } else {
+    const unsigned e = (__float_as_uint(v) >> 23) & 0xffu;
+    return e - 77u < 100u;  // 2^-50 .. 2^50
   }
 }
 
+// Factor entries M(row_i, kb + k), k < kbn <= 16, for slots i < cnt of 2 N rows r0 + dir i: half a warp
+// reads one row, so a warp's load touches two lines (by one row per lane it touched 32).
+template <typename P, int N, typename TX>
+__device__ __forceinline__ void solve_fetch(TX (&t)[N], const typename P::S* M, int n,
+                                            const int* rmap, int r0, int dir, int cnt, int kb,
+                                            int kbn) {
+  const int k = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    const int i = 2 * j + h;
+    t[j] = i < cnt && k < kbn ? (TX)P::ld(&M[rmap[r0 + dir * i] * n + kb + k]) : TX(0);
+  }
+}
+// ... to shared memory, slot i at tr + i SP.
+template <int N, typename TX>
+__device__ __forceinline__ void solve_stage(TX* tr, const TX (&t)[N], int cnt) {
+  const int k = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
+#pragma unroll
+  for (int j = 0; j < N; j++)
+    if (2 * j + h < cnt) tr[(2 * j + h) * SP + k] = t[j];
+}
+
+// One diagonal block (16 rows, lane li = row, half a warp per right-hand side), dg = the lane's row of
+// it, d and r its diagonal entry and the reciprocal. FULL: 16 rows. UPPER: x / d without a division on
+// the chain: q = x r, then one correction with the exact remainder x - q d (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990). Returns whether every quotient of
+// an active lane was in the range where that holds.
+template <typename TX, bool UPPER, bool FULL>
+__device__ __forceinline__ bool solve_diag(const TX (&dg)[16], TX d, TX r, int kbn, bool act, TX& x) {
+  const int lane = threadIdx.x & 31, li = lane & 15;
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const int k = UPPER ? 15 - i : i;
+    if (FULL || k < kbn) {  // uniform
+      if (UPPER) {
+        const TX q = x * r, y = fma(fma(-q, d, x), r, q);
+        if (li == k) x = y;
+      }
+      const TX xk = __shfl_sync(0xffffffffu, x, (lane & 16) | k);
+      if (UPPER ? li < k : li > k) x = fma(-dg[k], xk, x);
+    }
+  }
+  return !UPPER || !act || (mid_range(d) && (x == TX(0) || mid_range(x)));
+}
+
 // X (n x nrhs, pitch nrhs, already in the factor's row order, i.e. P b)
-// <- U^-1 L^-1 X with the stored factors in M. 16-row blocks: warp 0 solves
-// the diagonal block (lanes = rows, two right-hand sides per pass, values
-// passed by shuffles), then all threads update the remaining rows.
-template <typename P, typename TX>
-__device__ void block_solve(const typename P::S* M, int p, int n, const int* rmap, TX* X,
-                            int nrhs) {
-  const int BT = blockDim.x;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// <- U^-1 L^-1 X with the stored factors in M, by blocks of 16 rows. Warp 0
+// carries the chain: block b's diagonal solve, and the update of block b + 1's
+// rows by it, in registers. Warp 1 brings the two 16 x 16 tiles that warp 0
+// needs next into shared memory (buf, the staging space of the factorization,
+// free by now: the tiles behind the warps' own pieces), its loads issued a
+// block ahead. The other warps update all later rows, one block behind, their
+// loads issued a pass ahead. One barrier per block.
+// What bounds it: warp 0's instructions, a few hundred per block at four to
+// five clocks each. With loads, both updates and a division per row in its
+// path a block took 6200 clocks (FP32, n = 264, one CTA alone on its SM), now 4100; 5400 and 3000 at
+// n = 128. FP64, batches of n up to 256: the solves' share of the SM time 1.67 -> 0.73 G clocks.
+// Not inlined: spills cost an L2 round trip each here, since shared memory
+// leaves the L1 next to nothing.
+template <typename P, typename TX, bool UPPER>
+__device__ __noinline__ void block_tri(const typename P::S* M, int n, const int* rmap, TX* X,
+                                       int nrhs, TX* buf) {
+  constexpr int TILE = 16 * SP;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = blockDim.x >> 5;
   const int li = lane & 15, half = lane >> 4;
-  for (int kb = 0; kb < n; kb += 16) {
-    const int kbn = min(16, n - kb);
-    if (warp == 0) {
-      // lane's row of the diagonal block in registers (16 loads in flight)
-      const typename P::S* lrow = M + (size_t)rmap[kb + min(li, kbn - 1)] * p + kb;
-      TX lv[16];
+  const int nblk = (n + 15) / 16;
+  // buf holds 33 n values: (n - 17) SP for the passes of warps 1.. (at most n - 17 rows lie beyond the
+  // first two blocks, backward with a first block of one row), and two sets of two tiles and 16
+  // reciprocals, which need n >= 52. In smaller systems, and in CTAs of two warps, warp 0 reads M
+  // itself and warp 1 updates rows too.
+  const bool direct = n < 52 || NW < 4;
+  const int R0 = direct ? 1 : 2, NR = NW - R0;  // the warps that update rows
+  TX* const slots = buf + (n - 17) * SP;
+  TX* const tr = buf + (warp - R0) * 32 * SP;
+  auto block_at = [&](int b) { return 16 * (UPPER ? nblk - 1 - b : b); };
+  auto width_at = [&](int kb) { return min(16, n - kb); };
+  auto slot_at = [&](int par) { return slots + (par & 1) * (2 * TILE + 16); };
+  // rows beyond block b and the one after it
+  auto beyond = [&](int b) {
+    return b + 1 < nblk ? (UPPER ? block_at(b + 1) : n - block_at(b + 1) - width_at(block_at(b + 1))) : 0;
+  };
+  auto row_at = [&](int b, int r) {
+    const int k1 = block_at(b + 1);
+    return UPPER ? k1 - 1 - r : k1 + width_at(k1) + r;
+  };
+  auto barrier = [&] { asm volatile("bar.sync 0;" ::: "memory"); };  // one per block in both roles
+  if (warp == 0) {
+    TX dg[16], d = TX(1), rcp = TX(1), x0 = TX(0), x1 = TX(0);
+    barrier();
+#pragma unroll 1
+    for (int b = 0; b < nblk; b++) {
+      const int kb = block_at(b), kbn = width_at(kb), i = min(li, kbn - 1);
+      const bool a0 = li < kbn && half < nrhs, a1 = li < kbn && half + 2 < nrhs;
+      TX* const xr = X + (kb + li) * nrhs + half;
+      x0 = a0 ? xr[0] : TX(0);
+      x1 = a1 ? xr[2] : TX(0);
+      const typename P::S* const row = M + rmap[kb + i] * n;  // the lane's row of the factors
+      if (b > 0) {  // its terms of the previous block
+        const int kp = block_at(b - 1), np = width_at(kp);
+        const TX* const xblk = X + kp * nrhs;
+        const int c0 = min(half, nrhs - 1), c1 = min(half + 2, nrhs - 1);
+        if (direct) {
 #pragma unroll
-      for (int k = 0; k < 16; k++) lv[k] = k < kbn ? (TX)P::ld(&lrow[k]) : TX(0);
-      for (int c0 = 0; c0 < nrhs; c0 += 2) {
-        const int c = c0 + half;
-        const bool act = li < kbn && c < nrhs;
-        TX xi = act ? X[(kb + li) * nrhs + c] : TX(0);
+          for (int k = 0; k < 16; k++) dg[k] = k < np ? (TX)P::ld(&row[kp + k]) : TX(0);
+        } else {
+          const TX* sl = slot_at(b - 1) + TILE + i * SP;
 #pragma unroll
-        for (int k = 0; k < 15; k++) {
-          if (k + 1 < kbn) {
-            const TX xk = __shfl_sync(0xffffffffu, xi, (lane & 16) | k);
-            if (act && li > k) xi = fma(-lv[k], xk, xi);
+          for (int k = 0; k < 16; k++) dg[k] = sl[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+          if (k < np) {
+            x0 = fma(-dg[k], xblk[k * nrhs + c0], x0);
+            if (nrhs > 2) x1 = fma(-dg[k], xblk[k * nrhs + c1], x1);
+          }
+      }
+      if (direct) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) dg[k] = k < kbn ? (TX)P::ld(&row[kb + k]) : TX(0);
+        if (UPPER) d = (TX)P::ld(&row[kb + i]), rcp = TX(1) / d;
+      } else {
+        const TX* sl = slot_at(b - 1);
+#pragma unroll
+        for (int k = 0; k < 16; k++) dg[k] = sl[i * SP + k];
+        if (UPPER) d = sl[i * SP + i], rcp = sl[2 * TILE + i];
+      }
+      const TX v0 = x0, v1 = x1;
+      bool ok;
+      if (kbn == 16) {
+        ok = solve_diag<TX, UPPER, true>(dg, d, rcp, 16, a0, x0);
+        if (nrhs > 2) ok &= solve_diag<TX, UPPER, true>(dg, d, rcp, 16, a1, x1);
+      } else {
+        ok = solve_diag<TX, UPPER, false>(dg, d, rcp, kbn, a0, x0);
+        if (nrhs > 2) ok &= solve_diag<TX, UPPER, false>(dg, d, rcp, kbn, a1, x1);
+      }
+      if (UPPER && __any_sync(0xffffffffu, !ok)) {  // with divisions
+        x0 = v0;
+        x1 = v1;
+#pragma unroll 1
+        for (int k = kbn - 1; k >= 0; k--) {
+          const TX f = (TX)P::ld(&row[kb + k]);
+          if (li == k) x0 = x0 / f, x1 = x1 / f;
+          const TX y0 = __shfl_sync(0xffffffffu, x0, (lane & 16) | k);
+          const TX y1 = __shfl_sync(0xffffffffu, x1, (lane & 16) | k);
+          if (li < k) x0 = fma(-f, y0, x0), x1 = fma(-f, y1, x1);
+        }
+      }
+      if (a0) xr[0] = x0;
+      if (a1) xr[2] = x1;
+      barrier();
+    }
+  } else if (warp < R0) {  // warp 1: the tiles
+    TX td[8], ts[8];       // diagonal tile of block b + 1, and its tile against block b
+    {
+      const int k1 = block_at(0), w1 = width_at(k1);
+      solve_fetch<P>(td, M, n, rmap, k1, 1, w1, k1, w1);
+    }
+#pragma unroll 1
+    for (int b = -1; b < nblk; b++) {
+      if (b + 1 < nblk) {
+        TX* const sl = slot_at(b);
+        const int w1 = width_at(block_at(b + 1));
+        solve_stage(sl, td, w1);
+        if (b >= 0) solve_stage(sl + TILE, ts, w1);
+        __syncwarp();
+        if (UPPER && lane < w1) sl[2 * TILE + lane] = TX(1) / sl[lane * SP + lane];
+      }
+      if (b + 2 < nblk) {
+        const int k2 = block_at(b + 2), w2 = width_at(k2), k1 = block_at(b + 1);
+        solve_fetch<P>(td, M, n, rmap, k2, 1, w2, k2, w2);
+        solve_fetch<P>(ts, M, n, rmap, k2, 1, w2, k1, width_at(k1));
+      }
+      barrier();
+    }
+  } else {
+    TX t[16];  // a pass of 32 rows
+    auto fetch_pass = [&](int b, int r0) {
+      const int rest = beyond(b), kb = block_at(b);
+      if (r0 < rest)
+        solve_fetch<P>(t, M, n, rmap, row_at(b, r0), UPPER ? -1 : 1, min(32, rest - r0), kb,
+                       width_at(kb));
+    };
+    fetch_pass(0, 32 * (warp - R0));
+    barrier();
+#pragma unroll 1
+    for (int b = 0; b < nblk; b++) {
+      barrier();
+      const int kb = block_at(b), kbn = width_at(kb);
+      const TX* const xblk = X + kb * nrhs;
+      const int rest = beyond(b);
+#pragma unroll 1
+      for (int r0 = 32 * (warp - R0); r0 < rest; r0 += 32 * NR) {
+        __syncwarp();
+        solve_stage(tr, t, min(32, rest - r0));
+        __syncwarp();
+        fetch_pass(b, r0 + 32 * NR);
+        if (r0 + lane < rest) {
+          TX* const xi = X + row_at(b, r0 + lane) * nrhs;
+          const TX* const f = tr + lane * SP;
+#pragma unroll 1
+          for (int c = 0; c < nrhs; c++) {
+            TX s = xi[c];
+            if (kbn == 16) {
+#pragma unroll
+              for (int k = 0; k < 16; k++) s = fma(-f[k], xblk[k * nrhs + c], s);
+            } else {
+#pragma unroll 1
+              for (int k = 0; k < kbn; k++) s = fma(-f[k], xblk[k * nrhs + c], s);
+            }
+            xi[c] = s;
           }
         }
-        if (act) X[(kb + li) * nrhs + c] = xi;
       }
+      if (b + 1 < nblk) fetch_pass(b + 1, 32 * (warp - R0));
     }
-    __syncthreads();
-    const int rest = n - kb - kbn;
-    for (int r = tid; r < rest; r += BT)
-      solve_row_update<P, TX>(M + (size_t)rmap[kb + kbn + r] * p + kb, kbn,
-                              X + (size_t)(kb + kbn + r) * nrhs, X + (size_t)kb * nrhs, nrhs);
-    __syncthreads();
   }
-  for (int kb = (n - 1) / 16 * 16; kb >= 0; kb -= 16) {
-    const int kbn = min(16, n - kb);
-    if (warp == 0) {
-      const typename P::S* urow = M + (size_t)rmap[kb + min(li, kbn - 1)] * p + kb;
-      TX uv[16];
-#pragma unroll
-      for (int k = 0; k < 16; k++) uv[k] = k < kbn ? (TX)P::ld(&urow[k]) : TX(1);
-      for (int c0 = 0; c0 < nrhs; c0 += 2) {
-        const int c = c0 + half;
-        const bool act = li < kbn && c < nrhs;
-        TX xi = act ? X[(kb + li) * nrhs + c] : TX(0);
-#pragma unroll
-        for (int k = 15; k >= 0; k--) {
-          if (k < kbn) {
-            if (act && li == k) xi = xi / uv[k];
-            const TX xk = __shfl_sync(0xffffffffu, xi, (lane & 16) | k);
-            if (act && li < k) xi = fma(-uv[k], xk, xi);
-          }
-        }
-        if (act) X[(kb + li) * nrhs + c] = xi;
-      }
-    }
-    __syncthreads();
-    for (int r = tid; r < kb; r += BT)
-      solve_row_update<P, TX>(M + (size_t)rmap[r] * p + kb, kbn, X + (size_t)r * nrhs,
-                              X + (size_t)kb * nrhs, nrhs);
-    __syncthreads();
-  }
+  __syncthreads();
+}
+
+template <typename P, typename TX>
+__device__ void block_solve(const typename P::S* M, int n, const int* rmap, TX* X, int nrhs, TX* buf) {
+  block_tri<P, TX, false>(M, n, rmap, X, nrhs, buf);
+  block_tri<P, TX, true>(M, n, rmap, X, nrhs, buf);
 }
 
 struct BatchArgs {
@@ -622,7 +925,7 @@ __device__ double refine_eta(const double* rv, const double* xv, int n, int nrhs
 // w <- A^-1 w through the stored factors of scale * A: an FP32 solve of
 // P w / max|w| (the preconditioner of GMRES-IR).
 template <typename P>
-__device__ void precondition(const typename P::S* M, int n, const int* rmap, double* w, float* dv,
+__device__ void precondition(const typename P::S* M, int n, const int* rmap, float* st, double* w, float* dv,
                              float scale, Shared& sh) {
   const int BT = blockDim.x;
   double m = 0.0;
@@ -631,7 +934,7 @@ __device__ void precondition(const typename P::S* M, int n, const int* rmap, dou
   const double inv = m > 0 ? 1.0 / m : 0.0;
   for (int i = threadIdx.x; i < n; i += BT) dv[i] = (float)(w[rmap[i]] * inv);
   __syncthreads();
-  block_solve<P, float>(M, n, n, rmap, dv, 1);
+  block_solve<P, float>(M, n, rmap, dv, 1, st);
   for (int i = threadIdx.x; i < n; i += BT) w[i] = (double)dv[i] * m * (double)scale;
   __syncthreads();
 }
@@ -643,7 +946,7 @@ __device__ void precondition(const typename P::S* M, int n, const int* rmap, dou
 // Returns the steps taken.
 template <typename P>
 __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int c,
-                            const typename P::S* M, const int* rmap, const double* rv, double* xv,
+                            const typename P::S* M, const int* rmap, float* st, const double* rv, double* xv,
                             float* dv, float scale, double* w, double* H, double* V, int mcap,
                             Shared& sh) {
   const int tid = threadIdx.x, BT = blockDim.x;
@@ -652,7 +955,7 @@ __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int 
   double* sn = cs + GM_M + 1;
   for (int i = tid; i < n; i += BT) w[i] = rv[(size_t)i * nrhs + c];
   __syncthreads();
-  precondition<P>(M, n, rmap, w, dv, scale, sh);
+  precondition<P>(M, n, rmap, st, w, dv, scale, sh);
   double s = 0.0;
   for (int i = tid; i < n; i += BT) s += w[i] * w[i];
   const double beta = sqrt(block_sum_d(s, sh.red));
@@ -664,7 +967,7 @@ __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int 
   for (int j = 0; j < mcap; j++) {
     residual_rows<1, true>(Ai, n, V + (size_t)j * n, nullptr, w);  // w = A v_j
     __syncthreads();
-    precondition<P>(M, n, rmap, w, dv, scale, sh);
+    precondition<P>(M, n, rmap, st, w, dv, scale, sh);
     for (int i = 0; i <= j; i++) {
       const double* vi = V + (size_t)i * n;
       double hs = 0.0;
@@ -835,7 +1138,7 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
       xv[idx] = Bi[(size_t)rmap[i] * nrhs + c];
     }
     __syncthreads();
-    block_solve<P, double>(M, n, n, rmap, xv, nrhs);
+    block_solve<P, double>(M, n, rmap, xv, nrhs, reinterpret_cast<double*>(st));
     for (int idx = tid; idx < n * nrhs; idx += BT) Xi[idx] = xv[idx];
     if (tid == 0) {
       a.status[sidx] = 0;
@@ -876,7 +1179,7 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
     }
     __syncthreads();
     if (tid == 0) pc.mark(3);
-    block_solve<P, float>(M, n, n, rmap, dv, nrhs);
+    block_solve<P, float>(M, n, rmap, dv, nrhs, reinterpret_cast<float*>(st));
     if (tid == 0) pc.mark(2);
     // (scale A) d = r / rmax  =>  A (scale d rmax) = r
     for (int idx = tid; idx < n * nrhs; idx += BT)
@@ -900,7 +1203,7 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
                                           (size_t)blockIdx.x * a.scratch_bytes + GM_V_OFFSET);
     for (int outer = 0; outer < GM_OUTER && !ok; outer++) {
       for (int c = 0; c < nrhs; c++)
-        gsteps += gmres_column<P>(Ai, n, nrhs, c, M, rmap, rv, xv, dv, scale, w, H, V, mcap, sh);
+        gsteps += gmres_column<P>(Ai, n, nrhs, c, M, rmap, reinterpret_cast<float*>(st), rv, xv, dv, scale, w, H, V, mcap, sh);
       residual_all(Ai, n, nrhs, xv, Bi, Xi);
       rv = Xi;
       __syncthreads();
