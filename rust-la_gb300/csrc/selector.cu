@@ -148,22 +148,23 @@ struct RowStats {
 template <int PF>
 __device__ __forceinline__ void load_row_f64(double (&x)[PF], const double* __restrict__ row, int n,
                                              int lane);
-__device__ __forceinline__ void load_row_f32(float (&x)[16], const float* row, int n, int lane);
+template <int MS>
+__device__ __forceinline__ void load_row_f32(float (&x)[MS], const float* row, int n, int lane);
 
 // One Lanczos pass over the rows of warp `warp` (rows warp, warp + NWp, ...):
 // t1[r] = a_r . qj and acc += a_r t1[r] (this lane's columns). FIRST: the rows
 // come from A in FP64 (converted to FP32 and stored in af), and the row and
 // column statistics of pass 0 are taken on the way. The next row's loads are
-// issued before the current row is reduced.
-template <bool FIRST>
+// issued before the current row is reduced. MS: slots of 32 columns (n <= 32 MS).
+template <bool FIRST, int MS>
 __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float* af, int n,
                                              const float* qj, const float* q0, float* t1,
                                              float (&acc)[16], float (&cs)[16], float (&sq)[16],
                                              RowStats& st, int warp, int lane, int NWp) {
-  // Prefetched slots per lane: all 16 from the FP32 copy; 8 (columns < 256)
+  // Prefetched slots per lane: all of them from the FP32 copy; up to 8 (columns < 256)
   // from A in FP64, whose wider raw values would not fit the register budget.
   // The rest of a wider FP64 row is loaded when it is used.
-  constexpr int PF = FIRST ? 8 : 16;
+  constexpr int PF = FIRST && MS > 8 ? 8 : MS;
   using L = typename std::conditional<FIRST, double, float>::type;
   L xn[PF];
   if (warp < n) {
@@ -171,9 +172,9 @@ __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float
     else load_row_f32(xn, af + (size_t)warp * n, n, lane);
   }
   for (int r = warp; r < n; r += NWp) {
-    float x[16];
+    float x[MS];
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
+    for (int m = 0; m < MS; m++) {
       if constexpr (FIRST) {
         const int k = lane + 32 * m;
         x[m] = m < PF ? la_f64_to_f32(xn[m < PF ? m : 0])
@@ -189,7 +190,7 @@ __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float
     float* fr = af + (size_t)r * n;
     float s = 0, rs = 0, f2 = 0, am = 0;
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
+    for (int m = 0; m < MS; m++) {
       const int k = lane + 32 * m;
       if (k < n) {
         s = fmaf(x[m], qj[k], s);
@@ -205,7 +206,7 @@ __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float
     if (FIRST) {  // the diagonal a_rr: slot r / 32 of lane r % 32
       float xdg = x[0];
 #pragma unroll
-      for (int m = 1; m < 16; m++) xdg = m == (r >> 5) ? x[m] : xdg;
+      for (int m = 1; m < MS; m++) xdg = m == (r >> 5) ? x[m] : xdg;
       di = fabsf(__shfl_sync(0xffffffffu, xdg, r & 31));
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -218,7 +219,7 @@ __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float
     }
     const float q0r = q0[r];
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
+    for (int m = 0; m < MS; m++) {
       acc[m] = fmaf(x[m], s, acc[m]);
       if (FIRST) {
         cs[m] += fabsf(x[m]);
@@ -243,7 +244,7 @@ __device__ __forceinline__ void feature_rows(const double* __restrict__ a, float
   }
 }
 
-// A row's entries k = lane + 32 m (m < PF resp. 16, k < n; zero beyond n)
+// A row's entries k = lane + 32 m (m < PF resp. MS, k < n; zero beyond n)
 // into registers, all loads issued before any is used.
 template <int PF>
 __device__ __forceinline__ void load_row_f64(double (&x)[PF], const double* __restrict__ row, int n,
@@ -254,9 +255,10 @@ __device__ __forceinline__ void load_row_f64(double (&x)[PF], const double* __re
     x[m] = k < n ? __ldg(row + k) : 0.0;
   }
 }
-__device__ __forceinline__ void load_row_f32(float (&x)[16], const float* row, int n, int lane) {
+template <int MS>
+__device__ __forceinline__ void load_row_f32(float (&x)[MS], const float* row, int n, int lane) {
 #pragma unroll
-  for (int m = 0; m < 16; m++) {
+  for (int m = 0; m < MS; m++) {
     const int k = lane + 32 * m;
     x[m] = k < n ? row[k] : 0.f;
   }
@@ -330,8 +332,10 @@ __device__ double tridiag_min_eig_warp(const double* al, const double* be, int k
 }
 
 constexpr int FEAT_CTAS_PER_SM = 4;  // 4 CTAs of 4 warps: four systems in flight per SM
+// Systems are taken from a ticket, largest first: dealt out in turn, the CTAs' shares of 3000 systems
+// of 16 to 512 rows differed so much that 56 % of the warps were there on average.
 
-// 16 features per system (one CTA per system). FP64 arithmetic is slow on
+// 16 features per system (one CTA per system), systems by decreasing n. FP64 arithmetic is slow on
 // this GPU, so A_i is read in FP64 once and rounded to an FP32 copy in the
 // CTA's global scratch slice; every statistic and matrix-vector product works
 // in FP32 on that copy (dot products of length n accumulate in FP64). One
@@ -345,8 +349,10 @@ constexpr int FEAT_CTAS_PER_SM = 4;  // 4 CTAs of 4 warps: four systems in fligh
 // sigma_min^2 from above. The asymmetry feature is the probe
 // ||A q0 - A^T q0|| / ||A q0||.
 __global__ void __launch_bounds__(128, 4)
-features_kernel(const double* __restrict__ A, const SysRec* __restrict__ sys, int count,
-                float* __restrict__ F, float* __restrict__ scratch) {
+features_kernel(const double* __restrict__ A, const SysRec* __restrict__ sys,
+                const int* __restrict__ order, int* ticket, int count, float* __restrict__ F,
+                float* __restrict__ scratch) {
+  __shared__ int s_next;
   __shared__ double red[2][8];
   int rpar = 0;
   __shared__ float q[LK + 1][512];
@@ -361,7 +367,11 @@ features_kernel(const double* __restrict__ A, const SysRec* __restrict__ sys, in
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NWp = blockDim.x >> 5;
   float* af = scratch + (size_t)blockIdx.x * 512 * 512;
-  for (int i = blockIdx.x; i < count; i += gridDim.x) {
+  for (;;) {
+    if (tid == 0) s_next = atomicAdd(ticket, 1);
+    __syncthreads();
+    if (s_next >= count) return;
+    const int i = order[s_next];
     const SysRec d = sys[i];
     const int n = d.n;
     const double* a = A + d.a;
@@ -385,10 +395,19 @@ features_kernel(const double* __restrict__ A, const SysRec* __restrict__ sys, in
       // Rows are software-pipelined per warp (feature_rows): the next row's
       // loads are issued before the current row's reduction, so the memory
       // latency overlaps the shuffles.
-      if (j == 0)
-        feature_rows<true>(a, af, n, q[0], q[0], t1, acc, cs, sq, st, warp, lane, NWp);
-      else
-        feature_rows<false>(a, af, n, q[j], q[0], t1, acc, cs, sq, st, warp, lane, NWp);
+      // Only as many column slots as the system has: with all sixteen for every n, a third of the
+      // instructions at n = 264 were for columns that do not exist.
+      const auto rows = [&](auto ms) {
+        constexpr int MS = decltype(ms)::value;
+        if (j == 0)
+          feature_rows<true, MS>(a, af, n, q[0], q[0], t1, acc, cs, sq, st, warp, lane, NWp);
+        else
+          feature_rows<false, MS>(a, af, n, q[j], q[0], t1, acc, cs, sq, st, warp, lane, NWp);
+      };
+      if (n <= 128) rows(std::integral_constant<int, 4>());
+      else if (n <= 256) rows(std::integral_constant<int, 8>());
+      else if (n <= 384) rows(std::integral_constant<int, 12>());
+      else rows(std::integral_constant<int, 16>());
       // t2 = A^T t1: sum the warps' column partials
 #pragma unroll
       for (int m = 0; m < 16; m++)
@@ -948,19 +967,31 @@ la_status la_batch_features_device(la_ctx ctx, const double* d_a, const la_batch
     h[i] = {(long long)systems[i].a_offset, (long long)systems[i].b_offset, systems[i].n,
             systems[i].nrhs};
   }
+  // Queue order: decreasing n (a counting sort), then the ticket, behind the records.
+  std::vector<int> first(514, 0), order((size_t)count + 1);
+  for (int i = 0; i < count; i++) first[513 - h[i].n]++;
+  for (int k = 1; k < 514; k++) first[k] += first[k - 1];
+  for (int i = 0; i < count; i++) order[first[512 - h[i].n]++] = i;
+  order[count] = 0;
   SysRec* d = nullptr;
   float* scr = nullptr;
   const int grid = std::min(count, ctx->sm_count * FEAT_CTAS_PER_SM);
-  LA_TRY(la_device_alloc(ctx, reinterpret_cast<void**>(&d), count * sizeof(SysRec)));
+  LA_TRY(la_device_alloc(ctx, reinterpret_cast<void**>(&d),
+                         count * sizeof(SysRec) + order.size() * sizeof(int)));
+  int* const d_order = reinterpret_cast<int*>(d + count);
   la_status s = la_device_alloc(ctx, reinterpret_cast<void**>(&scr),
                                 (size_t)grid * 512 * 512 * sizeof(float));
   if (s == LA_OK) {
     cudaError_t e = cudaMemcpyAsync(d, h.data(), count * sizeof(SysRec), cudaMemcpyHostToDevice,
                                     ctx->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(d_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice,
+                          ctx->stream);
     if (e != cudaSuccess) s = la_cuda_fail(ctx, e, "features upload");
   }
   if (s == LA_OK) {
-    features_kernel<<<grid, 128, 0, ctx->stream>>>(d_a, d, count, d_features, scr);
+    features_kernel<<<grid, 128, 0, ctx->stream>>>(d_a, d, d_order, d_order + count, count,
+                                                   d_features, scr);
     ctx->launches++;
     s = la_check_launch(ctx, "features_kernel");
   }
