@@ -311,6 +311,8 @@ la_status launch_lu_solve(la_ctx ctx, bool exact, const double* LU, size_t ld, d
                           size_t ldx, int n, int nrhs);
 la_status launch_permute_rows(la_ctx ctx, const uint64_t* d_piv, const double* B, size_t ldb,
                               double* X, size_t ldx, int m, int nrhs);
+la_status launch_permute_cols(la_ctx ctx, const uint64_t* d_piv, const double* X, double* Y, size_t ld,
+                              int n);
 la_status launch_identity_permuted(la_ctx ctx, const uint64_t* d_piv, double* X, size_t ldx,
                                    int m);
 la_status launch_det(la_ctx ctx, const double* LU, size_t ld, int n, int pospivsign,

@@ -101,6 +101,90 @@ constexpr int SPLIT_MIN_MN = 64 * 64;  // smaller updates: one FMA launch is no 
 // Block width for R remaining rows.
 int lu_block(int R) { return R > 3072 ? 256 : R > 1024 ? 128 : LU_BASE; }
 
+// Workspace of the split products (digits of both operands) that a product may ask for.
+constexpr size_t SPLIT_WS_MAX = (size_t)4 << 30;
+
+// C (M x N) -= A B as a split product, in pieces of whole tiles that the workspace takes.
+la_status split_update(la_ctx ctx, int M, int N, int K, const double* A, size_t lda, const double* B,
+                       size_t ldb, double* C, size_t ldc, void* ws, size_t ws_bytes) {
+  int rb = M, cb = N;
+  auto half = [](int x, int q) { return std::max(q, ((x + 1) / 2 + q - 1) / q * q); };
+  while (gemm_split_ws(rb, cb, K, false) > ws_bytes && (rb > 128 || cb > 64)) {
+    if (rb > 128 && rb >= cb) rb = half(rb, 128);
+    else if (cb > 64) cb = half(cb, 64);
+    else rb = half(rb, 128);
+  }
+  la_status s = LA_OK;
+  for (int r = 0; r < M && s == LA_OK; r += rb)
+    for (int c = 0; c < N && s == LA_OK; c += cb)
+      s = launch_gemm_split(ctx, ctx->stream, -1, std::min(rb, M - r), std::min(cb, N - c), K,
+                            A + (size_t)r * lda, lda, B + c, ldb, false, C + (size_t)r * ldc + c, ldc,
+                            false, ws, ws_bytes);
+  return s;
+}
+
+// X <- U^-1 L^-1 X for many right-hand sides: blocks of up to SOLVE_BASE rows by the wavefront kernel,
+// and between them split products, recursively, so that most terms are in few products of large K.
+// What bounds the wavefront here is the FP64 pipe (n^2 nrhs FMAs at two per clock and SM: 1.7 ms of
+// 2.4 at n = nrhs = 1000); the products do theirs on the tensor cores, with one rounding each.
+// `id`: X is the identity on entry; row r of L^-1 ends at column r, so the forward half leaves the
+// columns beyond out. (Against the permuted identity every column's zeros and single entries sent most
+// tiles to the FMA chains: 4.89 ms for the inverse of order 1000 instead of 3.84.)
+constexpr int SOLVE_BASE = 256;  // 128: 4.02 ms
+// Inverses, ms, wavefront and blocked: n = 500 1.64, 1.67; 600 2.10, 2.19; 700 2.65, 2.55; 800 3.28,
+// 2.92; 1000 4.98, 3.82; 2500 42.3, 14.7.
+constexpr size_t INVERSE_BLOCKED_N = 672;
+struct BlockedSolve {
+  la_ctx ctx;
+  const double* A;
+  size_t ld;
+  double* X;
+  size_t ldx;
+  int nrhs;
+  bool id;
+  void* ws;
+  size_t ws_bytes;
+
+  static int middle(int r0, int r1) { return r0 + ((r1 - r0 + 1) / 2 + 63) / 64 * 64; }
+  // The first nc columns of X[r0:r1] -= A[r0:r1, k0:k1] X[k0:k1].
+  la_status update(int r0, int r1, int k0, int k1, int nc) {
+    if (nc <= 0) return LA_OK;
+    const double* a = A + (size_t)r0 * ld + k0;
+    const double* x = X + (size_t)k0 * ldx;
+    const la_status s = split_update(ctx, r1 - r0, nc, k1 - k0, a, ld, x, ldx, X + (size_t)r0 * ldx, ldx,
+                                     ws, ws_bytes);
+    if (s != LA_UNSUPPORTED) return s;
+    return launch_gemm(ctx, GM_FMA_SUB, r1 - r0, nc, k1 - k0, a, ld, x, ldx, X + (size_t)r0 * ldx, ldx);
+  }
+  la_status block(bool upper, int r0, int r1, int nc) {
+    return launch_tri_wave(ctx, false, upper, upper, A + (size_t)r0 * ld + r0, ld, X + (size_t)r0 * ldx,
+                           ldx, r1 - r0, nc);
+  }
+  la_status lower(int r0, int r1) {
+    if (r1 - r0 <= SOLVE_BASE) return block(false, r0, r1, id ? r1 : nrhs);
+    const int mid = middle(r0, r1);
+    LA_TRY(lower(r0, mid));
+    if (!id) {
+      LA_TRY(update(mid, r1, r0, mid, nrhs));
+      return lower(mid, r1);
+    }
+    // The last 64 columns end in as many rows: their terms are an FMA product of K = 64. (Elements of
+    // few terms do not fit the split product, and one such tile is a chain of all K: 590 us at K = 512.)
+    const int c = mid - 64;
+    LA_TRY(update(mid, r1, r0, mid, c));
+    LA_TRY(launch_gemm_narrow(ctx, GM_FMA_SUB, r1 - mid, 64, 64, A + (size_t)mid * ld + c, ld,
+                              X + (size_t)c * ldx + c, ldx, X + (size_t)mid * ldx + c, ldx));
+    return lower(mid, r1);
+  }
+  la_status upper(int r0, int r1) {
+    if (r1 - r0 <= SOLVE_BASE) return block(true, r0, r1, nrhs);
+    const int mid = middle(r0, r1);
+    LA_TRY(upper(mid, r1));
+    LA_TRY(update(r0, mid, mid, r1, nrhs));
+    return upper(r0, mid);
+  }
+};
+
 struct FastLu {
   la_ctx ctx;
   double* A;
@@ -124,19 +208,8 @@ struct FastLu {
     const int M = r1 - r0, N = c1 - c0, K = k1 - k0;
     if (M <= 0 || N <= 0) return LA_OK;
     if (ws && K >= 32 && (size_t)M * N >= SPLIT_MIN_MN) {
-      int rb = M, cb = N;
-      auto half = [](int x, int q) { return std::max(q, ((x + 1) / 2 + q - 1) / q * q); };
-      while (gemm_split_ws(rb, cb, K, false) > ws_bytes && (rb > 128 || cb > 64)) {
-        if (rb > 128 && rb >= cb) rb = half(rb, 128);
-        else if (cb > 64) cb = half(cb, 64);
-        else rb = half(rb, 128);
-      }
-      la_status s = LA_OK;
-      for (int r = r0; r < r1 && s == LA_OK; r += rb)
-        for (int c = c0; c < c1 && s == LA_OK; c += cb)
-          s = launch_gemm_split(ctx, ctx->stream, -1, std::min(rb, r1 - r), std::min(cb, c1 - c), K,
-                                at(r, k0), ld, at(k0, c), ld, false, at(r, c), ld, false, ws,
-                                ws_bytes);
+      const la_status s = split_update(ctx, M, N, K, at(r0, k0), ld, at(k0, c0), ld, at(r0, c0), ld, ws,
+                                       ws_bytes);
       if (s != LA_UNSUPPORTED) return s;
     }
     if (N <= 64 && K <= 64)
@@ -413,8 +486,23 @@ la_status lu_non_singular(la_lu h, int* out) {
 // X (m x nrhs, pitch ldx) holds B(piv,:) on entry and the solution on exit
 // (lu.rs:256-275; the loops run over the first n rows).
 la_status lu_solve_inplace(la_ctx ctx, la_lu h, double* X, size_t ldx, int nrhs) {
-  return launch_lu_solve(ctx, h->arith == LA_ARITH_EXACT, h->d_lu, h->ld, X, ldx, (int)h->n,
-                         nrhs);
+  const int n = (int)h->n;
+  // Where the blocked solve is the faster one. Device solve, us, wavefront and blocked: n = 512: 512
+  // right-hand sides 439, 429; 1000: 751, 594. n = 1000: 256: 766, 922; 512: 1321, 959; 1000: 2466, 1299.
+  // n = 2500: 192: 2835, 2922; 256: 3643, 2958. n = 6000: 64: 5497, 6553; 128: 10042, 6915; 1000: 74520,
+  // 9991. Backward errors 4 to 10 times smaller. Without memory for the digits: the wavefront.
+  if (h->arith == LA_ARITH_FAST && ctx->solve_wave > 0 && !ctx->split_ws && n >= 512 && nrhs >= 64 &&
+      (long long)n * nrhs >= 500000) {
+    const int half = BlockedSolve::middle(0, n);
+    DevBuf ws(ctx);
+    const size_t bytes = gemm_split_ws(half, nrhs, half, false);
+    if (bytes <= SPLIT_WS_MAX && ws.alloc(bytes) == LA_OK) {
+      BlockedSolve s{ctx, h->d_lu, h->ld, X, ldx, nrhs, false, ws.p, bytes};
+      LA_TRY(s.lower(0, n));
+      return s.upper(0, n);
+    }
+  }
+  return launch_lu_solve(ctx, h->arith == LA_ARITH_EXACT, h->d_lu, h->ld, X, ldx, n, nrhs);
 }
 
 la_status check_ctx(la_ctx ctx) {
@@ -424,8 +512,6 @@ la_status check_ctx(la_ctx ctx) {
   return LA_OK;
 }
 
-// Workspace of the split products (digits of both operands) that a product may ask for.
-constexpr size_t SPLIT_WS_MAX = (size_t)4 << 30;
 
 // Device solve shared by the host and device entry points: d_b (pitch ldb) ->
 // d_x (pitch ldx); both may be unaligned, an aligned work buffer is used.
@@ -670,9 +756,26 @@ la_status la_matrix_inverse(la_ctx ctx, const double* a, size_t m, size_t n, dou
     const size_t ldw = pad4(n);
     DevBuf Xw(ctx);
     s = Xw.alloc(n * ldw * sizeof(double));
-    if (s == LA_OK) s = launch_identity_permuted(ctx, h->d_piv, Xw.d(), ldw, (int)n);
-    if (s == LA_OK) s = lu_solve_inplace(ctx, h, Xw.d(), ldw, (int)n);
-    if (s == LA_OK) s = la_copy_to_host(ctx, out, Xw.d(), ldw, n, n);
+    // U^-1 L^-1 by blocks, then the columns in their order: A^-1 = (LU)^-1 P.
+    DevBuf ws(ctx);
+    const double* inv = Xw.d();
+    if (s == LA_OK && h->arith == LA_ARITH_FAST && ctx->solve_wave > 0 && n >= INVERSE_BLOCKED_N) {
+      const int half = BlockedSolve::middle(0, (int)n);
+      const size_t bytes = std::max(gemm_split_ws(half, (int)n, half, false), n * ldw * sizeof(double));
+      if (bytes <= SPLIT_WS_MAX && ws.alloc(bytes) == LA_OK) {
+        BlockedSolve b{ctx, h->d_lu, h->ld, Xw.d(), ldw, (int)n, true, ws.p, bytes};
+        s = launch_identity_permuted(ctx, nullptr, Xw.d(), ldw, (int)n);
+        if (s == LA_OK) s = b.lower(0, (int)n);
+        if (s == LA_OK) s = b.upper(0, (int)n);
+        if (s == LA_OK) s = launch_permute_cols(ctx, h->d_piv, Xw.d(), ws.d(), ldw, (int)n);
+        inv = ws.d();
+      }
+    }
+    if (inv == Xw.d()) {
+      if (s == LA_OK) s = launch_identity_permuted(ctx, h->d_piv, Xw.d(), ldw, (int)n);
+      if (s == LA_OK) s = lu_solve_inplace(ctx, h, Xw.d(), ldw, (int)n);
+    }
+    if (s == LA_OK) s = la_copy_to_host(ctx, out, inv, ldw, n, n);
     if (s == LA_OK) s = la_sync_and_check(ctx, "inverse");
   }
   la_lu_free(h);

@@ -339,14 +339,21 @@ __global__ void permute_rows_kernel(const uint64_t* __restrict__ piv, const doub
   }
 }
 
-// X = I(piv, :) for inverse (mod.rs:1036 solves against Matrix::id).
+// Y(:, piv[c]) = X(:, c), one row per CTA: written in any order, but within a row of L2 lines.
+__global__ void permute_cols_kernel(const uint64_t* __restrict__ piv, const double* __restrict__ X,
+                                    double* __restrict__ Y, size_t ld, int n) {
+  const size_t r = (size_t)blockIdx.x * ld;
+  for (int c = threadIdx.x; c < n; c += blockDim.x) Y[r + piv[c]] = X[r + c];
+}
+
+// X = I(piv, :) for inverse (mod.rs:1036 solves against Matrix::id); I without piv.
 __global__ void identity_permuted_kernel(const uint64_t* __restrict__ piv, double* X, size_t ldx,
                                          int m) {
   size_t total = (size_t)m * m;
   for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
        idx += (size_t)gridDim.x * blockDim.x) {
     int i = (int)(idx / m), j = (int)(idx % m);
-    X[(size_t)i * ldx + j] = (piv[i] == (uint64_t)j) ? 1.0 : 0.0;
+    X[(size_t)i * ldx + j] = ((piv ? piv[i] : (uint64_t)i) == (uint64_t)j) ? 1.0 : 0.0;
   }
 }
 
@@ -531,6 +538,13 @@ la_status launch_identity_permuted(la_ctx ctx, const uint64_t* d_piv, double* X,
                                                                                   m);
   ctx->launches++;
   return la_check_launch(ctx, "identity_permuted_kernel");
+}
+
+la_status launch_permute_cols(la_ctx ctx, const uint64_t* d_piv, const double* X, double* Y, size_t ld,
+                              int n) {
+  permute_cols_kernel<<<n, 256, 0, ctx->stream>>>(d_piv, X, Y, ld, n);
+  ctx->launches++;
+  return la_check_launch(ctx, "permute_cols_kernel");
 }
 
 la_status launch_det(la_ctx ctx, const double* LU, size_t ld, int n, int pospivsign,
