@@ -1,6 +1,6 @@
 // Triangular solves of LUDecomposition::solve (src/decomp/lu.rs:256-275).
 //
-// Two schedules that apply every term in the same order, so their results are
+// Three schedules that apply every term in the same order, so their results are
 // bit-identical:
 //
 // Wavefront (default). One persistent launch per triangle. The rows are cut
@@ -17,6 +17,9 @@
 // block lane by lane with shuffles, stores x and publishes (release). The
 // critical path per block is one tile application and one 32-step diagonal
 // solve; the rest of the update work fills the other SMs.
+//
+// Chain (up to CHAIN_MAX_NRHS right-hand sides). The wavefront with 128 rows of
+// one column per item; see solve_chain_kernel.
 //
 // Block steps. One launch per 16-row block step: for the finished block
 // [k0, k1),
@@ -367,9 +370,287 @@ solve_wave_kernel(const T* __restrict__ LU, size_t ld, T* X, size_t ldx, int n, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// The wavefront for few right-hand sides: an item is 128 rows of one column, one warp to each of its
+// four 32-row blocks, in the order of the solve.
+//
+// What bounds a solve with few columns is the chain through all n rows: per row a shuffle and one FP64
+// FMA (64 clocks of a sub-partition for a warp, whatever its active lanes). With one block per item
+// every 32 rows also paid a hand-over through L2 (store, fence, release, poll, load: 2500 clocks) and,
+// after it, the whole tile against the block before (2000). Here three of four hand-overs are through
+// shared memory, eight rows at a time, so a warp has taken all but the last eight terms when the warp
+// before it is done. Each warp stays on its own sub-partition, so that the chain has a pipe to itself.
+//   * Every element takes its terms in the same order by the same operations: the same bits as the
+//     other two schedules.
+//   * A solved value is its own flag: xs holds a NaN that no computation here gives until it is
+//     written (a value with these very bits is handed on as the default NaN).
+//   * Tiles come by cp.async, one ahead, row-major with 16 bytes of padding: reading 16 bytes of its
+//     row per lane is free of bank conflicts.
+// Both triangles (us, one block per item and now): n = 512 213, 159; 1000 389, 278; 4096 1521, 1030;
+// 8192 3107, 2067.
+constexpr int CB = 4;                          // blocks of WB rows per item
+template <typename T>
+struct ChainTile {
+  static constexpr int VN = 16 / (int)sizeof(T);
+  static constexpr int P = WB + VN;            // pitch
+  static constexpr size_t SMEM = (size_t)CB * 2 * WB * P * sizeof(T);
+};
+template <typename T>
+__device__ __forceinline__ bool unset(T v) {
+  if constexpr (sizeof(T) == 8) return __double_as_longlong(v) == -1ll;
+  else return __float_as_int(v) == -1;
+}
+template <typename T>
+__device__ __forceinline__ T unset_value() {
+  if constexpr (sizeof(T) == 8) return __longlong_as_double(-1ll);
+  else return __int_as_float(-1);
+}
+template <typename T>
+__device__ __forceinline__ T settable(T v) {
+  if constexpr (sizeof(T) == 8) return unset(v) ? __longlong_as_double(0x7ff8000000000000ll) : v;
+  else return unset(v) ? __int_as_float(0x7fc00000) : v;
+}
+// Blocks of the column known to be solved, in order: counter w of the four counts its block of each
+// item. As wave_wait, until that is at least `need`; -1 after an error or without progress.
+__device__ __forceinline__ int chain_wait(const int* p, int need, int* err) {
+  const unsigned full = 0xffffffffu;
+  const int w = threadIdx.x & (CB - 1);
+  unsigned long long t0 = 0;
+  for (unsigned spins = 1;; spins++) {
+    const int done = __reduce_min_sync(full, CB * wave_ld_acquire(p + w) + w);
+    if (done >= need) return done;
+    if ((spins & 63u) == 0) {
+      int bad = 0;
+      if ((threadIdx.x & 31) == 0) {
+        if (*reinterpret_cast<volatile int*>(err) != 0) {
+          bad = 1;
+        } else {
+          const unsigned long long now = wave_time();
+          if (t0 == 0) t0 = now;
+          else if (now - t0 > WAVE_WAIT_NS) {
+            atomicCAS(err, 0, (int)DERR_TRSV_TIMEOUT);
+            bad = 1;
+          }
+        }
+      }
+      if (__shfl_sync(full, bad, 0)) return -1;
+    }
+  }
+}
+// The tile of rows [r0, r0 + sb) against columns [k0, k0 + kbs) to shared memory, zeros around it; 16
+// bytes per copy, or one element where rows are not 16-byte aligned.
+template <typename T>
+__device__ __forceinline__ void chain_fetch(T* tile, const T* __restrict__ LU, size_t ld, int r0, int sb,
+                                            int k0, int kbs, bool vec) {
+  constexpr int VN = ChainTile<T>::VN, P = ChainTile<T>::P;
+  const int lane = threadIdx.x & 31;
+  if (vec) {
+    constexpr int PER = WB / VN;  // copies per row
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int idx = lane + 32 * j, r = idx / PER, k = idx % PER * VN;
+      const int have = r < sb ? max(0, min(VN, kbs - k)) : 0;
+      const T* src = have ? LU + (size_t)(r0 + r) * ld + k0 + k : LU;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(tile + r * P + k)),
+                   "l"(src), "r"(have * (int)sizeof(T)));
+    }
+  } else {
+    for (int r = 0; r < WB; r++) {
+      const int have = r < sb && lane < kbs;
+      const T* src = have ? LU + (size_t)(r0 + r) * ld + k0 + lane : LU;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(tile + r * P + lane)),
+                   "l"(src), "n"(sizeof(T)), "r"(have ? (int)sizeof(T) : 0));
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// Entries [k, k + VN) of the lane's row.
+template <typename T>
+__device__ __forceinline__ void chain_row(T (&l)[ChainTile<T>::VN], const T* row, int k) {
+  const int4 v = *reinterpret_cast<const int4*>(row + k);
+  memcpy(l, &v, 16);
+}
+
+template <typename T, bool EXACT, bool UPPER, bool DIVL>
+__global__ void __launch_bounds__(CB * 32)
+solve_chain_kernel(const T* __restrict__ LU, size_t ld, T* X, size_t ldx, int n, int nrhs, int nb,
+                   bool vec, int* ticket, int* prog, int* err) {
+  constexpr int VN = ChainTile<T>::VN, P = ChainTile<T>::P;
+  extern __shared__ __align__(16) char chain_smem[];
+  __shared__ T xs_[CB * WB];
+  __shared__ int s_item, s_fail_;
+  volatile T* const xs = xs_;
+  volatile int* const s_fail = &s_fail_;
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  T* const tiles = reinterpret_cast<T*>(chain_smem) + (size_t)w * 2 * WB * P;
+  const int items = (nb + CB - 1) / CB * nrhs;
+  for (;;) {
+    if (tid == 0) {
+      s_item = atomicAdd(ticket, 1);
+      s_fail_ = 0;
+    }
+    xs[tid] = unset_value<T>();
+    __syncthreads();
+    const int t = s_item;
+    if (t >= items) return;
+    const int q = t / nrhs, col = t - q * nrhs, o = CB * q + w;
+    int* const pg = prog + CB * col;
+    bool fail = false;  // warp-uniform
+    if (o < nb) {
+      const int b = UPPER ? nb - 1 - o : o;
+      const int r0 = b * WB, sb = min(WB, n - r0);
+      auto fetch = [&](int s) {
+        const int k0 = (UPPER ? nb - 1 - s : s) * WB;
+        chain_fetch<T>(tiles + (s & 1) * WB * P, LU, ld, r0, sb, k0, min(WB, n - k0), vec);
+      };
+      T x = lane < sb ? __ldcg(X + (size_t)(r0 + lane) * ldx + col) : T(0);
+      T xn = T(0);
+      bool have_xn = false;
+      int known = 0;
+      fetch(0);
+      for (int s = 0; s <= o && !fail; s++) {
+        const int kb = UPPER ? nb - 1 - s : s;
+        const int kbs = min(WB, n - kb * WB);
+        if (s < o) {
+          fetch(s + 1);
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const T* const row = tiles + (s & 1) * WB * P + lane * P;
+        T l[VN];
+        if (s < CB * q) {
+          T xc = xn;
+          if (!have_xn) {
+            if (known < s + 1) {
+              known = chain_wait(pg, s + 1, err);
+              if (known < 0) {
+                fail = true;
+                break;
+              }
+            }
+            xc = lane < kbs ? __ldcg(X + (size_t)(kb * WB + lane) * ldx + col) : T(0);
+          }
+          have_xn = s + 1 < CB * q && known >= s + 2;
+          if (have_xn) {
+            const int kn = UPPER ? kb - 1 : kb + 1;
+            xn = lane < min(WB, n - kn * WB) ? __ldcg(X + (size_t)(kn * WB + lane) * ldx + col) : T(0);
+          }
+#pragma unroll
+          for (int i = 0; i < WB; i += VN) {
+            const int k0 = UPPER ? WB - VN - i : i;
+            chain_row<T>(l, row, k0);
+#pragma unroll
+            for (int j = 0; j < VN; j++) {
+              const int e = UPPER ? VN - 1 - j : j;
+              const T xk = __shfl_sync(full, xc, k0 + e);
+              if (k0 + e < kbs) x = apply<EXACT, T>(x, xk, l[e]);
+            }
+          }
+        } else if (s < o) {
+          // the warps before this one, eight rows at a time
+#pragma unroll 1
+          for (int i = 0; i < WB; i += 8) {
+            const int k0 = UPPER ? WB - 8 - i : i;
+            T xc;
+            for (unsigned spins = 1;; spins++) {
+              xc = xs[(s & (CB - 1)) * WB + k0 + (lane & 7)];
+              if (__all_sync(full, !unset(xc))) break;
+              if ((spins & 63u) == 0 && __any_sync(full, *s_fail)) {
+                fail = true;
+                break;
+              }
+            }
+            if (fail) break;
+#pragma unroll
+            for (int h = 0; h < 8; h += VN) {
+              const int kh = k0 + (UPPER ? 8 - VN - h : h);
+              chain_row<T>(l, row, kh);
+#pragma unroll
+              for (int j = 0; j < VN; j++) {
+                const int e = UPPER ? VN - 1 - j : j;
+                const T xk = __shfl_sync(full, xc, (kh + e) & 7);
+                if (kh + e < kbs) x = apply<EXACT, T>(x, xk, l[e]);
+              }
+            }
+          }
+        } else {
+          // FAST: the reciprocals off the chain; EXACT divides on it (see solve_wave_kernel).
+          constexpr bool DIV = UPPER || DIVL;
+          const T dd = DIV && lane < sb ? row[lane] : T(1);
+          const T rcp = DIV && !EXACT ? T(1) / dd : T(1);
+#pragma unroll
+          for (int i = 0; i < WB; i += VN) {
+            const int k0 = UPPER ? WB - VN - i : i;
+            chain_row<T>(l, row, k0);
+#pragma unroll
+            for (int j = 0; j < VN; j++) {
+              const int k = k0 + (UPPER ? VN - 1 - j : j);
+              if (k < sb) {  // uniform
+                if (DIV) {
+                  const T v = quot<EXACT>(x, dd, rcp);  // every lane's, row k's is taken
+                  if (lane == k) x = v;
+                }
+                const T xk = __shfl_sync(full, x, k);
+                if (UPPER ? lane < k : lane > k) x = apply<EXACT, T>(x, xk, l[k - k0]);
+              }
+              if (k % 8 == (UPPER ? 0 : 7) && lane / 8 == k / 8) xs[w * WB + lane] = settable(x);
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (!fail) {
+        if (lane < sb) X[(size_t)(r0 + lane) * ldx + col] = x;
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) wave_st_release(pg + w, q + 1);
+      } else if (lane == 0) {
+        *s_fail = 1;
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    if (__syncthreads_or(fail ? 1 : 0)) return;
+  }
+}
+
+// Right-hand sides up to which the chain's items are one column each; above, four columns per item
+// share each tile's load and the FP64 pipes are busy anyway. Both triangles, us, four columns and one:
+// n = 8192: 16 right-hand sides 4053, 3412; 24: 4731, 4593; 32: 5609, 5839. n = 4096: 24: 1912, 1471;
+// 64: 2842, 2980.
+constexpr int CHAIN_MAX_NRHS = 24;
+
+// One triangle by solve_chain_kernel.
+template <typename T, bool EXACT, bool UPPER, bool DIVL>
+la_status chain(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int nrhs) {
+  static_assert(2 + CB * CHAIN_MAX_NRHS <= 2 + 2 * SOLVE_WAVE_MAX_GROUPS, "progress counters");
+  const auto kernel = solve_chain_kernel<T, EXACT, UPPER, DIVL>;
+  const size_t smem = ChainTile<T>::SMEM;
+  LA_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int nb = (n + WB - 1) / WB;
+  int* const sync = ctx->d_solve_sync;
+  LA_CUDA(ctx, cudaMemsetAsync(sync, 0, (2 + CB * (size_t)nrhs) * sizeof(int), ctx->stream));
+  const long long items = (long long)((nb + CB - 1) / CB) * nrhs;
+  const int cps = ctx->solve_wave > 0 ? ctx->solve_wave : 2;
+  const int grid = (int)std::min<long long>(items, (long long)cps * ctx->sm_count);
+  const bool vec = ld % ChainTile<T>::VN == 0 && reinterpret_cast<uintptr_t>(LU) % 16 == 0;
+  kernel<<<grid, CB * 32, smem, ctx->stream>>>(LU, ld, X, ldx, n, nrhs, nb, vec, sync, sync + 2,
+                                               ctx->d_err);
+  ctx->launches++;
+  return la_check_launch(ctx, "solve_chain_kernel");
+}
+
 template <typename T, bool EXACT>
 la_status solve_wave(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int nrhs) {
   const int nb = (n + WB - 1) / WB;
+  if (nrhs <= CHAIN_MAX_NRHS) {
+    LA_TRY((chain<T, EXACT, false, false>(ctx, LU, ld, X, ldx, n, nrhs)));
+    return chain<T, EXACT, true, false>(ctx, LU, ld, X, ldx, n, nrhs);
+  }
   const int groups = (nrhs + WC - 1) / WC;
   int* tickets = ctx->d_solve_sync;
   int* prog_l = tickets + 2;
@@ -392,6 +673,7 @@ la_status solve_wave(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n
 template <bool EXACT, bool UPPER, bool DIVL>
 la_status tri_wave(la_ctx ctx, const double* T, size_t ld, double* X, size_t ldx, int n,
                    int nrhs) {
+  if (nrhs <= CHAIN_MAX_NRHS) return chain<double, EXACT, UPPER, DIVL>(ctx, T, ld, X, ldx, n, nrhs);
   const int nb = (n + WB - 1) / WB;
   const int per = WC * SOLVE_WAVE_MAX_GROUPS;
   for (int c0 = 0; c0 < nrhs; c0 += per) {
