@@ -302,24 +302,31 @@ __global__ void lu_finish_kernel(const int* __restrict__ ipiv, uint64_t* piv, in
   __syncthreads();
   for (int j = threadIdx.x; j < kmin; j += blockDim.x)
     if (LU[(size_t)j * ld + j] == T(0)) atomicOr(&zero, 1);
-  if (threadIdx.x == 0) {
-    int pos = 1;
-    for (int j = 0; j < kmin; j++) {
-      int p = ipiv[j];
-      if (p != j) {
+  // One warp replays: 32 interchanges are loaded at once, ahead of the chain
+  // (two shared-memory accesses per interchange; with the load in it, n = 1000
+  // took 55 us).
+  if (threadIdx.x < 32) {
+    int swaps = 0;
+    int next = (int)threadIdx.x < kmin ? ipiv[threadIdx.x] : 0;
+    for (int j0 = 0; j0 < kmin; j0 += 32) {
+      const int mine = next, cnt = min(32, kmin - j0);
+      if (j0 + 32 + (int)threadIdx.x < kmin) next = ipiv[j0 + 32 + threadIdx.x];
+      swaps += __popc(__ballot_sync(0xffffffffu, (int)threadIdx.x < cnt && mine != j0 + (int)threadIdx.x));
+      for (int i = 0; i < cnt; i++) {
+        const int j = j0 + i, p = __shfl_sync(0xffffffffu, mine, i);
+        if (threadIdx.x != 0 || p == j) continue;
         if (in_smem) {
-          int t = sperm[p];
+          const int t = sperm[p];
           sperm[p] = sperm[j];
           sperm[j] = t;
         } else {
-          uint64_t t = piv[p];
+          const uint64_t t = piv[p];
           piv[p] = piv[j];
           piv[j] = t;
         }
-        pos = !pos;
       }
     }
-    flags[0] = pos;
+    if (threadIdx.x == 0) flags[0] = !(swaps & 1);
   }
   __syncthreads();
   if (in_smem)
@@ -358,13 +365,25 @@ __global__ void identity_permuted_kernel(const uint64_t* __restrict__ piv, doubl
 }
 
 // det (lu.rs:224-232): one thread multiplies U's diagonal in ascending order,
-// the reference's exact sequence of roundings.
-__global__ void det_kernel(const double* LU, size_t ld, int n, int pospivsign, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double d = pospivsign ? 1.0 : -1.0;
-    for (int j = 0; j < n; j++) d = d * LU[(size_t)j * ld + j];
-    out[0] = d;
+// the reference's exact sequence of roundings. The diagonal comes through
+// shared memory, a thread to each entry: n dependent products bound it (64
+// clocks each), where n loads in one thread's path took 48 us at n = 512.
+constexpr int DET_T = 256, DET_CHUNK = 1024;
+__global__ void __launch_bounds__(DET_T)
+det_kernel(const double* LU, size_t ld, int n, int pospivsign, double* out) {
+  __shared__ double diag[DET_CHUNK];
+  double d = pospivsign ? 1.0 : -1.0;
+  for (int j0 = 0; j0 < n; j0 += DET_CHUNK) {
+    const int cnt = min(DET_CHUNK, n - j0);
+    for (int i = threadIdx.x; i < cnt; i += DET_T) diag[i] = LU[(size_t)(j0 + i) * ld + j0 + i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int i = 0; i < cnt; i++) d = d * diag[i];
+    }
+    __syncthreads();
   }
+  if (threadIdx.x == 0) out[0] = d;
 }
 
 // get_l (which 0, lu.rs:184-202), get_u (1, :204-215), get_p (2, :217-220),
@@ -549,7 +568,7 @@ la_status launch_permute_cols(la_ctx ctx, const uint64_t* d_piv, const double* X
 
 la_status launch_det(la_ctx ctx, const double* LU, size_t ld, int n, int pospivsign,
                      double* d_out) {
-  det_kernel<<<1, 32, 0, ctx->stream>>>(LU, ld, n, pospivsign, d_out);
+  det_kernel<<<1, DET_T, 0, ctx->stream>>>(LU, ld, n, pospivsign, d_out);
   ctx->launches++;
   return la_check_launch(ctx, "det_kernel");
 }
