@@ -140,10 +140,15 @@ trsm_cols8_kernel(double* A, const double* S, size_t ld, int j0, int jb, int c_b
   const int tid = threadIdx.x, col = tid % TC8, r0 = tid / TC8;  // r0 0..31
   const int c = c_begin + blockIdx.x * TC8 + col;
   const bool ok = c < c_end;
-  for (int idx = tid; idx < jb * MAX_PANEL_W; idx += TC8_T) {
-    const int i = idx / MAX_PANEL_W, k = idx % MAX_PANEL_W;
-    if (k < i) L[i][k] = A[(size_t)(j0 + i) * ld + j0 + k];
+  constexpr int PER = MAX_PANEL_W * MAX_PANEL_W / TC8_T;
+  double l[PER];  // all loads in flight together
+#pragma unroll
+  for (int q = 0; q < PER; q++) {
+    const int i = (tid + q * TC8_T) / MAX_PANEL_W, k = tid % MAX_PANEL_W;
+    l[q] = i < jb && k < i ? A[(size_t)(j0 + i) * ld + j0 + k] : 0.0;
   }
+#pragma unroll
+  for (int q = 0; q < PER; q++) L[(tid + q * TC8_T) / MAX_PANEL_W][tid % MAX_PANEL_W] = l[q];
   for (int i = r0; i < jb; i += TC8_T / TC8) {
     x[i][col] = ok ? A[(size_t)(j0 + i) * ld + c] : 0.0;
     if (EXACT) xs[i][col] = ok ? S[(size_t)(j0 + i) * ld + c] : 0.0;
