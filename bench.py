@@ -12,10 +12,10 @@ count 2/3 n^3 + 2 n^2 nrhs (factor + solve).
   e2e   : the public host-pointer API (la_lu_new + la_lu_solve) from pinned
           host memory; the copy of A and B to the device and of X back are
           inside the timed region.
-  roofline : the trailing-update FP64 GEMM (the dominant kernel), its
-          algorithmic flops over its device time (per-phase CUDA events inside
-          the library, from two extra untimed factorizations), against this
-          GPU's FP64 FMA rate measured live.
+  roofline : the trailing updates between blocks (split FP16 products, the
+          dominant kernel), 36 FP16 products per algorithmic FP64 product over
+          their device time (per-phase CUDA events inside the library, from two
+          extra untimed factorizations), against the measured dense tensor rate.
   cpu_baseline : the oracle (a single-threaded restatement of the reference's
           left-looking LUDecomposition::new) timed on a bounded prefix of the
           same factorization on this host.
@@ -63,25 +63,28 @@ def lu_solve_flops(n, nrhs):
     return 2.0 / 3.0 * n ** 3 + 2.0 * n ** 2 * nrhs
 
 
-def trailing_gemm_launches(n, w, lookahead=True):
-    """(M, N, K) of every trailing-update GEMM launch of one LU of a square n
-    with panel width w, as the library issues them: with lookahead each panel
-    updates the next panel's columns first and the rest in a second launch."""
+def trailing_updates(n):
+    """(M, N, K) of every trailing update between the blocks of one FAST LU of a square n: blocks of
+    256 columns while more than 3072 rows remain, 128 above 1024, then 64 (lu_block in lu_api.cu)."""
     out = []
-    for j0 in range(0, n, w):
-        jb = min(w, n - j0)
-        j1 = j0 + jb
-        if j1 >= n:
-            break
-        jbn = min(w, n - j1)
-        m = n - j1
-        if lookahead:
-            out.append((m, jbn, jb))
-            if n - (j1 + jbn) > 0:
-                out.append((m, n - (j1 + jbn), jb))
-        else:
-            out.append((m, n - j1, jb))
+    j0 = 0
+    while j0 < n:
+        rows = n - j0
+        jb = min(256 if rows > 3072 else 128 if rows > 1024 else 64, rows)
+        if j0 + jb < n:
+            out.append((rows - jb, rows - jb, jb))
+        j0 += jb
     return out
+
+
+def measured_fp16_peak():
+    """Dense FP16 tensor rate (TFLOP/s): the BF16 burst rate (the same pipe) measured on these GPUs,
+    from the peaks file beside this script, else one earlier measurement of it."""
+    try:
+        with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")) as f:
+            return float(json.load(f)["bf16_tflops"]), "measured cuBLAS BF16 burst rate"
+    except (OSError, ValueError, KeyError):
+        return 1900.0, "one earlier measurement of the BF16 burst rate"
 
 
 def gemm_algorithmic(launches):
@@ -92,11 +95,13 @@ def gemm_algorithmic(launches):
     return flops, flops / len(launches), nbytes / len(launches)
 
 
-# DRAM traffic of the trailing-update GEMM (gemm_f64_tma_kernel) measured by
-# ncu (dram__bytes_read.sum + dram__bytes_write.sum) over all 253 launches of
-# one n = 8192 factorization of this benchmark's matrix: bytes per launch
-# (mean). Summary and command: profiles/gemm_f64_tma_traffic_n8192.md.
-GEMM_TRAFFIC_BYTES_PER_LAUNCH = 156961959
+SPLIT_PRODUCTS = 36  # FP16 products per FP64 product (pairs of eight digits up to the eighth weight)
+
+# DRAM traffic of the trailing updates' product kernel (gemm_split_kernel) measured by ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum) over its launches in one n = 8192 factorization of a
+# matrix of this size: bytes per launch (mean, with the smaller updates inside the blocks).
+# Summary and command: profiles/gemm_split_n8192.md.
+GEMM_TRAFFIC_BYTES_PER_LAUNCH = None
 
 
 def event_ms(torch, fn, reps=5, warmup=1):
@@ -859,21 +864,23 @@ def run_ours(args):
                                        nrhs, n, nrhs)
 
     # roofline of the trailing-update GEMM: all its launches of one factorization
-    gl = trailing_gemm_launches(n, panel_w, lookahead=bool(ctx.get_option(la_gpu.OPT_LOOKAHEAD)))
+    gl = trailing_updates(n)
     flops_gemm, flops_per_launch, bytes_per_launch = gemm_algorithmic(gl)
     gemm_ms = phases[3] / PK
-    achieved = flops_gemm / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else None
+    fp64_rate = flops_gemm / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else None
+    achieved = SPLIT_PRODUCTS * fp64_rate if fp64_rate else None
+    fp16_peak, fp16_source = measured_fp16_peak()
     roof = {
-        "bound": "fp64", "compute_pipe": "FP64 FMA (DFMA): GB300 has no faster FP64 path "
-                                         "(no FP64 tensor-core rate above it)",
-        "kernel": "gemm_f64_tma_kernel (trailing update A22 -= L21*U12)",
-        "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
-        "frac": (achieved / fp64_peak) if achieved else None,
-        "peak_source": "FP64 FMA issue rate measured live in this process "
-                       "(la_probe_fp64_peak); the measured-peaks file has no FP64 figure",
+        "bound": "tensor", "compute_pipe": "FP16 tensor cores (tcgen05 kind::f16): each FP64 product is "
+                                           "36 exact products of 8-bit digits",
+        "kernel": "gemm_split_kernel with its digit and guard kernels (trailing update A22 -= L21*U12)",
+        "achieved": achieved, "peak": fp16_peak, "unit": "TFLOP/s",
+        "frac": (achieved / fp16_peak) if achieved else None,
+        "peak_source": fp16_source,
+        "fp64_tflops": fp64_rate, "fp64_fma_peak_tflops": fp64_peak,
         "traffic": GEMM_TRAFFIC_BYTES_PER_LAUNCH,
-        "traffic_unit": "DRAM bytes per launch (mean over the factorization's launches), one "
-                        "ncu capture of the same n=8192 factorization",
+        "traffic_unit": "DRAM bytes per launch (mean over the kernel's launches, smaller updates "
+                        "included), one ncu capture of an n=8192 factorization",
         "launches_per_factorization": len(gl),
         "algorithmic_flops_per_launch": flops_per_launch,
         "algorithmic_bytes_per_launch": bytes_per_launch,
@@ -882,8 +889,8 @@ def run_ours(args):
                                        "row_panel_trsm": phases[2] / PK,
                                        "trailing_gemm": phases[3] / PK, "finish": phases[4] / PK,
                                        "note": "device time per phase from 2 untimed, profiled "
-                                               "factorizations; the panel overlaps the "
-                                               "trailing update"},
+                                               "factorizations; finish holds the updates inside "
+                                               "the blocks too"},
     }
 
     # end-to-end through the host-pointer API, copies included

@@ -77,7 +77,7 @@ typedef enum la_option {
   /* 1: record per-phase device times of each LU (la_ctx_last_phase_ms). */
   LA_OPT_PROFILE = 4,
   /* 1 (default): factor the next panel on a second stream while the rest of
-   * the trailing update runs (EXACT LU, mixed LU, Cholesky, QR); 0: strictly
+   * the trailing update runs (EXACT LU, mixed LU, EXACT Cholesky); 0: strictly
    * one phase after the other. Results are bit-identical either way. */
   LA_OPT_LOOKAHEAD = 5,
   /* 1 (default): the FP32 panels of the mixed LU and the panels of the FAST LU

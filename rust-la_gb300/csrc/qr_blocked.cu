@@ -26,7 +26,7 @@
 //                      (the column before its reflection against each later
 //                      column of the block) and the owner of the diagonal row
 //                      publishes that row; every CTA then sums the parts in
-//                      rank order and forms a, u0 = q - a and
+//                      the same order and forms a, u0 = q - a and
 //                      u.t_c = x.t_c - a t_c[diag] identically. At the end the
 //                      block goes back to A with zeros above the diagonal of
 //                      its top square (whose final content is kept in rsave),
@@ -110,6 +110,9 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
   for (int k = 0; k < nb; k++) {
     const int par = k & 1, jc = p.j + k, w = nb - k;
     const int lr0 = max(0, jc - r0);  // first local row at or below the diagonal
+    // sums over parts: L neighbouring lanes per column, L the largest power of two that fits
+    const int L = min(32, 1 << (31 - __clz(QPT / w)));
+    const int col = tid / L, sub = tid % L;
     // x (column k) against columns k..nb-1 (the first is x.x). Thread t takes
     // column k + t % w of the rows lr0 + t / w + G i: every lane of an FP64
     // instruction does useful work whatever w is.
@@ -123,11 +126,13 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
       }
       red[tid] = sacc;
       __syncthreads();
-      if (tid < w) {
-        double t = 0.0;
-        for (int g = 0; g < G; g++) t += red[g * w + tid];
-        mine[tid] = t;
-      }
+      // L lanes per column, then a tree: the G parts one after the other were 19 dependent additions
+      // per column on average, 256 of them in the last.
+      double t = 0.0;
+      if (col < w)
+        for (int g = sub; g < G; g += L) t += red[g * w + col];
+      for (int o = L / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (col < w && sub == 0) mine[col] = t;
       __syncthreads();
     }
     for (int idx = tid; idx < w * CL; idx += QPT) {
@@ -141,18 +146,20 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
         st_remote_f64(remote_addr(&own[par][c], (uint32_t)dst), P[(jc - r0) * QNBP + k + c]);
       }
     cluster_sync();
-    // identical in every CTA: the sums in rank order, a, u0 and the factors
-    if (tid < w) {
+    // identical in every CTA: the sums in one order, a, u0 and the factors
+    {
       double t = 0.0;
-      for (int q = 0; q < CL; q++) t += xch[par][q][tid];
-      tot[tid] = t;
+      if (col < w)
+        for (int q = sub; q < CL; q += L) t += xch[par][q][col];
+      for (int o = L / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (col < w && sub == 0) tot[col] = t;
     }
     __syncthreads();
     const double q = own[par][0];
     const double a = q > 0.0 ? -sqrt(tot[0]) : sqrt(tot[0]);
     const double u0 = q - a;
     if (a != 0.0 && tid > 0 && tid < w) fac[tid] = (tot[tid] - a * own[par][tid]) / (a * u0);
-    if (rank == 0 && tid == 0) {
+    if (rank == 0 && tid == QPT - 1) {  // its own division, in a warp without factors
       p.rdiag[jc] = a;
       p.tau[k] = a != 0.0 ? -1.0 / (a * u0) : 0.0;
     }
