@@ -572,11 +572,11 @@ __device__ __forceinline__ bool solve_diag(const TX (&dg)[16], TX d, TX r, int k
 // block ahead. The other warps update all later rows, one block behind, their
 // loads issued a pass ahead. One barrier per block.
 // What bounds it: warp 0's instructions, a few hundred per block at four to
-// five clocks each. With loads, both updates and a division per row in its
-// path a block took 6200 clocks (FP32, n = 264, one CTA alone on its SM), now 4100; 5400 and 3000 at
-// n = 128. FP64, batches of n up to 256: the solves' share of the SM time 1.67 -> 0.73 G clocks.
-// Not inlined: spills cost an L2 round trip each here, since shared memory
-// leaves the L1 next to nothing.
+// five clocks each, and 64 clocks for each of its FP64 ones. Batches of n up to
+// 256: the solves' share of the SM time 1.67 -> 0.73 G clocks (with loads, both
+// updates and a division per row in warp 0's path before).
+// A function of its own: with 224 KB of shared memory taken the L1 is next to
+// nothing, and a spill in a loop costs an L2 round trip.
 template <typename P, typename TX, bool UPPER>
 __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int* rmap, TX* X,
                                        int nrhs, TX* buf) {
@@ -737,10 +737,108 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
   __syncthreads();
 }
 
+// One row of a block step of the triangular solves: x_i -= f * X_blk over all
+// nrhs right-hand sides, with the row's kbn (<= 16) factor entries f loaded
+// once (16 independent loads in flight) and the block's solved values X_blk
+// read from shared memory (the same address across the warp: a broadcast).
+template <typename P, typename TX>
+__device__ __forceinline__ void solve_row_shared(const typename P::S* frow, int kbn, TX* xi,
+                                                 const TX* xblk, int nrhs) {
+  TX f[16];
+#pragma unroll
+  for (int k = 0; k < 16; k++) f[k] = k < kbn ? (TX)P::ld(&frow[k]) : TX(0);
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    if (c < nrhs) {
+      TX s = xi[c];
+#pragma unroll
+      for (int k = 0; k < 16; k++)
+        if (k < kbn) s = fma(-f[k], xblk[k * nrhs + c], s);
+      xi[c] = s;
+    }
+  }
+}
+
+// X (n x nrhs, pitch nrhs, already in the factor's row order, i.e. P b)
+// <- U^-1 L^-1 X with the stored factors in M. 16-row blocks: warp 0 solves
+// the diagonal block (lanes = rows, two right-hand sides per pass, values
+// passed by shuffles), then all threads update the remaining rows.
+template <typename P, typename TX>
+__device__ void block_solve_shared(const typename P::S* M, int p, int n, const int* rmap, TX* X,
+                            int nrhs) {
+  const int BT = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int li = lane & 15, half = lane >> 4;
+  for (int kb = 0; kb < n; kb += 16) {
+    const int kbn = min(16, n - kb);
+    if (warp == 0) {
+      // lane's row of the diagonal block in registers (16 loads in flight)
+      const typename P::S* lrow = M + (size_t)rmap[kb + min(li, kbn - 1)] * p + kb;
+      TX lv[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) lv[k] = k < kbn ? (TX)P::ld(&lrow[k]) : TX(0);
+      for (int c0 = 0; c0 < nrhs; c0 += 2) {
+        const int c = c0 + half;
+        const bool act = li < kbn && c < nrhs;
+        TX xi = act ? X[(kb + li) * nrhs + c] : TX(0);
+#pragma unroll
+        for (int k = 0; k < 15; k++) {
+          if (k + 1 < kbn) {
+            const TX xk = __shfl_sync(0xffffffffu, xi, (lane & 16) | k);
+            if (act && li > k) xi = fma(-lv[k], xk, xi);
+          }
+        }
+        if (act) X[(kb + li) * nrhs + c] = xi;
+      }
+    }
+    __syncthreads();
+    const int rest = n - kb - kbn;
+    for (int r = tid; r < rest; r += BT)
+      solve_row_shared<P, TX>(M + (size_t)rmap[kb + kbn + r] * p + kb, kbn,
+                              X + (size_t)(kb + kbn + r) * nrhs, X + (size_t)kb * nrhs, nrhs);
+    __syncthreads();
+  }
+  for (int kb = (n - 1) / 16 * 16; kb >= 0; kb -= 16) {
+    const int kbn = min(16, n - kb);
+    if (warp == 0) {
+      const typename P::S* urow = M + (size_t)rmap[kb + min(li, kbn - 1)] * p + kb;
+      TX uv[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) uv[k] = k < kbn ? (TX)P::ld(&urow[k]) : TX(1);
+      for (int c0 = 0; c0 < nrhs; c0 += 2) {
+        const int c = c0 + half;
+        const bool act = li < kbn && c < nrhs;
+        TX xi = act ? X[(kb + li) * nrhs + c] : TX(0);
+#pragma unroll
+        for (int k = 15; k >= 0; k--) {
+          if (k < kbn) {
+            if (act && li == k) xi = xi / uv[k];
+            const TX xk = __shfl_sync(0xffffffffu, xi, (lane & 16) | k);
+            if (act && li < k) xi = fma(-uv[k], xk, xi);
+          }
+        }
+        if (act) X[(kb + li) * nrhs + c] = xi;
+      }
+    }
+    __syncthreads();
+    for (int r = tid; r < kb; r += BT)
+      solve_row_shared<P, TX>(M + (size_t)rmap[r] * p + kb, kbn, X + (size_t)r * nrhs,
+                              X + (size_t)kb * nrhs, nrhs);
+    __syncthreads();
+  }
+}
+
+// FP64 plans have 255 registers per thread and take block_tri. The mixed kernel has 128 (four 4-warp
+// CTAs per SM), in which block_tri and the calls to it spill: 3000 systems of n in [16, 256] took 5.26
+// ms in 4 x 4 warps with it and 3.87 without.
 template <typename P, typename TX>
 __device__ void block_solve(const typename P::S* M, int n, const int* rmap, TX* X, int nrhs, TX* buf) {
-  block_tri<P, TX, false>(M, n, rmap, X, nrhs, buf);
-  block_tri<P, TX, true>(M, n, rmap, X, nrhs, buf);
+  if constexpr (sizeof(TX) == 8) {
+    block_tri<P, TX, false>(M, n, rmap, X, nrhs, buf);
+    block_tri<P, TX, true>(M, n, rmap, X, nrhs, buf);
+  } else {
+    block_solve_shared<P, TX>(M, n, n, rmap, X, nrhs);
+  }
 }
 
 struct BatchArgs {
