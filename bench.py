@@ -101,7 +101,7 @@ SPLIT_PRODUCTS = 36  # FP16 products per FP64 product (pairs of eight digits up 
 # (dram__bytes_read.sum + dram__bytes_write.sum) over its launches in one n = 8192 factorization of a
 # matrix of this size: bytes per launch (mean, with the smaller updates inside the blocks).
 # Summary and command: profiles/gemm_split_n8192.md.
-GEMM_TRAFFIC_BYTES_PER_LAUNCH = None
+GEMM_TRAFFIC_BYTES_PER_LAUNCH = 69851569
 
 
 def event_ms(torch, fn, reps=5, warmup=1):

@@ -64,9 +64,14 @@ laswp_lists_kernel(T* A, size_t ld, const int* __restrict__ swaps, int lists, in
   constexpr int G = 256 / SW_COLS, PER = 2 * MAX_PANEL_W / G;  // move groups, moves per thread
   const int c = c0 + blockIdx.x * SW_COLS + threadIdx.x % SW_COLS;
   const int g = threadIdx.x / SW_COLS;
-  const bool ok = c < c1 && !aborted(err);
+  // every list's length at once; lists without moves cost nothing then
+  __shared__ int s_cnt[SWAP_LISTS];
+  if ((int)threadIdx.x < lists) s_cnt[threadIdx.x] = aborted(err) ? 0 : swaps[threadIdx.x * SWAP_STRIDE];
+  __syncthreads();
+  const bool ok = c < c1;
   for (int s = 0; s < lists; s++, swaps += SWAP_STRIDE) {
-    const int cnt = swaps[0];
+    const int cnt = s_cnt[s];
+    if (cnt == 0) continue;
     T v[PER];
 #pragma unroll
     for (int i = 0; i < PER; i++)
