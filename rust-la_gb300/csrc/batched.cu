@@ -13,9 +13,10 @@
 //   integers and the final map is the permutation P (lu.rs:245-254);
 //   solves for B_i and writes X_i.
 // Per 16-column panel: the panel is staged in shared memory in the arithmetic
-// type, factored column by column in registers (panel_regs), written back; U12 = L11^-1 A12 is solved with each column in
-// registers; A22 -= L21 U12 is register-tiled (a thread holds 4x4 of A22 and
-// its rows of L21, all loads of a tile are issued before its FMAs).
+// type, factored column by column in registers (panel_regs), written back;
+// U12 = L11^-1 A12 is solved with each column in registers; A22 -= L21 U12 is
+// register-tiled (a thread holds 4x4 of A22 and its rows of L21, all loads of a
+// tile are issued before its FMAs).
 // The working matrix is stored in the system's factor precision: FP64 (plain
 // pass), FP32, BF16 or FP8 e4m3 (mixed pass; FP8 with a power-of-two scale of
 // A_i), with FP32 arithmetic for the low precisions. Narrower storage keeps
@@ -226,18 +227,19 @@ __device__ __forceinline__ int panel_best(unsigned long long key, int pos) {
 }
 
 // Factors the staged panel (prow rows, jb columns, staged row s of logical position s) with each
-// thread's RPT rows in registers, on the CTA's first W warps; staged rows hold the factors on return, perm the row at each
-// position, and rmap[0..jb) takes the row interchanges (prow <= 32 RPT W). The other warps skip it:
-// fewer warps with more rows each repeat less of a column's search, and one warp needs no barrier.
+// thread's RPT rows in registers, on the CTA's first W warps; staged rows hold the factors on return,
+// perm the row at each position, and rmap[0..jb) takes the row interchanges (prow <= 32 RPT W). The
+// other warps skip it: fewer warps with more rows each repeat less of a column's search, and one warp
+// needs no barrier.
 //   Column jj sits in register slot 0 (the window moves by one slot per column, so there is one copy
 //   of the loop body and every register index is static). Each warp's best candidate writes its row
 //   to its place in st, one barrier, then every warp picks the winner from the warps' candidates and
-//   takes the pivot row from st. A row's multiplier goes to st as it is formed. Written as in the
-//   loop of block_lu that this replaces: the same operations on every value.
+//   takes the pivot row from st. A row's multiplier goes to st as it is formed. Every value takes the
+//   operations of the loop over rows in st that block_lu keeps for taller panels.
 //   What bounds it: the chain of one column (two warp reductions, a barrier, the reciprocal, the next
-//   column). With the rows in shared memory, a 64-bit shuffle tree and a serial scan of the warps'
-//   candidates, a column took 3700 clocks in FP32 (n up to 512, two CTAs per SM) and 4500 in FP64 (n up
-//   to 256); now 1900 and 2800, at four to five clocks per instruction of a warp.
+//   column) at four to five clocks per instruction of a warp. With the rows in shared memory, a 64-bit
+//   shuffle tree and a serial scan of the warps' candidates, a column took 3700 clocks in FP32 (n up to
+//   512, two CTAs per SM) and 4500 in FP64 (n up to 256); now 1900 and 2800.
 template <typename R, int RPT>
 __device__ __forceinline__ void panel_regs(R* st, int prow, int jb, int W, int* perm, int* rmap,
                                         Shared* shp) {
@@ -387,9 +389,9 @@ __device__ void block_lu(typename P::S* M, int p, int n, int* rmap, typename P::
       spos[r] = r;
     }
     __syncthreads();
-    // Warps and rows per thread of the panel. FP32: four rows per thread from 65 rows on. FP64: the
-    // updates take the FP64 pipes, so the rows go over as many warps as there are. Beyond four rows per
-    // thread (two-warp CTAs with n > 256) they stay in st.
+    // Warps and rows per thread of the panel: two rows per thread in FP32 from 33 rows on; in FP64 the
+    // updates take the FP64 pipes, so the rows go over as many warps as there are. Panels beyond two
+    // rows per thread of the CTA stay in st.
     const int rpt = sizeof(R) == 8 ? (prow + BT - 1) / BT : (prow + 31) / 32;
     const int PR = rpt <= 1 ? 1 : 2, W = (prow + 32 * PR - 1) / (32 * PR);
     if (W <= NW) {

@@ -3,7 +3,7 @@
 // Three schedules that apply every term in the same order, so their results are
 // bit-identical:
 //
-// Wavefront (default). One persistent launch per triangle. The rows are cut
+// Wavefront (more right-hand sides than the chain takes). One persistent launch per triangle. The rows are cut
 // into 32-row blocks and the right-hand sides into groups of 4 columns; a work
 // item is (row block, column group), taken by CTAs from an atomic ticket in
 // dependency order (forward: top block first; backward: bottom block first),
@@ -31,7 +31,7 @@
 // 32-column chunks. Used for more than 4 * SOLVE_WAVE_MAX_GROUPS right-hand
 // sides or when the wavefront is switched off.
 //
-// Order of the terms of row i (both schedules): forward (unit L, lu.rs:257-263)
+// Order of the terms of row i (every schedule): forward (unit L, lu.rs:257-263)
 // ascending k; backward (U, lu.rs:266-275) descending k, then the division by
 // u_ii. EXACT applies each term as x_i = x_i - x_k * l_ik without fusion and
 // divides; FAST uses FMA and multiplies by the reciprocal of u_ii (quot).
