@@ -33,8 +33,11 @@
 // leading two digits by mma.sync (a few microseconds, where the FMA tile of K = 256 takes 1 ms; as
 // FP32 FMAs they took 65 us for K = 700, a tenth of the FMA tiles that may follow). Every other
 // tile (graded or sparse operands, values that are not finite or beyond 2^+-400) goes on a list that
-// the epilogue warps work off at the end of the product (fma_tiles), with FMA chains in ascending k
-// and 64 x 64 tiles as in gemm_f64.cu.
+// the epilogue warps work off at the end of the product (fma_tiles), with FMA chains in ascending k,
+// in pieces small enough that every SM has some. Where all tiles are on the list (graded along k), us,
+// by the FMA kernels of gemm_f64.cu alone, with 64 x 64 pieces here, and now: 100 x 64 x 100 88, 115,
+// 57; 64 x 1936 x 436 1967, 2209, 333; 2048^3 14253, 15371, 14265; 4096^3 109.8 ms, 118.5, 113.3 (the
+// sums that reject the tiles are 2 % of it).
 //
 // Measured on 8192^3 (A and B N(0,1)): 24.0 ms against 876.6 ms by FMA, 36 x 2 x 8192^3 FP16
 // operations in all, 1.65 PFLOP/s; rms error against quadruple precision 5 to 17 times smaller than
@@ -80,8 +83,7 @@ constexpr int EXP_LIMIT = 400;        // |ea|, |eb| the digits are used for
 constexpr int LARGE_BITS = 4;         // "large": exponent within 4 of the largest (2^-5 of the scale)
 constexpr float GUARD = 0.0021f;      // 2^-8.9
 constexpr int CNT_BAD = -(1 << 29);   // count of a row the digits cannot represent
-constexpr int FT = 64, FK = 16;       // FMA tiles: 64 x 64 in slabs of 16 k
-static_assert(2 * 2 * FK * FT * 8 <= EPI_BYTES, "the FMA slabs reuse the epilogue's buffer");
+constexpr int FR = 64, FC = 16, FK = 32;  // FMA pieces: up to 64 rows, 16 columns, slabs of 32 k
 
 using la_tma::mbar_init;
 using la_tma::smem_u32;
@@ -435,14 +437,20 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 
 // fits[tile] (see the head of the file), and the list of the others. A warp per tile compares the
 // counts; the tiles they do not decide are summed by the whole CTA, one after the other.
-constexpr int GUARD_T = 256;
-__global__ void __launch_bounds__(GUARD_T)
+// The sums are a chain of loads through L2. Where K is long, SETS = 2 sets of 8 warps take every second
+// slab of k each, two slabs' loads in flight (7 tiles of K = 1936: 177 us with one set, 76 with two); for
+// short ones, of a few slabs, one set leaves room for two CTAs per SM.
+constexpr int GUARD_W = 8;  // warps of a set, tiles of a CTA at most
+constexpr int GUARD_LONG_K = 1024;
+template <int SETS>
+__global__ void __launch_bounds__(SETS * GUARD_W * 32)
 guard_kernel(const __grid_constant__ SplitArgs p) {
   la_pdl_wait();
   la_pdl_trigger();
-  __shared__ int s_sum[GUARD_T / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  {
+  __shared__ int s_sum[GUARD_W];
+  __shared__ float s_acc[SETS > 1 ? 32 : 1][GUARD_W * 32];  // the second set's sums
+  const int tid = threadIdx.x, lane = tid & 31, set = tid / (GUARD_W * 32), warp = tid / 32 % GUARD_W;
+  if (set == 0) {
     const int t = blockIdx.x * p.per_cta + warp;
     int sum = 0;
     if (warp < p.per_cta && t < p.tiles) {
@@ -471,7 +479,7 @@ guard_kernel(const __grid_constant__ SplitArgs p) {
     if (lane == 0) s_sum[warp] = sum;
   }
   __syncthreads();
-  for (int w = 0; w < GUARD_T / 32; w++) {
+  for (int w = 0; w < GUARD_W; w++) {
     if (!s_sum[w]) continue;
     const int t = blockIdx.x * p.per_cta + w;
     int tm, tn;
@@ -484,7 +492,8 @@ guard_kernel(const __grid_constant__ SplitArgs p) {
     const int row0 = tm * PM + warp / 2 * 32 + g, col0 = tn * PN + warp % 2 * 32 + g;
     const size_t sa = (size_t)p.M * p.kp, sb = (size_t)p.N * p.kp;
     float acc[2][4][4] = {};
-    for (int k0 = 0; k0 < p.K; k0 += 32) {
+#pragma unroll SETS
+    for (int k0 = 32 * set; k0 < p.K; k0 += 32 * SETS) {
       uint4 a[4], b[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) {
@@ -499,18 +508,23 @@ guard_kernel(const __grid_constant__ SplitArgs p) {
           mma_16816(acc[i][j], a[2 * i].z, a[2 * i + 1].z, a[2 * i].w, a[2 * i + 1].w, b[j].z, b[j].w);
         }
     }
+    float* const other = &s_acc[0][tid % (GUARD_W * 32)];
+    if (SETS > 1) {
+      if (set != 0)
+#pragma unroll
+        for (int i = 0; i < 32; i++) other[i * GUARD_W * 32] = acc[i / 16][i / 4 % 4][i % 4];
+      __syncthreads();
+    }
     const float need = GUARD * sqrtf((float)p.K);
     bool ok = true;
+    if (set == 0)
 #pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int r = row0 + 16 * i + 8 * (e >> 1);
-          const int c = col0 - g + 8 * j + 2 * (lane & 3) + (e & 1);
-          if (r < p.M && c < p.N) ok = ok && acc[i][j][e] >= need;
-        }
+      for (int i = 0; i < 32; i++) {
+        const int r = row0 + i / 16 * 16 + i % 4 / 2 * 8;
+        const int c = col0 - g + i / 4 % 4 * 8 + 2 * (lane & 3) + i % 2;
+        const float v = acc[i / 16][i / 4 % 4][i % 4] + (SETS > 1 ? other[i * GUARD_W * 32] : 0.f);
+        if (r < p.M && c < p.N) ok = ok && v >= need;
+      }
     const bool fit = __syncthreads_and(ok ? 1 : 0) != 0;
     if (tid == 0) {
       p.fits[t] = fit ? 1 : 0;
@@ -555,80 +569,129 @@ __device__ __forceinline__ double round_sum(Sum96 a, int sc) {
   return hi == 0u ? 0.0 : __hiloint2double((int)rh, (int)rl);
 }
 
-__device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_T) : "memory"); }
+// The listed tiles by FMA chains in ascending k, in pieces of 16 NI rows and 16 columns. Each of four
+// groups of four epilogue warps takes pieces of its own, with its own barrier and buffers: one warp per
+// sub-partition with 2 NI chains per thread keeps the FP64 pipe (two FMAs per clock and SM) busy by
+// itself, and while one group fetches or waits the others have the pipe. Slabs come by 8-byte cp.async
+// (any alignment), one ahead, into the stages' shared memory: nothing is in flight there any more.
+constexpr int FG_T = 128;                      // threads of a group
+constexpr int FSLAB = FK * (FR + FC);          // doubles of a slab: A [k][row ^ k], B [k][column ^ k]
+static_assert((size_t)(EPI_T / FG_T) * 2 * FSLAB * 8 <= (size_t)NST * PST_BYTES, "slabs in the stages");
 
-// The listed tiles by FMA chains in ascending k, in halves of 64 x 64, by the epilogue's 512
-// threads: thread (tx, ty) owns rows ty + 32 i and columns tx + 16 j. The next slab's values wait in
-// registers while the present one is used; the FP64 pipe (two FMAs per clock) hides the rest. buf:
-// two slabs of A and of B.
-template <int MODE>
-__device__ __noinline__ void fma_tiles(const SplitArgs& p, double* buf, int tid) {
-  double(*as)[FK][FT] = reinterpret_cast<double(*)[FK][FT]>(buf);
-  double(*bs)[FK][FT] = reinterpret_cast<double(*)[FK][FT]>(buf + 2 * FK * FT);
-  const int items = 2 * p.splits * *reinterpret_cast<volatile int*>(p.list);
-  const int tx = tid & 15, ty = tid >> 4;
-  for (int it = blockIdx.x; it < items; it += gridDim.x) {
+// Set where a wait of an epilogue warp gave up.
+__device__ __forceinline__ volatile int& gave_up() {
+  __shared__ volatile int flag;
+  return flag;
+}
+// The group's barrier; whether `ok` holds in all of its threads.
+__device__ __forceinline__ bool group_all(int g, bool ok) {
+  unsigned r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n"
+      " barrier.cta.red.and.aligned.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u), "r"(1 + g), "n"(FG_T)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(1 + g), "n"(FG_T) : "memory");
+}
+__device__ __forceinline__ void fetch8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
+// Pieces of the first tile, which is the largest: row pieces of 16 NI, column pieces.
+__device__ __forceinline__ int piece_rows(const SplitArgs& p, int R) { return (min(PM, p.M) + R - 1) / R; }
+__device__ __forceinline__ int piece_cols(const SplitArgs& p) { return (min(PN, p.N) + FC - 1) / FC; }
+
+template <int MODE, int NI>
+__device__ __forceinline__ void fma_pieces(const SplitArgs& p, double* smem, int tid, int count) {
+  const int g = tid / FG_T, t = tid % FG_T, tx = t & 7, ty = t >> 3;
+  double* const buf = smem + g * 2 * FSLAB;
+  const int hn = piece_cols(p), per = piece_rows(p, 16 * NI) * hn;
+  const int items = count * p.splits * per;
+  for (int it = g * gridDim.x + blockIdx.x; it < items; it += EPI_T / FG_T * gridDim.x) {
+    const int q = it % per, z = it / per % p.splits;
     int tm, tn;
-    tile_at(p, p.list[1 + it / (2 * p.splits)], tm, tn);
-    const int z = it / 2 % p.splits;
+    tile_at(p, p.list[1 + it / (per * p.splits)], tm, tn);
+    const int m0 = tm * PM + q / hn * 16 * NI, n0 = tn * PN + q % hn * FC;
+    if (m0 >= p.M || n0 >= p.N) continue;
     const int kb = z * p.kper, ke = min(p.K, kb + p.kper);
-    double* C = p.C + z * p.czs;
-    const int m0 = tm * PM + (it & 1) * FT, n0 = tn * PN;
-    double acc[2][4], ra[2], rb[2];
+    double* const C = p.C + z * p.czs;
+    auto fetch = [&](int k0, double* slab) {
+#pragma unroll 4
+      for (int j = 0; j < 4 * NI; j++) {
+        const int k = t % FK, r = t / FK + j * (FG_T / FK);
+        const bool in = m0 + r < p.M && k0 + k < ke;
+        fetch8(slab + k * FR + (r ^ k), in ? p.A + (size_t)(m0 + r) * p.lda + k0 + k : p.A, in);
+      }
+      double* const b = slab + FK * FR;
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+      for (int j = 0; j < FK * FC / FG_T; j++) {
+        const int e = t + j * FG_T;
+        const int k = p.b_rows ? e % FK : e / FC, c = p.b_rows ? e / FK : e % FC;
+        const bool in = n0 + c < p.N && k0 + k < ke;
+        const size_t at = p.b_rows ? (size_t)(n0 + c) * p.ldb + k0 + k : (size_t)(k0 + k) * p.ldb + n0 + c;
+        fetch8(b + k * FC + (c ^ (k % FC)), in ? p.B + at : p.B, in);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    group_sync(g);  // the buffers' last readers are done
+    fetch(kb, buf);
+    double acc[NI][2];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int r = m0 + ty + 32 * i, c = n0 + tx + 16 * j;
+    for (int i = 0; i < NI; i++)
+#pragma unroll
+      for (int j = 0; j < 2; j++) {
+        const int r = m0 + ty + 16 * i, c = n0 + tx + 8 * j;
         acc[i][j] = MODE != 0 && r < p.M && c < p.N ? C[(size_t)r * p.ldc + c] : 0.0;
       }
-    auto fetch = [&](int k0) {
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int e = tid + q * EPI_T;
-        const int r = e / FK, k = e % FK;
-        ra[q] = m0 + r < p.M && k0 + k < ke ? p.A[(size_t)(m0 + r) * p.lda + k0 + k] : 0.0;
-        if (p.b_rows)
-          rb[q] = n0 + r < p.N && k0 + k < ke ? p.B[(size_t)(n0 + r) * p.ldb + k0 + k] : 0.0;
-        else
-          rb[q] = n0 + e % FT < p.N && k0 + e / FT < ke
-                      ? p.B[(size_t)(k0 + e / FT) * p.ldb + n0 + e % FT] : 0.0;
-      }
-    };
-    epi_sync();  // the buffer's last users are done
-    fetch(kb);
     for (int k0 = kb, b = 0; k0 < ke; k0 += FK, b ^= 1) {
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int e = tid + q * EPI_T;
-        as[b][e % FK][(e / FK) ^ (e % FK)] = ra[q];
-        const int k = p.b_rows ? e % FK : e / FT, c = p.b_rows ? e / FK : e % FT;
-        bs[b][k][c ^ k] = rb[q];
-      }
-      epi_sync();  // the other buffer's readers of two slabs ago are done, too
-      if (k0 + FK < ke) fetch(k0 + FK);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      group_sync(g);  // the slab is there, and the other buffer's readers are done
+      if (k0 + FK < ke) fetch(k0 + FK, buf + (b ^ 1) * FSLAB);
+      const double *as = buf + b * FSLAB, *bs = as + FK * FR;
       const int kn = min(FK, ke - k0);
 #pragma unroll 4
       for (int k = 0; k < kn; k++) {
-        double a[2], v[4];
+        double a[NI], v[2];
 #pragma unroll
-        for (int i = 0; i < 2; i++) a[i] = as[b][k][(ty + 32 * i) ^ k];
+        for (int i = 0; i < NI; i++) a[i] = as[k * FR + ((ty + 16 * i) ^ k)];
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = bs[b][k][(tx + 16 * j) ^ k];
+        for (int j = 0; j < 2; j++) v[j] = bs[k * FC + ((tx + 8 * j) ^ (k % FC))];
 #pragma unroll
-        for (int i = 0; i < 2; i++)
+        for (int i = 0; i < NI; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fma(MODE < 0 ? -a[i] : a[i], v[j], acc[i][j]);
+          for (int j = 0; j < 2; j++) acc[i][j] = fma(MODE < 0 ? -a[i] : a[i], v[j], acc[i][j]);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < NI; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int r = m0 + ty + 32 * i, c = n0 + tx + 16 * j;
+      for (int j = 0; j < 2; j++) {
+        const int r = m0 + ty + 16 * i, c = n0 + tx + 8 * j;
         if (r < p.M && c < p.N) C[(size_t)r * p.ldc + c] = acc[i][j];
       }
   }
+}
+
+// The pieces are as high as the number of them allows: the most loaded SM decides (R rows of 16 columns
+// take it 8 R clocks per k), and a lower piece loads more per FMA.
+template <int MODE>
+__device__ __noinline__ void fma_tiles(const SplitArgs& p, double* epi, int tid) {
+  double* const smem = epi - NST * PST_BYTES / sizeof(double);
+  const int count = *reinterpret_cast<volatile int*>(p.list);
+  if (!group_all(tid / FG_T, gave_up() == 0)) return;
+  const long long n = (long long)count * p.splits * piece_cols(p);
+  auto cost = [&](int R) {
+    return ((n * piece_rows(p, R) + gridDim.x - 1) / (int)gridDim.x) * (R + 2);
+  };
+  const long long c64 = cost(64), c32 = cost(32), c16 = cost(16);
+  if (c64 <= c32 && c64 <= c16) fma_pieces<MODE, 4>(p, smem, tid, count);
+  else if (c32 <= c16) fma_pieces<MODE, 2>(p, smem, tid, count);
+  else fma_pieces<MODE, 1>(p, smem, tid, count);
 }
 
 // MODE -1: C -= A B, 0: C = A B, 1: C += A B.
@@ -641,12 +704,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
   extern __shared__ __align__(1024) unsigned char split_raw[];
   __shared__ __align__(8) uint64_t full[NST], empty[NST], acc_full[2], acc_empty[2], last;
   __shared__ uint32_t tmem_holder;
-  __shared__ volatile int s_fail;
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(split_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int total = p.tiles * p.splits;
-  // The grid has a CTA for every FMA half of small products; without FMA tiles they are done here.
+  // The grid has a CTA for every FMA piece of small products; without FMA tiles they are done here.
   if (blockIdx.x >= total && *reinterpret_cast<volatile int*>(p.list) == 0) return;
   // Item t: tile t % tiles of piece t / tiles, whose stages are s0, s0 + 1, ... (nst of them).
   auto item = [&](int t, int& tile, int& z, int& s0) {
@@ -666,7 +728,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
       mbar_init(&acc_empty[h], EPI_WARPS);
     }
     mbar_init(&last, 1);
-    s_fail = 0;
+    gave_up() = 0;
     la_tma::mbar_init_fence();
   }
   if (warp == 0) {
@@ -698,7 +760,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
         for (int s = 0; s < nst; s++, n++) {
           const int b = n % NST;
           if (n >= NST && !sw_wait(&empty[b], (uint32_t)((n / NST - 1) & 1), p.err)) {
-            s_fail = 1;
             ok = false;
             break;
           }
@@ -746,10 +807,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
               }
             if (end) tc_commit(&acc_full[h]);
           }
-          if (!ok) {
-            s_fail = 1;
-            break;
-          }
+          if (!ok) break;
           tc_commit(&empty[b]);
           if (end) chunk++;
         }
@@ -837,8 +895,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant_
         __syncwarp();
       }
     }
-    if (!ok) s_fail = 1;
-    // every epilogue warp comes here, whatever its waits gave, and the list is the same for all
+    if (!ok) gave_up() = 1;
+    // Every epilogue warp comes here, whatever its waits gave, and the list is the same for all. A warp
+    // whose waits all ended has seen the last of the CTA's MMAs complete, and with them its copies.
+    __syncwarp();
     if (*reinterpret_cast<volatile int*>(p.list) != 0)
       fma_tiles<MODE>(p, reinterpret_cast<double*>(smem + NST * PST_BYTES), tid);
   }
@@ -873,11 +933,17 @@ la_status launch_product(la_ctx ctx, cudaStream_t st, const CUtensorMap& ta, con
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SPLIT_SMEM);
   });
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaFuncSetAttribute(gemm_split)");
-  e = la_launch(ctx, guard_kernel, dim3((p.tiles + p.per_cta - 1) / p.per_cta), dim3(GUARD_T), 0, st,
-                p);
+  const bool lng = p.K >= GUARD_LONG_K;
+  e = la_launch(ctx, lng ? guard_kernel<2> : guard_kernel<1>, dim3((p.tiles + p.per_cta - 1) / p.per_cta),
+                dim3((lng ? 2 : 1) * GUARD_W * 32), 0, st, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "guard_kernel launch");
-  e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(std::min(2 * p.tiles * p.splits, ctx->sm_count)),
-                dim3(SPLIT_T), SPLIT_SMEM, st, ta, tb, p);
+  // CTAs beyond the tiles are for the FMA pieces (up to 32 of a tile) and leave at once without any. In
+  // the factorizations, chains of dependent launches with updates of K <= 256, each of them also keeps the
+  // next kernel's CTAs from being placed early: Cholesky of order 4099 7.70 ms with 32 CTAs at least,
+  // 7.74 with 64, 8.27 with 120, 9.5 with all 152.
+  const int items = p.tiles * p.splits, most = ctx->pdl_now && p.K <= 256 ? 32 : ctx->sm_count;
+  const int grid = std::min(std::max(2 * items, std::min(32 * items, most)), ctx->sm_count);
+  e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(grid), dim3(SPLIT_T), SPLIT_SMEM, st, ta, tb, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "gemm_split_kernel launch");
   ctx->launches += 2;
   return la_check_launch(ctx, "gemm_split_kernel");
@@ -975,7 +1041,7 @@ la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N,
   p.cb = sb.cnt;
   p.prefetch = mode != 0;
   // tiles per CTA of the guard: one while that leaves SMs free, up to eight
-  p.per_cta = std::min(GUARD_T / 32, 1 + p.tiles / (4 * ctx->sm_count));
+  p.per_cta = std::min(GUARD_W, 1 + p.tiles / (4 * ctx->sm_count));
   p.da = sa.dig;
   p.db = sb.dig;
   p.kp = kp;
