@@ -267,6 +267,7 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
                            size_t ldt, int cols);
 la_status launch_panel(la_ctx ctx, cudaStream_t stream, bool exact, double* A, double* S,
                        size_t ld, int m, int j0, int jb, int* d_ipiv, unsigned* bar_base);
+constexpr int PANEL64_ROWS = 8192;  // most rows of a FAST panel on one cluster (EXACT: half of them)
 la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t stream, double* A, const double* S,
                                  size_t ld, int m, int j0, int jb, int* d_ipiv);
 // C -= A B or C = A B (mode GM_FMA_SUB, GM_FMA_ZERO) with tiles of 16 columns.

@@ -78,7 +78,8 @@ constexpr size_t GEMM_SMEM_WITH_PANEL = 78 * 1024;
 
 // FAST factorization of h->d_lu in place. Blocks of LU_BASE = 64 columns are factored in panels of at
 // most 32:
-//   panel : cluster kernel (panel_cluster64.cu), the cooperative one (lu_panel.cu) beyond 8192 rows
+//   panel : cluster kernel (panel_cluster64.cu); beyond 8192 rows the cooperative one (lu_panel.cu), on
+//           all 64 columns
 //   swaps of the panel on all other columns
 //   inner : triangular solve and FMA update of the block's remaining columns (32 x 32, K = 32)
 // and a wider block is its left half, that half's triangular solve and update of the right half,
@@ -238,11 +239,16 @@ struct FastLu {
       t.end(ctx->stream, b, PH_OTHER);
       return factor(mid, b1);
     }
-    for (int j0 = b0; j0 < b1; j0 += W) {
-      const int jb = std::min(W, b1 - j0), j1 = j0 + jb;
+    for (int j0 = b0, jb; j0 < b1; j0 += jb) {
+      // The cooperative kernel takes the block in one piece (in halves, with the swaps, triangle and
+      // update between them, 50000 x 64 took 845 us instead of 769, 9000 x 33 290 instead of 262).
+      const bool cluster = ctx->cluster_panels && (ctx->panel_ctas == 0 || ctx->split_ws) &&
+                           m - j0 <= PANEL64_ROWS;
+      jb = std::min(cluster ? W : ctx->panel_width, b1 - j0);
+      const int j1 = j0 + jb;
       size_t b = t.begin(ctx->stream);
       la_status s = LA_UNSUPPORTED;
-      if (ctx->cluster_panels && (ctx->panel_ctas == 0 || ctx->split_ws))
+      if (cluster)
         s = launch_panel_cluster64(ctx, ctx->stream, A, nullptr, ld, m, j0, jb, ipiv);
       if (s == LA_UNSUPPORTED)
         s = launch_panel(ctx, ctx->stream, false, A, nullptr, ld, m, j0, jb, ipiv, &bar_base);

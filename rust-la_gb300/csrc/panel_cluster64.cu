@@ -467,7 +467,8 @@ la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t st, double* A, const d
                                  int m, int j0, int jb, int* d_ipiv) {
   const int R = m - j0;
   if (R <= 0 || jb <= 0) return LA_OK;
-  if (jb > PW || R > PMAXC * (S ? 256 : 512)) return LA_UNSUPPORTED;
+  static_assert(PANEL64_ROWS == PMAXC * 512, "rows of the largest CTA");
+  if (jb > PW || R > PANEL64_ROWS / (S ? 2 : 1)) return LA_UNSUPPORTED;
   // 32 rows per CTA until the cluster is full (R = 256: 51 us, with 128 rows per CTA 82)
   int C = 1;
   while (C < PMAXC && R > C * 32) C *= 2;
