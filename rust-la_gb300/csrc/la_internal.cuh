@@ -153,6 +153,7 @@ struct la_lu_handle {
   uint64_t* d_piv = nullptr;     // permutation vector (lu.rs piv), length m
   int pospivsign = 1;
   int zero_diag = 0;             // an exact 0 on U's diagonal (j < min(m,n))
+  int uneven = 0;                // sampled rows of U that lie unevenly (see lu_finish_kernel)
   int arith = LA_ARITH_FAST;
   // Mixed-precision factorization: FP32 factors (d_lu32, pitch ld32) of the
   // FP64 matrix kept in d_lu (used for residuals); null for plain FP64.
@@ -302,10 +303,12 @@ la_status launch_trsv_wave_f32(la_ctx ctx, const float* LU, size_t ld, const dou
 la_status launch_invert_diag_f32f(la_ctx ctx, const float* LU, size_t ld, int n, float* dinv);
 la_status launch_trsv_wave_f32f(la_ctx ctx, const float* LU, size_t ld, const float* dinv,
                                 float* X, size_t ldx, int n, int nrhs, int* sync);
-la_status launch_lu_finish(la_ctx ctx, la_lu h, int* d_flags);
+// d_uneven (square FP64 factors, else null): how many sampled rows of U lie unevenly.
+la_status launch_lu_finish(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven);
 // Enqueues the whole factorization of h (no readback, no synchronization);
-// lu_finish writes {pospivsign, zero-on-diagonal} to d_flags.
-la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags);
+// lu_finish writes {pospivsign, zero-on-diagonal} to d_flags and, where asked
+// for, the uneven rows to d_uneven.
+la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven);
 la_status launch_tri_wave(la_ctx ctx, bool exact, bool upper, bool divide, const double* T,
                           size_t ld, double* X, size_t ldx, int n, int nrhs);
 la_status launch_lu_solve(la_ctx ctx, bool exact, const double* LU, size_t ld, double* X,

@@ -135,6 +135,8 @@ constexpr int SOLVE_BASE = 256;  // 128: 4.02 ms
 // Inverses, ms, wavefront and blocked: n = 500 1.64, 1.67; 600 2.10, 2.19; 700 2.65, 2.55; 800 3.28,
 // 2.92; 1000 4.98, 3.82; 2500 42.3, 14.7.
 constexpr size_t INVERSE_BLOCKED_N = 672;
+constexpr size_t SOLVE_BLOCKED_N = 512;
+constexpr int SOLVE_UNEVEN = 1;  // of up to 31 sampled rows: a few scattered ones reach most tiles
 struct BlockedSolve {
   la_ctx ctx;
   const double* A;
@@ -270,7 +272,7 @@ struct FastLu {
   }
 };
 
-la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
+la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
   FastLu f(ctx, h);
   const int m = f.m, n = f.n, kmin = std::min(m, n);
   cudaStream_t st = ctx->stream;
@@ -303,7 +305,7 @@ la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
   }
   ctx->pdl_now = false;
   size_t b = f.t.begin(st);
-  LA_TRY(launch_lu_finish(ctx, h, d_flags));
+  LA_TRY(launch_lu_finish(ctx, h, d_flags, d_uneven));
   f.t.end(st, b, PH_OTHER);
   if (f.t.on) {
     LA_CUDA(ctx, cudaStreamSynchronize(st));
@@ -324,8 +326,8 @@ la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
 // columns >= j2 and reads L21 (columns < j1) and U12 (rows < j1).
 }  // namespace
 
-la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
-  if (h->arith != LA_ARITH_EXACT) return lu_fast_enqueue(ctx, h, d_flags);
+la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
+  if (h->arith != LA_ARITH_EXACT) return lu_fast_enqueue(ctx, h, d_flags, d_uneven);
   const bool exact = true;
   const int m = (int)h->m, n = (int)h->n;
   const size_t ld = h->ld;
@@ -430,7 +432,7 @@ la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags) {
   }
   // m < n: the columns right of the last panel got their triangular update above.
   size_t b = t.begin(ms);
-  LA_TRY(launch_lu_finish(ctx, h, d_flags));
+  LA_TRY(launch_lu_finish(ctx, h, d_flags, d_uneven));
   t.end(ms, b, PH_OTHER);
   if (t.on) {
     LA_CUDA(ctx, cudaStreamSynchronize(ms));
@@ -445,13 +447,15 @@ namespace {
 
 la_status lu_factor(la_ctx ctx, la_lu h) {
   int* d_flags = reinterpret_cast<int*>(ctx->d_small);
-  LA_TRY(lu_factor_enqueue(ctx, h, d_flags));
+  const bool look = h->arith == LA_ARITH_FAST && h->m == h->n && h->n >= SOLVE_BLOCKED_N;
+  LA_TRY(lu_factor_enqueue(ctx, h, d_flags, look ? d_flags + 2 : nullptr));
   int* flags = static_cast<int*>(ctx->h_pinned);
-  LA_CUDA(ctx, cudaMemcpyAsync(flags, d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+  LA_CUDA(ctx, cudaMemcpyAsync(flags, d_flags, 3 * sizeof(int), cudaMemcpyDeviceToHost,
                                ctx->stream));
   LA_TRY(la_sync_and_check(ctx, "lu factorization"));
   h->pospivsign = flags[0];
   h->zero_diag = flags[1];
+  if (look) h->uneven = flags[2];
   return LA_OK;
 }
 
@@ -497,8 +501,13 @@ la_status lu_solve_inplace(la_ctx ctx, la_lu h, double* X, size_t ldx, int nrhs)
   // right-hand sides 439, 429; 1000: 751, 594. n = 1000: 256: 766, 922; 512: 1321, 959; 1000: 2466, 1299.
   // n = 2500: 192: 2835, 2922; 256: 3643, 2958. n = 6000: 64: 5497, 6553; 128: 10042, 6915; 1000: 74520,
   // 9991. Backward errors 4 to 10 times smaller. Without memory for the digits: the wavefront.
-  if (h->arith == LA_ARITH_FAST && ctx->solve_wave > 0 && !ctx->split_ws && n >= 512 && nrhs >= 64 &&
-      (long long)n * nrhs >= 500000) {
+  // Where U's rows lie unevenly the products' tiles are FMA chains, and the blocked solve pays from 800000
+  // on. Columns over 16 powers of ten: n = 512: 1000: 754, 728; n = 1000: 500: 1293, 1376; 1000: 2468, 1989;
+  // n = 4096: 128: 4885, 6006; 256: 9182, 7316. Banded: n = 512: 1000: 754, 823; 1500: 1083, 1042; n = 1000:
+  // 500: 1292, 1506; 1000: 2471, 2156; n = 6000: 128: 10071, 11817; 256: 19407, 12227.
+  const long long elements = (long long)n * nrhs;
+  if (h->arith == LA_ARITH_FAST && ctx->solve_wave > 0 && !ctx->split_ws && n >= (int)SOLVE_BLOCKED_N &&
+      nrhs >= 64 && elements >= (h->uneven <= SOLVE_UNEVEN ? 500000 : 800000)) {
     const int half = BlockedSolve::middle(0, n);
     DevBuf ws(ctx);
     const size_t bytes = gemm_split_ws(half, nrhs, half, false);

@@ -293,16 +293,43 @@ trsm_block_kernel(float* A, size_t ld, int j0, int jbo, int c_begin, int c_end) 
 // The swap list (LAPACK ipiv form) is replayed in order on a permutation
 // vector (lu.rs:147-149), the sign flips once per real swap (lu.rs:151), and
 // U's diagonal is scanned for an exact zero (lu.rs:177).
+// Whether the entries [c0, c1) of a row lie unevenly: one of their quarters has hardly any (1 in 32)
+// within 2^-5 of the row's largest, as where they fall off along the row (columns or rows of very
+// different size) or the matrix is banded. Whole warp.
+__device__ bool uneven_row(const double* row, int c0, int c1) {
+  const int lane = threadIdx.x & 31;
+  auto exp_of = [&](int c) { return (int)(__double_as_longlong(row[c]) >> 52) & 0x7ff; };
+  int top = 0;
+#pragma unroll 8
+  for (int c = c0 + lane; c < c1; c += 32) top = max(top, exp_of(c));
+  top = __reduce_max_sync(0xffffffffu, top);
+  bool uneven = false;
+  for (int q = 0; q < 4; q++) {
+    const int a = c0 + (int)((long long)(c1 - c0) * q / 4), b = c0 + (int)((long long)(c1 - c0) * (q + 1) / 4);
+    int large = 0;
+#pragma unroll 8
+    for (int c = a + lane; c < b; c += 32) large += exp_of(c) >= top - 4;
+    uneven |= __reduce_add_sync(0xffffffffu, large) * 32 < b - a;
+  }
+  return uneven;
+}
+
+// uneven (may be null): how many of LU_SAMPLES rows of U lie unevenly, for the choice of the solve. Each
+// warp without a part in the replay looks at one meanwhile. (L's rows need no look: where they are uneven
+// the blocked forward half is still the faster one.)
+constexpr int LU_SAMPLES = 31;
+constexpr int LU_FINISH_T = 32 * (LU_SAMPLES + 1);
+constexpr int LU_SAMPLE_MIN = 256;  // entries of a row that is looked at
 template <typename T>
 __global__ void lu_finish_kernel(const int* __restrict__ ipiv, uint64_t* piv, int m, int kmin,
-                                 const T* LU, size_t ld, int* flags, int smem_rows,
+                                 const T* LU, size_t ld, int* flags, int* uneven, int smem_rows,
                                  const int* err) {
   extern __shared__ int sperm[];  // permutation in shared memory when m fits
-  __shared__ int zero, s_abort;
+  __shared__ int zero, s_abort, s_uneven;
   if (threadIdx.x == 0) s_abort = aborted(err);
   __syncthreads();
   if (s_abort) return;  // the host reports the error; flags and piv are not used
-  if (threadIdx.x == 0) zero = 0;
+  if (threadIdx.x == 0) zero = s_uneven = 0;
   const bool in_smem = m <= smem_rows;
   if (in_smem) {
     for (int i = threadIdx.x; i < m; i += blockDim.x) sperm[i] = i;
@@ -337,11 +364,20 @@ __global__ void lu_finish_kernel(const int* __restrict__ ipiv, uint64_t* piv, in
       }
     }
     if (threadIdx.x == 0) flags[0] = !(swaps & 1);
+  } else if constexpr (sizeof(T) == 8) {
+    if (uneven) {  // a square matrix
+      const int i = (int)((2ll * (threadIdx.x / 32) - 1) * m / (2 * LU_SAMPLES));
+      if (m - 1 - i >= LU_SAMPLE_MIN && uneven_row(LU + (size_t)i * ld, i + 1, m) && threadIdx.x % 32 == 0)
+        atomicAdd(&s_uneven, 1);
+    }
   }
   __syncthreads();
   if (in_smem)
     for (int i = threadIdx.x; i < m; i += blockDim.x) piv[i] = (uint64_t)sperm[i];
-  if (threadIdx.x == 0) flags[1] = zero;
+  if (threadIdx.x == 0) {
+    flags[1] = zero;
+    if (uneven) *uneven = s_uneven;
+  }
 }
 
 // X = B(piv, :) (lu.rs:245-254).
@@ -525,7 +561,7 @@ la_status launch_trsm_rowpanel_f32(la_ctx ctx, float* A, size_t ld, int j0, int 
   return la_check_launch(ctx, "trsm_rowpanel_reg_kernel");
 }
 
-la_status launch_lu_finish(la_ctx ctx, la_lu h, int* d_flags) {
+la_status launch_lu_finish(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
   const int kmin = (int)std::min(h->m, h->n);
   const int smem_rows = 50000;  // 200 KB of int32 (opt-in); larger m replays in global memory
   static la_device_once configured;
@@ -542,13 +578,13 @@ la_status launch_lu_finish(la_ctx ctx, la_lu h, int* d_flags) {
   if (ce != cudaSuccess) return la_cuda_fail(ctx, ce, "cudaFuncSetAttribute(lu_finish)");
   const size_t smem = (size_t)std::min((int)h->m, smem_rows) * sizeof(int);
   if (h->d_lu32)
-    lu_finish_kernel<float><<<1, 1024, smem, ctx->stream>>>(h->d_ipiv, h->d_piv, (int)h->m, kmin,
-                                                            h->d_lu32, h->ld32, d_flags, smem_rows,
-                                                            ctx->d_err);
+    lu_finish_kernel<float><<<1, LU_FINISH_T, smem, ctx->stream>>>(h->d_ipiv, h->d_piv, (int)h->m, kmin,
+                                                            h->d_lu32, h->ld32, d_flags, nullptr,
+                                                            smem_rows, ctx->d_err);
   else
-    lu_finish_kernel<double><<<1, 1024, smem, ctx->stream>>>(h->d_ipiv, h->d_piv, (int)h->m, kmin,
-                                                             h->d_lu, h->ld, d_flags, smem_rows,
-                                                             ctx->d_err);
+    lu_finish_kernel<double><<<1, LU_FINISH_T, smem, ctx->stream>>>(h->d_ipiv, h->d_piv, (int)h->m, kmin,
+                                                             h->d_lu, h->ld, d_flags, d_uneven,
+                                                             smem_rows, ctx->d_err);
   ctx->launches++;
   return la_check_launch(ctx, "lu_finish_kernel");
 }

@@ -648,7 +648,7 @@ la_status la_lu_mixed_new_device(la_ctx ctx, const double* d_a, size_t lda, size
   ctx->launches++;
   s = la_check_launch(ctx, "f64_to_f32_kernel");
   if (s == LA_OK) s = mixed_factor(ctx, h, prec);
-  if (s == LA_OK) s = launch_lu_finish(ctx, h, reinterpret_cast<int*>(ctx->d_small));
+  if (s == LA_OK) s = launch_lu_finish(ctx, h, reinterpret_cast<int*>(ctx->d_small), nullptr);
   int* flags = static_cast<int*>(ctx->h_pinned);
   if (s == LA_OK) {
     e = cudaMemcpyAsync(flags, ctx->d_small, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);

@@ -114,7 +114,7 @@ extern "C" la_status la_lu_factor_noalloc(void* stream, double* d_a, size_t lda,
   h.d_ipiv = d_ipiv;
   h.d_piv = d_piv;
   h.arith = LA_ARITH_FAST;
-  LA_TRY(lu_factor_enqueue(&c, &h, d_flags));
+  LA_TRY(lu_factor_enqueue(&c, &h, d_flags, nullptr));
   if (cudaStreamSynchronize(c.stream) != cudaSuccess) return LA_CUDA_ERROR;
   int err = 0;
   if (cudaMemcpy(&err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
