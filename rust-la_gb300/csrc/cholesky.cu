@@ -50,6 +50,7 @@ struct Buf {
   explicit Buf(la_ctx c) : ctx(c) {}
   ~Buf() { la_device_free(ctx, p); }
   la_status alloc(size_t bytes) { return la_device_alloc(ctx, &p, bytes); }
+  bool try_alloc(size_t bytes) { return la_device_try_alloc(ctx, &p, bytes); }
   double* d() { return static_cast<double*>(p); }
 };
 
@@ -417,7 +418,7 @@ la_status chol_fast_factor(la_ctx ctx, la_chol h, int* d_flags) {
   FastChol f{ctx, h->d_l, h->ld, n, diag.d(), d_flags, nullptr, 0, Buf(ctx)};
   if (n > CHW) {
     f.ws_bytes = gemm_split_ws(n, n, std::min(chol_block(n), n), true);
-    if (ws.alloc(f.ws_bytes) == LA_OK) f.ws = ws.p;
+    if (ws.try_alloc(f.ws_bytes)) f.ws = ws.p;
   }
   struct PdlScope {
     la_ctx c;

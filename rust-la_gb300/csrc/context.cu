@@ -39,6 +39,14 @@ la_status la_device_alloc(la_ctx ctx, void** p, size_t bytes) {
   return LA_OK;
 }
 
+bool la_device_try_alloc(la_ctx ctx, void** p, size_t bytes) {
+  std::string before;
+  before.swap(ctx->last_error);
+  const bool ok = la_device_alloc(ctx, p, bytes) == LA_OK;
+  ctx->last_error.swap(before);
+  return ok;
+}
+
 void la_device_free(la_ctx ctx, void* p) {
   if (p) cudaFreeAsync(p, ctx->stream);
 }
@@ -55,7 +63,7 @@ la_status copy_host_2d(la_ctx ctx, void* dev, size_t ld, void* host, size_t rows
   const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
   void* dense = ld == cols || rows == 1 ? dev : nullptr;
   void* tmp = nullptr;
-  if (!dense && la_device_alloc(ctx, &tmp, rows * w) == LA_OK) dense = tmp;
+  if (!dense && la_device_try_alloc(ctx, &tmp, rows * w)) dense = tmp;
   cudaError_t e = cudaSuccess;
   if (!dense) {
     e = to_host ? cudaMemcpy2DAsync(host, w, dev, pitch, w, rows, kind, ctx->stream)

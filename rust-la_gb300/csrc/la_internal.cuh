@@ -204,6 +204,8 @@ cudaError_t la_launch(la_ctx ctx, void (*k)(KArgs...), dim3 grid, dim3 block, si
 la_status la_cuda_fail(la_ctx ctx, cudaError_t e, const char* what);
 la_status la_check_launch(la_ctx ctx, const char* what);
 la_status la_device_alloc(la_ctx ctx, void** p, size_t bytes);
+// The same for memory that the caller can do without: a refusal leaves no text in last_error.
+bool la_device_try_alloc(la_ctx ctx, void** p, size_t bytes);
 void la_device_free(la_ctx ctx, void* p);
 // Dense host matrix (rows x cols) <-> device memory of pitch ld, on the context's stream.
 la_status la_copy_to_device(la_ctx ctx, double* dev, size_t ld, const double* host, size_t rows,

@@ -29,6 +29,7 @@ struct DevBuf {
   explicit DevBuf(la_ctx c) : ctx(c) {}
   ~DevBuf() { la_device_free(ctx, p); }
   la_status alloc(size_t bytes) { return la_device_alloc(ctx, &p, bytes); }
+  bool try_alloc(size_t bytes) { return la_device_try_alloc(ctx, &p, bytes); }
   double* d() { return static_cast<double*>(p); }
 };
 
@@ -283,7 +284,7 @@ la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
   if (!f.ws && m > LU_BASE && n > LU_BASE) {
     const int nb = std::min(lu_block(m), kmin);
     f.ws_bytes = gemm_split_ws(m, n, nb, false);
-    if (own.alloc(f.ws_bytes) == LA_OK) f.ws = own.p;
+    if (own.try_alloc(f.ws_bytes)) f.ws = own.p;
   }
   struct PdlScope {
     la_ctx c;
@@ -511,7 +512,7 @@ la_status lu_solve_inplace(la_ctx ctx, la_lu h, double* X, size_t ldx, int nrhs)
     const int half = BlockedSolve::middle(0, n);
     DevBuf ws(ctx);
     const size_t bytes = gemm_split_ws(half, nrhs, half, false);
-    if (bytes <= SPLIT_WS_MAX && ws.alloc(bytes) == LA_OK) {
+    if (bytes <= SPLIT_WS_MAX && ws.try_alloc(bytes)) {
       BlockedSolve s{ctx, h->d_lu, h->ld, X, ldx, nrhs, false, ws.p, bytes};
       LA_TRY(s.lower(0, n));
       return s.upper(0, n);
@@ -559,7 +560,7 @@ la_status gemm_device_common(la_ctx ctx, const double* d_a, size_t lda, const do
     const size_t kc = std::max<size_t>(128, SPLIT_WS_MAX / (16 * (m + n)) / 128 * 128);
     DevBuf ws(ctx);
     const size_t bytes = gemm_split_ws((int)m, (int)n, (int)std::min(k, kc), false);
-    if (bytes <= 2 * SPLIT_WS_MAX && ws.alloc(bytes) == LA_OK) {
+    if (bytes <= 2 * SPLIT_WS_MAX && ws.try_alloc(bytes)) {
       la_status s = LA_OK;
       for (size_t k0 = 0; k0 < k && s == LA_OK; k0 += kc)
         s = launch_gemm_split(ctx, ctx->stream, k0 ? 1 : 0, (int)m, (int)n,
@@ -777,7 +778,7 @@ la_status la_matrix_inverse(la_ctx ctx, const double* a, size_t m, size_t n, dou
     if (s == LA_OK && h->arith == LA_ARITH_FAST && ctx->solve_wave > 0 && n >= INVERSE_BLOCKED_N) {
       const int half = BlockedSolve::middle(0, (int)n);
       const size_t bytes = std::max(gemm_split_ws(half, (int)n, half, false), n * ldw * sizeof(double));
-      if (bytes <= SPLIT_WS_MAX && ws.alloc(bytes) == LA_OK) {
+      if (bytes <= SPLIT_WS_MAX && ws.try_alloc(bytes)) {
         BlockedSolve b{ctx, h->d_lu, h->ld, Xw.d(), ldw, (int)n, true, ws.p, bytes};
         s = launch_identity_permuted(ctx, nullptr, Xw.d(), ldw, (int)n);
         if (s == LA_OK) s = b.lower(0, (int)n);

@@ -434,6 +434,7 @@ struct DevBuf {
   explicit DevBuf(la_ctx c) : ctx(c) {}
   ~DevBuf() { la_device_free(ctx, p); }
   la_status alloc(size_t doubles) { return la_device_alloc(ctx, &p, doubles * sizeof(double)); }
+  bool try_alloc(size_t doubles) { return la_device_try_alloc(ctx, &p, doubles * sizeof(double)); }
   double* d() const { return static_cast<double*>(p); }
 };
 
@@ -455,10 +456,9 @@ void split_plan_tc(la_ctx ctx, int tiles, int K, int* splits, int* kper) {
   *splits = (K + *kper - 1) / *kper;
 }
 // Digits for products against up to n columns of m rows; without the memory: FMA products.
-la_status alloc_split(la_ctx ctx, DevBuf& buf, int m, int n, SplitWs* ws) {
+void alloc_split(la_ctx ctx, DevBuf& buf, int m, int n, SplitWs* ws) {
   ws->bytes = std::max(gemm_split_ws(QB, n, m, false), gemm_split_ws(m, n, QB, false));
-  if (la_tma::get_encoder(ctx) && buf.alloc((ws->bytes + 7) / 8) == LA_OK) ws->p = buf.p;
-  return LA_OK;
+  if (la_tma::get_encoder(ctx) && buf.try_alloc((ws->bytes + 7) / 8)) ws->p = buf.p;
 }
 
 // The block's [G | W] = V' T[j:, cols] on the tensor cores: rows below the top square by split
@@ -565,7 +565,7 @@ la_status qr_blocked_factor(la_ctx ctx, double* A, size_t ld, int m, int n, doub
   LA_TRY(w2.alloc((size_t)QB * ldw));
   DevBuf dig(ctx);
   SplitWs ws;
-  LA_TRY(alloc_split(ctx, dig, m, n, &ws));
+  alloc_split(ctx, dig, m, n, &ws);
   struct PdlScope {
     la_ctx c;
     ~PdlScope() { c->pdl_now = false; }
@@ -626,7 +626,7 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
   // Digits of the products, where the columns are many (get_q).
   DevBuf dig(ctx);
   SplitWs ws;
-  if (cols >= 2 * QB) LA_TRY(alloc_split(ctx, dig, m, cols, &ws));
+  if (cols >= 2 * QB) alloc_split(ctx, dig, m, cols, &ws);
   struct PdlScope {
     la_ctx c;
     ~PdlScope() { c->pdl_now = false; }
