@@ -1,4 +1,5 @@
 // Context, device memory and error plumbing of liblagpu.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -54,28 +55,43 @@ void la_device_free(la_ctx ctx, void* p) {
 // Host matrices (rows x cols, dense) to and from device memory of pitch ld. Two-dimensional copies of
 // pageable memory go row by row inside the runtime: 50 MB (2500 rows) took 43 ms to the host, where
 // one contiguous copy takes 2 (3 into memory that was never touched). So a dense device side is
-// copied in one piece, and any other goes through a dense buffer and a copy on the device; without
-// memory for that, the two-dimensional copy.
+// copied in one piece, and any other through a dense buffer of about STAGE_BYTES, whole rows at a time,
+// and copies on the device (9001 rows to the host 24.0 ms in one piece, 24.4 in five); without memory for
+// that, the two-dimensional copy.
 namespace {
+constexpr size_t STAGE_BYTES = (size_t)128 << 20;
+
+cudaError_t copy_staged(la_ctx ctx, char* dev, size_t pitch, char* host, size_t w, size_t rows,
+                        bool to_host, void* tmp, size_t tmp_rows) {
+  for (size_t r = 0; r < rows; r += tmp_rows) {
+    const size_t n = std::min(tmp_rows, rows - r);
+    char *d = dev + r * pitch, *h = host + r * w;
+    const cudaError_t e = to_host ? cudaMemcpy2DAsync(tmp, w, d, pitch, w, n, cudaMemcpyDeviceToDevice, ctx->stream)
+                                  : cudaMemcpyAsync(tmp, h, n * w, cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) return e;
+    const cudaError_t f = to_host ? cudaMemcpyAsync(h, tmp, n * w, cudaMemcpyDeviceToHost, ctx->stream)
+                                  : cudaMemcpy2DAsync(d, pitch, tmp, w, w, n, cudaMemcpyDeviceToDevice, ctx->stream);
+    if (f != cudaSuccess) return f;
+  }
+  return cudaSuccess;
+}
+
 la_status copy_host_2d(la_ctx ctx, void* dev, size_t ld, void* host, size_t rows, size_t cols,
                        bool to_host) {
   const size_t w = cols * sizeof(double), pitch = ld * sizeof(double);
   const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-  void* dense = ld == cols || rows == 1 ? dev : nullptr;
+  const size_t tmp_rows = std::min(rows, STAGE_BYTES / std::max<size_t>(w, 1) + 1);
   void* tmp = nullptr;
-  if (!dense && la_device_try_alloc(ctx, &tmp, rows * w)) dense = tmp;
   cudaError_t e = cudaSuccess;
-  if (!dense) {
+  if (ld == cols || rows == 1)
+    e = to_host ? cudaMemcpyAsync(host, dev, rows * w, kind, ctx->stream)
+                : cudaMemcpyAsync(dev, host, rows * w, kind, ctx->stream);
+  else if (la_device_try_alloc(ctx, &tmp, tmp_rows * w))
+    e = copy_staged(ctx, static_cast<char*>(dev), pitch, static_cast<char*>(host), w, rows, to_host, tmp,
+                    tmp_rows);
+  else
     e = to_host ? cudaMemcpy2DAsync(host, w, dev, pitch, w, rows, kind, ctx->stream)
                 : cudaMemcpy2DAsync(dev, pitch, host, w, w, rows, kind, ctx->stream);
-  } else {
-    if (to_host && tmp)
-      e = cudaMemcpy2DAsync(tmp, w, dev, pitch, w, rows, cudaMemcpyDeviceToDevice, ctx->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(to_host ? host : dense, to_host ? dense : host, rows * w, kind, ctx->stream);
-    if (e == cudaSuccess && !to_host && tmp)
-      e = cudaMemcpy2DAsync(dev, pitch, tmp, w, w, rows, cudaMemcpyDeviceToDevice, ctx->stream);
-  }
   la_device_free(ctx, tmp);
   return e == cudaSuccess ? LA_OK : la_cuda_fail(ctx, e, to_host ? "copy to host" : "copy to device");
 }
