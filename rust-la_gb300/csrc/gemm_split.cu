@@ -999,7 +999,7 @@ la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N,
                             double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes, int splits,
                             int kper, size_t czs) {
   if (M <= 0 || N <= 0) return LA_OK;
-  if (K <= 0 || K > (1 << 20) || (tri && M != N)) return LA_UNSUPPORTED;
+  if (K <= 0 || K > SPLIT_MAX_K || (tri && M != N)) return LA_UNSUPPORTED;
   if (splits > 1 && (mode != 0 || kper % (CHUNK_STAGES * PK) || (long long)(splits - 1) * kper >= K ||
                      (long long)splits * kper < K))
     return LA_UNSUPPORTED;

@@ -243,7 +243,9 @@ la_status launch_gemm_lower(la_ctx ctx, int M, int K, const double* A, size_t ld
 // (0) or += A B (1); A M x K, B K x N, or N x K rows of B' when b_rows; any alignment. tri: the
 // square C's part at or below the diagonal, in tiles. ws: gemm_split_ws bytes of device memory,
 // used until the product is done (same: B' is A). splits > 1 (mode 0): K in pieces of kper, a
-// multiple of 128, piece z's product to C + z czs. LA_UNSUPPORTED: nothing launched.
+// multiple of 128, piece z's product to C + z czs. LA_UNSUPPORTED: nothing launched (K > SPLIT_MAX_K,
+// a workspace too small, no encoder).
+constexpr int SPLIT_MAX_K = 1 << 20;
 size_t gemm_split_ws(int M, int N, int K, bool same);
 la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
                             const double* A, size_t lda, const double* B, size_t ldb, bool b_rows,

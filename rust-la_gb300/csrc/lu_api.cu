@@ -556,8 +556,10 @@ la_status gemm_device_common(la_ctx ctx, const double* d_a, size_t lda, const do
   if (mode == GM_FMA_ZERO && n > 16 && k >= 32) {
     // On the tensor cores from 32 k and 17 columns on: one FMA tile of 64 x 64 x 32 keeps an SM busy
     // for 33 us, while the split product's three launches of one tile take about 15 us in all
-    // (8192^3: 27.9 ms against 876 ms). In slabs of K whose digits fit the workspace.
-    const size_t kc = std::max<size_t>(128, SPLIT_WS_MAX / (16 * (m + n)) / 128 * 128);
+    // (8192^3: 24.0 ms against 876 ms). In slabs of K whose digits fit the workspace and whose sums fit
+    // the product's integers (2 x 1048736 x 17: 61 ms, as one FMA tile 1048).
+    const size_t kc = std::min<size_t>(
+        SPLIT_MAX_K, std::max<size_t>(128, SPLIT_WS_MAX / (16 * (m + n)) / 128 * 128));
     DevBuf ws(ctx);
     const size_t bytes = gemm_split_ws((int)m, (int)n, (int)std::min(k, kc), false);
     if (bytes <= 2 * SPLIT_WS_MAX && ws.try_alloc(bytes)) {
