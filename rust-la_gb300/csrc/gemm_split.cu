@@ -28,8 +28,8 @@
 //     sum_k |a_ik b_kj| >= 2^-8.9 sqrt(K),
 // where the error left out is no larger than the chain's. guard_kernel decides it per tile, in two
 // steps. The split kernels count, per row and column, the entries within 2^-5 of the scale; if the
-// smallest row count and the smallest column count exceed K by 2 sqrt(K) together, that many k have
-// both entries large, and the sum is at least 2 sqrt(K) 2^-10. Else the sums are formed from the
+// smallest row count and the smallest column count exceed K by 2^1.1 sqrt(K) together, that many k have
+// both entries large, and the sum is at least 2^1.1 sqrt(K) 2^-10. Else the sums are formed from the
 // leading two digits by mma.sync (a few microseconds, where the FMA tile of K = 256 takes 1 ms; as
 // FP32 FMAs they took 65 us for K = 700, a tenth of the FMA tiles that may follow). Every other
 // tile (graded or sparse operands, values that are not finite or beyond 2^+-400) goes on a list that
@@ -382,7 +382,7 @@ struct SplitArgs {
   size_t ldc;
   const int *ea, *ca, *eb, *cb;
   const __half *da, *db;  // the digits [SL][rows][kp]
-  int kp, joint;     // joint: 2 sqrt(K), rounded up
+  int kp, joint;     // joint: terms of 2^-10 that make the guard's sum
   int* fits;         // per tile: 1 where the digits hold what it needs
   int* list;         // [0] count, then the tiles left to fma_tiles
   int* err;
@@ -1045,7 +1045,7 @@ la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N,
   p.da = sa.dig;
   p.db = sb.dig;
   p.kp = kp;
-  p.joint = (int)std::ceil(2.0 * std::sqrt((double)K));
+  p.joint = (int)std::ceil(1024.0 * GUARD * std::sqrt((double)K));
   p.list = list;
   p.fits = list + 1 + p.tiles;
   p.err = ctx->d_err;
