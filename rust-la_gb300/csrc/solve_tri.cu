@@ -411,14 +411,19 @@ __device__ __forceinline__ T settable(T v) {
   else return unset(v) ? __int_as_float(0x7fc00000) : v;
 }
 // Blocks of the column known to be solved, in order: counter w of the four counts its block of each
-// item. As wave_wait, until that is at least `need`; -1 after an error or without progress.
+// item. As wave_wait, until that is at least `need`; -1 after an error or without progress. The lanes
+// acquire different counters and then read rows released under all four, which takes a __syncwarp: a
+// reduction orders no memory.
 __device__ __forceinline__ int chain_wait(const int* p, int need, int* err) {
   const unsigned full = 0xffffffffu;
   const int w = threadIdx.x & (CB - 1);
   unsigned long long t0 = 0;
   for (unsigned spins = 1;; spins++) {
     const int done = __reduce_min_sync(full, CB * wave_ld_acquire(p + w) + w);
-    if (done >= need) return done;
+    if (done >= need) {
+      __syncwarp();
+      return done;
+    }
     if ((spins & 63u) == 0) {
       int bad = 0;
       if ((threadIdx.x & 31) == 0) {
