@@ -244,13 +244,14 @@ la_status launch_gemm_lower(la_ctx ctx, int M, int K, const double* A, size_t ld
 // square C's part at or below the diagonal, in tiles. ws: gemm_split_ws bytes of device memory,
 // used until the product is done (same: B' is A). splits > 1 (mode 0): K in pieces of kper, a
 // multiple of 128, piece z's product to C + z czs. LA_UNSUPPORTED: nothing launched (K > SPLIT_MAX_K,
-// a workspace too small, no encoder).
+// a workspace too small, no encoder). misses: a device word of a chain of like products, zero before the
+// first; where they leave nearly all of their tiles to FMA chains, most of the following form no digits.
 constexpr int SPLIT_MAX_K = 1 << 20;
 size_t gemm_split_ws(int M, int N, int K, bool same);
 la_status launch_gemm_split(la_ctx ctx, cudaStream_t st, int mode, int M, int N, int K,
                             const double* A, size_t lda, const double* B, size_t ldb, bool b_rows,
                             double* C, size_t ldc, bool tri, void* ws, size_t ws_bytes,
-                            int splits = 1, int kper = 0, size_t czs = 0);
+                            int splits = 1, int kper = 0, size_t czs = 0, int* misses = nullptr);
 // C + z * czs = A[:, z kper : (z + 1) kper] B[z kper : (z + 1) kper, :] for z < splits
 // (fused, from zero); kper a multiple of 32, splits * kper >= K > (splits - 1) kper.
 la_status launch_gemm_splitk(la_ctx ctx, int M, int N, int K, const double* A, size_t lda,

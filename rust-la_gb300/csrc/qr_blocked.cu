@@ -442,6 +442,7 @@ struct DevBuf {
 struct SplitWs {
   void* p = nullptr;
   size_t bytes = 0;
+  int* misses = nullptr;  // of the blocks' V' T products, of their updates
 };
 // Whether a block of `rows` rows uses them against `right` columns (get_q: all of them; else those
 // right of the block): a whole 64-row square on top, and enough below and beside it that their
@@ -456,9 +457,14 @@ void split_plan_tc(la_ctx ctx, int tiles, int K, int* splits, int* kper) {
   *splits = (K + *kper - 1) / *kper;
 }
 // Digits for products against up to n columns of m rows; without the memory: FMA products.
-void alloc_split(la_ctx ctx, DevBuf& buf, int m, int n, SplitWs* ws) {
+la_status alloc_split(la_ctx ctx, DevBuf& buf, int m, int n, SplitWs* ws) {
   ws->bytes = std::max(gemm_split_ws(QB, n, m, false), gemm_split_ws(m, n, QB, false));
-  if (la_tma::get_encoder(ctx) && buf.try_alloc((ws->bytes + 7) / 8)) ws->p = buf.p;
+  const size_t words = (ws->bytes + 7) / 8;
+  if (!la_tma::get_encoder(ctx) || !buf.try_alloc(words + 1)) return LA_OK;
+  ws->p = buf.p;
+  ws->misses = reinterpret_cast<int*>(buf.d() + words);
+  LA_CUDA(ctx, cudaMemsetAsync(ws->misses, 0, 2 * sizeof(int), ctx->stream));
+  return LA_OK;
 }
 
 // The block's [G | W] = V' T[j:, cols] on the tensor cores: rows below the top square by split
@@ -472,7 +478,7 @@ la_status apply_vt_tc(la_ctx ctx, const SplitWs& ws, const double* vt, size_t ld
   if ((size_t)splits * pzs > part_cap) return LA_INVALID;
   LA_TRY(launch_gemm_split(ctx, ctx->stream, 0, QB, ncols, rows - QB, vt + QB, ldv,
                            T + (size_t)QB * ldt, ldt, false, part, ldp, false, ws.p, ws.bytes, splits,
-                           kper, pzs));
+                           kper, pzs, ws.misses));
   const cudaError_t e = la_launch(ctx, qr_wsum_top_kernel, dim3((ncols + WT_C - 1) / WT_C), dim3(256),
                                   0, ctx->stream, (const double*)part, ldp, pzs, splits, vt, ldv, T,
                                   ldt, ncols, nvc, wf, ldw);
@@ -565,7 +571,7 @@ la_status qr_blocked_factor(la_ctx ctx, double* A, size_t ld, int m, int n, doub
   LA_TRY(w2.alloc((size_t)QB * ldw));
   DevBuf dig(ctx);
   SplitWs ws;
-  alloc_split(ctx, dig, m, n, &ws);
+  LA_TRY(alloc_split(ctx, dig, m, n, &ws));
   struct PdlScope {
     la_ctx c;
     ~PdlScope() { c->pdl_now = false; }
@@ -597,7 +603,7 @@ la_status qr_blocked_factor(la_ctx ctx, double* A, size_t ld, int m, int n, doub
                            true, gj, true, vt.d(), ldv, Aj + nb, ld));
       LA_TRY(launch_gemm_split(ctx, ctx->stream, -1, rows - QB, ncols - nb, nb, Aj + (size_t)QB * ld,
                                ld, w2.d(), ldw, false, Aj + (size_t)QB * ld + nb, ld, false, ws.p,
-                               ws.bytes));
+                               ws.bytes, 1, 0, 0, ws.misses + 1));
       continue;
     }
     LA_TRY(apply_vt(ctx, vt.d(), ldv, nb, rows, Aj, ld, ncols, part.d(), pcap, wf.d(), ldw));
@@ -626,7 +632,7 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
   // Digits of the products, where the columns are many (get_q).
   DevBuf dig(ctx);
   SplitWs ws;
-  if (cols >= 2 * QB) alloc_split(ctx, dig, m, cols, &ws);
+  if (cols >= 2 * QB) LA_TRY(alloc_split(ctx, dig, m, cols, &ws));
   struct PdlScope {
     la_ctx c;
     ~PdlScope() { c->pdl_now = false; }
@@ -651,7 +657,7 @@ la_status qr_blocked_apply(la_ctx ctx, const double* A, size_t ld, int m, int dc
                            true, vt.d(), ldv, Tj, ldt));
       LA_TRY(launch_gemm_split(ctx, ctx->stream, -1, rows - QB, ncols, nb, vx.d() + (size_t)QB * QB,
                                QB, w2.d(), ldw, false, Tj + (size_t)QB * ldt, ldt, false, ws.p,
-                               ws.bytes));
+                               ws.bytes, 1, 0, 0, ws.misses + 1));
       continue;
     }
     LA_TRY(apply_vt(ctx, vt.d(), ldv, nb, rows, Tj, ldt, ncols, part.d(), pcap, wf.d(), ldw));
