@@ -18,7 +18,7 @@
 // critical path per block is one tile application and one 32-step diagonal
 // solve; the rest of the update work fills the other SMs.
 //
-// Chain (up to CHAIN_MAX_NRHS right-hand sides). The wavefront with 128 rows of
+// Chain (more than 32 rows, up to CHAIN_MAX_NRHS right-hand sides). The wavefront with 128 rows of
 // one column per item; see solve_chain_kernel.
 //
 // Block steps. One launch per 16-row block step: for the finished block
@@ -626,25 +626,29 @@ solve_chain_kernel(const T* __restrict__ LU, size_t ld, T* X, size_t ldx, int n,
 // Right-hand sides up to which the chain's items are one column each; above, four columns per item
 // share each tile's load and the FP64 pipes are busy anyway. Both triangles, us, four columns and one:
 // n = 8192: 16 right-hand sides 4053, 3412; 24: 4731, 4593; 32: 5609, 5839. n = 4096: 24: 1912, 1471;
-// 64: 2842, 2980.
+// 64: 2842, 2980. A single block has nothing to hand on, and the chain's body, unrolled over the block with
+// its divisions, is read from memory for one pass: whole calls at n = 24, us,
+// four-column items and chain: EXACT 53, 66; FAST 44, 44.
 constexpr int CHAIN_MAX_NRHS = 24;
+bool chained(int n, int nrhs) { return nrhs <= CHAIN_MAX_NRHS && n > WB; }
 
-// One triangle by solve_chain_kernel.
+// One triangle by solve_chain_kernel; ticket and prog (CB counters per right-hand side) are zero.
 template <typename T, bool EXACT, bool UPPER, bool DIVL>
-la_status chain(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int nrhs) {
-  static_assert(2 + CB * CHAIN_MAX_NRHS <= 2 + 2 * SOLVE_WAVE_MAX_GROUPS, "progress counters");
+la_status chain(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int nrhs, int* ticket,
+                int* prog) {
+  static_assert(2 * CB * CHAIN_MAX_NRHS <= 2 * SOLVE_WAVE_MAX_GROUPS, "progress counters");
   const auto kernel = solve_chain_kernel<T, EXACT, UPPER, DIVL>;
   const size_t smem = ChainTile<T>::SMEM;
-  LA_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static la_device_once configured;
+  LA_CUDA(ctx, configured.run([&](int) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  }));
   const int nb = (n + WB - 1) / WB;
-  int* const sync = ctx->d_solve_sync;
-  LA_CUDA(ctx, cudaMemsetAsync(sync, 0, (2 + CB * (size_t)nrhs) * sizeof(int), ctx->stream));
   const long long items = (long long)((nb + CB - 1) / CB) * nrhs;
   const int cps = ctx->solve_wave > 0 ? ctx->solve_wave : 2;
   const int grid = (int)std::min<long long>(items, (long long)cps * ctx->sm_count);
   const bool vec = ld % ChainTile<T>::VN == 0 && reinterpret_cast<uintptr_t>(LU) % 16 == 0;
-  kernel<<<grid, CB * 32, smem, ctx->stream>>>(LU, ld, X, ldx, n, nrhs, nb, vec, sync, sync + 2,
-                                               ctx->d_err);
+  kernel<<<grid, CB * 32, smem, ctx->stream>>>(LU, ld, X, ldx, n, nrhs, nb, vec, ticket, prog, ctx->d_err);
   ctx->launches++;
   return la_check_launch(ctx, "solve_chain_kernel");
 }
@@ -652,12 +656,14 @@ la_status chain(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int
 template <typename T, bool EXACT>
 la_status solve_wave(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n, int nrhs) {
   const int nb = (n + WB - 1) / WB;
-  if (nrhs <= CHAIN_MAX_NRHS) {
-    LA_TRY((chain<T, EXACT, false, false>(ctx, LU, ld, X, ldx, n, nrhs)));
-    return chain<T, EXACT, true, false>(ctx, LU, ld, X, ldx, n, nrhs);
+  int* tickets = ctx->d_solve_sync;
+  if (chained(n, nrhs)) {
+    const size_t counters = CB * (size_t)nrhs;  // of a triangle
+    LA_CUDA(ctx, cudaMemsetAsync(tickets, 0, (2 + 2 * counters) * sizeof(int), ctx->stream));
+    LA_TRY((chain<T, EXACT, false, false>(ctx, LU, ld, X, ldx, n, nrhs, tickets, tickets + 2)));
+    return chain<T, EXACT, true, false>(ctx, LU, ld, X, ldx, n, nrhs, tickets + 1, tickets + 2 + counters);
   }
   const int groups = (nrhs + WC - 1) / WC;
-  int* tickets = ctx->d_solve_sync;
   int* prog_l = tickets + 2;
   int* prog_u = prog_l + groups;
   LA_CUDA(ctx, cudaMemsetAsync(tickets, 0, (2 + 2 * (size_t)groups) * sizeof(int), ctx->stream));
@@ -678,7 +684,11 @@ la_status solve_wave(la_ctx ctx, const T* LU, size_t ld, T* X, size_t ldx, int n
 template <bool EXACT, bool UPPER, bool DIVL>
 la_status tri_wave(la_ctx ctx, const double* T, size_t ld, double* X, size_t ldx, int n,
                    int nrhs) {
-  if (nrhs <= CHAIN_MAX_NRHS) return chain<double, EXACT, UPPER, DIVL>(ctx, T, ld, X, ldx, n, nrhs);
+  if (chained(n, nrhs)) {
+    int* const sync = ctx->d_solve_sync;
+    LA_CUDA(ctx, cudaMemsetAsync(sync, 0, (2 + CB * (size_t)nrhs) * sizeof(int), ctx->stream));
+    return chain<double, EXACT, UPPER, DIVL>(ctx, T, ld, X, ldx, n, nrhs, sync, sync + 2);
+  }
   const int nb = (n + WB - 1) / WB;
   const int per = WC * SOLVE_WAVE_MAX_GROUPS;
   for (int c0 = 0; c0 < nrhs; c0 += per) {
