@@ -1,4 +1,6 @@
 // Context, device memory and error plumbing of liblagpu.
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -52,58 +54,71 @@ void la_device_free(la_ctx ctx, void* p) {
   if (p) cudaFreeAsync(p, ctx->stream);
 }
 
-// Host matrices (rows x cols, dense) to and from device memory of pitch ld. Two-dimensional copies of
-// pageable memory go row by row inside the runtime: 50 MB (2500 rows) took 43 ms to the host, where
-// one contiguous copy takes 2 (3 into memory that was never touched). So a dense device side is
-// copied in one piece, and any other through a dense buffer of about STAGE_BYTES, whole rows at a time,
-// and copies on the device (9001 rows to the host 24.0 ms in one piece, 24.4 in five); without memory for
-// that, the two-dimensional copy.
+// Host matrices (rows x cols, dense) to and from device memory of pitch ld.
+//
+// To the device: a dense device side is copied in one piece, any other through a dense buffer of about
+// STAGE_BYTES, whole rows at a time, and copies on the device; without memory for that, by a
+// two-dimensional copy (333 rows 50 us, staged 48; 1001: 119, 93; as part of small calls 5 us more).
+//
+// To the host: a two-dimensional copy. The GPU writes pageable memory itself, and a page that the process
+// has not touched is a fault of the GPU's for each of its rows, so the pages are touched before. 333 rows
+// and 2501 (50 MB), memory touched long before: 38 us, 0.34 ms; fresh: 95 us, 2.2 ms; fresh and not
+// touched here 1.0 ms, 31 ms; staged 49 us, 0.36 ms, fresh 222 us, 2.1 ms.
 namespace {
 constexpr size_t STAGE_BYTES = (size_t)128 << 20;
 
-cudaError_t copy_staged(la_ctx ctx, char* dev, size_t pitch, char* host, size_t w, size_t rows,
-                        bool to_host, void* tmp, size_t tmp_rows) {
+cudaError_t copy_staged(la_ctx ctx, char* dev, size_t pitch, const char* host, size_t w, size_t rows,
+                        void* tmp, size_t tmp_rows) {
   for (size_t r = 0; r < rows; r += tmp_rows) {
     const size_t n = std::min(tmp_rows, rows - r);
-    char *d = dev + r * pitch, *h = host + r * w;
-    const cudaError_t e = to_host ? cudaMemcpy2DAsync(tmp, w, d, pitch, w, n, cudaMemcpyDeviceToDevice, ctx->stream)
-                                  : cudaMemcpyAsync(tmp, h, n * w, cudaMemcpyHostToDevice, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(tmp, host + r * w, n * w, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpy2DAsync(dev + r * pitch, pitch, tmp, w, w, n, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e != cudaSuccess) return e;
-    const cudaError_t f = to_host ? cudaMemcpyAsync(h, tmp, n * w, cudaMemcpyDeviceToHost, ctx->stream)
-                                  : cudaMemcpy2DAsync(d, pitch, tmp, w, w, n, cudaMemcpyDeviceToDevice, ctx->stream);
-    if (f != cudaSuccess) return f;
   }
   return cudaSuccess;
 }
 
-la_status copy_host_2d(la_ctx ctx, void* dev, size_t ld, void* host, size_t rows, size_t cols,
-                       bool to_host) {
-  const size_t w = cols * sizeof(double), pitch = ld * sizeof(double);
-  const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
-  const size_t tmp_rows = std::min(rows, STAGE_BYTES / std::max<size_t>(w, 1) + 1);
-  void* tmp = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (ld == cols || rows == 1)
-    e = to_host ? cudaMemcpyAsync(host, dev, rows * w, kind, ctx->stream)
-                : cudaMemcpyAsync(dev, host, rows * w, kind, ctx->stream);
-  else if (la_device_try_alloc(ctx, &tmp, tmp_rows * w))
-    e = copy_staged(ctx, static_cast<char*>(dev), pitch, static_cast<char*>(host), w, rows, to_host, tmp,
-                    tmp_rows);
-  else
-    e = to_host ? cudaMemcpy2DAsync(host, w, dev, pitch, w, rows, kind, ctx->stream)
-                : cudaMemcpy2DAsync(dev, pitch, host, w, w, rows, kind, ctx->stream);
-  la_device_free(ctx, tmp);
-  return e == cudaSuccess ? LA_OK : la_cuda_fail(ctx, e, to_host ? "copy to host" : "copy to device");
+void touch_pages(char* p, size_t bytes) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
+    cudaGetLastError();
+    return;
+  }
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  for (size_t i = 0; i < bytes; i += page - (reinterpret_cast<uintptr_t>(p) + i) % page)
+    *const_cast<volatile char*>(p + i) = 0;
 }
 }  // namespace
 
 la_status la_copy_to_device(la_ctx ctx, double* dev, size_t ld, const double* host, size_t rows,
                             size_t cols) {
-  return copy_host_2d(ctx, dev, ld, const_cast<double*>(host), rows, cols, false);
+  const size_t w = cols * sizeof(double), pitch = ld * sizeof(double);
+  const size_t tmp_rows = std::min(rows, STAGE_BYTES / std::max<size_t>(w, 1) + 1);
+  void* tmp = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (ld == cols || rows == 1)
+    e = cudaMemcpyAsync(dev, host, rows * w, cudaMemcpyHostToDevice, ctx->stream);
+  else if (la_device_try_alloc(ctx, &tmp, tmp_rows * w))
+    e = copy_staged(ctx, reinterpret_cast<char*>(dev), pitch, reinterpret_cast<const char*>(host), w, rows,
+                    tmp, tmp_rows);
+  else
+    e = cudaMemcpy2DAsync(dev, pitch, host, w, w, rows, cudaMemcpyHostToDevice, ctx->stream);
+  la_device_free(ctx, tmp);
+  return e == cudaSuccess ? LA_OK : la_cuda_fail(ctx, e, "copy to device");
 }
+
 la_status la_copy_to_host(la_ctx ctx, double* host, const double* dev, size_t ld, size_t rows,
                           size_t cols) {
-  return copy_host_2d(ctx, const_cast<double*>(dev), ld, host, rows, cols, true);
+  const size_t w = cols * sizeof(double), pitch = ld * sizeof(double);
+  cudaError_t e = cudaSuccess;
+  if (ld == cols || rows == 1) {
+    e = cudaMemcpyAsync(host, dev, rows * w, cudaMemcpyDeviceToHost, ctx->stream);
+  } else {
+    touch_pages(reinterpret_cast<char*>(host), rows * w);
+    e = cudaMemcpy2DAsync(host, w, dev, pitch, w, rows, cudaMemcpyDeviceToHost, ctx->stream);
+  }
+  return e == cudaSuccess ? LA_OK : la_cuda_fail(ctx, e, "copy to host");
 }
 
 // Synchronizes the context's stream and turns a device-side error word into a status.
