@@ -92,6 +92,9 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
   __shared__ double own[2][QB];                // the diagonal row: q, then t_c
   __shared__ double red[QPT];
   __shared__ double mine[QB], tot[QB], fac[QB];
+  // A CTA's shared memory may be written by the others only once it has started: all arrive here, and
+  // wait before their first remote store.
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   la_pdl_wait();
   la_pdl_trigger();
   const int tid = threadIdx.x;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(QPT, 1) qr_panel_kernel(QrPanelArgs p) {
     P[lr * QNBP + c] = p.A[(size_t)(r0 + lr) * p.ld + p.j + c];
   }
   __syncthreads();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 
   for (int k = 0; k < nb; k++) {
     const int par = k & 1, jc = p.j + k, w = nb - k;
