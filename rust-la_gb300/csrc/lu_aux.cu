@@ -85,53 +85,14 @@ laswp_lists_kernel(T* A, size_t ld, const int* __restrict__ swaps, int lists, in
 }
 
 // ---- row-panel triangular update: U12 = L11^{-1} A12 ----------------------
-// Rows [j0, j0+jb), columns [c_begin, c_end), one 32-column strip per CTA (FP32
-// blocks wider than 32 rows). Column sweep over k (one barrier per k): row k is
-// finished, then every row i > k of the block takes its k-th term by FMA, i.e.
-// each element receives its terms in ascending k, like lu.rs:124-128.
-constexpr int TR_COLS = 32;
-constexpr int LP = MAX_PANEL_W + 1;  // padded row of the triangular block in shared memory
-template <typename T>
-constexpr size_t trsm_smem() {
-  return (size_t)(MAX_PANEL_W * LP + MAX_PANEL_W * TR_COLS) * sizeof(T);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-trsm_rowpanel_kernel(T* A, size_t ld, int j0, int jb, int c_begin, int c_end) {
-  extern __shared__ __align__(16) double dsm_raw[];
-  T* dsm = reinterpret_cast<T*>(dsm_raw);
-  T(*L)[LP] = reinterpret_cast<T(*)[LP]>(dsm);
-  T(*xa)[TR_COLS] = reinterpret_cast<T(*)[TR_COLS]>(dsm + MAX_PANEL_W * LP);
-  const int tx = threadIdx.x % TR_COLS, ty = threadIdx.x / TR_COLS;  // ty 0..7
-  const int c = c_begin + blockIdx.x * TR_COLS + tx;
-  const bool ok = c < c_end;
-  for (int idx = threadIdx.x; idx < jb * jb; idx += 256) {
-    int i = idx / jb, k = idx % jb;
-    L[i][k] = A[(size_t)(j0 + i) * ld + j0 + k];
-  }
-  for (int i = ty; i < jb; i += 8) {
-    size_t off = (size_t)(j0 + i) * ld + c;
-    xa[i][tx] = ok ? A[off] : T(0);
-  }
-  __syncthreads();
-  for (int k = 0; k < jb; k++) {
-    __syncthreads();
-    const T uk = xa[k][tx];
-    for (int i = ty; i < jb; i += 8)
-      if (i > k) xa[i][tx] = fma(-L[i][k], uk, xa[i][tx]);
-  }
-  __syncthreads();
-  if (ok)
-    for (int i = ty; i < jb; i += 8) A[(size_t)(j0 + i) * ld + c] = xa[i][tx];
-}
-
+// Rows [j0, j0 + jb) of columns [c_begin, c_end). Row k is finished, then every row i > k of the block
+// takes its k-th term, i.e. each element receives its terms in ascending k, like lu.rs:124-128.
+//
 // FP64 form, jb <= 64: 8 columns per CTA. With two FP64 FMAs per clock an SM needs 16 clocks
 // for one warp's FMA, so the 64 x 64 triangle costs 0.5 us a column and the strip's width sets the
-// latency: the 32-column CTAs of the kernel above took 49 us however few columns there were. Row k
-// is final when step k starts; the rows below take its term, neighbouring items (row, column) on
-// neighbouring threads, so that no lane idles but in the last warp. The same FMAs in the same
-// order as above, so the same bits.
+// latency: CTAs of 32 columns took 49 us however few columns there were. Row k is final when step k
+// starts; the rows below take its term, neighbouring items (row, column) on neighbouring threads, so
+// that no lane idles but in the last warp.
 // EXACT: the running sums s from S, row k formed as a - s at its step, terms added unfused.
 constexpr int TC8 = 8;
 constexpr int TC8_T = 256;
@@ -182,8 +143,7 @@ trsm_cols8_kernel(double* A, const double* S, size_t ld, int j0, int jb, int c_b
 
 // FP32 form for the mixed LU's 32-row blocks (jb <= 32, FMA): one thread per
 // column holds the column's jb values in registers and applies the terms in
-// ascending k (the same FMAs in the same order as the kernel above, so the
-// same bits), with the unit-lower block broadcast from shared memory. No
+// ascending k, with the unit-lower block broadcast from shared memory. No
 // barrier inside the sweep: at FP32 rates the barriers, not the FMAs, were the
 // cost of the 32-step sweep.
 constexpr int TRR_W = 32;
@@ -524,35 +484,21 @@ la_status launch_trsm_block_f32(la_ctx ctx, float* A, size_t ld, int j0, int jbo
   return la_check_launch(ctx, "trsm_block_kernel");
 }
 
-template <typename T>
-la_status launch_trsm_t(la_ctx ctx, bool exact, T* A, T* S, size_t ld, int j0, int jb,
-                        int c_begin, int c_end) {
-  if (c_end <= c_begin) return LA_OK;
-  if (sizeof(T) == 8) {
-    const cudaError_t e =
-        la_launch(ctx, exact ? trsm_cols8_kernel<true> : trsm_cols8_kernel<false>,
-                  dim3((c_end - c_begin + TC8 - 1) / TC8), dim3(TC8_T), 0, ctx->stream,
-                  reinterpret_cast<double*>(A), reinterpret_cast<const double*>(S), ld, j0, jb,
-                  c_begin, c_end);
-    if (e != cudaSuccess) return la_cuda_fail(ctx, e, "trsm_cols8_kernel launch");
-    ctx->launches++;
-    return la_check_launch(ctx, "trsm_cols8_kernel");
-  }
-  dim3 grid((c_end - c_begin + TR_COLS - 1) / TR_COLS);
-  trsm_rowpanel_kernel<float><<<grid, 256, trsm_smem<float>(), ctx->stream>>>(
-      reinterpret_cast<float*>(A), ld, j0, jb, c_begin, c_end);
-  ctx->launches++;
-  return la_check_launch(ctx, "trsm_rowpanel_kernel");
-}
-
 la_status launch_trsm_rowpanel(la_ctx ctx, bool exact, double* A, double* S, size_t ld, int j0,
                                int jb, int c_begin, int c_end) {
-  return launch_trsm_t<double>(ctx, exact, A, S, ld, j0, jb, c_begin, c_end);
+  if (c_end <= c_begin) return LA_OK;
+  const cudaError_t e =
+      la_launch(ctx, exact ? trsm_cols8_kernel<true> : trsm_cols8_kernel<false>,
+                dim3((c_end - c_begin + TC8 - 1) / TC8), dim3(TC8_T), 0, ctx->stream, A,
+                (const double*)S, ld, j0, jb, c_begin, c_end);
+  if (e != cudaSuccess) return la_cuda_fail(ctx, e, "trsm_cols8_kernel launch");
+  ctx->launches++;
+  return la_check_launch(ctx, "trsm_cols8_kernel");
 }
 la_status launch_trsm_rowpanel_f32(la_ctx ctx, float* A, size_t ld, int j0, int jb, int c_begin,
                                    int c_end) {
-  if (jb > TRR_W) return launch_trsm_t<float>(ctx, false, A, nullptr, ld, j0, jb, c_begin, c_end);
   if (c_end <= c_begin) return LA_OK;
+  if (jb > TRR_W) return LA_INVALID;
   const int grid = (c_end - c_begin + TRR_T - 1) / TRR_T;
   const cudaError_t e = la_launch(ctx, trsm_rowpanel_reg_kernel, dim3(grid), dim3(TRR_T), 0,
                                   ctx->stream, A, ld, j0, jb, c_begin, c_end);

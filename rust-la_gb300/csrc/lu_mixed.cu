@@ -460,19 +460,9 @@ la_status mixed_factor(la_ctx ctx, la_lu h, int prec) {
     ctx->stream = saved;
     return st;
   };
-  // U12 = L11^-1 A12 for rows [j0, j1o) on columns [c0, c1): one blocked
-  // launch (the outer panel is at most 256 rows).
+  // U12 = L11^-1 A12 for rows [j0, j1o) on columns [c0, c1).
   auto outer_trsm = [&](int j0, int j1o, int c0, int c1) -> la_status {
-    if (j1o - j0 <= 256) return launch_trsm_block_f32(ctx, A, ld, j0, j1o - j0, c0, c1);
-    for (int i0 = j0; i0 < j1o; i0 += WI) {
-      const int ib = std::min(WI, j1o - i0);
-      const int i1 = i0 + ib;
-      LA_TRY(launch_trsm_rowpanel_f32(ctx, A, ld, i0, ib, c0, c1));
-      if (i1 < j1o)
-        LA_TRY(launch_gemm_f32(ctx, GM_FMA_SUB, j1o - i1, c1 - c0, ib, A + (size_t)i1 * ld + i0, ld,
-                               A + (size_t)i0 * ld + c0, ld, A + (size_t)i1 * ld + c0, ld));
-    }
-    return LA_OK;
+    return launch_trsm_block_f32(ctx, A, ld, j0, j1o - j0, c0, c1);
   };
   // A22 -= L21 U12 for rows >= j1o on columns [c0, c1). L21 is copied once per
   // outer panel (pack_l) before the next panel's row swaps can permute it:
