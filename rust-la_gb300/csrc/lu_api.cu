@@ -3,7 +3,8 @@
 //
 // FAST arithmetic: lu_fast_enqueue below. EXACT arithmetic: blocked right-looking LU
 // (panel width W, default 64), for each panel [j0, j1 = j0 + jb):
-//   panel  : cooperative kernel, pivots + L21/U11 of the panel (lu_panel.cu)
+//   panel  : pivots + L21/U11 of the panel, on one cluster in halves of 32 columns up to 4096 rows
+//            (panel_cluster64.cu), else by the cooperative kernel (lu_panel.cu)
 //   laswp  : the panel's row swaps on the other columns (lu.rs:140-145)
 //   trsm   : U12 = L11^{-1} A12 for rows [j0, j1)
 //   gemm   : S22 += L21 * U12
@@ -329,7 +330,6 @@ la_status lu_fast_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
 
 la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
   if (h->arith != LA_ARITH_EXACT) return lu_fast_enqueue(ctx, h, d_flags, d_uneven);
-  const bool exact = true;
   const int m = (int)h->m, n = (int)h->n;
   const size_t ld = h->ld;
   const int kmin = std::min(m, n);
@@ -338,23 +338,18 @@ la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
   cudaStream_t ms = ctx->stream, ss = ctx->side_stream;
   double* A = h->d_lu;
   DevBuf S(ctx);
-  if (exact) {
-    LA_TRY(S.alloc((size_t)m * ld * sizeof(double)));
-    LA_CUDA(ctx, cudaMemsetAsync(S.p, 0, (size_t)m * ld * sizeof(double), ms));
-  }
+  LA_TRY(S.alloc((size_t)m * ld * sizeof(double)));
+  LA_CUDA(ctx, cudaMemsetAsync(S.p, 0, (size_t)m * ld * sizeof(double), ms));
   LA_CUDA(ctx, cudaMemsetAsync(ctx->d_bar, 0, sizeof(unsigned), ms));
   unsigned bar_base = 0;
   PhaseTimer t(ctx);
-  const int gmode = exact ? GM_EXACT_ADD : GM_FMA_SUB;
   auto trailing = [&](int j0, int jb, int c0, int c1, size_t min_smem) -> la_status {
     // rows [j0+jb, m), columns [c0, c1)
     const int j1 = j0 + jb;
     if (j1 >= m || c1 <= c0) return LA_OK;
-    const double* L21 = A + (size_t)j1 * ld + j0;
-    const double* U12 = A + (size_t)j0 * ld + c0;
-    double* C = exact ? S.d() + (size_t)j1 * ld + c0 : A + (size_t)j1 * ld + c0;
     size_t b = t.begin(ms);
-    la_status st = launch_gemm(ctx, gmode, m - j1, c1 - c0, jb, L21, ld, U12, ld, C, ld, min_smem);
+    la_status st = launch_gemm(ctx, GM_EXACT_ADD, m - j1, c1 - c0, jb, A + (size_t)j1 * ld + j0, ld,
+                               A + (size_t)j0 * ld + c0, ld, S.d() + (size_t)j1 * ld + c0, ld, min_smem);
     t.end(ms, b, PH_GEMM);
     return st;
   };
@@ -373,18 +368,18 @@ la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
       st = launch_panel_cluster64(ctx, s, A, S.d(), ld, m, j0, h0, h->d_ipiv);
     lists = 1;
     if (st == LA_UNSUPPORTED)
-      return launch_panel(ctx, s, exact, A, S.d(), ld, m, j0, jb, h->d_ipiv, &bar_base);
+      return launch_panel(ctx, s, true, A, S.d(), ld, m, j0, jb, h->d_ipiv, &bar_base);
     LA_TRY(st);
     if (h0 == jb) return LA_OK;
-    LA_TRY(launch_laswp(ctx, exact, A, S.d(), ld, j0, j0 + jb, j0, h0));
-    LA_TRY(launch_trsm_rowpanel(ctx, exact, A, S.d(), ld, j0, h0, jm, j0 + jb));
+    LA_TRY(launch_laswp(ctx, true, A, S.d(), ld, j0, j0 + jb, j0, h0));
+    LA_TRY(launch_trsm_rowpanel(ctx, true, A, S.d(), ld, j0, h0, jm, j0 + jb));
     if (jm < m)
       LA_TRY(launch_gemm_narrow(ctx, GM_EXACT_ADD, m - jm, jb - h0, h0, A + (size_t)jm * ld + j0, ld,
                                 A + (size_t)j0 * ld + jm, ld, S.d() + (size_t)jm * ld + jm, ld));
     ctx->swap_list = 1;
     LA_TRY(launch_panel_cluster64(ctx, s, A, S.d(), ld, m, jm, jb - h0, h->d_ipiv));
     lists = 2;
-    return launch_laswp(ctx, exact, A, S.d(), ld, j0, j0 + jb, jm, jb - h0);
+    return launch_laswp(ctx, true, A, S.d(), ld, j0, j0 + jb, jm, jb - h0);
   };
   auto panel = [&](cudaStream_t s, int j0, int jb) -> la_status {
     cudaStream_t saved = ctx->stream;
@@ -406,14 +401,14 @@ la_status lu_factor_enqueue(la_ctx ctx, la_lu h, int* d_flags, int* d_uneven) {
     la_status sw = LA_OK;
     for (int l = 0; l < lists && sw == LA_OK; l++) {
       ctx->swap_list = l;
-      sw = launch_laswp(ctx, exact, A, S.d(), ld, 0, n, j0, jb);
+      sw = launch_laswp(ctx, true, A, S.d(), ld, 0, n, j0, jb);
     }
     ctx->swap_list = 0;
     LA_TRY(sw);
     t.end(ms, b, PH_SWAP);
     if (j1 < n) {
       b = t.begin(ms);
-      LA_TRY(launch_trsm_rowpanel(ctx, exact, A, S.d(), ld, j0, jb, j1, n));
+      LA_TRY(launch_trsm_rowpanel(ctx, true, A, S.d(), ld, j0, jb, j1, n));
       t.end(ms, b, PH_TRSM);
     }
     if (j1 >= kmin) break;  // no next panel
@@ -527,7 +522,6 @@ la_status check_ctx(la_ctx ctx) {
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "cudaSetDevice");
   return LA_OK;
 }
-
 
 // Device solve shared by the host and device entry points: d_b (pitch ldb) ->
 // d_x (pitch ldx); both may be unaligned, an aligned work buffer is used.
