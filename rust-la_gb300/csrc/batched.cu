@@ -507,35 +507,29 @@ __device__ void block_lu(typename P::S* M, int p, int n, int* rmap, typename P::
   __syncthreads();
 }
 
-// Whether |v| is far from both ends of the range, so that products with another such value and the
-// remainders below are exact where they have to be.
-template <typename T>
-__device__ __forceinline__ bool mid_range(T v) {
-  if constexpr (sizeof(T) == 8) {
-    const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
-    return e - 523u < 1000u;  // 2^-500 .. 2^500
-  } else {
-    const unsigned e = (__float_as_uint(v) >> 23) & 0xffu;
-    return e - 77u < 100u;  // 2^-50 .. 2^50
-  }
+// Whether |v| is within 2^-500 .. 2^500, so that products with another such value and the remainders
+// below are exact where they have to be.
+__device__ __forceinline__ bool mid_range(double v) {
+  const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
+  return e - 523u < 1000u;
 }
 
 // Factor entries M(row_i, kb + k), k < kbn <= 16, for slots i < cnt of 2 N rows r0 + dir i: half a warp
 // reads one row, so a warp's load touches two lines (by one row per lane it touched 32).
-template <typename P, int N, typename TX>
-__device__ __forceinline__ void solve_fetch(TX (&t)[N], const typename P::S* M, int n,
+template <typename P, int N>
+__device__ __forceinline__ void solve_fetch(double (&t)[N], const typename P::S* M, int n,
                                             const int* rmap, int r0, int dir, int cnt, int kb,
                                             int kbn) {
   const int k = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
 #pragma unroll
   for (int j = 0; j < N; j++) {
     const int i = 2 * j + h;
-    t[j] = i < cnt && k < kbn ? (TX)P::ld(&M[rmap[r0 + dir * i] * n + kb + k]) : TX(0);
+    t[j] = i < cnt && k < kbn ? P::ld(&M[rmap[r0 + dir * i] * n + kb + k]) : 0.0;
   }
 }
 // ... to shared memory, slot i at tr + i SP.
-template <int N, typename TX>
-__device__ __forceinline__ void solve_stage(TX* tr, const TX (&t)[N], int cnt) {
+template <int N>
+__device__ __forceinline__ void solve_stage(double* tr, const double (&t)[N], int cnt) {
   const int k = threadIdx.x & 15, h = (threadIdx.x >> 4) & 1;
 #pragma unroll
   for (int j = 0; j < N; j++)
@@ -547,22 +541,23 @@ __device__ __forceinline__ void solve_stage(TX* tr, const TX (&t)[N], int cnt) {
 // the chain: q = x r, then one correction with the exact remainder x - q d (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990). Returns whether every quotient of
 // an active lane was in the range where that holds.
-template <typename TX, bool UPPER, bool FULL>
-__device__ __forceinline__ bool solve_diag(const TX (&dg)[16], TX d, TX r, int kbn, bool act, TX& x) {
+template <bool UPPER, bool FULL>
+__device__ __forceinline__ bool solve_diag(const double (&dg)[16], double d, double r, int kbn, bool act,
+                                           double& x) {
   const int lane = threadIdx.x & 31, li = lane & 15;
 #pragma unroll
   for (int i = 0; i < 16; i++) {
     const int k = UPPER ? 15 - i : i;
     if (FULL || k < kbn) {  // uniform
       if (UPPER) {
-        const TX q = x * r, y = fma(fma(-q, d, x), r, q);
+        const double q = x * r, y = fma(fma(-q, d, x), r, q);
         if (li == k) x = y;
       }
-      const TX xk = __shfl_sync(0xffffffffu, x, (lane & 16) | k);
+      const double xk = __shfl_sync(0xffffffffu, x, (lane & 16) | k);
       if (UPPER ? li < k : li > k) x = fma(-dg[k], xk, x);
     }
   }
-  return !UPPER || !act || (mid_range(d) && (x == TX(0) || mid_range(x)));
+  return !UPPER || !act || (mid_range(d) && (x == 0.0 || mid_range(x)));
 }
 
 // X (n x nrhs, pitch nrhs, already in the factor's row order, i.e. P b)
@@ -579,9 +574,9 @@ __device__ __forceinline__ bool solve_diag(const TX (&dg)[16], TX d, TX r, int k
 // updates and a division per row in warp 0's path before).
 // A function of its own: with 224 KB of shared memory taken the L1 is next to
 // nothing, and a spill in a loop costs an L2 round trip.
-template <typename P, typename TX, bool UPPER>
-__device__ __noinline__ void block_tri(const typename P::S* M, int n, const int* rmap, TX* X,
-                                       int nrhs, TX* buf) {
+template <typename P, bool UPPER>
+__device__ __noinline__ void block_tri(const typename P::S* M, int n, const int* rmap, double* X,
+                                       int nrhs, double* buf) {
   constexpr int TILE = 16 * SP;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = blockDim.x >> 5;
   const int li = lane & 15, half = lane >> 4;
@@ -592,8 +587,8 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
   // itself and warp 1 updates rows too.
   const bool direct = n < 52 || NW < 4;
   const int R0 = direct ? 1 : 2, NR = NW - R0;  // the warps that update rows
-  TX* const slots = buf + (n - 17) * SP;
-  TX* const tr = buf + (warp - R0) * 32 * SP;
+  double* const slots = buf + (n - 17) * SP;
+  double* const tr = buf + (warp - R0) * 32 * SP;
   auto block_at = [&](int b) { return 16 * (UPPER ? nblk - 1 - b : b); };
   auto width_at = [&](int kb) { return min(16, n - kb); };
   auto slot_at = [&](int par) { return slots + (par & 1) * (2 * TILE + 16); };
@@ -607,25 +602,25 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
   };
   auto barrier = [&] { asm volatile("bar.sync 0;" ::: "memory"); };  // one per block in both roles
   if (warp == 0) {
-    TX dg[16], d = TX(1), rcp = TX(1), x0 = TX(0), x1 = TX(0);
+    double dg[16], d = 1.0, rcp = 1.0, x0 = 0.0, x1 = 0.0;
     barrier();
 #pragma unroll 1
     for (int b = 0; b < nblk; b++) {
       const int kb = block_at(b), kbn = width_at(kb), i = min(li, kbn - 1);
       const bool a0 = li < kbn && half < nrhs, a1 = li < kbn && half + 2 < nrhs;
-      TX* const xr = X + (kb + li) * nrhs + half;
-      x0 = a0 ? xr[0] : TX(0);
-      x1 = a1 ? xr[2] : TX(0);
+      double* const xr = X + (kb + li) * nrhs + half;
+      x0 = a0 ? xr[0] : 0.0;
+      x1 = a1 ? xr[2] : 0.0;
       const typename P::S* const row = M + rmap[kb + i] * n;  // the lane's row of the factors
       if (b > 0) {  // its terms of the previous block
         const int kp = block_at(b - 1), np = width_at(kp);
-        const TX* const xblk = X + kp * nrhs;
+        const double* const xblk = X + kp * nrhs;
         const int c0 = min(half, nrhs - 1), c1 = min(half + 2, nrhs - 1);
         if (direct) {
 #pragma unroll
-          for (int k = 0; k < 16; k++) dg[k] = k < np ? (TX)P::ld(&row[kp + k]) : TX(0);
+          for (int k = 0; k < 16; k++) dg[k] = k < np ? P::ld(&row[kp + k]) : 0.0;
         } else {
-          const TX* sl = slot_at(b - 1) + TILE + i * SP;
+          const double* sl = slot_at(b - 1) + TILE + i * SP;
 #pragma unroll
           for (int k = 0; k < 16; k++) dg[k] = sl[k];
         }
@@ -638,32 +633,32 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
       }
       if (direct) {
 #pragma unroll
-        for (int k = 0; k < 16; k++) dg[k] = k < kbn ? (TX)P::ld(&row[kb + k]) : TX(0);
-        if (UPPER) d = (TX)P::ld(&row[kb + i]), rcp = TX(1) / d;
+        for (int k = 0; k < 16; k++) dg[k] = k < kbn ? P::ld(&row[kb + k]) : 0.0;
+        if (UPPER) d = P::ld(&row[kb + i]), rcp = 1.0 / d;
       } else {
-        const TX* sl = slot_at(b - 1);
+        const double* sl = slot_at(b - 1);
 #pragma unroll
         for (int k = 0; k < 16; k++) dg[k] = sl[i * SP + k];
         if (UPPER) d = sl[i * SP + i], rcp = sl[2 * TILE + i];
       }
-      const TX v0 = x0, v1 = x1;
+      const double v0 = x0, v1 = x1;
       bool ok;
       if (kbn == 16) {
-        ok = solve_diag<TX, UPPER, true>(dg, d, rcp, 16, a0, x0);
-        if (nrhs > 2) ok &= solve_diag<TX, UPPER, true>(dg, d, rcp, 16, a1, x1);
+        ok = solve_diag<UPPER, true>(dg, d, rcp, 16, a0, x0);
+        if (nrhs > 2) ok &= solve_diag<UPPER, true>(dg, d, rcp, 16, a1, x1);
       } else {
-        ok = solve_diag<TX, UPPER, false>(dg, d, rcp, kbn, a0, x0);
-        if (nrhs > 2) ok &= solve_diag<TX, UPPER, false>(dg, d, rcp, kbn, a1, x1);
+        ok = solve_diag<UPPER, false>(dg, d, rcp, kbn, a0, x0);
+        if (nrhs > 2) ok &= solve_diag<UPPER, false>(dg, d, rcp, kbn, a1, x1);
       }
       if (UPPER && __any_sync(0xffffffffu, !ok)) {  // with divisions
         x0 = v0;
         x1 = v1;
 #pragma unroll 1
         for (int k = kbn - 1; k >= 0; k--) {
-          const TX f = (TX)P::ld(&row[kb + k]);
+          const double f = P::ld(&row[kb + k]);
           if (li == k) x0 = x0 / f, x1 = x1 / f;
-          const TX y0 = __shfl_sync(0xffffffffu, x0, (lane & 16) | k);
-          const TX y1 = __shfl_sync(0xffffffffu, x1, (lane & 16) | k);
+          const double y0 = __shfl_sync(0xffffffffu, x0, (lane & 16) | k);
+          const double y1 = __shfl_sync(0xffffffffu, x1, (lane & 16) | k);
           if (li < k) x0 = fma(-f, y0, x0), x1 = fma(-f, y1, x1);
         }
       }
@@ -672,7 +667,7 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
       barrier();
     }
   } else if (warp < R0) {  // warp 1: the tiles
-    TX td[8], ts[8];       // diagonal tile of block b + 1, and its tile against block b
+    double td[8], ts[8];  // diagonal tile of block b + 1, and its tile against block b
     {
       const int k1 = block_at(0), w1 = width_at(k1);
       solve_fetch<P>(td, M, n, rmap, k1, 1, w1, k1, w1);
@@ -680,12 +675,12 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
 #pragma unroll 1
     for (int b = -1; b < nblk; b++) {
       if (b + 1 < nblk) {
-        TX* const sl = slot_at(b);
+        double* const sl = slot_at(b);
         const int w1 = width_at(block_at(b + 1));
         solve_stage(sl, td, w1);
         if (b >= 0) solve_stage(sl + TILE, ts, w1);
         __syncwarp();
-        if (UPPER && lane < w1) sl[2 * TILE + lane] = TX(1) / sl[lane * SP + lane];
+        if (UPPER && lane < w1) sl[2 * TILE + lane] = 1.0 / sl[lane * SP + lane];
       }
       if (b + 2 < nblk) {
         const int k2 = block_at(b + 2), w2 = width_at(k2), k1 = block_at(b + 1);
@@ -695,7 +690,7 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
       barrier();
     }
   } else {
-    TX t[16];  // a pass of 32 rows
+    double t[16];  // a pass of 32 rows
     auto fetch_pass = [&](int b, int r0) {
       const int rest = beyond(b), kb = block_at(b);
       if (r0 < rest)
@@ -708,7 +703,7 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
     for (int b = 0; b < nblk; b++) {
       barrier();
       const int kb = block_at(b), kbn = width_at(kb);
-      const TX* const xblk = X + kb * nrhs;
+      const double* const xblk = X + kb * nrhs;
       const int rest = beyond(b);
 #pragma unroll 1
       for (int r0 = 32 * (warp - R0); r0 < rest; r0 += 32 * NR) {
@@ -717,11 +712,11 @@ __device__ __noinline__ void block_tri(const typename P::S* M, int n, const int*
         __syncwarp();
         fetch_pass(b, r0 + 32 * NR);
         if (r0 + lane < rest) {
-          TX* const xi = X + row_at(b, r0 + lane) * nrhs;
-          const TX* const f = tr + lane * SP;
+          double* const xi = X + row_at(b, r0 + lane) * nrhs;
+          const double* const f = tr + lane * SP;
 #pragma unroll 1
           for (int c = 0; c < nrhs; c++) {
-            TX s = xi[c];
+            double s = xi[c];
             if (kbn == 16) {
 #pragma unroll
               for (int k = 0; k < 16; k++) s = fma(-f[k], xblk[k * nrhs + c], s);
@@ -832,15 +827,12 @@ __device__ void block_solve_shared(const typename P::S* M, int p, int n, const i
 
 // FP64 plans have 255 registers per thread and take block_tri. The mixed kernel has 128 (four 4-warp
 // CTAs per SM), in which block_tri and the calls to it spill: 3000 systems of n in [16, 256] took 5.26
-// ms in 4 x 4 warps with it and 3.87 without.
-template <typename P, typename TX>
-__device__ void block_solve(const typename P::S* M, int n, const int* rmap, TX* X, int nrhs, TX* buf) {
-  if constexpr (sizeof(TX) == 8) {
-    block_tri<P, TX, false>(M, n, rmap, X, nrhs, buf);
-    block_tri<P, TX, true>(M, n, rmap, X, nrhs, buf);
-  } else {
-    block_solve_shared<P, TX>(M, n, n, rmap, X, nrhs);
-  }
+// ms in 4 x 4 warps with it and 3.87 with block_solve_shared.
+template <typename P>
+__device__ void block_solve(const typename P::S* M, int n, const int* rmap, double* X, int nrhs,
+                            double* buf) {
+  block_tri<P, false>(M, n, rmap, X, nrhs, buf);
+  block_tri<P, true>(M, n, rmap, X, nrhs, buf);
 }
 
 struct BatchArgs {
@@ -1025,7 +1017,7 @@ __device__ double refine_eta(const double* rv, const double* xv, int n, int nrhs
 // w <- A^-1 w through the stored factors of scale * A: an FP32 solve of
 // P w / max|w| (the preconditioner of GMRES-IR).
 template <typename P>
-__device__ void precondition(const typename P::S* M, int n, const int* rmap, float* st, double* w, float* dv,
+__device__ void precondition(const typename P::S* M, int n, const int* rmap, double* w, float* dv,
                              float scale, Shared& sh) {
   const int BT = blockDim.x;
   double m = 0.0;
@@ -1034,7 +1026,7 @@ __device__ void precondition(const typename P::S* M, int n, const int* rmap, flo
   const double inv = m > 0 ? 1.0 / m : 0.0;
   for (int i = threadIdx.x; i < n; i += BT) dv[i] = (float)(w[rmap[i]] * inv);
   __syncthreads();
-  block_solve<P, float>(M, n, rmap, dv, 1, st);
+  block_solve_shared<P, float>(M, n, n, rmap, dv, 1);
   for (int i = threadIdx.x; i < n; i += BT) w[i] = (double)dv[i] * m * (double)scale;
   __syncthreads();
 }
@@ -1046,7 +1038,7 @@ __device__ void precondition(const typename P::S* M, int n, const int* rmap, flo
 // Returns the steps taken.
 template <typename P>
 __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int c,
-                            const typename P::S* M, const int* rmap, float* st, const double* rv, double* xv,
+                            const typename P::S* M, const int* rmap, const double* rv, double* xv,
                             float* dv, float scale, double* w, double* H, double* V, int mcap,
                             Shared& sh) {
   const int tid = threadIdx.x, BT = blockDim.x;
@@ -1055,7 +1047,7 @@ __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int 
   double* sn = cs + GM_M + 1;
   for (int i = tid; i < n; i += BT) w[i] = rv[(size_t)i * nrhs + c];
   __syncthreads();
-  precondition<P>(M, n, rmap, st, w, dv, scale, sh);
+  precondition<P>(M, n, rmap, w, dv, scale, sh);
   double s = 0.0;
   for (int i = tid; i < n; i += BT) s += w[i] * w[i];
   const double beta = sqrt(block_sum_d(s, sh.red));
@@ -1067,7 +1059,7 @@ __device__ int gmres_column(const double* __restrict__ Ai, int n, int nrhs, int 
   for (int j = 0; j < mcap; j++) {
     residual_rows<1, true>(Ai, n, V + (size_t)j * n, nullptr, w);  // w = A v_j
     __syncthreads();
-    precondition<P>(M, n, rmap, st, w, dv, scale, sh);
+    precondition<P>(M, n, rmap, w, dv, scale, sh);
     for (int i = 0; i <= j; i++) {
       const double* vi = V + (size_t)i * n;
       double hs = 0.0;
@@ -1232,13 +1224,13 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
   if (tid == 0) pc.mark(1);
   for (int i = tid; i < n; i += BT) a.piv[d.poff + i] = rmap[i];
 
-  if (!MIXED) {
+  if constexpr (!MIXED) {
     for (int idx = tid; idx < n * nrhs; idx += BT) {
       const int i = idx / nrhs, c = idx - i * nrhs;
       xv[idx] = Bi[(size_t)rmap[i] * nrhs + c];
     }
     __syncthreads();
-    block_solve<P, double>(M, n, rmap, xv, nrhs, reinterpret_cast<double*>(st));
+    block_solve<P>(M, n, rmap, xv, nrhs, st);
     for (int idx = tid; idx < n * nrhs; idx += BT) Xi[idx] = xv[idx];
     if (tid == 0) {
       a.status[sidx] = 0;
@@ -1279,7 +1271,7 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
     }
     __syncthreads();
     if (tid == 0) pc.mark(3);
-    block_solve<P, float>(M, n, rmap, dv, nrhs, reinterpret_cast<float*>(st));
+    block_solve_shared<P, float>(M, n, n, rmap, dv, nrhs);
     if (tid == 0) pc.mark(2);
     // (scale A) d = r / rmax  =>  A (scale d rmax) = r
     for (int idx = tid; idx < n * nrhs; idx += BT)
@@ -1303,7 +1295,7 @@ __device__ void process_system(const BatchArgs& a, int sidx, const SysDesc& d, S
                                           (size_t)blockIdx.x * a.scratch_bytes + GM_V_OFFSET);
     for (int outer = 0; outer < GM_OUTER && !ok; outer++) {
       for (int c = 0; c < nrhs; c++)
-        gsteps += gmres_column<P>(Ai, n, nrhs, c, M, rmap, reinterpret_cast<float*>(st), rv, xv, dv, scale, w, H, V, mcap, sh);
+        gsteps += gmres_column<P>(Ai, n, nrhs, c, M, rmap, rv, xv, dv, scale, w, H, V, mcap, sh);
       residual_all(Ai, n, nrhs, xv, Bi, Xi);
       rv = Xi;
       __syncthreads();
