@@ -63,11 +63,12 @@ int la_abi_version(void);
 
 /* Options (la_ctx_set_option). */
 typedef enum la_option {
-  /* LU arithmetic. LA_ARITH_FAST (default): blocked right-looking LU with
-   * fused multiply-add. LA_ARITH_EXACT: the same blocked kernels carry each
-   * element's partial sum separately and add terms in the reference's order
-   * without fusion, so LU factors, pivots, det and solve results are
-   * bit-identical to src/decomp/lu.rs (at about half the FP64 rate). Also
+  /* LU arithmetic. LA_ARITH_FAST (default): blocked LU whose updates run on the
+   * tensor cores by exact splitting into FP16 digits where the operands allow it
+   * (one rounding per update) and by fused multiply-add elsewhere.
+   * LA_ARITH_EXACT: blocked kernels carry each element's partial sum separately
+   * and add terms in the reference's order without fusion, so LU factors,
+   * pivots, det and solve results are bit-identical to src/decomp/lu.rs. Also
    * selects the summation of la_matrix_mul (mod.rs:957-980 order when EXACT). */
   LA_OPT_ARITH = 1,
   /* Panel width of the blocked LU (16, 32 or 64). */
@@ -80,9 +81,10 @@ typedef enum la_option {
    * the trailing update runs (EXACT LU, mixed LU, EXACT Cholesky); 0: strictly
    * one phase after the other. Results are bit-identical either way. */
   LA_OPT_LOOKAHEAD = 5,
-  /* 1 (default): the FP32 panels of the mixed LU and the panels of the FAST LU
-   * run on one thread-block cluster (distributed shared memory); 0: the
-   * cooperative multi-CTA kernel. The LU's results are the same bits. */
+  /* 1 (default): the FP32 panels of the mixed LU and the FP64 panels of the LU
+   * (FAST up to 8192 rows, EXACT up to 4096) run on one thread-block cluster
+   * (distributed shared memory); 0: the cooperative multi-CTA kernel. The LU's
+   * results are the same bits. */
   LA_OPT_CLUSTER_PANEL = 6,
   /* Batch plans (read when a plan is built): largest Krylov basis (0-20) of
    * the GMRES-IR stage that a LA_BATCH_MIXED plan runs on a system whose
@@ -104,25 +106,24 @@ typedef enum la_option {
    * la_lu_solve_auto_device) report a stall before their first correction. */
   LA_OPT_INJECT_ALLOC_FAIL = 10,
   LA_OPT_INJECT_IR_STALL = 11,
-  /* Limit, in microseconds, of the grid-barrier wait of the cooperative panel
-   * kernel (1 to 10,000,000; 0 = the default of 2 s). A CTA whose wait runs
-   * out records the failure and returns, every other CTA sees it and returns,
+  /* Limit, in microseconds, of the waits of the FP64 panel kernels (the grid
+   * barrier of the cooperative one, the exchange of the cluster's; 1 to
+   * 10,000,000; 0 = the default of 2 s). A CTA whose wait runs out records the failure and returns, every other CTA sees it and returns,
    * the kernels queued behind the panel that would use its row interchanges
    * return at entry, and the call reports LA_TIMEOUT; the context stays
    * usable. */
   LA_OPT_WAIT_LIMIT_US = 12,
   /* Failure injection for tests (0 = off; reads back what is left): the k-th
-   * launch of the cooperative panel kernel from now makes its CTAs wait for
+   * launch of an FP64 panel kernel from now makes its CTAs wait for
    * one arrival more than there are CTAs, so that the wait runs out (after
    * LA_OPT_WAIT_LIMIT_US) exactly as when a CTA cannot reach the barrier. */
   LA_OPT_INJECT_PANEL_STALL = 13,
-  /* 1 (default): in the mixed LU, the chain of inner-panel kernels (32-column
-   * panel, row swaps, triangular solve, rank-32 update) and the serial part
-   * between outer panels (row swaps, the next panel's triangular solve, U12
-   * scale and packing, tensor-core update) are launched with programmatic
-   * stream serialization, so that each kernel is scheduled while the one
-   * before it finishes and waits on the device for its results; 0: ordinary
-   * stream order. Results are bit-identical either way. */
+  /* 1 (default): chains of kernels that wait for one another are launched with
+   * programmatic stream serialization, so that each kernel is scheduled while
+   * the one before it finishes and waits on the device for its results: the
+   * mixed LU's inner panels and the serial part between its outer ones, the
+   * FAST LU and Cholesky throughout, the panels of the EXACT LU, the blocked
+   * QR; 0: ordinary stream order. Results are bit-identical either way. */
   LA_OPT_PDL = 14
 } la_option;
 

@@ -338,7 +338,7 @@ la_status chol_check_ctx(la_ctx ctx) {
 
 // FAST factorization of h->d_l (see the head of the file). Block widths as in the LU: an update's
 // cost is the split product's epilogue, so wide blocks where there are many rows. n = 4099 with 5
-// right-hand sides: 8.1 ms, of them 2.7 in the panels, 1.9 in the split products and 1.8 in the
+// right-hand sides: 7.6 ms, of them 2.7 in the panels, 1.9 in the split products and 1.8 in the
 // solves (64-column panels with FP64 FMA updates beside them: 31.9 ms).
 struct FastChol {
   la_ctx ctx;

@@ -393,7 +393,7 @@ la_status launch_gemm(la_ctx ctx, int mode, int M, int N, int K, const double* A
   return launch_bn<64>(ctx, mode, M, N, K, A, lda, B, ldb, C, ldc, min_smem);
 }
 
-// C -= A B (GM_FMA_SUB) or C = A B (GM_FMA_ZERO) by tiles of 64 x 16: an SM needs 33 us for a
+// C -= A B (GM_FMA_SUB) or C += A B (GM_EXACT_ADD) by tiles of 64 x 16: an SM needs 33 us for a
 // 64 x 64 tile of 32 k, whatever part of it exists, and 8 us for one of these.
 la_status launch_gemm_narrow(la_ctx ctx, int mode, int M, int N, int K, const double* A, size_t lda,
                              const double* B, size_t ldb, double* C, size_t ldc) {

@@ -102,21 +102,21 @@ struct la_context {
   cudaStream_t side_stream = nullptr;    // high priority: lookahead panels
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int lookahead = 1;
-  int cluster_panels = 1;                // FP32 panels on one thread-block cluster
+  int cluster_panels = 1;                // LA_OPT_CLUSTER_PANEL: panels on one thread-block cluster
   int batch_gmres = 0;                   // Krylov steps per GMRES correction in batch plans (0: off)
   int solve_wave = 2;                    // CTAs per SM of the wavefront solve (0: block steps)
   int inject_alloc_at = 0;               // the n-th device allocation from now fails (0: none)
   int inject_ir_stall = 0;               // this many refinement calls report a stall at once
   int inject_panel_stall = 0;            // the n-th FP64 panel launch from now waits for a CTA too many
-  long long wait_limit_us = 0;           // limit of the panel's grid-barrier wait (0: 2 s)
+  long long wait_limit_us = 0;           // limit of the FP64 panels' waits (0: 2 s)
   int sm_count = 0;
   size_t smem_optin = 0;
   int arith = LA_ARITH_FAST;
   int panel_width = 64;
   int panel_ctas = 0;
   int profile = 0;
-  int pdl = 1;                           // LA_OPT_PDL: dependent launches in the mixed LU's panel chain
-  bool pdl_now = false;                  // set while that chain is being enqueued
+  int pdl = 1;                           // LA_OPT_PDL: dependent launches in chains of kernels
+  bool pdl_now = false;                  // set while such a chain is being enqueued
   std::string last_error;
   uint64_t launches = 0;
   double phase_ms[5] = {0, 0, 0, 0, 0};
@@ -276,7 +276,7 @@ la_status launch_panel(la_ctx ctx, cudaStream_t stream, bool exact, double* A, d
 constexpr int PANEL64_ROWS = 8192;  // most rows of a FAST panel on one cluster (EXACT: half of them)
 la_status launch_panel_cluster64(la_ctx ctx, cudaStream_t stream, double* A, const double* S,
                                  size_t ld, int m, int j0, int jb, int* d_ipiv);
-// C -= A B or C = A B (mode GM_FMA_SUB, GM_FMA_ZERO) with tiles of 16 columns.
+// C -= A B (mode GM_FMA_SUB) or the EXACT carry C += A B (GM_EXACT_ADD) with tiles of 16 columns.
 la_status launch_gemm_narrow(la_ctx ctx, int mode, int M, int N, int K, const double* A, size_t lda,
                              const double* B, size_t ldb, double* C, size_t ldc);
 // The row moves of panel [j0, j0 + jb) (the current list) on columns [c0, j0) and [j0 + jb, c1).

@@ -90,7 +90,7 @@ constexpr size_t GEMM_SMEM_WITH_PANEL = 78 * 1024;
 // cost is the epilogue's per element of C, about the same for K = 64 and K = 256; so blocks are
 // wide where there are many rows (lu_block), and 64 columns where the launches of the wider
 // blocks' inner steps would cost more than they save. Every launch is a dependent one, so that only
-// their execution adds up. Measured, factor + solve with 16 right-hand sides at n = 8192: 54.9 ms
+// their execution adds up. Measured, factor + solve with 16 right-hand sides at n = 8192: 53.5 ms
 // (64-column blocks throughout: 69.3 ms in the same build but for the guard of the split products;
 // FP64 FMA updates beside a cooperative panel: 328 ms).
 //

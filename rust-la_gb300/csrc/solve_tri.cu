@@ -627,8 +627,8 @@ solve_chain_kernel(const T* __restrict__ LU, size_t ld, T* X, size_t ldx, int n,
 // share each tile's load and the FP64 pipes are busy anyway. Both triangles, us, four columns and one:
 // n = 8192: 16 right-hand sides 4053, 3412; 24: 4731, 4593; 32: 5609, 5839. n = 4096: 24: 1912, 1471;
 // 64: 2842, 2980. A single block has nothing to hand on, and the chain's body, unrolled over the block with
-// its divisions, is read from memory for one pass: whole calls at n = 24, us,
-// four-column items and chain: EXACT 53, 66; FAST 44, 44.
+// its divisions, is read from memory for one pass: whole calls at n = 24, us, four columns and one: EXACT
+// 53, 66; FAST 44, 44.
 constexpr int CHAIN_MAX_NRHS = 24;
 bool chained(int n, int nrhs) { return nrhs <= CHAIN_MAX_NRHS && n > WB; }
 
