@@ -963,10 +963,12 @@ la_status launch_product(la_ctx ctx, cudaStream_t st, const CUtensorMap& ta, con
                 dim3((lng ? 2 : 1) * GUARD_W * 32), 0, st, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "guard_kernel launch");
   // CTAs beyond the tiles are for the FMA pieces (up to 32 of a tile) and leave at once without any. In
-  // the factorizations, chains of dependent launches with updates of K <= 256, each of them also keeps the
-  // next kernel's CTAs from being placed early: Cholesky of order 4099 7.70 ms with 32 CTAs at least,
-  // 7.74 with 64, 8.27 with 120, 9.5 with all 152.
-  const int items = p.tiles * p.splits, most = ctx->pdl_now && p.K <= 256 ? 32 : ctx->sm_count;
+  // the factorizations, chains of dependent launches, each of them also keeps the kernels around this one
+  // from being placed early: Cholesky of order 4099 (K <= 256) 7.70 ms with 32 CTAs at least, 7.74 with 64,
+  // 8.27 with 120, 9.5 with all 152; QR of order 1000 (K = rows) 6.35 ms with 32, 6.37 with 112, 6.48 with
+  // 128, 6.67 with all, and 9.04, 8.20, 8.13, 8.18 where the pieces are needed.
+  const int items = p.tiles * p.splits;
+  const int most = !ctx->pdl_now ? ctx->sm_count : p.K <= 256 ? 32 : std::max(32, ctx->sm_count - 40);
   const int grid = std::min(std::max(2 * items, std::min(32 * items, most)), ctx->sm_count);
   e = la_launch(ctx, gemm_split_kernel<MODE>, dim3(grid), dim3(SPLIT_T), SPLIT_SMEM, st, ta, tb, p);
   if (e != cudaSuccess) return la_cuda_fail(ctx, e, "gemm_split_kernel launch");
