@@ -79,6 +79,8 @@ cudaError_t copy_staged(la_ctx ctx, char* dev, size_t pitch, const char* host, s
   return cudaSuccess;
 }
 
+// A write to each page that leaves its bytes as they are: the result may go where an argument came from,
+// and the stream may not have taken that yet.
 void touch_pages(char* p, size_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) {
@@ -87,7 +89,7 @@ void touch_pages(char* p, size_t bytes) {
   }
   static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
   for (size_t i = 0; i < bytes; i += page - (reinterpret_cast<uintptr_t>(p) + i) % page)
-    *const_cast<volatile char*>(p + i) = 0;
+    __atomic_fetch_or(p + i, 0, __ATOMIC_RELAXED);
 }
 }  // namespace
 
